@@ -195,6 +195,7 @@ struct GemmArgs {
   bool f16 = false;     // TC operand type: FP16 (true) or BF16
   int plan = 0;         // TC ring plan: 0 by N (N ≤ 64: two tiles per CTA, one CTA per SM), 1: N ≤ 64,
                         // one tile per CTA and two CTAs per SM (256 TMEM columns each)
+  bool twos = false;    // TC, FP16, N ≤ 64, plan 0: the matrix is 2·[count = 2] instead of the count
 };
 
 void gemm_simt(const GemmArgs& a, cudaStream_t st);

@@ -54,6 +54,12 @@ __device__ __forceinline__ uint32_t f16sub_pair_of(uint32_t word, int q)
   const uint32_t src = (q < 5) ? word : (word >> 10);
   return src & (0x00030003u << (2 * f16sub_shift(q)));
 }
+// The same pair with every count x replaced by 2·[x = 2] (the high bit of its field alone).
+__device__ __forceinline__ uint32_t f16sub_twos_of(uint32_t word, int q)
+{
+  const uint32_t src = (q < 5) ? word : (word >> 10);
+  return src & (0x00020002u << (2 * f16sub_shift(q)));
+}
 // 2^−2s for the element at K index kidx (K-tiles start at multiples of 64; element j of a
 // 16-element word is K index ≡ j mod 16, pair q = j / 2).
 __device__ __forceinline__ float f16sub_kscale(int64_t kidx)
@@ -68,10 +74,11 @@ __device__ __forceinline__ float f16sub_kunscale(int64_t kidx)
 }
 constexpr float kF16SubUnscale = 16777216.0f;   // 2^24
 
-template <bool F16>
+template <bool F16, bool TWOS = false>
 __device__ __forceinline__ uint32_t pair_of(uint32_t word, int q)
 {
-  if constexpr (F16) return f16sub_pair_of(word, q);
+  if constexpr (F16 && TWOS) return f16sub_twos_of(word, q);
+  else if constexpr (F16) return f16sub_pair_of(word, q);
   else return bf16pair_of(word, q);
 }
 
@@ -92,12 +99,6 @@ __device__ __forceinline__ void f32pair_of(uint32_t word, int q, float& even, fl
   const uint32_t p = bf16pair_of(word, q);
   even = __uint_as_float(p << 16);
   odd = __uint_as_float(p & 0xFFFF0000u);
-}
-
-// Count of element e (0..15) of a word, as an integer.
-__device__ __forceinline__ uint32_t count_at(uint32_t word, int e)
-{
-  return (word >> ((e & 1) * 16 + 2 * (e >> 1))) & 3u;
 }
 
 }  // namespace slemm

@@ -1,173 +1,230 @@
 // extra.cu — GEBV prediction (src/pred.cpp:4-141) and the GRAMMAR-Gamma per-variant terms of
-// slemm_gamma (bin/slemm_gamma.py:302-325) as packed-genotype passes with FP64 accumulation.
+// slemm_gamma (bin/slemm_gamma.py:302-325) as exact packed-genotype products.
 //
 // GEBV: tgv = Σ_j (flip_j ? 2 − x_j : x_j)·α_j = Cnt·α' + 2·Σ_{flip} α_j with α'_j = ±α_j, one
-// pass over the individual-major copy (thread = individual, K = SNPs).
+// pass over the individual-major copy (rows = individuals, K = SNPs).
 //
 // Score terms, with x = allele-1 count = 2 − count (pgenlib's convention) and z = count − gm:
 //   x − x̄ = −z, so xy = −zᵀy and xx = ‖(I − QQᵀ)(rr∘z)‖²
 //        = Σ rr²z² − Σ_l (Q_lᵀ(rr∘z))²,
 //   Σ rr²z² = (S1 + 2·S2) − 2·gm·S1 + gm²·Σrr²   (count² = count + 2·[count = 2])
 // where S1 = Σ rr²·count, S2 = Σ rr²·[count = 2], and Q_lᵀ(rr∘z) = Σ rr·Q_l·count − gm·Σ rr·Q_l.
-// One pass over the SNP-major copy (thread = SNP) accumulates Σ y·count, S1, S2 and the c
-// projections in FP64.
+// Two passes over the SNP-major copy (rows = SNPs, K = individuals): the counts against
+// [y | rr² | rr·Q_l], and 2·[count = 2] (the high bit of each packed field) against rr².  When
+// every rr is 1 (slemm_gamma's is_one_rr case) S1 and S2 are the SNP's integer class counts, and one
+// pass against [y | Q_l] does.
+//
+// Exact products on the tensor cores.  A dense column v is cut into slices of 11 bits,
+//   v·2^e = q_0 + 2^−11·q_1 + 2^−22·q_2 + …,   q_p integers, |q_p| ≤ 2^10,
+// with e such that max|v|·2^e lies in [2^9, 2^10): six slices hold an FP64 column to 2^−65 of its
+// largest value, four hold an FP32 one to 2^−43.  Slices are exact in FP16 and a count is at most
+// 2, so a product row's sum over 8,192 K-elements is an integer of at most 2^24: the FP32
+// accumulators are exact whatever their order.  K is therefore split every 128 K-tiles at the
+// latest, the partials are added as 64-bit integers, and only the last combination of the slices
+// rounds (in FP64).  Bound by the narrow tensor-core pass (its decoders).  GB300's FP64 pipe ran the
+// same sums by an FMA per genotype and column: at n = 100,000, m = 50,000 the GEBV took 18,988 µs
+// and takes 829 µs, the score terms with three covariates and residual weights 112,698 µs and
+// 1,221 µs, with the same or a smaller error against 64-bit sums.
 #include "internal.h"
 #include "decode.cuh"
+#include "reduce.cuh"
 
 namespace slemm {
 
-constexpr int kXStage = 8;   // tiles per shared-memory stage
+constexpr int kSliceBits = 11;
+constexpr int kSlicesF64 = 6;
+constexpr int kSlicesF32 = 4;
+constexpr int kExactKTiles = 8192 / kTileK;   // K-tiles of one exact FP32 partial sum
+constexpr int kXRows = 2048;                  // K-elements of one block of the operand kernels
+constexpr int kXThreads = 256;
 
-// tgv_partial[s][i] = Σ_{SNPs in split s} count[i,j]·alpha[j]
-__global__ void __launch_bounds__(128)
-gebv_kernel(const uint4* __restrict__ GT, int64_t K_tiles, const double* __restrict__ alpha,
-            int tiles_per_split, int64_t n_pad, double* __restrict__ part)
+// e with amax·2^e in [2^9, 2^10) (0 for a zero or non-finite column)
+__host__ __device__ inline int slice_exp(double amax)
 {
-  __shared__ double sa[kXStage * kTileK];
-  const int t = threadIdx.x;
-  const int64_t mt = blockIdx.x;
-  const int s = blockIdx.y;
-  const int64_t kt0 = (int64_t)s * tiles_per_split, kt1 = min64(K_tiles, kt0 + tiles_per_split);
-  double acc = 0.0;
-  for (int64_t ks = kt0; ks < kt1; ks += kXStage) {
-    const int nt = (int)min64(kXStage, kt1 - ks);
-    __syncthreads();
-    for (int q = t; q < nt * kTileK; q += 128) sa[q] = alpha[ks * kTileK + q];
-    __syncthreads();
-    for (int u = 0; u < nt; ++u) {
-      const uint4 pk = GT[(mt * K_tiles + ks + u) * 128 + t];
-      const uint32_t w4[4] = {pk.x, pk.y, pk.z, pk.w};
+  if (!(amax > 0.0) || !isfinite(amax)) return 0;
+  int E;
+  frexp(amax, &E);
+  return 10 - E;
+}
+
+// Slices 0 … S−1 of v·2^e into rows row0 … row0 + S − 1 of the FP16 operand at K-element kidx, times
+// the 2^−2s its K position takes (f16sub_pair_of).
+template <int S>
+__device__ __forceinline__ void store_slices(double v, int e, __half* __restrict__ B, int64_t K_pad, int row0,
+                                             int64_t kidx)
+{
+  double r = ldexp(v, e);
+  const float ks = f16sub_kscale(kidx);
 #pragma unroll
-      for (int w = 0; w < 4; ++w) {
+  for (int p = 0; p < S; ++p) {
+    const double q = rint(r);
+    B[(int64_t)(row0 + p) * K_pad + kidx] = __float2half_rn(__fmul_rn((float)q, ks));
+    r = (r - q) * (double)(1 << kSliceBits);   // exact
+  }
+}
+
+// Σ_p 2^−11p·(Σ_splits D[s][row0 + p][r]) — the column's product with row r, in units of 2^−e
+template <int S>
+__device__ __forceinline__ double gather_slices(const float* __restrict__ D, int splits, int kp, int64_t M_pad,
+                                                int row0, int64_t r)
+{
+  long long sum[S] = {};
+  for (int s = 0; s < splits; ++s)
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          float xe, xo;
-          f32pair_of(w4[w], q, xe, xo);
-          const int kk = u * kTileK + w * 16 + 2 * q;
-          acc = fma((double)xe, sa[kk], acc);
-          acc = fma((double)xo, sa[kk + 1], acc);
-        }
-      }
+    for (int p = 0; p < S; ++p) sum[p] += (long long)D[((int64_t)s * kp + row0 + p) * M_pad + r];
+  double v = 0.0;
+#pragma unroll
+  for (int p = S - 1; p >= 0; --p) v = v * (1.0 / (1 << kSliceBits)) + (double)sum[p];
+  return v;
+}
+
+// GEBV operand: rows 0 … 5 the slices of alpha (0 past m), rows 6 … 15 zero
+__global__ void __launch_bounds__(kXThreads)
+gebv_operand_kernel(const double* __restrict__ alpha, int64_t m, int64_t m_pad, int e, __half* __restrict__ B)
+{
+  const int64_t j = (int64_t)blockIdx.x * kXThreads + threadIdx.x;
+  if (j >= m_pad) return;
+  store_slices<kSlicesF64>(j < m ? alpha[j] : 0.0, e, B, m_pad, 0, j);
+#pragma unroll
+  for (int q = kSlicesF64; q < 16; ++q) B[(int64_t)q * m_pad + j] = __float2half_rn(0.f);
+}
+
+__global__ void __launch_bounds__(kXThreads)
+gebv_finish_kernel(const float* __restrict__ D, int splits, int kp, int64_t n_pad, int64_t n, int e, double shift,
+                   double* __restrict__ tgv)
+{
+  const int64_t i = (int64_t)blockIdx.x * kXThreads + threadIdx.x;
+  if (i < n) tgv[i] = shift + ldexp(gather_slices<kSlicesF64>(D, splits, kp, n_pad, 0, i), -e);
+}
+
+// Score columns: 0 = y, l = 1 … cq: rr·Q_{l−1}, cq + 1 = rr² (FP32 values), i < n; rr == nullptr: all 1
+// and no last column.
+__device__ __forceinline__ float score_column(const float* __restrict__ y, const float* __restrict__ rr,
+                                              const float* __restrict__ Q, int64_t n_pad, int cq, int c, int64_t i)
+{
+  if (c == 0) return y[i];
+  const float r = rr ? rr[i] : 1.f;
+  return __fmul_rn(r, c <= cq ? Q[(int64_t)(c - 1) * n_pad + i] : r);
+}
+
+// Block partials of each column's sum and largest magnitude (∞ for a non-finite value):
+// sums[c][blk], amax[c][blk]; grid (blocks, C).
+__global__ void __launch_bounds__(kXThreads)
+score_stats_kernel(const float* __restrict__ y, const float* __restrict__ rr, const float* __restrict__ Q, int64_t n,
+                   int64_t n_pad, int cq, double* __restrict__ sums, double* __restrict__ amax, int nblk)
+{
+  __shared__ double sh[32];
+  const int c = blockIdx.y;
+  const int64_t i0 = (int64_t)blockIdx.x * kXRows, i1 = min64(n, i0 + kXRows);
+  DF acc;
+  float mx = 0.f;
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += kXThreads) {
+    const float v = score_column(y, rr, Q, n_pad, cq, c, i);
+    df_add(acc, v);
+    mx = fmaxf(mx, isfinite(v) ? fabsf(v) : INFINITY);
+  }
+  const double s = block_sum_d(df_value(acc), sh);
+  __syncthreads();
+  double w = mx;
+  for (int o = 16; o; o >>= 1) w = fmax(w, __shfl_down_sync(0xffffffffu, w, o));
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = w;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int q = 1; q < kXThreads / 32; ++q) w = fmax(w, sh[q]);
+    sums[(int64_t)c * nblk + blockIdx.x] = s;
+    amax[(int64_t)c * nblk + blockIdx.x] = w;
+  }
+}
+
+// Operand of the count pass (N1 rows: column c's slices in rows 4c …, the rest zero) and of the
+// count-2 pass (16 rows: rr²'s slices, the rest zero).  Blocks y < C write column y of the first,
+// y = C the second (rr given), y > C one zero row of the first each.  A non-finite column is stored as zeros
+// (its terms come out NaN through its sum in the finish).
+__global__ void __launch_bounds__(kXThreads)
+score_operand_kernel(const float* __restrict__ y, const float* __restrict__ rr, const float* __restrict__ Q, int64_t n,
+                     int64_t n_pad, int cq, int C, const double* __restrict__ amax, int nblk, __half* __restrict__ B1,
+                     __half* __restrict__ B2)
+{
+  __shared__ double sa;
+  const int b = blockIdx.y;
+  const int64_t i0 = (int64_t)blockIdx.x * kXRows, i1 = min64(n_pad, i0 + kXRows);
+  if (b > C) {
+    for (int64_t i = i0 + threadIdx.x; i < i1; i += kXThreads)
+      B1[(int64_t)(kSlicesF32 * C + b - C - 1) * n_pad + i] = __float2half_rn(0.f);
+    return;
+  }
+  if (b == C && !rr) return;
+  const int c = b < C ? b : C - 1;
+  if (threadIdx.x < 32) {
+    const double v = warp_max_partials(amax + (int64_t)c * nblk, nblk);
+    if (threadIdx.x == 0) sa = v;
+  }
+  __syncthreads();
+  const int e = slice_exp(sa);
+  const bool fine = isfinite(sa);
+  __half* B = b < C ? B1 : B2;
+  const int row0 = b < C ? kSlicesF32 * c : 0;
+  for (int64_t i = i0 + threadIdx.x; i < i1; i += kXThreads) {
+    const float v = (i < n && fine) ? score_column(y, rr, Q, n_pad, cq, c, i) : 0.f;
+    store_slices<kSlicesF32>((double)v, e, B, n_pad, row0, i);
+    if (b == C)
+      for (int q = kSlicesF32; q < 16; ++q) B2[(int64_t)q * n_pad + i] = __float2half_rn(0.f);
+  }
+}
+
+// xy, xx per SNP from the exact sums, MAC filter → NaN.
+constexpr int kMaxScoreCols = 16;   // y, rr² and at most 14 projection columns
+__global__ void __launch_bounds__(kXThreads)
+score_finish_kernel(const float* __restrict__ D1, int splits1, int kp1, const float* __restrict__ D2, int splits2,
+                    int kp2, int64_t m_pad, int64_t m, int64_t n, const int32_t* __restrict__ n1,
+                    const int32_t* __restrict__ n2, int cq, int C, const double* __restrict__ sums,
+                    const double* __restrict__ amax, int nblk, int mac, float* __restrict__ xy, float* __restrict__ xx)
+{
+  __shared__ double ssum[kMaxScoreCols];
+  __shared__ int sexp[kMaxScoreCols];
+  for (int c = threadIdx.x >> 5; c < C; c += kXThreads / 32) {
+    const double s = warp_sum_partials(sums + (int64_t)c * nblk, nblk);
+    const double a = warp_max_partials(amax + (int64_t)c * nblk, nblk);
+    if ((threadIdx.x & 31) == 0) {
+      ssum[c] = isfinite(a) ? s : NAN;
+      sexp[c] = slice_exp(a);
     }
   }
-  part[(int64_t)s * n_pad + mt * 128 + t] = acc;
-}
-
-__global__ void gebv_finish_kernel(const double* __restrict__ part, int splits, int64_t n_pad, int64_t n,
-                                   double shift, double* __restrict__ tgv)
-{
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double s = shift;
-  for (int q = 0; q < splits; ++q) s += part[(int64_t)q * n_pad + i];
-  tgv[i] = s;
-}
-
-// Per SNP row (thread): acc[0] = Σ y·x, acc[1] = S1, acc[2] = S2, acc[3+l] = Σ rr·Q_l·x.
-// B rows: 0 = y, 1 = rr², 2.. = rr·Q_l (row stride K_pad); C = 2 + c rows, c ≤ 16.
-template <int C>
-__global__ void __launch_bounds__(128)
-score_kernel(const uint4* __restrict__ G, int64_t K_tiles, const float* __restrict__ B, int64_t K_pad,
-             int tiles_per_split, int64_t m_pad, double* __restrict__ part)
-{
-  __shared__ float sb[kXStage * kTileK][C];
-  const int t = threadIdx.x;
-  const int64_t mt = blockIdx.x;
-  const int s = blockIdx.y;
-  const int64_t kt0 = (int64_t)s * tiles_per_split, kt1 = min64(K_tiles, kt0 + tiles_per_split);
-  double acc[C + 1];
-#pragma unroll
-  for (int q = 0; q <= C; ++q) acc[q] = 0.0;
-  for (int64_t ks = kt0; ks < kt1; ks += kXStage) {
-    const int nt = (int)min64(kXStage, kt1 - ks);
-    __syncthreads();
-    for (int q = t; q < nt * kTileK * C; q += 128) {
-      const int r = q / (nt * kTileK), kk = q % (nt * kTileK);
-      sb[kk][r] = B[(int64_t)r * K_pad + ks * kTileK + kk];
-    }
-    __syncthreads();
-    for (int u = 0; u < nt; ++u) {
-      const uint4 pk = G[(mt * K_tiles + ks + u) * 128 + t];
-      const uint32_t w4[4] = {pk.x, pk.y, pk.z, pk.w};
-#pragma unroll
-      for (int w = 0; w < 4; ++w) {
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const uint32_t cnt = count_at(w4[w], e);
-          if (!cnt) continue;
-          const int kk = u * kTileK + w * 16 + e;
-          const double x = (double)cnt;
-          acc[0] = fma(x, (double)sb[kk][0], acc[0]);
-          const double r2 = (double)sb[kk][1];
-          acc[1] = fma(x, r2, acc[1]);
-          if (cnt == 2u) acc[2] += r2;
-#pragma unroll
-          for (int l = 2; l < C; ++l) acc[l + 1] = fma(x, (double)sb[kk][l], acc[l + 1]);
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int q = 0; q <= C; ++q) part[((int64_t)s * (C + 1) + q) * m_pad + mt * 128 + t] = acc[q];
-}
-
-// xy, xx per SNP from the accumulated sums (FP64), MAC filter → NaN.
-__global__ void score_finish_kernel(const double* __restrict__ part, int splits, int nacc, int64_t m_pad,
-                                    int64_t m, int64_t n, const int64_t* __restrict__ pc, int c,
-                                    double sum_y, double sum_r2, const double* __restrict__ sum_rq,
-                                    int mac, float* __restrict__ xy, float* __restrict__ xx)
-{
-  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  __syncthreads();
+  const int64_t j = (int64_t)blockIdx.x * kXThreads + threadIdx.x;
   if (j >= m) return;
-  double a[3 + 64];
-  for (int q = 0; q < nacc; ++q) {
-    double s = 0.0;
-    for (int p = 0; p < splits; ++p) s += part[((int64_t)p * nacc + q) * m_pad + j];
-    a[q] = s;
-  }
-  const double s_a1 = 2.0 * (double)n - (double)pc[j];   // Σ x with x = 2 − count
+  const double pc = (double)n1[j] + 2.0 * (double)n2[j];
+  const double s_a1 = 2.0 * (double)n - pc;   // Σ x with x = 2 − count
   if (s_a1 <= mac || 2.0 * (double)n - s_a1 <= mac) {
     xy[j] = __int_as_float(0x7fc00000);
     xx[j] = __int_as_float(0x7fc00000);
     return;
   }
-  const double gm = (double)pc[j] / (double)n;
-  xy[j] = (float)(-(a[0] - gm * sum_y));
-  double v = (a[1] + 2.0 * a[2]) - 2.0 * gm * a[1] + gm * gm * sum_r2;
-  for (int l = 0; l < c; ++l) {
-    const double ql = a[3 + l] - gm * sum_rq[l];
+  const double gm = pc / (double)n;
+  auto sum_of = [&](int c) {
+    return ldexp(gather_slices<kSlicesF32>(D1, splits1, kp1, m_pad, kSlicesF32 * c, j), -sexp[c]);
+  };
+  xy[j] = (float)(-(sum_of(0) - gm * ssum[0]));
+  double v;
+  if (D2 != nullptr) {
+    const double S1 = sum_of(C - 1);
+    const double S2x2 = ldexp(gather_slices<kSlicesF32>(D2, splits2, kp2, m_pad, 0, j), -sexp[C - 1]);   // 2·S2
+    v = (S1 + S2x2) - 2.0 * gm * S1 + gm * gm * ssum[C - 1];
+  } else {
+    v = (pc + 2.0 * (double)n2[j]) - 2.0 * gm * pc + gm * gm * (double)n;
+  }
+  for (int c = 1; c <= cq; ++c) {
+    const double ql = sum_of(c) - gm * ssum[c];
     v -= ql * ql;
   }
   xx[j] = (float)v;
 }
 
-// The same xy, xx from the tensor-core product when every rr is 1 (slemm_gamma's is_one_rr
-// case): out[l·m + j] = Z_hᵀv_l for the columns v = [y | Q_0 … Q_{c−1}] with Z_h centred by the
-// handle's gm_h; Σx·y and Σx·Q_l follow as out + gm_h·Σv, and Σx², the only rr-weighted sums, are
-// the integer counts pc + 2·n2.  Centred by the true mean gm = pc/n in FP64, as the FP64 kernel.
-__global__ void score_finish_tc_kernel(const float* __restrict__ out, int64_t m, int64_t n, int c,
-                                       const float* __restrict__ gmh, const int64_t* __restrict__ pc,
-                                       const int32_t* __restrict__ n2, double sum_y,
-                                       const double* __restrict__ sum_q, int mac, float* __restrict__ xy,
-                                       float* __restrict__ xx)
+// Split-K count of an exact product over K_tiles K-tiles: at most kExactKTiles of them each.
+static int exact_splits(int64_t M_pad, int64_t K_tiles, int N)
 {
-  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= m) return;
-  const double s_a1 = 2.0 * (double)n - (double)pc[j];
-  if (s_a1 <= mac || 2.0 * (double)n - s_a1 <= mac) {
-    xy[j] = __int_as_float(0x7fc00000);
-    xx[j] = __int_as_float(0x7fc00000);
-    return;
-  }
-  const double gm = (double)pc[j] / (double)n;
-  const double dg = (double)gmh[j] - gm;   // Σx·v − gm·Σv = out + (gm_h − gm)·Σv
-  xy[j] = (float)(-((double)out[j] + dg * sum_y));
-  double v = ((double)pc[j] + 2.0 * (double)n2[j]) - 2.0 * gm * (double)pc[j] + gm * gm * (double)n;
-  for (int l = 0; l < c; ++l) {
-    const double ql = (double)out[(int64_t)(1 + l) * m + j] + dg * sum_q[l];
-    v -= ql * ql;
-  }
-  xx[j] = (float)v;
+  return choose_splits(M_pad / gemm_tc_rows_per_cta(N, 0), K_tiles, 1, num_sms(),
+                       (int)ceil_div(K_tiles, kExactKTiles));
 }
 
 }  // namespace slemm
@@ -184,45 +241,36 @@ int slemm_gpu_gebv(slemm_geno* g, const double* alpha, const uint8_t* flip, doub
       SLEMM_THROW(SLEMM_ERR_UNSUPPORTED, "slemm_gpu_gebv reads the packed copies directly and is not available on a "
                                          "trait view; create a handle with the keep list instead");
     cudaStream_t st = g->stream;
-    std::vector<double> a(g->m_pad, 0.0);
-    double shift = 0.0;
+    std::vector<double> a(g->m);
+    double shift = 0.0, amax = 0.0;
     for (int64_t j = 0; j < g->m; ++j) {
       CHECK_ARG(std::isfinite(alpha[j]), "non-finite SNP effect");
       const bool f = flip && flip[j];
       a[j] = f ? -alpha[j] : alpha[j];
       if (f) shift += 2.0 * alpha[j];
+      amax = std::max(amax, std::fabs(alpha[j]));
     }
-    const int64_t M_tiles = g->n_pad / kTileM, K_tiles = g->m_pad / kTileK;
-    const int splits = choose_splits(M_tiles, K_tiles, 8, num_sms());
-    const int tps = (int)ceil_div(K_tiles, splits);
-    DevBuf d_a(st), d_part(st), d_out(st);
+    const int e = slice_exp(amax);
+    const int64_t K_tiles = g->m_pad / kTileK;
+    const int N = 16, kp = 8;
+    const int splits = exact_splits(g->n_pad, K_tiles, N);
+    DevBuf d_a(st), d_out(st);
     d_a.ensure(a.size() * sizeof(double));
-    d_part.ensure((size_t)splits * g->n_pad * sizeof(double));
     d_out.ensure((size_t)g->n * sizeof(double));
+    __half* B = (__half*)g->ws_B.ensure((size_t)N * g->m_pad * sizeof(__half));
+    float* D = (float*)g->ws_D.ensure((size_t)splits * kp * g->n_pad * sizeof(float));
     CUDA_TRY(cudaMemcpyAsync(d_a.p, a.data(), a.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-    gebv_kernel<<<dim3((unsigned)M_tiles, splits), 128, 0, st>>>(g->GT.as<uint4>(), K_tiles, d_a.as<double>(), tps,
-                                                                 g->n_pad, d_part.as<double>());
+    gebv_operand_kernel<<<(unsigned)ceil_div(g->m_pad, kXThreads), kXThreads, 0, st>>>(d_a.as<double>(), g->m, g->m_pad,
+                                                                                      e, B);
     LAUNCH_CHECK();
-    gebv_finish_kernel<<<(unsigned)ceil_div(g->n, 256), 256, 0, st>>>(d_part.as<double>(), splits, g->n_pad, g->n,
-                                                                      shift, d_out.as<double>());
+    gemm_tc({g->GT.as<uint8_t>(), g->n_pad, g->m_pad, B, N, D, splits, g->err.as<int>(), kp, 1, true}, st);
+    gebv_finish_kernel<<<(unsigned)ceil_div(g->n, kXThreads), kXThreads, 0, st>>>(D, splits, kp, g->n_pad, g->n, e, shift,
+                                                                                 d_out.as<double>());
     LAUNCH_CHECK();
     CUDA_TRY(cudaMemcpyAsync(tgv, d_out.p, g->n * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    check_device_error(g);
   });
 }
-
-}  // extern "C"
-
-template <int C>
-static void launch_score(slemm_geno* g, const float* B, int64_t K_pad, int splits, int tps, double* part)
-{
-  const int64_t M_tiles = g->m_pad / kTileM, K_tiles = g->n_pad / kTileK;
-  score_kernel<C><<<dim3((unsigned)M_tiles, splits), 128, 0, g->stream>>>(g->G.as<uint4>(), K_tiles, B, K_pad, tps,
-                                                                          g->m_pad, part);
-  LAUNCH_CHECK();
-}
-
-extern "C" {
 
 int slemm_gpu_score_terms(slemm_geno* g, const float* y, int mac, float* xy, float* xx)
 {
@@ -236,135 +284,45 @@ int slemm_gpu_score_terms(slemm_geno* g, const float* y, int mac, float* xy, flo
     CHECK_ARG(c <= 14, "score terms support up to 14 projection columns");
     cudaStream_t st = g->stream;
     const int64_t n = g->n, n_pad = g->n_pad;
-    // host-side B rows: y, rr², rr·Q_l (FP32), and the FP64 column sums
-    std::vector<float> rr(n_pad, 0.f), Q((size_t)n_pad * std::max(c, 1), 0.f);
-    CUDA_TRY(cudaMemcpyAsync(rr.data(), g->rr.p, n_pad * sizeof(float), cudaMemcpyDeviceToHost, st));
-    if (c) CUDA_TRY(cudaMemcpyAsync(Q.data(), g->Q.p, (size_t)n_pad * c * sizeof(float), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    bool one_rr = true;
-    for (int64_t i = 0; i < n && one_rr; ++i) one_rr = rr[i] == 1.0f;
-    if (one_rr) {
-      // the packed tensor-core product of [y | Q] (column-scaled FP16 hi+lo pieces, FP32 accumulation);
-      // the FP64 per-genotype kernel below serves general rr
-      const int k = 1 + c;
-      std::vector<float> V((size_t)k * n);
-      double sum_y = 0.0;
-      std::vector<double> sum_q(std::max(c, 1), 0.0);
-      for (int64_t i = 0; i < n; ++i) {
-        V[i] = y[i];
-        sum_y += (double)y[i];
-      }
-      for (int l = 0; l < c; ++l)
-        for (int64_t i = 0; i < n; ++i) {
-          const float q = Q[(size_t)l * n_pad + i];
-          V[(size_t)(1 + l) * n + i] = q;
-          sum_q[l] += (double)q;
-        }
-      std::vector<int64_t> pc(g->m);
-      std::vector<int32_t> n2(g->m);
-      {
-        const int s2 = slemm_gpu_genotype_counts(g, pc.data(), nullptr, nullptr, n2.data());
-        if (s2 != SLEMM_OK) SLEMM_THROW(s2, "genotype counts failed");
-      }
-      DevBuf dV(st), dO(st), dpc(st), dn2(st), dsq(st), dxy(st), dxx(st);
-      dV.ensure(V.size() * sizeof(float));
-      dO.ensure((size_t)k * g->m * sizeof(float));
-      dpc.ensure(g->m * sizeof(int64_t));
-      dn2.ensure(g->m * sizeof(int32_t));
-      dsq.ensure(sum_q.size() * sizeof(double));
-      dxy.ensure(g->m * sizeof(float));
-      dxx.ensure(g->m * sizeof(float));
-      CUDA_TRY(cudaMemcpyAsync(dV.p, V.data(), V.size() * sizeof(float), cudaMemcpyHostToDevice, st));
-      CUDA_TRY(cudaMemcpyAsync(dpc.p, pc.data(), g->m * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-      CUDA_TRY(cudaMemcpyAsync(dn2.p, n2.data(), g->m * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-      CUDA_TRY(cudaMemcpyAsync(dsq.p, sum_q.data(), sum_q.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-      const int prec = g->prec;
-      g->prec = SLEMM_PREC_FP16X2;
-      try {
-        op_device(g, SLEMM_OP_RMATVEC, 0.f, dV.as<float>(), n, k, dO.as<float>(), g->m);
-      } catch (...) {
-        g->prec = prec;
-        throw;
-      }
-      g->prec = prec;
-      score_finish_tc_kernel<<<(unsigned)ceil_div(g->m, 256), 256, 0, st>>>(
-          dO.as<float>(), g->m, n, c, g->gm.as<float>(), dpc.as<int64_t>(), dn2.as<int32_t>(), sum_y,
-          dsq.as<double>(), mac, dxy.as<float>(), dxx.as<float>());
-      LAUNCH_CHECK();
-      CUDA_TRY(cudaMemcpyAsync(xy, dxy.p, g->m * sizeof(float), cudaMemcpyDeviceToHost, st));
-      CUDA_TRY(cudaMemcpyAsync(xx, dxx.p, g->m * sizeof(float), cudaMemcpyDeviceToHost, st));
-      CUDA_TRY(cudaStreamSynchronize(st));
-      return;
-    }
-    const int C = 2 + c;
-    std::vector<float> B((size_t)C * n_pad, 0.f);
-    double sum_y = 0.0, sum_r2 = 0.0;
-    std::vector<double> sum_rq(std::max(c, 1), 0.0);
-    for (int64_t i = 0; i < n; ++i) {
-      B[i] = y[i];
-      B[n_pad + i] = rr[i] * rr[i];
-      sum_y += (double)y[i];
-      sum_r2 += (double)rr[i] * rr[i];
-      for (int l = 0; l < c; ++l) {
-        const float v = rr[i] * Q[(size_t)l * n_pad + i];
-        B[(size_t)(2 + l) * n_pad + i] = v;
-        sum_rq[l] += (double)v;
-      }
-    }
-    const int64_t M_tiles = g->m_pad / kTileM, K_tiles = n_pad / kTileK;
-    const int splits = choose_splits(M_tiles, K_tiles, 8, num_sms());
-    const int tps = (int)ceil_div(K_tiles, splits);
-    DevBuf dB(st), dpart(st), dsrq(st), dxy(st), dxx(st), dpc(st);
-    dB.ensure(B.size() * sizeof(float));
-    dpart.ensure((size_t)splits * (C + 1) * g->m_pad * sizeof(double));
-    dsrq.ensure(sum_rq.size() * sizeof(double));
-    dxy.ensure(g->m * sizeof(float));
-    dxx.ensure(g->m * sizeof(float));
-    dpc.ensure(g->m * sizeof(int64_t));
-    std::vector<int64_t> pc(g->m);
-    {
-      int s2 = slemm_gpu_genotype_counts(g, pc.data(), nullptr, nullptr, nullptr);
-      if (s2 != SLEMM_OK) SLEMM_THROW(s2, "genotype counts failed");
-    }
-    CUDA_TRY(cudaMemcpyAsync(dpc.p, pc.data(), g->m * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(dB.p, B.data(), B.size() * sizeof(float), cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(dsrq.p, sum_rq.data(), sum_rq.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-    double* part = dpart.as<double>();
-    switch (C) {
-      case 2: launch_score<2>(g, dB.as<float>(), n_pad, splits, tps, part); break;
-      case 3: launch_score<3>(g, dB.as<float>(), n_pad, splits, tps, part); break;
-      case 4: launch_score<4>(g, dB.as<float>(), n_pad, splits, tps, part); break;
-      case 5: launch_score<5>(g, dB.as<float>(), n_pad, splits, tps, part); break;
-      case 6: launch_score<6>(g, dB.as<float>(), n_pad, splits, tps, part); break;
-      case 8: launch_score<8>(g, dB.as<float>(), n_pad, splits, tps, part); break;
-      default: {
-        // widths 7 and 9..16: pad the B rows up to the next supported width with zero rows
-        const int Cp = C <= 8 ? 8 : 16;
-        std::vector<float> Bp((size_t)Cp * n_pad, 0.f);
-        std::copy(B.begin(), B.end(), Bp.begin());
-        DevBuf dBp(st), dpp(st);
-        dBp.ensure(Bp.size() * sizeof(float));
-        dpp.ensure((size_t)splits * (Cp + 1) * g->m_pad * sizeof(double));
-        CUDA_TRY(cudaMemcpyAsync(dBp.p, Bp.data(), Bp.size() * sizeof(float), cudaMemcpyHostToDevice, st));
-        if (Cp == 8) launch_score<8>(g, dBp.as<float>(), n_pad, splits, tps, dpp.as<double>());
-        else launch_score<16>(g, dBp.as<float>(), n_pad, splits, tps, dpp.as<double>());
-        score_finish_kernel<<<(unsigned)ceil_div(g->m, 256), 256, 0, st>>>(
-            dpp.as<double>(), splits, Cp + 1, g->m_pad, g->m, n, dpc.as<int64_t>(), c, sum_y, sum_r2,
-            dsrq.as<double>(), mac, dxy.as<float>(), dxx.as<float>());
-        LAUNCH_CHECK();
-        CUDA_TRY(cudaMemcpyAsync(xy, dxy.p, g->m * sizeof(float), cudaMemcpyDeviceToHost, st));
-        CUDA_TRY(cudaMemcpyAsync(xx, dxx.p, g->m * sizeof(float), cudaMemcpyDeviceToHost, st));
-        CUDA_TRY(cudaStreamSynchronize(st));
-        return;
-      }
-    }
-    score_finish_kernel<<<(unsigned)ceil_div(g->m, 256), 256, 0, st>>>(
-        part, splits, C + 1, g->m_pad, g->m, n, dpc.as<int64_t>(), c, sum_y, sum_r2, dsrq.as<double>(), mac,
-        dxy.as<float>(), dxx.as<float>());
+    const float* rr = g->rr_one ? nullptr : g->rr.as<float>();
+    const int C = 1 + c + (rr ? 1 : 0);
+    const int64_t K_tiles = n_pad / kTileK;
+    const int nblk = (int)ceil_div(n_pad, kXRows);
+    const int kp1 = (int)round_up(kSlicesF32 * C, 8), kp2 = 8;
+    const int N1 = (int)round_up(kp1, 16), N2 = 16;
+    const int sp1 = exact_splits(g->m_pad, K_tiles, N1), sp2 = exact_splits(g->m_pad, K_tiles, N2);
+    DevBuf dy(st), dstat(st), dcnt(st), dout(st);
+    float* yv = (float*)dy.ensure((size_t)n * sizeof(float));
+    double* sums = (double*)dstat.ensure((size_t)2 * C * nblk * sizeof(double));
+    double* amax = sums + (size_t)C * nblk;
+    int64_t* pc = (int64_t*)dcnt.ensure((size_t)g->m * (sizeof(int64_t) + 2 * sizeof(int32_t)));
+    int32_t* n1 = reinterpret_cast<int32_t*>(pc + g->m);
+    int32_t* n2 = n1 + g->m;
+    float* oxy = (float*)dout.ensure((size_t)2 * g->m * sizeof(float));
+    float* oxx = oxy + g->m;
+    __half* B1 = (__half*)g->ws_B.ensure((size_t)(N1 + N2) * n_pad * sizeof(__half));
+    __half* B2 = B1 + (size_t)N1 * n_pad;
+    const size_t d1 = (size_t)sp1 * kp1 * g->m_pad, d2 = (size_t)sp2 * kp2 * g->m_pad;
+    float* D1 = (float*)g->ws_D.ensure((d1 + d2) * sizeof(float));
+    float* D2 = D1 + d1;
+    CUDA_TRY(cudaMemcpyAsync(yv, y, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, st));
+    row_counts_device(g, pc, n1, n2);
+    const float* Q = g->Q.as<float>();
+    score_stats_kernel<<<dim3(nblk, C), kXThreads, 0, st>>>(yv, rr, Q, n, n_pad, c, sums, amax, nblk);
     LAUNCH_CHECK();
-    CUDA_TRY(cudaMemcpyAsync(xy, dxy.p, g->m * sizeof(float), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaMemcpyAsync(xx, dxx.p, g->m * sizeof(float), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
+    score_operand_kernel<<<dim3(nblk, C + 1 + N1 - kSlicesF32 * C), kXThreads, 0, st>>>(yv, rr, Q, n, n_pad, c, C, amax, nblk,
+                                                                                      B1, B2);
+    LAUNCH_CHECK();
+    const uint8_t* G = g->G.as<uint8_t>();
+    int* err = g->err.as<int>();
+    gemm_tc({G, g->m_pad, n_pad, B1, N1, D1, sp1, err, kp1, 1, true}, st);
+    if (rr) gemm_tc({G, g->m_pad, n_pad, B2, N2, D2, sp2, err, kp2, 1, true, 0, true}, st);
+    score_finish_kernel<<<(unsigned)ceil_div(g->m, kXThreads), kXThreads, 0, st>>>(
+        D1, sp1, kp1, rr ? D2 : nullptr, sp2, kp2, g->m_pad, g->m, n, n1, n2, c, C, sums, amax, nblk, mac, oxy, oxx);
+    LAUNCH_CHECK();
+    CUDA_TRY(cudaMemcpyAsync(xy, oxy, (size_t)g->m * sizeof(float), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaMemcpyAsync(xx, oxx, (size_t)g->m * sizeof(float), cudaMemcpyDeviceToHost, st));
+    check_device_error(g);
   });
 }
 

@@ -261,7 +261,7 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
       : "memory");
 }
 
-template <int PK, int S, int SB, int KT, bool F16, int TM>
+template <int PK, int S, int SB, int KT, bool F16, int TM, bool TWOS>
 __global__ void __launch_bounds__(tc_max_threads(TM), tc_min_blocks(TM))
 gemm_tc_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMap tmapB,
                float* __restrict__ D, int64_t M_pad, int K_tiles, int tiles_per_split, int N, int sub,
@@ -440,7 +440,7 @@ gemm_tc_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMa
 #pragma unroll
         for (int w = 0; w < 4; ++w)
 #pragma unroll
-          for (int q = 0; q < 8; ++q) v[w * 8 + q] = pair_of<F16>(words[w], q);
+          for (int q = 0; q < 8; ++q) v[w * 8 + q] = pair_of<F16, TWOS>(words[w], q);
         if (kk == 0 && i >= S) {   // the stage that last used this A slot has been consumed
           got = mbar_wait(&done[(i - S) % BS], (uint32_t)((i - S) / BS) & 1, err, 64, abort_flag, 64);
           if (!__all_sync(0xffffffffu, got)) {
@@ -549,7 +549,7 @@ static void configure_once()
   done.fetch_or(bit);
 }
 
-template <int PK, int S, int SB, int KT, bool F16, int TM = 512>
+template <int PK, int S, int SB, int KT, bool F16, int TM = 512, bool TWOS = false>
 static void launch_tc(const GemmArgs& a, cudaStream_t st)
 {
   const TcPlan<PK, S, SB, KT> P = plan_tc<PK, S, SB, KT, TM>(a.N);
@@ -573,15 +573,14 @@ static void launch_tc(const GemmArgs& a, cudaStream_t st)
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) SLEMM_THROW(SLEMM_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
 
-  configure_once<gemm_tc_kernel<PK, S, SB, KT, F16, TM>>();
+  configure_once<gemm_tc_kernel<PK, S, SB, KT, F16, TM, TWOS>>();
   CHECK_ARG(a.kp % 8 == 0 && a.pieces >= 1 && a.pieces * a.kp <= a.N, "bad piece layout");
   // Each CTA allocates TM of the SM's 512 TMEM columns: request enough shared memory that at most
   // 512 / TM CTAs are resident per SM, so no allocation ever has to wait for another CTA's release.
   const size_t smem = std::max<size_t>(P.total, TM == 512 ? 120 * 1024 : 80 * 1024);
   dim3 grid((unsigned)Mc, (unsigned)a.splits);
-  gemm_tc_kernel<PK, S, SB, KT, F16, TM><<<grid, P.threads(), smem, st>>>(a.A, map, a.D, a.M_pad, K_tiles, tps, a.N,
-                                                                       P.sub, a.kp, a.pieces, a.err,
-                                                                       g_withhold_b.exchange(-1));
+  gemm_tc_kernel<PK, S, SB, KT, F16, TM, TWOS><<<grid, P.threads(), smem, st>>>(
+      a.A, map, a.D, a.M_pad, K_tiles, tps, a.N, P.sub, a.kp, a.pieces, a.err, g_withhold_b.exchange(-1));
   LAUNCH_CHECK();
 }
 
@@ -589,8 +588,10 @@ void gemm_tc(const GemmArgs& a, cudaStream_t st)
 {
   CHECK_ARG(a.N >= 16 && a.N <= 256 && a.N % 16 == 0, "TC path needs N in [16,256], N%16==0");
   CHECK_ARG(a.plan == 0 || (a.plan == 1 && a.N <= kNarrowN), "unknown tensor-core plan");
+  CHECK_ARG(!a.twos || (a.f16 && a.N <= kNarrowN && a.plan == 0), "the count-2 matrix has an FP16 plan for N <= 64 only");
   if (a.f16) {
-    if (a.N > kNarrowN) launch_tc<4, 3, 6, 1, true>(a, st);
+    if (a.twos) launch_tc<6, 3, 0, 2, true, 512, true>(a, st);
+    else if (a.N > kNarrowN) launch_tc<4, 3, 6, 1, true>(a, st);
     else if (a.plan == 1) launch_tc<6, 3, 0, 2, true, 256>(a, st);
     else launch_tc<6, 3, 0, 2, true>(a, st);
   } else {

@@ -15,6 +15,7 @@ struct slemm_geno {
   slemm::DevBuf Q;                // n_pad × c column-major, zero padded rows
   int c = 0;
   bool weights_set = false;
+  bool rr_one = false;            // every rr of set_weights is 1
   int prec = SLEMM_PREC_FP16X2;
   int per_vector = 0;
   int lanczos_mode = 0;           // SLEMM_LANCZOS_* bits of the seeds run on this handle

@@ -1,0 +1,67 @@
+"""GEBV and the GWAS score terms against extended- and double-precision sums, at the edges of the
+exact product's tiles and of its 8,192-element partial sums."""
+import numpy as np
+import pytest
+
+from conftest import make_case
+from slemm_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,m", [(1, 1), (257, 127), (300, 8192), (129, 8193), (1000, 16640)])
+def test_gebv_exact_products(gpu, n, m):
+    from slemm_gb300 import api
+    rows, _, dec = make_case(n, m, seed=n + m, missing=0.02)
+    rng = np.random.default_rng(m)
+    alpha = rng.standard_normal(m) * 10.0 ** rng.uniform(-12, 2, m)
+    flip = (rng.random(m) < 0.5).astype(np.uint8)
+    with api.Genotypes(rows, n) as g:
+        got = g.gebv(alpha, flip)
+    x = dec.astype(np.longdouble)
+    want = (np.where(flip[:, None] == 1, 2 - x, x) * alpha.astype(np.longdouble)[:, None]).sum(0)
+    # the slices resolve 2^-65 of max|alpha|; the shift 2·Σalpha is a running FP64 sum of m terms and
+    # the last combination rounds a few times
+    assert np.abs(got - want).max() <= 2.0 ** -52 * 4 * m * np.abs(alpha).max()
+
+
+@pytest.mark.parametrize("value", [0.7, -1.0, 2.0 ** -1060, 1e300])
+def test_gebv_largest_partial_sums(gpu, value):
+    """Every count 2 and every effect the same: the partial sums reach their bound of 2^24."""
+    from slemm_gb300 import api
+    n, m = 130, 8192 + 64
+    with api.Genotypes(synth.encode_bed(np.full((m, n), 2, np.uint8)), n) as g:
+        got = g.gebv(np.full(m, value))
+    want = 2.0 * m * value
+    assert np.abs(got - want).max() <= 2.0 ** -51 * abs(want)
+
+
+@pytest.mark.parametrize("n,m,c,unit", [(255, 1, 0, False), (8192, 130, 1, False), (8200, 257, 14, False),
+                                        (20001, 300, 3, False), (8200, 257, 14, True), (513, 129, 0, True)])
+def test_score_terms_exact_products(gpu, n, m, c, unit):
+    from slemm_gb300 import api
+    rows, _, dec = make_case(n, m, seed=n + c, missing=0.01)
+    rng = np.random.default_rng(n)
+    y = (rng.standard_normal(n) * 3 + 1).astype(np.float32)
+    rr = np.ones(n, np.float32) if unit else (1 / np.sqrt(10.0 ** rng.uniform(-3, 3, n))).astype(np.float32)
+    X = np.column_stack([np.ones(n)] + [rng.standard_normal(n) for _ in range(c)])[:, :c]
+    Q = np.linalg.qr(rr[:, None] * X)[0].astype(np.float32) if c else np.zeros((n, 0), np.float32)
+    x = dec.astype(np.float64)
+    gm = x.mean(1)
+    with api.Genotypes(rows, n) as g:
+        g.set_weights(gm.astype(np.float32), np.ones(m, np.float32), rr)
+        g.set_projection(Q)
+        xy, xx = g.score_terms(y, 0)
+        bad = y.copy()
+        bad[n // 2] = np.nan
+        nan_xy, same_xx = g.score_terms(bad, 0)
+    z = x - gm[:, None]
+    want_xy = -(z @ y.astype(np.float64))
+    # the columns as the kernel takes them: rr·Q_l and rr² rounded to FP32
+    r2 = (rr * rr).astype(np.float64)
+    rq = (rr[:, None] * Q).astype(np.float64)
+    want_xx = (z * z) @ r2 - ((z @ rq) ** 2).sum(1)
+    # FP32 rounding of the result, and the FP64 cancellation of the centring terms
+    assert np.all(np.abs(xy - want_xy) <= 2.0 ** -23 * np.abs(want_xy) + 1e-12 * np.abs(y).sum())
+    assert np.all(np.abs(xx - want_xx) <= 2.0 ** -23 * np.abs(want_xx) + 1e-12 * r2.sum())
+    assert np.all(np.isnan(nan_xy)) and np.array_equal(same_xx, xx)
