@@ -196,6 +196,8 @@ struct GemmArgs {
   int plan = 0;         // TC ring plan: 0 by N (N ≤ 64: two tiles per CTA, one CTA per SM), 1: N ≤ 64,
                         // one tile per CTA and two CTAs per SM (256 TMEM columns each)
   bool twos = false;    // TC, FP16, N ≤ 64, plan 0: the matrix is 2·[count = 2] instead of the count
+  int groups = 1;       // TC: products of as many operands B[grp] (N rows each, one after the other) with
+                        // the same matrix, partials [groups][splits][kp][M_pad]
 };
 
 void gemm_simt(const GemmArgs& a, cudaStream_t st);

@@ -358,13 +358,13 @@ gemm_tc_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMa
         uint64_t* full = (SB > 0) ? &b_full[s] : &st_full[s];
         if (i >= BS && !mbar_wait(&done[s], (round - 1) & 1, err, 16, abort_flag, 128)) break;
         if (*abort_flag) break;
-        if (i == withhold && blockIdx.x == 0 && blockIdx.y == 0) {   // test support: the stage never fills
+        if (i == withhold && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {   // test support: the stage never fills
           ++issued;
           continue;
         }
         mbar_arrive_expect_tx(full, (uint32_t)KT * bytes);
         for (int kk = 0; kk < KT; ++kk)
-          tma_load_2d(sB + ((size_t)s * KT + kk) * N * 128, &tmapB, (kt0 + i * KT + kk) * kTileK, 0, full);
+          tma_load_2d(sB + ((size_t)s * KT + kk) * N * 128, &tmapB, (kt0 + i * KT + kk) * kTileK, (int)blockIdx.z * N, full);
         ++issued;
       }
       if (*abort_flag)
@@ -468,7 +468,7 @@ gemm_tc_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMa
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (ok) {
         // column c of D = Σ_p accumulator column p·kp + c (the pieces of c): kp columns per split
-        float* Dbase = D + ((size_t)split * kp) * M_pad + (mt0 + tsub) * 128 + r;
+        float* Dbase = D + (((size_t)blockIdx.z * gridDim.y + split) * kp) * M_pad + (mt0 + tsub) * 128 + r;
         const uint32_t tl = tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)(tsub * N);
         for (int c0 = 0; c0 < kp; c0 += 8) {
           float acc[8] = {};
@@ -562,7 +562,7 @@ static void launch_tc(const GemmArgs& a, cudaStream_t st)
   const int tps = (int)(ceil_div(ceil_div(K_tiles, a.splits), KT) * KT);   // whole stages per split
 
   CUtensorMap map;
-  const cuuint64_t dims[2] = {(cuuint64_t)a.K_pad, (cuuint64_t)a.N};
+  const cuuint64_t dims[2] = {(cuuint64_t)a.K_pad, (cuuint64_t)a.N * a.groups};
   const cuuint64_t strides[1] = {(cuuint64_t)a.K_pad * 2};
   const cuuint32_t box[2] = {64, (cuuint32_t)a.N};
   const cuuint32_t estr[2] = {1, 1};
@@ -578,7 +578,7 @@ static void launch_tc(const GemmArgs& a, cudaStream_t st)
   // Each CTA allocates TM of the SM's 512 TMEM columns: request enough shared memory that at most
   // 512 / TM CTAs are resident per SM, so no allocation ever has to wait for another CTA's release.
   const size_t smem = std::max<size_t>(P.total, TM == 512 ? 120 * 1024 : 80 * 1024);
-  dim3 grid((unsigned)Mc, (unsigned)a.splits);
+  dim3 grid((unsigned)Mc, (unsigned)a.splits, (unsigned)a.groups);
   gemm_tc_kernel<PK, S, SB, KT, F16, TM, TWOS><<<grid, P.threads(), smem, st>>>(
       a.A, map, a.D, a.M_pad, K_tiles, tps, a.N, P.sub, a.kp, a.pieces, a.err, g_withhold_b.exchange(-1));
   LAUNCH_CHECK();

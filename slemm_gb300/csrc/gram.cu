@@ -1,0 +1,610 @@
+// gram.cu — projected Gram blocks of SNP rows, and the batched factorisation of their systems
+// (the windows of --lmm and the blocks of slemm_gwa).
+//
+// With P = I − QQᵀ, z_j = x_j − gm_j the centred counts of SNP j and t_j = Qᵀ(rr∘z_j),
+//   G_jk = (P(rr∘z_j))ᵀ(P(rr∘z_k)) = Σ_i rr_i²·x_ij·z_ik − gm_j·h_k − t_jᵀt_k,   h_k = Σ_i rr_i²·z_ik.
+// h and t come from one exact pass over the packed matrix (gram_stats), so a Gram block is one
+// packed product of SNP rows with columns that are read straight from the packed rows, and no
+// dense FP32 column of n individuals is ever formed.  In general the columns are rr²∘z_k,
+// column-scaled FP16 hi+lo; with every rr 1 they are the counts themselves, one FP16 piece whose
+// product is an exact integer, and Σ_i x_ij·z_ik = Σ_i x_ij·x_ik − p_j·gm_k with p_j = Σ_i x_ij.  Forming U = rr∘P(rr∘z) as FP32
+// columns instead (centre, project, scale, measure, split: nine passes over n × columns floats)
+// took 38 of the 82 ms of slemm_gwa at n = 50,021 with 20,011 variants and 4,000 model SNPs, and
+// 31 of the 73 ms of --lmm with 30 windows of 1,000 SNPs at n = 50,000.
+#include "gram.h"
+#include "decode.cuh"
+#include "reduce.cuh"
+
+namespace slemm {
+
+// ---- per-SNP statistics ------------------------------------------------------------------------
+__global__ void __launch_bounds__(256)
+gram_stats_kernel(const double* __restrict__ dots, const double* __restrict__ twos, const double* __restrict__ tot,
+                  int64_t m, int64_t n, const int64_t* __restrict__ pc, const int32_t* __restrict__ n2,
+                  const float* __restrict__ gmf, int yb, int cq, GramStats s)
+{
+  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= m) return;
+  const double p = (double)pc[j], gm = (double)gmf[j];
+  double h, xx;
+  if (twos != nullptr) {   // the last column is rr²
+    const double S1 = dots[(int64_t)(yb + cq) * m + j], R = tot[yb + cq];
+    h = S1 - gm * R;
+    xx = (S1 + twos[j]) - 2.0 * gm * S1 + gm * gm * R;
+  } else {
+    h = p - gm * (double)n;
+    xx = (p + 2.0 * (double)n2[j]) - 2.0 * gm * p + gm * gm * (double)n;
+  }
+  for (int l = 0; l < cq; ++l) {
+    const double t = dots[(int64_t)(yb + l) * m + j] - gm * tot[yb + l];
+    s.t[(int64_t)l * s.ld + j] = (float)t;
+    xx -= t * t;
+  }
+  float a, b;
+  split_double(h, a, b);
+  s.h[j] = make_float2(a, b);
+  split_double(twos != nullptr ? 0.0 : p, a, b);
+  s.p[j] = make_float2(a, b);
+  s.gm[j] = gmf[j];
+  s.xy[j] = yb ? dots[j] - gm * tot[0] : 0.0;
+  s.xx[j] = xx;
+}
+
+void gram_stats(slemm_geno* g, const float* gm, const float* y, const float* rr, const float* Q, int cq,
+                GramStatsBuf& out)
+{
+  cudaStream_t st = g->stream;
+  const int64_t m = g->m;
+  const ExactCols cols{y, rr, Q, g->n_pad, cq};
+  const int C = cols.count();
+  DevBuf d(st), dc(st);
+  double* dots = (double*)d.ensure(((size_t)(C + 1) * m + C) * sizeof(double));
+  double* twos = rr ? dots + (size_t)C * m : nullptr;
+  double* tot = dots + (size_t)(C + 1) * m;
+  int64_t* pc = (int64_t*)dc.ensure((size_t)m * (sizeof(int64_t) + 2 * sizeof(int32_t)));
+  int32_t* n1 = reinterpret_cast<int32_t*>(pc + m);
+  row_counts_device(g, pc, n1, n1 + m);
+  if (C > 0) exact_dots(g, cols, dots, tot, twos);
+  const GramStats s = out.make(m, cq, st);
+  gram_stats_kernel<<<(unsigned)ceil_div(m, 256), 256, 0, st>>>(dots, twos, tot, m, g->n, pc, n1 + m, gm, y ? 1 : 0, cq,
+                                                                 s);
+  LAUNCH_CHECK();
+}
+
+// dst SNP k = src SNP idx[k]
+__global__ void gram_stats_gather_kernel(GramStats src, const int64_t* __restrict__ idx, int64_t cnt, int cq, GramStats dst)
+{
+  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= cnt) return;
+  const int64_t j = idx[k];
+  dst.gm[k] = src.gm[j];
+  dst.h[k] = src.h[j];
+  dst.p[k] = src.p[j];
+  dst.xy[k] = src.xy[j];
+  dst.xx[k] = src.xx[j];
+  for (int l = 0; l < cq; ++l) dst.t[(int64_t)l * dst.ld + k] = src.t[(int64_t)l * src.ld + j];
+}
+
+void gram_stats_gather(const GramStats& src, const int64_t* d_idx, int64_t cnt, int cq, GramStatsBuf& out, cudaStream_t st)
+{
+  const GramStats s = out.make(cnt, cq, st);
+  gram_stats_gather_kernel<<<(unsigned)ceil_div(cnt, 256), 256, 0, st>>>(src, d_idx, cnt, cq, s);
+  LAUNCH_CHECK();
+}
+
+// ---- Gram blocks ----------------------------------------------------------------------------------
+// Operand of the columns SNP j0 … j0 + ncols − 1, group by group: column c is row c % kc of group
+// c / kc, a group's rows kc … kp − 1 are zero.  UNIT: N = kp rows of counts per group.  Otherwise
+// N = 2·kp rows, pieces hi and lo of rr²·z·2^e.  Each value is stored times the 2^−2s of its K position
+// (f16sub_pair_of).  A thread writes 8 K-elements (half of a packed word): 16-byte stores, 512
+// contiguous bytes per warp.  Bound by the 16-bit operand it writes.
+template <bool UNIT>
+__global__ void __launch_bounds__(256)
+gram_operand_kernel(const uint32_t* __restrict__ G, int64_t K_tiles, int64_t j0, int64_t ncols, int kc, int kp,
+                    const float* __restrict__ gm, const float* __restrict__ rr, float scale, __half* __restrict__ B)
+{
+  const int64_t q8 = (int64_t)blockIdx.x * 256 + threadIdx.x;   // K-elements 8·q8 …
+  const int64_t K_pad = K_tiles * kTileK;
+  if (q8 * 8 >= K_pad) return;
+  const int grp = blockIdx.z, r = blockIdx.y;
+  const int N = UNIT ? kp : 2 * kp;
+  __half* dst = B + ((int64_t)grp * N + r) * K_pad + q8 * 8;
+  const int64_t c = (int64_t)grp * kc + r;
+  uint4 hi = make_uint4(0u, 0u, 0u, 0u), lo = hi;
+  if (r < kc && c < ncols) {
+    const int64_t j = j0 + c, kt = q8 >> 3;
+    const int w = (int)(q8 & 7) >> 1, h = (int)(q8 & 1);
+    const uint32_t word = G[((j / 128 * K_tiles + kt) * 128 + j % 128) * 4 + w];
+    float zv[3], rv[8];
+    if constexpr (!UNIT) {
+      const float g = gm[j];
+#pragma unroll
+      for (int x = 0; x < 3; ++x) zv[x] = __fsub_rn((float)x, g);
+      const float4 r0 = *reinterpret_cast<const float4*>(rr + q8 * 8);
+      const float4 r1 = *reinterpret_cast<const float4*>(rr + q8 * 8 + 4);
+      rv[0] = r0.x, rv[1] = r0.y, rv[2] = r0.z, rv[3] = r0.w;
+      rv[4] = r1.x, rv[5] = r1.y, rv[6] = r1.z, rv[7] = r1.w;
+    }
+    uint32_t ph[4], pl[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {   // element pair q = 4h + p of the word
+      const int q = 4 * h + p, s = f16sub_shift(q);
+      const uint32_t xe = (word >> (2 * q)) & 3u, xo = (word >> (16 + 2 * q)) & 3u;
+      if constexpr (UNIT) {
+        // x·2^−2s in FP16: exponent field 14 + x − 2s (x = 1, 2), or zero
+        const uint32_t be = xe ? (14u + xe - 2u * s) << 10 : 0u, bo = xo ? (14u + xo - 2u * s) << 10 : 0u;
+        ph[p] = be | (bo << 16);
+      } else {
+        const float ks = __uint_as_float((uint32_t)(127 - 2 * s) << 23);
+        const float ve = __fmul_rn(__fmul_rn(__fmul_rn(rv[2 * p], rv[2 * p]), xe == 0 ? zv[0] : xe == 1 ? zv[1] : zv[2]),
+                                   scale);
+        const float vo = __fmul_rn(__fmul_rn(__fmul_rn(rv[2 * p + 1], rv[2 * p + 1]),
+                                             xo == 0 ? zv[0] : xo == 1 ? zv[1] : zv[2]),
+                                   scale);
+        const float he = rintf(ve), ho = rintf(vo);
+        ph[p] = (uint32_t)__half_as_ushort(__float2half_rn(__fmul_rn(he, ks))) |
+                ((uint32_t)__half_as_ushort(__float2half_rn(__fmul_rn(ho, ks))) << 16);
+        pl[p] = (uint32_t)__half_as_ushort(__float2half_rn(__fmul_rn(__fsub_rn(ve, he), ks))) |
+                ((uint32_t)__half_as_ushort(__float2half_rn(__fmul_rn(__fsub_rn(vo, ho), ks))) << 16);
+      }
+    }
+    hi = make_uint4(ph[0], ph[1], ph[2], ph[3]);
+    if constexpr (!UNIT) lo = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+  }
+  *reinterpret_cast<uint4*>(dst) = hi;
+  if constexpr (!UNIT) *reinterpret_cast<uint4*>(dst + (int64_t)kp * K_pad) = lo;
+}
+
+// out[c·ldo + i] = Σ_splits D·isc − gm_row·h_c − p_row·gm_c − t_rowᵀt_c for product row i (SNP r0 + i)
+// and column c (SNP c0 + c); double-float sums.  Rows past the matrix are left alone.
+__global__ void __launch_bounds__(256)
+gram_finish_kernel(const float* __restrict__ D, int splits, int kp, int64_t rows, int64_t nrows, int kc, float isc,
+                   GramStats rs, int64_t r0, GramStats cs, int64_t c0, int cq, float* __restrict__ out, int64_t ldo)
+{
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= nrows) return;
+  const int64_t c = blockIdx.y;
+  const int grp = (int)(c / kc), cc = (int)(c % kc);
+  const float* Dc = D + ((int64_t)grp * splits * kp + cc) * rows + i;
+  DF a;
+  for (int s = 0; s < splits; ++s) df_add(a, __fmul_rn(Dc[(int64_t)s * kp * rows], isc));
+  const float2 h = cs.h[c0 + c], p = rs.p[r0 + i];
+  const float gr = rs.gm[r0 + i], gc = cs.gm[c0 + c];
+  df_fma(a, -gr, h.x);
+  df_fma(a, -p.x, gc);
+  a.lo = __fmaf_rn(-gr, h.y, __fmaf_rn(-p.y, gc, a.lo));
+  for (int l = 0; l < cq; ++l) df_fma(a, -rs.t[(int64_t)l * rs.ld + r0 + i], cs.t[(int64_t)l * cs.ld + c0 + c]);
+  out[c * ldo + i] = __fadd_rn(a.hi, a.lo);
+}
+
+// Split-K count of a product of `ctas` CTAs without splits: the count whose CTAs fill the last wave
+// best, each with at least 48 K-tiles (a CTA's ramp and epilogue cost about eight).
+static int gram_splits(int64_t ctas, int64_t K_tiles, int64_t min_splits)
+{
+  int best = (int)min_splits;
+  double best_eff = -1.0;
+  for (int64_t s = min_splits; s == min_splits || K_tiles / s >= 48; ++s) {
+    const double waves = (double)(ctas * s) / num_sms();
+    const double eff = waves / std::ceil(waves) * (1.0 - 8.0 / (8.0 + (double)K_tiles / s));
+    if (eff > best_eff + 1e-9) {
+      best_eff = eff;
+      best = (int)s;
+    }
+    if (s > 64) break;
+  }
+  return best;
+}
+
+void gram_block(slemm_geno* g, const GramSide& R, int64_t r0, int64_t rows, const GramSide& C, int64_t c0, int64_t ncols,
+                int cq, const float* rr, float rr_max, float* out, int64_t ldo)
+{
+  CHECK_ARG(r0 % kPadRows == 0 && rows % kPadRows == 0 && r0 + rows <= round_up(R.m, kPadRows), "row range not aligned");
+  if (ncols <= 0) return;
+  cudaStream_t st = g->stream;
+  const int64_t K_pad = g->n_pad, K_tiles = K_pad / kTileK;
+  const bool unit = rr == nullptr;
+  // |rr²·z| ≤ 2·max rr²: the bound lies in [2^10, 2^11) after scaling (ops.cu, f16_exp)
+  int e = 0;
+  if (!unit) {
+    int E = 0;
+    std::frexp(2.0 * (double)rr_max * (double)rr_max, &E);
+    e = std::max(-120, std::min(120, 11 - E));
+  }
+  // N ≤ 160 keeps two row tiles, each with its own MMA-issuing thread, in one CTA
+  const int most = unit ? 160 : 80;
+  const int64_t groups = ceil_div(ncols, most);
+  const int kc = (int)ceil_div(ncols, groups);
+  const int kp = (int)round_up(kc, unit ? 16 : 8);
+  const int N = unit ? kp : 2 * kp;
+  // as many groups per launch as 256 MB of operand and 512 MB of a split's partials hold (at least one)
+  const int64_t per = std::max<int64_t>(1, std::min({groups, ((int64_t)256 << 20) / ((int64_t)N * K_pad * 2),
+                                                     ((int64_t)512 << 20) / ((int64_t)kp * rows * 4)}));
+  const int64_t rctas = rows / gemm_tc_rows_per_cta(N, 0);
+  const int64_t nrows = std::min(rows, R.m - r0);
+  const uint8_t* A = R.G + (size_t)(r0 / kTileM) * K_tiles * kTileBytes;
+  for (int64_t g0 = 0; g0 < groups; g0 += per) {
+    const int ng = (int)std::min(per, groups - g0);
+    const int64_t first = g0 * kc, nc = std::min<int64_t>((int64_t)ng * kc, ncols - first);
+    // an integer partial sum of 2^22 elements is at most 2^24: exact in FP32
+    const int splits = gram_splits(rctas * ng, K_tiles, ceil_div(K_pad, (int64_t)1 << 22));
+    __half* B = (__half*)g->ws_B.ensure((size_t)ng * N * K_pad * sizeof(__half));
+    float* D = (float*)g->ws_D.ensure((size_t)ng * splits * kp * rows * sizeof(float));
+    const dim3 og((unsigned)ceil_div(K_pad / 8, 256), kp, ng);
+    const uint32_t* Gc = reinterpret_cast<const uint32_t*>(C.G);
+    if (unit)
+      gram_operand_kernel<true><<<og, 256, 0, st>>>(Gc, K_tiles, c0 + first, nc, kc, kp, nullptr, nullptr, 1.f, B);
+    else
+      gram_operand_kernel<false><<<og, 256, 0, st>>>(Gc, K_tiles, c0 + first, nc, kc, kp, C.stats.gm, rr,
+                                                     (float)std::ldexp(1.0, e), B);
+    LAUNCH_CHECK();
+    GemmArgs a{A, rows, K_pad, B, N, D, splits, g->err.as<int>(), kp, unit ? 1 : 2, true};
+    a.groups = ng;
+    gemm_tc(a, st);
+    gram_finish_kernel<<<dim3((unsigned)ceil_div(nrows, 256), (unsigned)nc), 256, 0, st>>>(
+        D, splits, kp, rows, nrows, kc, (float)std::ldexp(1.0, -e), R.stats, r0, C.stats, c0 + first, cq,
+        out + first * ldo, ldo);
+    LAUNCH_CHECK();
+  }
+}
+
+// ---- batched factorisation ----------------------------------------------------------------------------
+// System b is the s×s matrix M_b = A_b + diag(ridge_b) with t_b further rows Z_b below it, all rows
+// FP32 and contiguous: row r < s at A + b·strideA + r·ld + offA[b], row s + r at
+// Z + (offZ[b] + r)·ld + offA[b].  The right-looking panels of spd_panels turn the rows of A
+// (strictly below each diagonal tile) into L's and the rows of Z into L⁻¹Z's columns,
+// Z_r ← L⁻¹z_r: one TRSM and one update serve both, so the quadratic forms z_rᵀM⁻¹z_r are row norms
+// of the result and a system's work spreads over all its row tiles.  The diagonal tiles' factors go
+// to Ld (a panel's CTAs all read the tile, so it stays as it was); the upper triangle of A keeps the
+// matrix.  One CTA per system factoring alone (a chain of 1,000 columns on one SM) took 20.4 ms for 7
+// systems of 1,000 and its triangular solves another 13.4 ms.
+constexpr int kPT = 128;   // panel width and row-tile height
+
+struct SpdRows {
+  float* A;
+  int64_t strideA;
+  float* Z;
+  const int64_t* offA;
+  const int64_t* offZ;
+  const int* t;
+  int64_t ld;
+  int s;
+  // first element (column 0) of row r ≥ 0 of row tile `tile` counted from row c0 of A, or null past the
+  // end; A's rows and Z's are tiled separately
+  __device__ float* row(int b, int c0, int tile, int r) const
+  {
+    const int nA = (s - c0 + kPT - 1) / kPT;
+    if (tile < nA) {
+      const int i = c0 + tile * kPT + r;
+      return i < s ? A + (int64_t)b * strideA + (int64_t)i * ld + offA[b] : nullptr;
+    }
+    const int i = (tile - nA) * kPT + r;
+    return i < t[b] ? Z + (offZ[b] + i) * ld + offA[b] : nullptr;
+  }
+};
+
+// Panel k0: every CTA factors the diagonal tile (tk ≤ 128 columns) and solves its own 128 rows
+// against it in the same sweep: thread (tx, ty) holds elements (ty + 16a, tx + 16b) of both tiles, and a
+// column is published through shared memory, one barrier per column.  Bound by that chain of 128
+// steps (about 20 µs), not by its arithmetic: so the rows ride along instead of a launch of
+// their own.
+__global__ void __launch_bounds__(256)
+spd_panel_kernel(SpdRows S, const float* __restrict__ ridge, int k0, float* __restrict__ Ld, int* __restrict__ status)
+{
+  __shared__ float scol[2][kPT], srow[2][kPT];
+  const int b = blockIdx.y, tile = blockIdx.x;
+  const int tk = min(kPT, S.s - k0), c0 = k0 + tk;
+  const int nA = (S.s - c0 + kPT - 1) / kPT;
+  const int ntiles = nA + (S.t[b] + kPT - 1) / kPT;
+  if (tile >= ntiles && tile > 0) return;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  // D, R: Σ l·l over the columns done so far; a column's own value is subtracted from once, when its
+  // turn comes (Dv, Rv: the values of the next 16 columns, loaded a block ahead)
+  float D[8][8] = {}, R[8][8] = {}, Dv[8], Rv[8];
+  auto load = [&](int jb) {
+    const int j = tx + 16 * jb;
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+      const int i = ty + 16 * a;
+      const float* rrow = tile < ntiles ? S.row(b, c0, tile, i) : nullptr;
+      float v = 0.f;
+      if (i < tk && j <= i) v = S.A[(int64_t)b * S.strideA + (int64_t)(k0 + i) * S.ld + S.offA[b] + k0 + j];
+      if (i == j) v = i < tk ? v + ridge[(int64_t)b * S.s + k0 + i] : 1.f;
+      Dv[a] = v;
+      Rv[a] = (rrow && j < tk) ? rrow[k0 + j] : 0.f;
+    }
+  };
+  load(0);
+  bool bad = false;
+#pragma unroll
+  for (int jb = 0; jb < 8; ++jb) {
+    float dv[8], rv[8];
+#pragma unroll
+    for (int a = 0; a < 8; ++a) dv[a] = Dv[a], rv[a] = Rv[a];
+    if (jb < 7) load(jb + 1);
+    for (int jj = 0; jj < 16; ++jj) {
+      const int j = 16 * jb + jj, buf = jj & 1;
+      if (tx == jj) {
+#pragma unroll
+        for (int a = 0; a < 8; ++a) {
+          scol[buf][ty + 16 * a] = dv[a] - D[a][jb];
+          srow[buf][ty + 16 * a] = rv[a] - R[a][jb];
+        }
+      }
+      __syncthreads();
+      const float d = scol[buf][j];
+      bad = bad || !(d > 0.f);
+      const float piv = sqrtf(fmaxf(d, 1e-30f)), inv = 1.f / piv;
+      float lk[8];
+#pragma unroll
+      for (int q = jb; q < 8; ++q) lk[q] = scol[buf][tx + 16 * q] * inv;
+      const bool own = tx == jj;
+      const bool right = tx > jj;   // column tx + 16·jb lies right of j
+#pragma unroll
+      for (int a = 0; a < 8; ++a) {
+        const float rl = srow[buf][ty + 16 * a] * inv;
+        if (own) R[a][jb] = rl;
+        else if (right) R[a][jb] = fmaf(rl, lk[jb], R[a][jb]);
+#pragma unroll
+        for (int q = jb + 1; q < 8; ++q) R[a][q] = fmaf(rl, lk[q], R[a][q]);
+      }
+#pragma unroll
+      for (int a = jb; a < 8; ++a) {
+        const float li = scol[buf][ty + 16 * a] * inv;
+        if (own) D[a][jb] = (ty + 16 * a == j) ? piv : li;
+        else if (right) D[a][jb] = fmaf(li, lk[jb], D[a][jb]);
+#pragma unroll
+        for (int q = jb + 1; q < 8; ++q) D[a][q] = fmaf(li, lk[q], D[a][q]);
+      }
+    }
+  }
+  if (tile < ntiles) {
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+      float* rrow = S.row(b, c0, tile, ty + 16 * a);
+      if (!rrow) continue;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (tx + 16 * q < tk) rrow[k0 + tx + 16 * q] = R[a][q];
+    }
+  }
+  if (tile == 0) {
+    if (bad && threadIdx.x == 0) atomicOr(status, 1);
+    float* L = Ld + ((int64_t)b * ((S.s + kPT - 1) / kPT) + k0 / kPT) * kPT * kPT;
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+      for (int q = 0; q < 8; ++q) L[(ty + 16 * a) * kPT + tx + 16 * q] = (tx + 16 * q <= ty + 16 * a) ? D[a][q] : 0.f;
+  }
+}
+
+// Trailing update after panel k0: C[I, J] −= P_I·P_Jᵀ over the panel's tk columns, for A's row tiles
+// (J ≤ I, the lower triangle alone) and Z's (every J).  128×128 per CTA, 8×8 per thread, the panels
+// through shared memory 32 columns at a time (stride 129: no bank conflicts either way).  Bound by FP32
+// FMA issue.
+__global__ void __launch_bounds__(256)
+spd_update_kernel(SpdRows S, int k0)
+{
+  __shared__ float Pa[32][kPT + 1], Pb[32][kPT + 1];
+  const int b = blockIdx.y;
+  const int tk = min(kPT, S.s - k0), c0 = k0 + tk;
+  const int nA = (S.s - c0 + kPT - 1) / kPT;
+  const int nZ = (S.t[b] + kPT - 1) / kPT;
+  const int tri = nA * (nA + 1) / 2;
+  const int q = blockIdx.x;
+  int ti, tj;
+  if (q < tri) {
+    ti = (int)((sqrtf(8.f * (float)q + 1.f) - 1.f) * 0.5f);
+    while ((ti + 1) * (ti + 2) / 2 <= q) ++ti;
+    while (ti * (ti + 1) / 2 > q) --ti;
+    tj = q - ti * (ti + 1) / 2;
+  } else {
+    if (q - tri >= nA * nZ) return;
+    ti = nA + (q - tri) / nA;
+    tj = (q - tri) % nA;
+  }
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  float acc[8][8] = {};
+  for (int u0 = 0; u0 < tk; u0 += 32) {
+    for (int e = threadIdx.x; e < 32 * kPT; e += 256) {
+      const int u = e & 31, r = e >> 5;
+      const bool cu = u0 + u < tk;
+      const float* ra = S.row(b, c0, ti, r);
+      const float* rb = S.row(b, c0, tj, r);
+      Pa[u][r] = (cu && ra) ? ra[k0 + u0 + u] : 0.f;
+      Pb[u][r] = (cu && rb) ? rb[k0 + u0 + u] : 0.f;
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int u = 0; u < 32; ++u) {
+      float x[8], y[8];
+#pragma unroll
+      for (int v = 0; v < 8; ++v) {
+        x[v] = Pa[u][ty + 16 * v];
+        y[v] = Pb[u][tx + 16 * v];
+      }
+#pragma unroll
+      for (int v = 0; v < 8; ++v)
+#pragma unroll
+        for (int w = 0; w < 8; ++w) acc[v][w] = fmaf(x[v], y[w], acc[v][w]);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
+    float* row = S.row(b, c0, ti, ty + 16 * v);
+    if (!row) continue;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      const int j = tj * kPT + tx + 16 * w;   // column c0 + j
+      if (c0 + j < S.s && (ti >= nA || j <= ti * kPT + ty + 16 * v)) row[c0 + j] -= acc[v][w];
+    }
+  }
+}
+
+// q[offZ[b] + r] = Σ_j Z_r[j]² (FP64 sum of the FP32 values), one warp per row of Z; grid (rows, systems)
+__global__ void __launch_bounds__(256)
+spd_norms_kernel(SpdRows S, double* __restrict__ q)
+{
+  const int b = blockIdx.y, r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= S.t[b]) return;
+  const float* z = S.Z + (S.offZ[b] + r) * S.ld + S.offA[b];
+  DF a;
+  for (int j = lane; j < S.s; j += 32) df_fma(a, z[j], z[j]);
+  double v = df_value(a);
+  for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (lane == 0) q[S.offZ[b] + r] = v;
+}
+
+// x ← L⁻ᵀy for the first row y of each system's Z (x[b·s …]): panels from the last, one CTA each.
+constexpr int kBackThreads = 512;
+__global__ void __launch_bounds__(kBackThreads)
+spd_back_kernel(SpdRows S, const float* __restrict__ Ld, float* __restrict__ x)
+{
+  extern __shared__ float sm[];
+  float* xs = sm;                     // s
+  float* L = sm + ((S.s + 31) & ~31);  // 128×129
+  float* red = L + kPT * (kPT + 1);   // 4×128
+  const int b = blockIdx.x, tid = threadIdx.x, s = S.s;
+  const int np = (s + kPT - 1) / kPT;
+  const float* y = S.Z + S.offZ[b] * S.ld + S.offA[b];
+  for (int j = tid; j < s; j += kBackThreads) xs[j] = y[j];
+  __syncthreads();
+  for (int p = np - 1; p >= 0; --p) {
+    const int k0 = p * kPT, tk = min(kPT, s - k0), c0 = k0 + tk;
+    const float* Lp = Ld + ((int64_t)b * np + p) * kPT * kPT;
+    for (int e = tid; e < kPT * kPT; e += kBackThreads) L[(e / kPT) * (kPT + 1) + e % kPT] = Lp[e];
+    const int j = tid & (kPT - 1), grp = tid / kPT;
+    float a = 0.f;
+    if (j < tk) {
+      const float* col = S.A + (int64_t)b * S.strideA + S.offA[b] + k0 + j;
+#pragma unroll 8
+      for (int i = c0 + grp; i < s; i += kBackThreads / kPT) a = fmaf(col[(int64_t)i * S.ld], xs[i], a);
+    }
+    red[grp * kPT + j] = a;
+    __syncthreads();
+    if (tid < 32) {   // L_kkᵀ x_k = rhs: lane holds elements lane + 32q
+      float v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int i = tid + 32 * q;
+        v[q] = i < tk ? xs[k0 + i] - (red[i] + red[kPT + i] + red[2 * kPT + i] + red[3 * kPT + i]) : 0.f;
+      }
+#pragma unroll
+      for (int q = 3; q >= 0; --q)
+        for (int l = 31; l >= 0; --l) {
+          const int jj = 32 * q + l;
+          if (jj >= tk) continue;
+          const float xj = __shfl_sync(0xffffffffu, v[q], l) / L[jj * (kPT + 1) + jj];
+          if (tid == l) v[q] = xj;
+#pragma unroll
+          for (int w = 0; w <= q; ++w) {
+            const int i = tid + 32 * w;
+            if (i < jj) v[w] = fmaf(-L[jj * (kPT + 1) + i], xj, v[w]);
+          }
+        }
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (tid + 32 * q < tk) xs[k0 + tid + 32 * q] = v[q];
+    }
+    __syncthreads();
+  }
+  for (int j = tid; j < s; j += kBackThreads) x[(int64_t)b * s + j] = xs[j];
+}
+
+// part[b·nblk + blk] = Σ_{i in block} x_i·(2z_i − (M x)_i) with M = A + diag(ridge): A's upper triangle
+// (kept by the factorisation) and its diagonal diag0, double-float products, FP64 per row.
+__global__ void __launch_bounds__(256)
+spd_quad_kernel(SpdRows S, const float* __restrict__ ridge, const float* __restrict__ diag0,
+                const float* __restrict__ z, const float* __restrict__ x, double* __restrict__ part)
+{
+  __shared__ double sh[32];
+  const int b = blockIdx.y, s = S.s, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float* xb = x + (int64_t)b * s;
+  double tot = 0.0;
+  for (int i = blockIdx.x * 64 + warp; i < min(s, (int)(blockIdx.x + 1) * 64); i += 8) {
+    const float* row = S.A + (int64_t)b * S.strideA + (int64_t)i * S.ld + S.offA[b];
+    DF a;
+    for (int j = i + 1 + lane; j < s; j += 32) df_fma(a, row[j], xb[j]);
+    double v = 2.0 * df_value(a);
+    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) {
+      const double xi = (double)xb[i];
+      v += ((double)diag0[(int64_t)b * s + i] + (double)ridge[(int64_t)b * s + i]) * xi;
+      tot += xi * (2.0 * (double)z[(int64_t)b * s + i] - v);
+    }
+  }
+  const double r = block_sum_d(tot, sh);
+  if (threadIdx.x == 0) part[(int64_t)b * gridDim.x + blockIdx.x] = r;
+}
+
+// diag0 = A's diagonal, z = A's row `which` (its own entries left of the diagonal by symmetry are the
+// same memory: the block is full), zrow = Z's first row ← z
+__global__ void __launch_bounds__(256)
+spd_take_kernel(SpdRows S, const int64_t* __restrict__ which, float* __restrict__ diag0, float* __restrict__ z)
+{
+  const int b = blockIdx.y, j = blockIdx.x * 256 + threadIdx.x;
+  if (j >= S.s) return;
+  const float* A = S.A + (int64_t)b * S.strideA + S.offA[b];
+  const float v = A[which[b] * S.ld + j];
+  diag0[(int64_t)b * S.s + j] = A[(int64_t)j * S.ld + j];
+  z[(int64_t)b * S.s + j] = v;
+  S.Z[S.offZ[b] * S.ld + S.offA[b] + j] = v;
+}
+
+static SpdRows rows_of(const SpdBatch& B)
+{
+  return SpdRows{B.A, B.strideA, B.Z, B.offA, B.offZ, B.t, B.ld, B.s};
+}
+
+// Factors the systems and solves their Z rows (see above); status gets 1 on a pivot that is not positive.
+static void spd_panels(const SpdBatch& B, const float* ridge, float* Ld, int* status, cudaStream_t st)
+{
+  const SpdRows S = rows_of(B);
+  const int nZ = (B.t_max + kPT - 1) / kPT;
+  for (int k0 = 0; k0 < B.s; k0 += kPT) {
+    const int c0 = std::min(k0 + kPT, B.s);
+    const int nA = (B.s - c0 + kPT - 1) / kPT;
+    spd_panel_kernel<<<dim3(std::max(1, nA + nZ), B.nb), 256, 0, st>>>(S, ridge, k0, Ld, status);
+    LAUNCH_CHECK();
+    const int tiles = nA * (nA + 1) / 2 + nA * nZ;
+    if (tiles == 0) continue;
+    spd_update_kernel<<<dim3(tiles, B.nb), 256, 0, st>>>(S, k0);
+    LAUNCH_CHECK();
+  }
+}
+
+static size_t ld_bytes(const SpdBatch& B) { return (size_t)B.nb * ceil_div(B.s, kPT) * kPT * kPT * sizeof(float); }
+
+void spd_row_norms(const SpdBatch& B, const float* ridge, double* q, int* status, cudaStream_t st)
+{
+  DevBuf d(st);
+  float* Ld = (float*)d.ensure(ld_bytes(B));
+  spd_panels(B, ridge, Ld, status, st);
+  if (B.t_max > 0) {
+    spd_norms_kernel<<<dim3((unsigned)ceil_div(B.t_max, 8), B.nb), 256, 0, st>>>(rows_of(B), q);
+    LAUNCH_CHECK();
+  }
+}
+
+int spd_quadform_blocks(int s) { return (int)ceil_div(s, 64); }
+
+void spd_quadforms(const SpdBatch& B, const float* ridge, const int64_t* which, double* part, int* status, cudaStream_t st)
+{
+  DevBuf d(st), dv(st);
+  float* Ld = (float*)d.ensure(ld_bytes(B));
+  float* diag0 = (float*)dv.ensure((size_t)3 * B.nb * B.s * sizeof(float));
+  float* z = diag0 + (size_t)B.nb * B.s;
+  float* x = z + (size_t)B.nb * B.s;
+  const SpdRows S = rows_of(B);
+  spd_take_kernel<<<dim3((unsigned)ceil_div(B.s, 256), B.nb), 256, 0, st>>>(S, which, diag0, z);
+  LAUNCH_CHECK();
+  spd_panels(B, ridge, Ld, status, st);
+  const size_t smem = (size_t)(((B.s + 31) & ~31) + kPT * (kPT + 1) + 4 * kPT) * sizeof(float);
+  CUDA_TRY(cudaFuncSetAttribute(spd_back_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  spd_back_kernel<<<B.nb, kBackThreads, smem, st>>>(S, Ld, x);
+  LAUNCH_CHECK();
+  spd_quad_kernel<<<dim3(spd_quadform_blocks(B.s), B.nb), 256, 0, st>>>(S, ridge, diag0, z, x, part);
+  LAUNCH_CHECK();
+}
+
+}  // namespace slemm

@@ -1,0 +1,74 @@
+// gram.h — projected Gram blocks of SNP rows and their batched systems (gram.cu).
+#pragma once
+
+#include "internal.h"
+
+namespace slemm {
+
+// Per-SNP statistics (device) with z = x − gm: h = Σ rr²·z and, when every rr is 1, p = Σ x (else 0), as
+// hi+lo FP32 pairs; t = Qᵀ(rr∘z) (cq × ld), xy = zᵀy (0 without y) and xx = ‖(I − QQᵀ)(rr∘z)‖².
+struct GramStats {
+  float* gm;
+  float2* h;
+  float2* p;
+  float* t;
+  double* xy;
+  double* xx;
+  int64_t ld;
+};
+struct GramStatsBuf {
+  DevBuf buf;
+  GramStats s{};
+  GramStats make(int64_t m, int cq, cudaStream_t st)
+  {
+    buf.stream = st;
+    buf.ordered = true;
+    s.ld = m;
+    s.xy = (double*)buf.ensure((size_t)m * (2 * sizeof(double) + 2 * sizeof(float2) + ((size_t)cq + 1) * sizeof(float)));
+    s.xx = s.xy + m;
+    s.h = reinterpret_cast<float2*>(s.xx + m);
+    s.p = s.h + m;
+    s.gm = reinterpret_cast<float*>(s.p + m);
+    s.t = s.gm + m;
+    return s;
+  }
+};
+
+// Statistics of every SNP of a handle at the centring values gm (m): y (n, may be nullptr), rr (n_pad,
+// nullptr: all 1), Q (n_pad × cq), all on the device.
+void gram_stats(slemm_geno* g, const float* gm, const float* y, const float* rr, const float* Q, int cq,
+                GramStatsBuf& out);
+void gram_stats_gather(const GramStats& src, const int64_t* d_idx, int64_t cnt, int cq, GramStatsBuf& out, cudaStream_t st);
+
+// A packed SNP-major copy of m rows (all with the same individuals) and its rows' statistics.
+struct GramSide {
+  const uint8_t* G;
+  int64_t m;
+  GramStats stats;
+};
+// out[c·ldo + i] = (P(rr∘z_{r0+i}))ᵀ(P(rr∘z_{c0+c})) for product rows r0 … r0 + rows − 1 of R (multiples
+// of 256; rows past R.m are not written) and columns c0 … c0 + ncols − 1 of C.  g gives the stream,
+// the work buffers and the individuals; rr (n_pad) == nullptr: all 1, else rr_max ≥ max|rr|.
+void gram_block(slemm_geno* g, const GramSide& R, int64_t r0, int64_t rows, const GramSide& C, int64_t c0, int64_t ncols,
+                int cq, const float* rr, float rr_max, float* out, int64_t ldo);
+
+// A batch of nb systems of s unknowns (layout in gram.cu); offA, offZ and t are device arrays.
+struct SpdBatch {
+  float* A;
+  int64_t strideA;
+  float* Z;
+  const int64_t* offA;
+  const int64_t* offZ;
+  const int* t;
+  int64_t ld;
+  int s, nb, t_max;
+};
+// q[offZ[b] + r] = z_rᵀ(A_b + diag(ridge_b))⁻¹z_r for every row z_r of Z_b; A and Z are overwritten.
+void spd_row_norms(const SpdBatch& B, const float* ridge, double* q, int* status, cudaStream_t st);
+// part[b·blocks …] sums to zᵀ(A_b + diag(ridge_b))⁻¹z with z the row which[b] of A_b (t = 1, Z has room for
+// one row per system).  With x an FP32 solution of M x = z, 2zᵀx − xᵀMx differs from zᵀM⁻¹z by
+// rᵀM⁻¹r only, r = z − Mx: accurate to the square of the solution's own error.
+int spd_quadform_blocks(int s);
+void spd_quadforms(const SpdBatch& B, const float* ridge, const int64_t* which, double* part, int* status, cudaStream_t st);
+
+}  // namespace slemm

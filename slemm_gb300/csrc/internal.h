@@ -16,6 +16,7 @@ struct slemm_geno {
   int c = 0;
   bool weights_set = false;
   bool rr_one = false;            // every rr of set_weights is 1
+  float rr_max = 0.f;             // its largest |rr|
   int prec = SLEMM_PREC_FP16X2;
   int per_vector = 0;
   int lanczos_mode = 0;           // SLEMM_LANCZOS_* bits of the seeds run on this handle
@@ -94,6 +95,24 @@ void op_device_mixed(slemm_geno* g, int kind, float tau0, const float* in, int64
 // prec (SLEMM_PREC_FP16X2, BF16X2 or BF16X3; ops.cu).
 void rows_product(slemm_geno* g, int64_t r0, int64_t rows, const float* U, int64_t ldu, int k, float* out,
                   int64_t ldo, int prec);
+
+// exact.cu — exact products of the packed counts with dense columns.
+// d_tgv[i] = shift + Σ_j count_ij·d_alpha[j] (FP64 effects, largest magnitude amax).
+void exact_gebv(slemm_geno* g, const double* d_alpha, double amax, double shift, double* d_tgv);
+// The columns of exact_dots over individuals i < n, FP32 values in this order: y (when given), rr·Q_l
+// for l < cq, rr² (when rr is given; rr == nullptr means every rr is 1).
+struct ExactCols {
+  const float* y;
+  const float* rr;
+  const float* Q;
+  int64_t ldq;
+  int cq;
+  int count() const { return (y ? 1 : 0) + cq + (rr ? 1 : 0); }
+};
+// dots[c·m + j] = Σ_i count_ij·column_c(i) for every SNP j, tot[c] = Σ_i column_c(i) (NaN for a column
+// with a non-finite value, and so its dots), and with rr given and twos != nullptr
+// twos[j] = 2·Σ_i rr_i²·[count_ij = 2].  Device pointers; at least one column.
+void exact_dots(slemm_geno* g, const ExactCols& a, double* dots, double* tot, double* twos);
 
 // reml.cu — orthonormal basis (FP64 column-pivoted QR) of an n×c matrix; returns the rank.
 int orthonormal_columns(const std::vector<double>& A, int64_t n, int c, std::vector<double>& Q);

@@ -12,16 +12,15 @@
 // xSx = ‖v‖²; xBx = (xSx − zᵀ(ZᵀZ + τ1·diag(1/gw))⁻¹z)/τ1 where Z holds the projected, rr-scaled
 // centred counts of the window_size markers around x (clamped at both ends) and z = Zᵀv.
 //
-// GB300 mapping: ZᵀZ and z come out of one packed tensor-core product per window,
-// Z_wdᵀ[U | rr∘v] with U = rr∘(I − QQᵀ)(rr∘Cc) — the centred counts Cc are read from the packed
-// copy, never materialised as a dense Z — using column-scaled FP16 hi+lo (≈ FP32 accuracy, like the
-// reference's SGEMM).  The windows' systems are then factored together, one CTA per window:
-// blocked FP32 Cholesky in global memory (L2-resident), then two steps of iterative refinement
-// with FP64 residuals, so the quadratic form is limited by the Gram's own accuracy, not by the
-// FP32 factorisation.
+// GB300 mapping: z is the row of x in its own window's ZᵀZ (x lies in the window), so each window is
+// one projected Gram block read straight from the packed rows (gram.cu).  The windows' systems are
+// factored together over all SMs by blocked FP32 panels; the quadratic form is taken as
+// 2zᵀx − xᵀMx of the FP32 solution against the kept matrix, which squares the solution's own
+// error away, so it is limited by the Gram's accuracy, not by the FP32 factorisation.
 #include "internal.h"
 #include "reduce.cuh"
 #include "dense.cuh"
+#include "gram.h"
 
 #include <algorithm>
 #include <memory>
@@ -74,85 +73,6 @@ static std::vector<int64_t> lmm_variants(const std::vector<float>& gm, int64_t n
   return std::vector<int64_t>(v.begin(), v.begin() + k);
 }
 
-// y ← L⁻¹y then y ← L⁻ᵀy (FP64 vector in shared memory, FP32 factor), one CTA.
-__device__ void chol_apply(const float* __restrict__ L, int s, int64_t lda, double* y)
-{
-  // forward: the thread that owns no row waits; columns processed in order
-  for (int j = 0; j < s; ++j) {
-    if (threadIdx.x == 0) y[j] /= (double)L[(int64_t)j * lda + j];
-    __syncthreads();
-    const double yj = y[j];
-    for (int i = j + 1 + threadIdx.x; i < s; i += blockDim.x) y[i] -= (double)L[(int64_t)j * lda + i] * yj;
-    __syncthreads();
-  }
-  // backward: y_j = (y_j − Σ_{i>j} L_ij y_i)/L_jj, dot products by block reduction
-  __shared__ double red[32];
-  for (int j = s - 1; j >= 0; --j) {
-    double part = 0.0;
-    for (int i = j + 1 + threadIdx.x; i < s; i += blockDim.x) part += (double)L[(int64_t)j * lda + i] * y[i];
-    const double tot = block_sum_d(part, red);
-    if (threadIdx.x == 0) y[j] = (y[j] - tot) / (double)L[(int64_t)j * lda + j];
-    __syncthreads();
-  }
-}
-
-// One CTA per system b: A_b = A + b·strideA + off[b] (s×s, ld lda, lower triangle used) plus
-// diag(d_b) is copied to F_b, factored, and q_b = z_bᵀx (z_b = column s of A_b) with x refined
-// twice against FP64 residuals of the original system.
-__global__ void __launch_bounds__(kCholThreads)
-spd_quadform_kernel(const float* __restrict__ A, int64_t lda, int64_t strideA, const int64_t* __restrict__ off,
-                    const float* __restrict__ d, int s, float* __restrict__ F, double* __restrict__ q,
-                    int* __restrict__ status)
-{
-  extern __shared__ double sm[];   // x (s), r (s)
-  __shared__ float S[kCholB][kCholB + 1];
-  __shared__ int bad;
-  __shared__ double red[32];
-  const int b = blockIdx.x;
-  const float* Ab = A + (int64_t)b * strideA + off[b];
-  const float* db = d + (int64_t)b * s;
-  const float* zb = Ab + (int64_t)s * lda;
-  float* Fb = F + (int64_t)b * s * s;
-  double* x = sm;
-  double* r = sm + s;
-  if (threadIdx.x == 0) bad = 0;
-  for (int64_t q2 = threadIdx.x; q2 < (int64_t)s * s; q2 += blockDim.x) {
-    const int i = (int)(q2 % s), j = (int)(q2 / s);
-    if (i >= j) Fb[(int64_t)j * s + i] = Ab[(int64_t)j * lda + i] + (i == j ? db[i] : 0.f);
-  }
-  __syncthreads();
-  const bool ok = chol_blocked(Fb, s, s, S, &bad);
-  if (!ok) {
-    if (threadIdx.x == 0) {
-      q[b] = 0.0;
-      atomicOr(status, 1);
-    }
-    return;
-  }
-  for (int i = threadIdx.x; i < s; i += blockDim.x) x[i] = (double)zb[i];
-  __syncthreads();
-  chol_apply(Fb, s, s, x);
-  for (int it = 0; it < 2; ++it) {
-    // r = z − (A + D)x in FP64, symmetric A from its lower triangle
-    for (int i = threadIdx.x; i < s; i += blockDim.x) {
-      double acc = (double)zb[i] - (double)db[i] * x[i];
-      for (int j = 0; j < s; ++j) {
-        const float a = (i >= j) ? Ab[(int64_t)j * lda + i] : Ab[(int64_t)i * lda + j];
-        acc -= (double)a * x[j];
-      }
-      r[i] = acc;
-    }
-    __syncthreads();
-    chol_apply(Fb, s, s, r);
-    for (int i = threadIdx.x; i < s; i += blockDim.x) x[i] += r[i];
-    __syncthreads();
-  }
-  double part = 0.0;
-  for (int i = threadIdx.x; i < s; i += blockDim.x) part += (double)zb[i] * x[i];
-  const double tot = block_sum_d(part, red);
-  if (threadIdx.x == 0) q[b] = tot;
-}
-
 }  // namespace slemm
 
 using namespace slemm;
@@ -192,7 +112,7 @@ extern "C" int slemm_gpu_lmm_quadforms(slemm_geno* g, const float* Py, float tau
     float* py = (float*)d_py.ensure(n * sizeof(float));
     double* sc = (double*)d_sc.ensure((size_t)4 * k * sizeof(double));
     DevBuf d_qt(st);
-    double* qtv = (double*)d_qt.ensure((size_t)g->c * std::max(k, window_size + 1) * sizeof(double));
+    double* qtv = (double*)d_qt.ensure((size_t)g->c * k * sizeof(double));
     CUDA_TRY(cudaMemcpyAsync(py, Py, n * sizeof(float), cudaMemcpyHostToDevice, st));
     centred_rows_kernel<<<dim3((unsigned)ceil_div(n, 256), k), 256, 0, st>>>(
         g->G.as<uint32_t>(), K_tiles, d_rows.as<int64_t>(), 0, g->gm.as<float>(), nullptr, n, V, n);
@@ -208,13 +128,18 @@ extern "C" int slemm_gpu_lmm_quadforms(slemm_geno* g, const float* Py, float tau
     lanczos_solve_device(S, 0.0, 1e-6, X, n, 0);
     col_dots(g, V, n, X, n, n, k, sc + k);
     col_dots(g, V, n, nullptr, 0, n, k, sc + 2 * k);
-    // windows: [ZᵀZ | Zᵀv] from the packed copy, one product per marker
+    // windows: the projected Gram of each marker's window, its own row of it kept as z
     const int ws = window_size;
-    DevBuf d_U(st), d_gram(st), d_F(st), d_d(st), d_q(st), d_status(st);
-    float* U = (float*)d_U.ensure((size_t)n * (ws + 1) * sizeof(float));
+    DevBuf d_gram(st), d_d(st), d_q(st), d_status(st), d_idx(st);
     const int64_t rows_max = round_up(ws, kPadRows) + kPadRows;
-    float* gram = (float*)d_gram.ensure((size_t)k * rows_max * (ws + 1) * sizeof(float));
-    std::vector<int64_t> wstart(k);
+    const int64_t stride = rows_max * (ws + 1);   // ws rows and the room for z
+    float* gram = (float*)d_gram.ensure((size_t)k * stride * sizeof(float));
+    const float* rr = g->rr_one ? nullptr : g->rr.as<float>();
+    GramStatsBuf stats;
+    gram_stats(g, g->gm.as<float>(), nullptr, rr, g->Q.as<float>(), g->c, stats);
+    const GramSide side{g->G.as<uint8_t>(), m, stats.s};
+    std::vector<int64_t> idx((size_t)3 * k);   // offA | offZ | which
+    std::vector<int> one(k, 1);
     std::vector<float> dd((size_t)k * ws);
     for (int c = 0; c < k; ++c) {
       const int64_t j = var[c];
@@ -222,51 +147,41 @@ extern "C" int slemm_gpu_lmm_quadforms(slemm_geno* g, const float* Py, float tau
       if (j < ws / 2) wds = 0;
       else if (j > m - ws / 2) wds = m - ws;
       else wds = j - ws / 2;
-      wstart[c] = wds;
       for (int t = 0; t < ws; ++t) dd[(size_t)c * ws + t] = tau1 / gw[wds + t];
-      // U = rr∘P(rr∘Cc) for the window's markers, then column ws = rr∘v
-      centred_rows_kernel<<<dim3((unsigned)ceil_div(n, 256), ws), 256, 0, st>>>(
-          g->G.as<uint32_t>(), K_tiles, nullptr, wds, g->gm.as<float>(), g->rr.as<float>(), n, U, n);
-      LAUNCH_CHECK();
-      proj_coeffs(g, U, n, ws, qtv);
-      proj_apply(g, U, n, ws, qtv);
-      CUDA_TRY(cudaMemcpyAsync(U + (size_t)ws * n, V + (size_t)c * n, n * sizeof(float), cudaMemcpyDeviceToDevice, st));
-      scale_rows_rr_kernel<<<dim3((unsigned)ceil_div(n, 256), ws + 1), 256, 0, st>>>(U, n, g->rr.as<float>(), n);
-      LAUNCH_CHECK();
       const int64_t r0 = wds / kPadRows * kPadRows;
       const int64_t r1 = std::min<int64_t>(round_up(wds + ws, kPadRows), g->m_pad);
-      rows_product(g, r0, r1 - r0, U, n, ws + 1, gram + (size_t)c * rows_max * (ws + 1), rows_max, SLEMM_PREC_FP16X2);
-      // this window's Gram starts at row wds − r0 of its block
-      wstart[c] = wds - r0;
+      gram_block(g, side, r0, r1 - r0, side, wds, ws, g->c, rr, g->rr_max, gram + (size_t)c * stride, rows_max);
+      idx[c] = wds - r0;   // this window's Gram starts at row wds − r0 of its block
+      idx[k + c] = (int64_t)c * (ws + 1);
+      idx[2 * k + c] = j - wds;
     }
     check_device_error(g);
-    // batched solves: q_c = zᵀ(ZᵀZ + D)⁻¹z
-    float* F = (float*)d_F.ensure((size_t)k * ws * ws * sizeof(float));
+    // batched systems: q_c = zᵀ(ZᵀZ + D)⁻¹z
     float* dvec = (float*)d_d.ensure((size_t)k * ws * sizeof(float));
-    double* q = (double*)d_q.ensure(k * sizeof(double));
-    int* status = (int*)d_status.ensure(sizeof(int));
+    const int nq = spd_quadform_blocks(ws);
+    double* q = (double*)d_q.ensure((size_t)k * nq * sizeof(double));
+    int* status = (int*)d_status.ensure(((size_t)k + 1) * sizeof(int));
+    int64_t* didx = (int64_t*)d_idx.ensure(idx.size() * sizeof(int64_t));
     CUDA_TRY(cudaMemcpyAsync(dvec, dd.data(), dd.size() * sizeof(float), cudaMemcpyHostToDevice, st));
+    CUDA_TRY(cudaMemcpyAsync(didx, idx.data(), idx.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), st));
-    const size_t smem = (size_t)2 * ws * sizeof(double);
-    CUDA_TRY(cudaFuncSetAttribute(spd_quadform_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    DevBuf d_off(st);
-    CUDA_TRY(cudaMemcpyAsync(d_off.ensure(k * sizeof(int64_t)), wstart.data(), k * sizeof(int64_t),
-                             cudaMemcpyHostToDevice, st));
-    spd_quadform_kernel<<<k, kCholThreads, smem, st>>>(gram, rows_max, rows_max * (ws + 1), d_off.as<int64_t>(), dvec,
-                                                       ws, F, q, status);
-    LAUNCH_CHECK();
-    std::vector<double> h(3 * k), hq(k);
+    CUDA_TRY(cudaMemcpyAsync(status + 1, one.data(), (size_t)k * sizeof(int), cudaMemcpyHostToDevice, st));
+    spd_quadforms({gram, stride, gram + (size_t)ws * rows_max, didx, didx + k, status + 1, rows_max, ws, k, 1}, dvec,
+                  didx + 2 * k, q, status, st);
+    std::vector<double> h(3 * k), hq((size_t)k * nq);
     int hs = 0;
     CUDA_TRY(cudaMemcpyAsync(h.data(), sc, 3 * k * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaMemcpyAsync(hq.data(), q, k * sizeof(double), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(cudaMemcpyAsync(hq.data(), q, hq.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaMemcpyAsync(&hs, status, sizeof(int), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaStreamSynchronize(st));
     if (hs) SLEMM_THROW(SLEMM_ERR_NUMERIC, "a window's ZᵀZ + τ1·diag(1/gw) is not positive definite in FP32");
     for (int c = 0; c < k; ++c) {
+      double qc = 0.0;
+      for (int b = 0; b < nq; ++b) qc += hq[(size_t)c * nq + b];
       xPy[c] = (float)h[c];
       xPx[c] = (float)h[k + c];
       xSx[c] = (float)h[2 * k + c];
-      xBx[c] = (float)((h[2 * k + c] - hq[c]) / (double)tau1);
+      xBx[c] = (float)((h[2 * k + c] - qc) / (double)tau1);
     }
   });
 }

@@ -1,0 +1,55 @@
+"""The projected Gram blocks and their batched systems (--lmm windows, slemm_gwa blocks) against the
+oracle, at the edges of the 128-column panels, of the 160- and 80-column operand groups and of the
+256-row product tiles, with and without residual weights."""
+import numpy as np
+import pytest
+
+from oracle import slemm_np as orc
+from slemm_gb300 import api, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _data(n, m, c, weighted, seed):
+    counts, _ = synth.simulate_counts(n, m, seed=seed)
+    rng = np.random.default_rng(seed)
+    rvec = rng.uniform(0.3, 3.0, n).astype(np.float32) if weighted else np.ones(n, np.float32)
+    X = np.column_stack([np.ones(n)] + [rng.standard_normal(n) for _ in range(c - 1)]).astype(np.float32)
+    return counts, synth.encode_bed(counts), rng.standard_normal(n).astype(np.float32), rvec, X
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("ws,n,c", [(2, 300, 1), (126, 700, 2), (128, 700, 0), (130, 1025, 3), (256, 700, 20),
+                                    (322, 700, 2)])
+def test_lmm_windows_at_panel_edges(gpu, weighted, ws, n, c):
+    m = 600
+    counts, rows, Py, rvec, X = _data(n, m, max(c, 1), weighted, seed=ws + n)
+    gm = orc.genotype_mean(orc.popcounts(counts), n)
+    gw = orc.snp_weights(gm, np.ones(m, np.float32))
+    rr = (1 / np.sqrt(rvec)).astype(np.float32)
+    Q = orc.qr_colpiv(rr[:, None] * X)[0][:, :c]
+    ref = orc.LMM_quadforms(counts, Py, rr, Q, gm, gw, 1.7, num_qf=9, window_size=ws)
+    with api.Genotypes(rows, n) as g:
+        g.set_weights(gm, gw, rr)
+        g.set_projection(Q.astype(np.float32))
+        r = g.LMM_quadforms(Py, 1.7, num_qf=9, window_size=ws)
+    assert r["variants"] == ref["variants"]
+    # FP32 Gram entries (2^-22 of the diagonal) in systems whose condition number is a few: the ridge
+    # is at least the diagonal's size here
+    assert np.allclose(r["xBx"], ref["xBx"], rtol=2e-5, atol=0)
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("block,n,c", [(4, 300, 1), (128, 1025, 2), (130, 700, 17), (322, 700, 2)])
+def test_gwa_blocks_at_panel_edges(gpu, weighted, block, n, c):
+    m, n_model = 1200, 500
+    counts, rows, y, R, X = _data(n, m, c, weighted, seed=block + n)
+    model = np.sort(np.random.default_rng(block).permutation(m)[:n_model])
+    ref = orc.gwa_windows(2 - counts, y, R, X, model, 0, m - 1, block, 1.5, n_model, 0.9, 0.4, 20)
+    with api.Genotypes(rows, n) as g:
+        got = g.gwa_windows(y, R, X, model, 0, m - 1, block, 1.5, n_model, 0.9, 0.4, 20)
+    ok = np.isfinite(ref[3])
+    assert np.array_equal(ok, np.isfinite(got[3]))
+    # the oracle is the script's float32: a few hundred FP32 products and sums per entry on both sides
+    for a, b in zip(got[:3], ref[:3]):
+        assert np.allclose(a[ok], b[ok], rtol=1e-3, atol=1e-5 * np.abs(b[ok]).max())
