@@ -51,7 +51,8 @@ extern "C" {
 #define SLEMM_PREC_BF16X2  1  /* tcgen05 BF16 MMA, dense side split hi+lo, FP32 accumulation     */
 #define SLEMM_PREC_BF16X3  2  /* tcgen05 BF16 MMA, dense side split hi+mid+lo (≈FP32 mantissa)   */
 #define SLEMM_PREC_FP16X2  3  /* tcgen05 FP16 MMA, dense side scaled by a power of two per column
-                                 and split hi+lo (22 mantissa bits) at the cost of hi+lo BF16     */
+                                 and split hi+lo (22 mantissa bits) at the cost of hi+lo BF16; at
+                                 most 32 columns: E4M3 MMA on five base-32 digits (24 bits)       */
 
 /* Largest number of fixed-effect covariates (columns of X, and so of the projection Q) a fit takes,
  * including the SNPs that --iter_weighting appends as fixed effects. */
@@ -350,7 +351,7 @@ int slemm_gpu_rmatvec_noalloc(slemm_geno* g, const float* v, int64_t ldv, int k,
  * fixed-rule count. */
 int slemm_gpu_set_autotune(slemm_geno* g, int on);
 /* The cached decisions: *rows = their number; for r < max_rows, info[7r …] = {device, N, pieces,
- * rule's splits, chosen splits, chosen plan (0: the default ring, 1: two CTAs per SM), candidates
+ * rule's splits, chosen splits, chosen plan (0: the default ring, 1: two CTAs per SM, 2: E4M3 digits), candidates
  * timed}, shape[2r …] = {K-tiles, padded rows},
  * ms[2r …] = {rule's ms per launch, chosen ms per launch}.  Any of info, shape, ms may be NULL. */
 int slemm_gpu_autotune_table(int max_rows, int* rows, int32_t* info, int64_t* shape, double* ms);

@@ -178,7 +178,8 @@ cudaMemPool_t own_pool(int device, Pool which);
 // D[M_pad × N] = Cnt[M_pad × K_pad] · B where the count matrix is a tiled 2-bit packed array
 // (tiles of kTileM rows × kTileK K-elements, 2048 contiguous bytes each, see geno.cu) and B is
 // either FP32 [k][K_pad] (SIMT) or 16-bit pieces [N][K_pad] (tensor cores: piece p of column c
-// in row p·kp + c, kp = k rounded up to 8, BF16 or FP16).  The raw product goes to partials
+// in row p·kp + c, kp = k rounded up to 8, BF16 or FP16; or 8-bit digits in the same layout, whose
+// K positions follow the decoded order of decode.cuh).  The raw product goes to partials
 // [splits][kp][M_pad] (FP32; the tensor-core epilogue adds a column's pieces before the store),
 // reduced by the finalize kernels of ops.cu.
 struct GemmArgs {
@@ -192,10 +193,11 @@ struct GemmArgs {
   int* err;             // device error word (bounded waits that gave up set bits here)
   int kp = 0;           // columns of D per split (TC: k rounded up to 8; SIMT: N)
   int pieces = 1;       // pieces per column (TC)
-  bool f16 = false;     // TC operand type: FP16 (true) or BF16
+  bool f16 = false;     // TC operand type: FP16 (true) or BF16, unless plan 2
   int plan = 0;         // TC ring plan: 0 by N (N ≤ 64: two tiles per CTA, one CTA per SM), 1: N ≤ 64,
-                        // one tile per CTA and two CTAs per SM (256 TMEM columns each)
-  bool twos = false;    // TC, FP16, N ≤ 64, plan 0: the matrix is 2·[count = 2] instead of the count
+                        // one tile per CTA and two CTAs per SM (256 TMEM columns each), 2: E4M3 digits
+                        // (N ≤ 160; a column is Σ_p 32^−p·digit_p)
+  bool twos = false;    // TC, plan 2: the matrix is 2·[count = 2] instead of the count
   int groups = 1;       // TC: products of as many operands B[grp] (N rows each, one after the other) with
                         // the same matrix, partials [groups][splits][kp][M_pad]
 };

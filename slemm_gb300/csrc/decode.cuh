@@ -13,6 +13,7 @@
 #include <cstdint>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <cuda_fp8.h>
 
 namespace slemm {
 
@@ -24,20 +25,6 @@ __device__ __forceinline__ uint32_t bf16pair_of(uint32_t word, int q)
   const float sc = 1.0f / (float)(1 << k);
   const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162*>(&bits);
   const __nv_bfloat162 r = __hfma2(v, __float2bfloat162_rn(sc), __float2bfloat162_rn(-128.0f * sc));
-  return *reinterpret_cast<const uint32_t*>(&r);
-}
-
-// The same pair as FP16: (src & (0x00030003 ≪ k)) | 0x64006400 is an FP16 pair whose halves are
-// 1024 + x·2^k (0x6400 is 1024, whose mantissa step is 1; x·2^k ≤ 128 stays inside the 10-bit
-// mantissa), and one HFMA2, v·2^−k − 1024·2^−k, gives x exactly.
-__device__ __forceinline__ uint32_t f16pair_of(uint32_t word, int q)
-{
-  const uint32_t src = (q < 4) ? word : (word >> 8);
-  const int k = 2 * (q & 3);
-  const uint32_t bits = (src & (0x00030003u << k)) | 0x64006400u;
-  const float sc = 1.0f / (float)(1 << k);
-  const __half2 v = *reinterpret_cast<const __half2*>(&bits);
-  const __half2 r = __hfma2(v, __float2half2_rn(sc), __float2half2_rn(-1024.0f * sc));
   return *reinterpret_cast<const uint32_t*>(&r);
 }
 
@@ -54,12 +41,6 @@ __device__ __forceinline__ uint32_t f16sub_pair_of(uint32_t word, int q)
   const uint32_t src = (q < 5) ? word : (word >> 10);
   return src & (0x00030003u << (2 * f16sub_shift(q)));
 }
-// The same pair with every count x replaced by 2·[x = 2] (the high bit of its field alone).
-__device__ __forceinline__ uint32_t f16sub_twos_of(uint32_t word, int q)
-{
-  const uint32_t src = (q < 5) ? word : (word >> 10);
-  return src & (0x00020002u << (2 * f16sub_shift(q)));
-}
 // 2^−2s for the element at K index kidx (K-tiles start at multiples of 64; element j of a
 // 16-element word is K index ≡ j mod 16, pair q = j / 2).
 __device__ __forceinline__ float f16sub_kscale(int64_t kidx)
@@ -74,23 +55,40 @@ __device__ __forceinline__ float f16sub_kunscale(int64_t kidx)
 }
 constexpr float kF16SubUnscale = 16777216.0f;   // 2^24
 
-template <bool F16, bool TWOS = false>
+template <bool F16>
 __device__ __forceinline__ uint32_t pair_of(uint32_t word, int q)
 {
-  if constexpr (F16 && TWOS) return f16sub_twos_of(word, q);
-  else if constexpr (F16) return f16sub_pair_of(word, q);
+  if constexpr (F16) return f16sub_pair_of(word, q);
   else return bf16pair_of(word, q);
 }
 
-// The 4 BF16 pairs of elements 8h … 8h+7 of a word (h = 0: pairs 0-3, h = 1: pairs 4-7).
-__device__ __forceinline__ uint4 bf16x8_of(uint32_t word, int h)
+// Four counts of a word as E4M3 bytes, by masking alone: a byte whose low two bits hold x is the
+// subnormal x·2^−9, and one whose bits 2, 3 hold x (mantissa and exponent zero elsewhere) reads as
+// x·2^−7 — x = 1 is the subnormal 4·2^−9, x = 2 the exponent field 1, 2^−6.  Group p = 0 … 3 of a
+// word is the mask 0x03 (p even) or 0x0C (p odd) on every byte of the word (p < 2) or of the
+// word shifted right by 4: four LOPs and one shift for 16 counts.  Byte b of group p is element
+// {2p, 8+2p, 2p+1, 9+2p}[b] of the word, the order the dense operand's K positions 4p + b follow, and
+// the operand carries 2^−2 at odd p; the accumulator is multiplied by 2^9.  TWOS: 2·[x = 2] instead of x.
+template <bool TWOS>
+__device__ __forceinline__ uint32_t f8_quad_of(uint32_t word, int p)
 {
-  uint4 r;
-  r.x = bf16pair_of(word, 4 * h + 0);
-  r.y = bf16pair_of(word, 4 * h + 1);
-  r.z = bf16pair_of(word, 4 * h + 2);
-  r.w = bf16pair_of(word, 4 * h + 3);
-  return r;
+  const uint32_t src = (p < 2) ? word : (word >> 4);
+  return src & ((p & 1) ? (TWOS ? 0x08080808u : 0x0C0C0C0Cu) : (TWOS ? 0x02020202u : 0x03030303u));
+}
+constexpr float kF8Unscale = 512.0f;   // 2^9
+
+// Four integers |d| ≤ 16 as E4M3 bytes (4 significant bits: exact), times 1 or 2^−2.
+__device__ __forceinline__ uint32_t e4m3x4(float d0, float d1, float d2, float d3, float s)
+{
+  const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(d0 * s, d1 * s), __NV_SATFINITE, __NV_E4M3);
+  const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(d2 * s, d3 * s), __NV_SATFINITE, __NV_E4M3);
+  return lo | (hi << 16);
+}
+// The 16 K positions of one word's elements d[0 … 15] in the decoded order.
+__device__ __forceinline__ uint4 e4m3_word(const float (&d)[16])
+{
+  return make_uint4(e4m3x4(d[0], d[8], d[1], d[9], 1.f), e4m3x4(d[2], d[10], d[3], d[11], 0.25f),
+                    e4m3x4(d[4], d[12], d[5], d[13], 1.f), e4m3x4(d[6], d[14], d[7], d[15], 0.25f));
 }
 
 // Exact FP32 counts of element pair q.

@@ -1,57 +1,63 @@
 // exact.cu — products of the packed counts with FP32 or FP64 columns whose sums are exact.
 //
-// A dense column v is cut into slices of 11 bits,
-//   v·2^e = q_0 + 2^−11·q_1 + 2^−22·q_2 + …,   q_p integers, |q_p| ≤ 2^10,
-// with e such that max|v|·2^e lies in [2^9, 2^10): six slices hold an FP64 column to 2^−65 of its
-// largest value, four hold an FP32 one to 2^−43.  Slices are exact in FP16 and a count is at most
-// 2, so a product row's sum over 8,192 K-elements is an integer of at most 2^24: the tensor cores'
-// FP32 accumulators are exact whatever their order.  K is therefore split every 128 K-tiles at the
-// latest, the partials are added as 64-bit integers, and only the last combination of the slices
-// rounds (in FP64).  Bound by the narrow tensor-core pass (its decoders).  GB300's FP64 pipe ran the
-// same sums by an FMA per genotype and column: at n = 100,000, m = 50,000 the GEBV took 18,988 µs
-// and takes 829 µs, the score terms with three covariates and residual weights 112,698 µs and
-// 1,221 µs, with the same or a smaller error against 64-bit sums.
+// A dense column v is cut into base-32 digits,
+//   v·2^e = d_0 + 2^−5·d_1 + 2^−10·d_2 + …,   d_p integers, |d_p| ≤ 16,
+// with e such that max|v|·2^e lies in [2^3, 2^4): 13 digits hold an FP64 column to 2^−65 of its
+// largest value, nine hold an FP32 one to 2^−45.  Digits are exact in E4M3 and a count is at most 2,
+// so a product row's sum over 2^19 K-elements is an integer of at most 2^24: the tensor cores' FP32
+// accumulators are exact whatever their order.  K is therefore split every 8,192 K-tiles at the
+// latest, the partials are added as 64-bit integers, and only the last combination of the digits
+// rounds (in FP64).  Bound by the narrow tensor-core pass.  GB300's FP64 pipe ran the same sums by an
+// FMA per genotype and column: at n = 100,000, m = 50,000 the GEBV took 18,988 µs and takes 593 µs, the
+// score terms with three covariates and residual weights 112,698 µs and 697 µs, with the same or a
+// smaller error against 64-bit sums.
 #include "internal.h"
 #include "decode.cuh"
 #include "reduce.cuh"
 
 namespace slemm {
 
-constexpr int kSliceBits = 11;
-constexpr int kSlicesF64 = 6;
-constexpr int kSlicesF32 = 4;
-constexpr int kExactKTiles = 8192 / kTileK;   // K-tiles of one exact FP32 partial sum
+constexpr int kDigitBits = 5;
+constexpr int kDigitsF64 = 13;
+constexpr int kDigitsF32 = 9;
+constexpr int kExactKTiles = (1 << 19) / kTileK;   // K-tiles of one exact FP32 partial sum
 constexpr int kXRows = 2048;                  // K-elements of one block of the operand kernels
 constexpr int kXThreads = 256;
 
-// e with amax·2^e in [2^9, 2^10) (0 for a zero or non-finite column)
-__host__ __device__ inline int slice_exp(double amax)
+// e with amax·2^e in [2^3, 2^4) (0 for a zero or non-finite column)
+__host__ __device__ inline int digit_exp(double amax)
 {
   if (!(amax > 0.0) || !isfinite(amax)) return 0;
   int E;
   frexp(amax, &E);
-  return 10 - E;
+  return 4 - E;
 }
 
-// Slices 0 … S−1 of v·2^e into rows row0 … row0 + S − 1 of the FP16 operand at K-element kidx, times
-// the 2^−2s its K position takes (f16sub_pair_of).
-template <int S>
-__device__ __forceinline__ void store_slices(double v, int e, __half* __restrict__ B, int64_t K_pad, int row0,
-                                             int64_t kidx)
+// Digits 0 … S−1 of the 16 values v[·]·2^e of K-elements kidx … kidx + 15 (one packed word) into rows
+// row0 … row0 + S − 1 of the operand.
+template <int S, class T>
+__device__ __forceinline__ void store_digits(const T (&v)[16], int e, uint8_t* __restrict__ B, int64_t K_pad,
+                                             int row0, int64_t kidx)
 {
-  double r = ldexp(v, e);
-  const float ks = f16sub_kscale(kidx);
+  T r[16];   // every step below is exact in the values' own type
 #pragma unroll
+  for (int u = 0; u < 16; ++u) r[u] = ldexp(v[u], e);
+#pragma unroll 1
   for (int p = 0; p < S; ++p) {
-    const double q = rint(r);
-    B[(int64_t)(row0 + p) * K_pad + kidx] = __float2half_rn(__fmul_rn((float)q, ks));
-    r = (r - q) * (double)(1 << kSliceBits);   // exact
+    float d[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      const T q = rint(r[u]);
+      d[u] = (float)q;
+      r[u] = (r[u] - q) * (T)(1 << kDigitBits);
+    }
+    *reinterpret_cast<uint4*>(B + (int64_t)(row0 + p) * K_pad + kidx) = e4m3_word(d);
   }
 }
 
-// Σ_p 2^−11p·(Σ_splits D[s][row0 + p][r]) — the column's product with row r, in units of 2^−e
+// Σ_p 2^−5p·(Σ_splits D[s][row0 + p][r]) — the column's product with row r, in units of 2^−e
 template <int S>
-__device__ __forceinline__ double gather_slices(const float* __restrict__ D, int splits, int kp, int64_t M_pad,
+__device__ __forceinline__ double gather_digits(const float* __restrict__ D, int splits, int kp, int64_t M_pad,
                                                 int row0, int64_t r)
 {
   long long sum[S] = {};
@@ -60,19 +66,21 @@ __device__ __forceinline__ double gather_slices(const float* __restrict__ D, int
     for (int p = 0; p < S; ++p) sum[p] += (long long)D[((int64_t)s * kp + row0 + p) * M_pad + r];
   double v = 0.0;
 #pragma unroll
-  for (int p = S - 1; p >= 0; --p) v = v * (1.0 / (1 << kSliceBits)) + (double)sum[p];
+  for (int p = S - 1; p >= 0; --p) v = v * (1.0 / (1 << kDigitBits)) + (double)sum[p];
   return v;
 }
 
-// GEBV operand: rows 0 … 5 the slices of alpha (0 past m), rows 6 … 15 zero
+// GEBV operand: rows 0 … 12 the digits of alpha (0 past m), rows 13 … 15 zero; 16 K-elements per thread
 __global__ void __launch_bounds__(kXThreads)
-gebv_operand_kernel(const double* __restrict__ alpha, int64_t m, int64_t m_pad, int e, __half* __restrict__ B)
+gebv_operand_kernel(const double* __restrict__ alpha, int64_t m, int64_t m_pad, int e, uint8_t* __restrict__ B)
 {
-  const int64_t j = (int64_t)blockIdx.x * kXThreads + threadIdx.x;
+  const int64_t j = ((int64_t)blockIdx.x * kXThreads + threadIdx.x) * 16;
   if (j >= m_pad) return;
-  store_slices<kSlicesF64>(j < m ? alpha[j] : 0.0, e, B, m_pad, 0, j);
+  double v[16];
 #pragma unroll
-  for (int q = kSlicesF64; q < 16; ++q) B[(int64_t)q * m_pad + j] = __float2half_rn(0.f);
+  for (int u = 0; u < 16; ++u) v[u] = j + u < m ? alpha[j + u] : 0.0;
+  store_digits<kDigitsF64>(v, e, B, m_pad, 0, j);
+  for (int q = kDigitsF64; q < 16; ++q) *reinterpret_cast<uint4*>(B + (int64_t)q * m_pad + j) = make_uint4(0u, 0u, 0u, 0u);
 }
 
 __global__ void __launch_bounds__(kXThreads)
@@ -80,7 +88,7 @@ gebv_finish_kernel(const float* __restrict__ D, int splits, int kp, int64_t n_pa
                    double* __restrict__ tgv)
 {
   const int64_t i = (int64_t)blockIdx.x * kXThreads + threadIdx.x;
-  if (i < n) tgv[i] = shift + ldexp(gather_slices<kSlicesF64>(D, splits, kp, n_pad, 0, i), -e);
+  if (i < n) tgv[i] = shift + ldexp(gather_digits<kDigitsF64>(D, splits, kp, n_pad, 0, i), -e);
 }
 
 // The columns of exact_dots (FP32 values), i < n.
@@ -122,7 +130,7 @@ dots_stats_kernel(ExactCols a, int64_t n, double* __restrict__ sums, double* __r
   }
 }
 
-// Column c's total (NaN when it holds a non-finite value) and slice exponent, one warp each.
+// Column c's total (NaN when it holds a non-finite value) and digit exponent, one warp each.
 __global__ void dots_scale_kernel(const double* __restrict__ sums, const double* __restrict__ amax, int nblk, int C,
                                   double* __restrict__ tot, int* __restrict__ exps)
 {
@@ -132,30 +140,30 @@ __global__ void dots_scale_kernel(const double* __restrict__ sums, const double*
   const double a = warp_max_partials(amax + (int64_t)c * nblk, nblk);
   if ((threadIdx.x & 31) == 0) {
     tot[c] = isfinite(a) ? s : NAN;
-    exps[c] = slice_exp(a);
+    exps[c] = digit_exp(a);
   }
 }
 
-// Operand of columns c0 … c0 + nc − 1: column c's slices in rows 4(c − c0) …, rows up to N zero.
+// Operand of columns c0 … c0 + nc − 1: column c's digits in rows 9(c − c0) …, rows up to N zero.
 // Blocks y < nc write a column, y ≥ nc one zero row each.  A non-finite column is stored as zeros (its
 // products come out NaN through its total).
 __global__ void __launch_bounds__(kXThreads)
 dots_operand_kernel(ExactCols a, int64_t n, int64_t n_pad, int c0, int nc, const double* __restrict__ tot,
-                    const int* __restrict__ exps, __half* __restrict__ B)
+                    const int* __restrict__ exps, uint8_t* __restrict__ B)
 {
   const int b = blockIdx.y;
-  const int64_t i0 = (int64_t)blockIdx.x * kXRows, i1 = min64(n_pad, i0 + kXRows);
+  const int64_t i = ((int64_t)blockIdx.x * kXThreads + threadIdx.x) * 16;
+  if (i >= n_pad) return;
   if (b >= nc) {
-    for (int64_t i = i0 + threadIdx.x; i < i1; i += kXThreads)
-      B[(int64_t)(kSlicesF32 * nc + b - nc) * n_pad + i] = __float2half_rn(0.f);
+    *reinterpret_cast<uint4*>(B + (int64_t)(kDigitsF32 * nc + b - nc) * n_pad + i) = make_uint4(0u, 0u, 0u, 0u);
     return;
   }
   const int c = c0 + b, e = exps[c];
   const bool fine = !isnan(tot[c]);
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += kXThreads) {
-    const float v = (i < n && fine) ? dot_column(a, c, i) : 0.f;
-    store_slices<kSlicesF32>((double)v, e, B, n_pad, kSlicesF32 * b, i);
-  }
+  float v[16];
+#pragma unroll
+  for (int u = 0; u < 16; ++u) v[u] = (i + u < n && fine) ? dot_column(a, c, i + u) : 0.f;
+  store_digits<kDigitsF32>(v, e, B, n_pad, kDigitsF32 * b, i);
 }
 
 // out[c0 + c][j] of the pass over columns c0 …; grid (rows, columns)
@@ -166,28 +174,28 @@ dots_gather_kernel(const float* __restrict__ D, int splits, int kp, int64_t m_pa
   const int64_t j = (int64_t)blockIdx.x * kXThreads + threadIdx.x;
   if (j >= m) return;
   const int c = c0 + blockIdx.y;
-  const double v = ldexp(gather_slices<kSlicesF32>(D, splits, kp, m_pad, kSlicesF32 * blockIdx.y, j), -exps[c]);
+  const double v = ldexp(gather_digits<kDigitsF32>(D, splits, kp, m_pad, kDigitsF32 * blockIdx.y, j), -exps[c]);
   out[(int64_t)blockIdx.y * m + j] = isnan(tot[c]) ? NAN : v;
 }
 
 // Split-K count of an exact product over K_tiles K-tiles: at most kExactKTiles of them each.
 static int exact_splits(int64_t M_pad, int64_t K_tiles, int N)
 {
-  return choose_splits(M_pad / gemm_tc_rows_per_cta(N, 0), K_tiles, 1, num_sms(),
+  return choose_splits(M_pad / gemm_tc_rows_per_cta(N, 2), K_tiles, 1, num_sms(),
                        (int)ceil_div(K_tiles, kExactKTiles));
 }
 
 void exact_gebv(slemm_geno* g, const double* d_alpha, double amax, double shift, double* d_tgv)
 {
   cudaStream_t st = g->stream;
-  const int e = slice_exp(amax);
-  const int N = 16, kp = 8;
+  const int e = digit_exp(amax);
+  const int N = 16, kp = 16;
   const int splits = exact_splits(g->n_pad, g->m_pad / kTileK, N);
-  __half* B = (__half*)g->ws_B.ensure((size_t)N * g->m_pad * sizeof(__half));
+  uint8_t* B = (uint8_t*)g->ws_B.ensure((size_t)N * g->m_pad);
   float* D = (float*)g->ws_D.ensure((size_t)splits * kp * g->n_pad * sizeof(float));
-  gebv_operand_kernel<<<(unsigned)ceil_div(g->m_pad, kXThreads), kXThreads, 0, st>>>(d_alpha, g->m, g->m_pad, e, B);
+  gebv_operand_kernel<<<(unsigned)ceil_div(g->m_pad, 16 * kXThreads), kXThreads, 0, st>>>(d_alpha, g->m, g->m_pad, e, B);
   LAUNCH_CHECK();
-  gemm_tc({g->GT.as<uint8_t>(), g->n_pad, g->m_pad, B, N, D, splits, g->err.as<int>(), kp, 1, true}, st);
+  gemm_tc({g->GT.as<uint8_t>(), g->n_pad, g->m_pad, B, N, D, splits, g->err.as<int>(), kp, 1, false, 2}, st);
   gebv_finish_kernel<<<(unsigned)ceil_div(g->n, kXThreads), kXThreads, 0, st>>>(D, splits, kp, g->n_pad, g->n, e, shift,
                                                                                d_tgv);
   LAUNCH_CHECK();
@@ -199,40 +207,38 @@ void exact_dots(slemm_geno* g, const ExactCols& a, double* dots, double* tot, do
   const int C = a.count();
   const int64_t n_pad = g->n_pad, K_tiles = n_pad / kTileK;
   const int nblk = (int)ceil_div(n_pad, kXRows);
-  // up to 16 columns fill one narrow pass (N = 64); more go 64 at a time through the wide plan
-  const int grp = C <= 16 ? C : 64;
-  const int kp = (int)round_up(kSlicesF32 * grp, 8), N = (int)round_up(kp, 16);
+  // up to 17 columns of nine digits fill one pass (N = 160)
+  const int grp = (int)ceil_div(C, ceil_div(C, 17));
+  const int kp = (int)round_up(kDigitsF32 * grp, 8), N = (int)round_up(kp, 16);
   const int splits = exact_splits(g->m_pad, K_tiles, N), splits2 = exact_splits(g->m_pad, K_tiles, 16);
   DevBuf dst(st);
   double* sums = (double*)dst.ensure((size_t)2 * C * nblk * sizeof(double) + C * sizeof(int));
   double* amax = sums + (size_t)C * nblk;
   int* exps = reinterpret_cast<int*>(amax + (size_t)C * nblk);
-  __half* B = (__half*)g->ws_B.ensure((size_t)std::max(N, 16) * n_pad * sizeof(__half));
-  float* D = (float*)g->ws_D.ensure(std::max((size_t)splits * kp, (size_t)splits2 * 8) * g->m_pad * sizeof(float));
+  uint8_t* B = (uint8_t*)g->ws_B.ensure((size_t)N * n_pad);
+  float* D = (float*)g->ws_D.ensure(std::max((size_t)splits * kp, (size_t)splits2 * 16) * g->m_pad * sizeof(float));
   const uint8_t* G = g->G.as<uint8_t>();
   int* err = g->err.as<int>();
-  const unsigned rows = (unsigned)ceil_div(g->m, kXThreads);
+  const unsigned rows = (unsigned)ceil_div(g->m, kXThreads), oblk = (unsigned)ceil_div(n_pad, 16 * kXThreads);
   dots_stats_kernel<<<dim3(nblk, C), kXThreads, 0, st>>>(a, g->n, sums, amax, nblk);
   LAUNCH_CHECK();
   dots_scale_kernel<<<(unsigned)ceil_div(C * 32, 128), 128, 0, st>>>(sums, amax, nblk, C, tot, exps);
   LAUNCH_CHECK();
   for (int c0 = 0; c0 < C; c0 += grp) {
     const int nc = std::min(grp, C - c0);
-    const int kpc = (int)round_up(kSlicesF32 * nc, 8), Nc = (int)round_up(kpc, 16);
-    const int sp = nc == grp ? splits : std::min(splits, exact_splits(g->m_pad, K_tiles, Nc));
-    const int spc = std::max(sp, (int)ceil_div(K_tiles, kExactKTiles));
-    dots_operand_kernel<<<dim3(nblk, nc + Nc - kSlicesF32 * nc), kXThreads, 0, st>>>(a, g->n, n_pad, c0, nc, tot, exps, B);
+    const int kpc = (int)round_up(kDigitsF32 * nc, 8), Nc = (int)round_up(kpc, 16);
+    dots_operand_kernel<<<dim3(oblk, nc + Nc - kDigitsF32 * nc), kXThreads, 0, st>>>(a, g->n, n_pad, c0, nc, tot, exps, B);
     LAUNCH_CHECK();
-    gemm_tc({G, g->m_pad, n_pad, B, Nc, D, spc, err, kpc, 1, true}, st);
-    dots_gather_kernel<<<dim3(rows, nc), kXThreads, 0, st>>>(D, spc, kpc, g->m_pad, g->m, c0, tot, exps,
+    gemm_tc({G, g->m_pad, n_pad, B, Nc, D, splits, err, kpc, 1, false, 2}, st);
+    dots_gather_kernel<<<dim3(rows, nc), kXThreads, 0, st>>>(D, splits, kpc, g->m_pad, g->m, c0, tot, exps,
                                                               dots + (size_t)c0 * g->m);
     LAUNCH_CHECK();
   }
   if (twos != nullptr) {   // 2·Σ rr²·[count = 2]: the last column (rr²) against the high bits
-    dots_operand_kernel<<<dim3(nblk, 1 + 16 - kSlicesF32), kXThreads, 0, st>>>(a, g->n, n_pad, C - 1, 1, tot, exps, B);
+    dots_operand_kernel<<<dim3(oblk, 1 + 16 - kDigitsF32), kXThreads, 0, st>>>(a, g->n, n_pad, C - 1, 1, tot, exps, B);
     LAUNCH_CHECK();
-    gemm_tc({G, g->m_pad, n_pad, B, 16, D, splits2, err, 8, 1, true, 0, true}, st);
-    dots_gather_kernel<<<dim3(rows, 1), kXThreads, 0, st>>>(D, splits2, 8, g->m_pad, g->m, C - 1, tot, exps, twos);
+    gemm_tc({G, g->m_pad, n_pad, B, 16, D, splits2, err, 16, 1, false, 2, true}, st);
+    dots_gather_kernel<<<dim3(rows, 1), kXThreads, 0, st>>>(D, splits2, 16, g->m_pad, g->m, C - 1, tot, exps, twos);
     LAUNCH_CHECK();
   }
 }

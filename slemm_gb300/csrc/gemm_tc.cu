@@ -8,6 +8,14 @@
 // one LOP and one HFMA2 each; FP16 pairs are the counts as FP16 subnormals, one LOP each, with
 // the matching power of two per K position in B and 2^24 in the epilogue (decode.cuh).
 //
+// Few columns (plan 2, kind::f8f6f4): an MMA of M = 128 takes the tensor pipe about 48 cycles
+// whatever its N is below 96, so a narrow FP16 product runs at the rate of its MMAs, two per 32
+// K-elements and row tile: 2.65 ms for the 7.5 GB of n = 500,000, m = 60,000, with 1 column as with 24.
+// E4M3 MMAs take 32 K-elements each, the counts are four masked bytes per LOP instead of two
+// halves, and the dense column is five base-32 digits instead of two halves: half the MMAs and
+// half the decode for the same 24 bits, and sums of integers that FP32 accumulates exactly.  Z_cᵀU of 4
+// columns at n = 200,003, m = 50,021: 990 → 584 µs (error against FP64 2.2e-7 → 1.6e-7).
+//
 // What limits tcgen05 here is the issuing thread, not the tensor pipe.  Measured on GB300: one
 // thread issuing M=128, N=144, K=16 BF16 MMAs back to back keeps the pipe full (72 cycles per
 // MMA, 8192 FLOP/clk per SM) whether A comes from TMEM or shared memory, but a barrier wait and
@@ -54,7 +62,12 @@ namespace slemm {
 // two K-tiles (eight MMAs per wait and commit; the small accumulators leave TMEM room for three
 // such stages): <6, 3, 0, 2>, where SB = 0 puts B on the A stages' own full barrier (the B
 // producer's expect_tx), which measured faster for narrow blocks than a separate B ring.
+// E4M3 digits read two K-tiles as one operand tile (128 bytes of K), so their stages are those of
+// the FP16 plans with twice the K: <6, 3, 0, 4> for N ≤ 64 and <4, 3, 6, 2> up to N = 160.
 constexpr int kPkg = 4;                // K-tiles per packed slot
+enum class Fmt { BF16, F16, F8 };
+// K-tiles of one operand tile (N rows × 128 bytes of K: 64 halves or 128 digits)
+constexpr int ktiles_per_op(Fmt f) { return f == Fmt::F8 ? 2 : 1; }
 constexpr int kNG = 3;                 // decoder groups (each keeps one stage in flight)
 constexpr int kMaxThreads = 64 + 2 * 32 + kNG * 2 * 128;   // SUB = 2
 // Threads of a one-tile CTA (the narrow plan that runs two CTAs per SM, 256 TMEM columns each).
@@ -65,14 +78,15 @@ constexpr int tc_min_blocks(int TM) { return TM == 512 ? 1 : 2; }
 constexpr uint64_t kWaitBudgetNs = 2000000000ull;   // 2 s per wait
 constexpr size_t kSmemBudget = 227 * 1024;
 
-template <int PK, int S, int SB, int KT>
+// U operand tiles per stage (KT K-tiles, or KT / 2 of digits).
+template <int PK, int S, int SB, int U>
 struct TcPlan {
   int N, sub;
   size_t b_off, pk_off, bar_off, total;
   __host__ __device__ TcPlan(int N_, int sub_) : N(N_), sub(sub_)
   {
-    b_off = 0;                                         // BS × KT × N·128 B (1024-aligned, N%8==0)
-    pk_off = b_off + (size_t)(SB > 0 ? SB : S) * KT * N * 128;   // PK × sub × kPkg × 2 KB
+    b_off = 0;                                         // BS × U × N·128 B (1024-aligned, N%8==0)
+    pk_off = b_off + (size_t)(SB > 0 ? SB : S) * U * N * 128;   // PK × sub × kPkg × 2 KB
     bar_off = pk_off + (size_t)PK * sub * kPkg * kTileBytes;
     total = bar_off + 512 + 1024;                      // barriers/slots + 1024-B base alignment
   }
@@ -83,15 +97,16 @@ struct TcPlan {
   __host__ __device__ uint32_t acol() const { return (uint32_t)(((sub * N + 31) / 32) * 32); }
 };
 
-// Two tiles when their accumulators and S A-stages of KT K-tiles fit the 512 TMEM columns, else one;
-// a plan with TM = 256 (two CTAs per SM) always has one tile.
-template <int PK, int S, int SB, int KT, int TM = 512>
-static TcPlan<PK, S, SB, KT> plan_tc(int N)
+// Two tiles when their accumulators and S A-stages of U operand tiles fit the 512 TMEM columns, else
+// one; a plan with TM = 256 (two CTAs per SM) always has one tile.
+template <int PK, int S, int SB, int U, int TM = 512>
+static TcPlan<PK, S, SB, U> plan_tc(int N)
 {
-  if (TM == 512 && (((2 * N + 31) / 32) * 32) + 2 * 32 * KT * S <= 512) return TcPlan<PK, S, SB, KT>(N, 2);
-  return TcPlan<PK, S, SB, KT>(N, 1);
+  if (TM == 512 && (((2 * N + 31) / 32) * 32) + 2 * 32 * U * S <= 512) return TcPlan<PK, S, SB, U>(N, 2);
+  return TcPlan<PK, S, SB, U>(N, 1);
 }
 constexpr int kNarrowN = 64;   // N ≤ 64 uses the deep ring
+constexpr int kDigitN = 160;   // largest N of the digit plans (two row tiles per CTA)
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p)
 {
@@ -207,16 +222,33 @@ __host__ __device__ constexpr uint32_t idesc_f16kind(int N, bool f16)
          | ((uint32_t)(128 >> 4) << 24);    // M / 16
 }
 
-// D[tmem] (+)= A[tmem] · B[smem]
-__device__ __forceinline__ void mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate)
+// Instruction descriptor of kind::f8f6f4: E4M3 × E4M3 → FP32, both K-major, M = 128.
+__host__ __device__ constexpr uint32_t idesc_f8kind(int N)
 {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+  return (1u << 4)                          // D format F32; A and B format 0: E4M3
+         | ((uint32_t)(N >> 3) << 17)       // N / 8
+         | ((uint32_t)(128 >> 4) << 24);    // M / 16
+}
+
+// D[tmem] (+)= A[tmem] · B[smem], K = 16 (kind::f16) or 32 (kind::f8f6f4)
+template <bool F8>
+__device__ __forceinline__ void mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                       uint32_t accumulate)
+{
+  if constexpr (F8)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
 }
 
 __device__ __forceinline__ void mma_commit(uint64_t* bar)
@@ -261,7 +293,7 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
       : "memory");
 }
 
-template <int PK, int S, int SB, int KT, bool F16, int TM, bool TWOS>
+template <int PK, int S, int SB, int KT, Fmt FMT, int TM, bool TWOS>
 __global__ void __launch_bounds__(tc_max_threads(TM), tc_min_blocks(TM))
 gemm_tc_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMap tmapB,
                float* __restrict__ D, int64_t M_pad, int K_tiles, int tiles_per_split, int N, int sub,
@@ -270,14 +302,16 @@ gemm_tc_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMa
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment of the shared-window address (SWIZZLE_128B tiles need it)
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  const TcPlan<PK, S, SB, KT> P(N, sub);
+  constexpr int KPO = ktiles_per_op(FMT);      // K-tiles per operand tile
+  constexpr int U = KT / KPO;                  // operand tiles per stage
+  const TcPlan<PK, S, SB, U> P(N, sub);
   uint8_t* sB = smem + P.b_off;
   uint8_t* sPk = smem + P.pk_off;
   uint64_t* pk_full = (uint64_t*)(smem + P.bar_off);
   uint64_t* pk_empty = pk_full + PK;
   constexpr int BS = SB > 0 ? SB : S;          // B stages (SB = 0: B rides on the A stages)
   static_assert(BS % S == 0, "the stage-done ring serves both rings");
-  static_assert(kPkg % KT == 0, "a stage's K-tiles lie in one packed slot");
+  static_assert(kPkg % KT == 0 && KT % KPO == 0, "a stage's K-tiles lie in one packed slot, in whole operand tiles");
   uint64_t* st_full = pk_empty + PK;
   uint64_t* done = st_full + S;                // done[i % BS]: the MMAs of stage i have completed
   uint64_t* b_full = done + BS;
@@ -350,7 +384,7 @@ gemm_tc_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMa
   } else if (warp == 1) {
     // ---------------- B producer (L2) ----------------
     if (lane == 0) {
-      const uint32_t bytes = (uint32_t)N * 128u;   // one K-tile of B
+      const uint32_t bytes = (uint32_t)N * 128u;   // one operand tile of B
       int issued = 0;
       for (int i = 0; i < ns; ++i) {
         const int s = i % BS;
@@ -362,9 +396,10 @@ gemm_tc_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMa
           ++issued;
           continue;
         }
-        mbar_arrive_expect_tx(full, (uint32_t)KT * bytes);
-        for (int kk = 0; kk < KT; ++kk)
-          tma_load_2d(sB + ((size_t)s * KT + kk) * N * 128, &tmapB, (kt0 + i * KT + kk) * kTileK, (int)blockIdx.z * N, full);
+        mbar_arrive_expect_tx(full, (uint32_t)U * bytes);
+        for (int kk = 0; kk < U; ++kk)
+          tma_load_2d(sB + ((size_t)s * U + kk) * N * 128, &tmapB, (kt0 + i * KT + kk * KPO) * kTileK,
+                      (int)blockIdx.z * N, full);
         ++issued;
       }
       if (*abort_flag)
@@ -378,12 +413,12 @@ gemm_tc_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMa
     // both tiles, or four column-group issuers, measured slower).
     const int t = warp - P.mma_warp0();
     if (lane == 0) {
-      const uint32_t idesc = idesc_f16kind(N, F16);
+      const uint32_t idesc = FMT == Fmt::F8 ? idesc_f8kind(N) : idesc_f16kind(N, FMT == Fmt::F16);
       const uint64_t bdesc0 = sw128_desc(smem_u32(sB));
-      const uint32_t bstep = (uint32_t)(N * 128) >> 4;          // descriptor units per B K-tile
+      const uint32_t bstep = (uint32_t)(N * 128) >> 4;          // descriptor units per B operand tile
       const uint32_t d_tmem = tmem_base + (uint32_t)(t * N);
-      const uint32_t a_base = tmem_base + acol + (uint32_t)(t * 32 * KT);
-      const uint32_t a_step = (uint32_t)(sub * 32 * KT);        // columns per A stage
+      const uint32_t a_base = tmem_base + acol + (uint32_t)(t * 32 * U);
+      const uint32_t a_step = (uint32_t)(sub * 32 * U);        // columns per A stage
       // Unrolled over one turn of the B ring (BS stages, a whole number of A-ring turns), so
       // ring slots, parities and descriptor offsets are constants: the issuing thread shares
       // its SM sub-partition with decoder warps, and every instruction it waits to issue
@@ -401,13 +436,13 @@ gemm_tc_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMa
           }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-          for (int kk = 0; kk < KT; ++kk) {
-            const uint64_t bd = bdesc0 + (uint64_t)((u * KT + kk) * bstep);
+          for (int kk = 0; kk < U; ++kk) {
+            const uint64_t bd = bdesc0 + (uint64_t)((u * U + kk) * bstep);
             const uint32_t ad = a_base + (uint32_t)(u % S) * a_step + (uint32_t)(kk * 32);
-            mma_bf16_ts(d_tmem, ad, bd, idesc, (i > 0 || kk > 0) ? 1u : 0u);
-            mma_bf16_ts(d_tmem, ad + 8, bd + 2, idesc, 1u);
-            mma_bf16_ts(d_tmem, ad + 16, bd + 4, idesc, 1u);
-            mma_bf16_ts(d_tmem, ad + 24, bd + 6, idesc, 1u);
+            mma_ts<FMT == Fmt::F8>(d_tmem, ad, bd, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+            mma_ts<FMT == Fmt::F8>(d_tmem, ad + 8, bd + 2, idesc, 1u);
+            mma_ts<FMT == Fmt::F8>(d_tmem, ad + 16, bd + 4, idesc, 1u);
+            mma_ts<FMT == Fmt::F8>(d_tmem, ad + 24, bd + 6, idesc, 1u);
           }
           mma_commit(&done[u]);   // frees A stage u % S and B stage u once these MMAs complete
         }
@@ -434,13 +469,23 @@ gemm_tc_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMa
       if (lane == 0) mbar_arrive(&pk_empty[sp]);
       bool ok = true;
 #pragma unroll
-      for (int kk = 0; kk < KT; ++kk) {
+      for (int kk = 0; kk < U; ++kk) {
         uint32_t v[32];
-        const uint32_t words[4] = {pk[kk].x, pk[kk].y, pk[kk].z, pk[kk].w};
 #pragma unroll
-        for (int w = 0; w < 4; ++w)
+        for (int t = 0; t < KPO; ++t) {
+          const uint4 pt = pk[kk * KPO + t];
+          const uint32_t words[4] = {pt.x, pt.y, pt.z, pt.w};
 #pragma unroll
-          for (int q = 0; q < 8; ++q) v[w * 8 + q] = pair_of<F16, TWOS>(words[w], q);
+          for (int w = 0; w < 4; ++w) {
+            if constexpr (FMT == Fmt::F8) {
+#pragma unroll
+              for (int q = 0; q < 4; ++q) v[t * 16 + w * 4 + q] = f8_quad_of<TWOS>(words[w], q);
+            } else {
+#pragma unroll
+              for (int q = 0; q < 8; ++q) v[w * 8 + q] = pair_of<FMT == Fmt::F16>(words[w], q);
+            }
+          }
+        }
         if (kk == 0 && i >= S) {   // the stage that last used this A slot has been consumed
           got = mbar_wait(&done[(i - S) % BS], (uint32_t)((i - S) / BS) & 1, err, 64, abort_flag, 64);
           if (!__all_sync(0xffffffffu, got)) {
@@ -449,7 +494,7 @@ gemm_tc_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMa
           }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
-        tmem_st32(tmem_base + ((uint32_t)(lq * 32) << 16) + acol + (uint32_t)(((s * sub + tsub) * KT + kk) * 32), v);
+        tmem_st32(tmem_base + ((uint32_t)(lq * 32) << 16) + acol + (uint32_t)(((s * sub + tsub) * U + kk) * 32), v);
       }
       if (!ok) break;
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -472,20 +517,23 @@ gemm_tc_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMa
         const uint32_t tl = tmem_base + ((uint32_t)(lq * 32) << 16) + (uint32_t)(tsub * N);
         for (int c0 = 0; c0 < kp; c0 += 8) {
           float acc[8] = {};
-          for (int p = 0; p < pieces; ++p) {
+          for (int q = 0; q < pieces; ++q) {   // digits from the last, each 1/32 of the one before
+            const int p = FMT == Fmt::F8 ? pieces - 1 - q : q;
             uint32_t o[8];
             tmem_ld8_nowait(tl + (uint32_t)(p * kp + c0), o);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int j = 0; j < 8; ++j) acc[j] = __fadd_rn(acc[j], __uint_as_float(o[j]));
+            for (int j = 0; j < 8; ++j)
+              acc[j] = FMT == Fmt::F8 ? __fmaf_rn(acc[j], 0.03125f, __uint_as_float(o[j]))
+                                      : __fadd_rn(acc[j], __uint_as_float(o[j]));
           }
           if (nk == 0) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) acc[j] = 0.f;
           }
-          if constexpr (F16) {   // the FP16 counts were x·2^(2s−24), the operand ·2^−2s
+          if constexpr (FMT != Fmt::BF16) {   // FP16 counts were x·2^(2s−24), the operand ·2^−2s; E4M3 likewise
 #pragma unroll
-            for (int j = 0; j < 8; ++j) acc[j] = __fmul_rn(acc[j], kF16SubUnscale);
+            for (int j = 0; j < 8; ++j) acc[j] = __fmul_rn(acc[j], FMT == Fmt::F16 ? kF16SubUnscale : kF8Unscale);
           }
 #pragma unroll
           for (int j = 0; j < 8; ++j) Dbase[(size_t)(c0 + j) * M_pad] = acc[j];
@@ -532,6 +580,7 @@ static PFN_encodeTiled get_encode()
 int gemm_tc_rows_per_cta(int N, int plan)
 {
   if (N <= kNarrowN && plan == 1) return kTileM;
+  if (plan == 2) return (N <= kNarrowN ? plan_tc<6, 3, 0, 2>(N).sub : plan_tc<4, 3, 6, 1>(N).sub) * kTileM;
   return (N <= kNarrowN ? plan_tc<6, 3, 0, 2>(N).sub : plan_tc<4, 3, 6, 1>(N).sub) * kTileM;
 }
 
@@ -549,13 +598,15 @@ static void configure_once()
   done.fetch_or(bit);
 }
 
-template <int PK, int S, int SB, int KT, bool F16, int TM = 512, bool TWOS = false>
+template <int PK, int S, int SB, int KT, Fmt FMT, int TM = 512, bool TWOS = false>
 static void launch_tc(const GemmArgs& a, cudaStream_t st)
 {
-  const TcPlan<PK, S, SB, KT> P = plan_tc<PK, S, SB, KT, TM>(a.N);
+  constexpr int U = KT / ktiles_per_op(FMT);
+  constexpr bool F8 = FMT == Fmt::F8;
+  const TcPlan<PK, S, SB, U> P = plan_tc<PK, S, SB, U, TM>(a.N);
   CHECK_ARG(a.M_pad % (P.sub * kTileM) == 0 && a.K_pad % 128 == 0, "unpadded operand");
   CHECK_ARG(((uintptr_t)a.A % 16) == 0 && ((uintptr_t)a.B % 16) == 0, "misaligned operand");
-  CHECK_ARG(P.total <= kSmemBudget && P.acol() + 32 * P.sub * S * KT <= TM, "no TMEM/shared-memory plan for this N");
+  CHECK_ARG(P.total <= kSmemBudget && P.acol() + 32 * P.sub * S * U <= TM, "no TMEM/shared-memory plan for this N");
   const int64_t Mc = a.M_pad / (P.sub * kTileM);
   const int K_tiles = (int)(a.K_pad / kTileK);
   CHECK_ARG(K_tiles % KT == 0, "K tiles not a multiple of the stage");
@@ -563,23 +614,26 @@ static void launch_tc(const GemmArgs& a, cudaStream_t st)
 
   CUtensorMap map;
   const cuuint64_t dims[2] = {(cuuint64_t)a.K_pad, (cuuint64_t)a.N * a.groups};
-  const cuuint64_t strides[1] = {(cuuint64_t)a.K_pad * 2};
-  const cuuint32_t box[2] = {64, (cuuint32_t)a.N};
+  const cuuint64_t strides[1] = {(cuuint64_t)a.K_pad * (F8 ? 1 : 2)};
+  const cuuint32_t box[2] = {F8 ? 128u : 64u, (cuuint32_t)a.N};
   const cuuint32_t estr[2] = {1, 1};
-  CUresult r = get_encode()(&map, F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
-                            const_cast<void*>(a.B), dims,
+  CUresult r = get_encode()(&map,
+                            F8                 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
+                            : FMT == Fmt::F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                               : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                            2, const_cast<void*>(a.B), dims,
                             strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) SLEMM_THROW(SLEMM_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
 
-  configure_once<gemm_tc_kernel<PK, S, SB, KT, F16, TM, TWOS>>();
+  configure_once<gemm_tc_kernel<PK, S, SB, KT, FMT, TM, TWOS>>();
   CHECK_ARG(a.kp % 8 == 0 && a.pieces >= 1 && a.pieces * a.kp <= a.N, "bad piece layout");
   // Each CTA allocates TM of the SM's 512 TMEM columns: request enough shared memory that at most
   // 512 / TM CTAs are resident per SM, so no allocation ever has to wait for another CTA's release.
   const size_t smem = std::max<size_t>(P.total, TM == 512 ? 120 * 1024 : 80 * 1024);
   dim3 grid((unsigned)Mc, (unsigned)a.splits, (unsigned)a.groups);
-  gemm_tc_kernel<PK, S, SB, KT, F16, TM, TWOS><<<grid, P.threads(), smem, st>>>(
+  gemm_tc_kernel<PK, S, SB, KT, FMT, TM, TWOS><<<grid, P.threads(), smem, st>>>(
       a.A, map, a.D, a.M_pad, K_tiles, tps, a.N, P.sub, a.kp, a.pieces, a.err, g_withhold_b.exchange(-1));
   LAUNCH_CHECK();
 }
@@ -587,17 +641,22 @@ static void launch_tc(const GemmArgs& a, cudaStream_t st)
 void gemm_tc(const GemmArgs& a, cudaStream_t st)
 {
   CHECK_ARG(a.N >= 16 && a.N <= 256 && a.N % 16 == 0, "TC path needs N in [16,256], N%16==0");
-  CHECK_ARG(a.plan == 0 || (a.plan == 1 && a.N <= kNarrowN), "unknown tensor-core plan");
-  CHECK_ARG(!a.twos || (a.f16 && a.N <= kNarrowN && a.plan == 0), "the count-2 matrix has an FP16 plan for N <= 64 only");
-  if (a.f16) {
-    if (a.twos) launch_tc<6, 3, 0, 2, true, 512, true>(a, st);
-    else if (a.N > kNarrowN) launch_tc<4, 3, 6, 1, true>(a, st);
-    else if (a.plan == 1) launch_tc<6, 3, 0, 2, true, 256>(a, st);
-    else launch_tc<6, 3, 0, 2, true>(a, st);
+  CHECK_ARG(a.plan == 0 || (a.plan == 1 && a.N <= kNarrowN) || (a.plan == 2 && a.N <= kDigitN),
+            "unknown tensor-core plan");
+  CHECK_ARG(!a.twos || a.plan == 2, "the count-2 matrix has digit plans only");
+  if (a.plan == 2) {
+    if (a.twos && a.N <= kNarrowN) launch_tc<6, 3, 0, 4, Fmt::F8, 512, true>(a, st);
+    else if (a.twos) SLEMM_THROW(SLEMM_ERR_ARG, "the count-2 matrix takes N <= 64");
+    else if (a.N > kNarrowN) launch_tc<4, 3, 6, 2, Fmt::F8>(a, st);
+    else launch_tc<6, 3, 0, 4, Fmt::F8>(a, st);
+  } else if (a.f16) {
+    if (a.N > kNarrowN) launch_tc<4, 3, 6, 1, Fmt::F16>(a, st);
+    else if (a.plan == 1) launch_tc<6, 3, 0, 2, Fmt::F16, 256>(a, st);
+    else launch_tc<6, 3, 0, 2, Fmt::F16>(a, st);
   } else {
-    if (a.N > kNarrowN) launch_tc<4, 3, 6, 1, false>(a, st);
-    else if (a.plan == 1) launch_tc<6, 3, 0, 2, false, 256>(a, st);
-    else launch_tc<6, 3, 0, 2, false>(a, st);
+    if (a.N > kNarrowN) launch_tc<4, 3, 6, 1, Fmt::BF16>(a, st);
+    else if (a.plan == 1) launch_tc<6, 3, 0, 2, Fmt::BF16, 256>(a, st);
+    else launch_tc<6, 3, 0, 2, Fmt::BF16>(a, st);
   }
 }
 

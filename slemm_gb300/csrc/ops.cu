@@ -30,6 +30,7 @@ namespace slemm {
 constexpr int kRedThreads = 256;
 static_assert(SLEMM_MAX_COVARIATES <= kRedThreads, "load_qt gives one covariate per thread");
 constexpr int kRowsPerBlock = 4096;   // rows handled by one block of the row-wise kernels
+static_assert(kRowsPerBlock == 16 * kRedThreads, "the digit kernels give each thread one packed word");
 
 // 4-wide accesses need rows % 4 == 0 (a vector never straddles the end), ld % 4 == 0 and a
 // 16-byte aligned base.
@@ -221,12 +222,18 @@ void col_dots(slemm_geno* g, const float* a, int64_t lda, const float* b, int64_
 // (≈4e-6 relative over 500,000 individuals) falls away and what remains is the lo piece's
 // rounding, ≤ 2^−23 of the column's largest value.  The products are scaled back by 2^−e
 // (exact).  BF16 shares FP32's exponent range and needs no scale.
-__device__ __forceinline__ int f16_exp(double bound)
+//
+// Digits (the same precision for at most kDigitCols columns) are a fixed-point split too: the column is
+// scaled into [2^3, 2^4) and written as five base-32 digits |d_p| ≤ 16, E4M3 bytes in the decoded
+// order of the counts (decode.cuh).  They resolve 2^−21 of a unit, ≤ 2^−24 of the column's largest
+// value, and every digit's sum is an exact integer.
+constexpr int kF16Top = 11, kDigitTop = 4;   // a column's bound times 2^e lies in [2^(top−1), 2^top)
+__device__ __forceinline__ int split_exp(double bound, int top)
 {
   if (!(bound > 0.0) || !isfinite(bound)) return 0;
   int E;
-  frexp(bound, &E);                       // bound = f·2^E, f ∈ [0.5, 1)
-  return max(-120, min(120, 11 - E));     // bound·2^e ∈ [2^10, 2^11)
+  frexp(bound, &E);                        // bound = f·2^E, f ∈ [0.5, 1)
+  return max(-120, min(120, top - E));
 }
 
 // max_b parts[c·nblk + b] by the 32 lanes of the calling warp (0 for no partials)
@@ -254,12 +261,12 @@ __device__ __forceinline__ float block_max_f(float v, float* sh)
 // measure pass's signed block extremes range[(c·nblk + b)·2 + {0, 1}] = {max x, max −x} over the
 // valid rows, the bound max(max x − μ, μ − min x) ≥ |x − μ|.  A column with a large mean keeps
 // the resolution of its spread.  The prologue and the finalize take the same e from this.
-__device__ __forceinline__ int f16_col_exp(const double* __restrict__ range, int nblk, int c, float mu)
+__device__ __forceinline__ int split_col_exp(const double* __restrict__ range, int nblk, int c, float mu, int top)
 {
   // by the 32 lanes of the calling warp
   const double hi = warp_max_partials(range + (int64_t)c * nblk * 2, nblk, 2, -INFINITY);
   const double nlo = warp_max_partials(range + (int64_t)c * nblk * 2 + 1, nblk, 2, -INFINITY);
-  return f16_exp(fmax(hi - (double)mu, nlo + (double)mu));
+  return split_exp(fmax(hi - (double)mu, nlo + (double)mu), top);
 }
 
 // Row of piece p of column c in a tensor-core operand whose pieces are kp rows apart.
@@ -348,7 +355,7 @@ __device__ __forceinline__ float column_mean(const double* __restrict__ mparts, 
 }
 
 // F16: the operand is stored as FP16 pieces of (x − μ)·2^e, e from the MEASURE pass's signed
-// extremes (f16_col_exp).  MEASURE also writes xmax[c][blk][2] = {max x, max −x} over the valid
+// extremes (split_col_exp).  MEASURE also writes xmax[c][blk][2] = {max x, max −x} over the valid
 // rows when xmax != nullptr.
 template <int V, bool MEASURE, bool F16 = false>
 __global__ void __launch_bounds__(kRedThreads)
@@ -373,7 +380,7 @@ prologue_indiv_kernel(const float* __restrict__ in, int64_t ld, int64_t n, int64
   if (!MEASURE && (mparts != nullptr || F16)) {
     if (threadIdx.x < 32) {   // warp 0 reduces the column's partials
       const float mu_ = mparts != nullptr ? column_mean(mparts, nblk, c, 1.0 / (double)n) : 0.f;
-      const int e = F16 ? f16_col_exp(xmax, nblk, c, mu_) : 0;
+      const int e = F16 ? split_col_exp(xmax, nblk, c, mu_, kF16Top) : 0;
       if (threadIdx.x == 0) {
         smu = mu_;
         ssc[0] = ldexpf(1.f, e);
@@ -440,7 +447,7 @@ prologue_indiv_kernel(const float* __restrict__ in, int64_t ld, int64_t n, int64
   }
   const double s = block_sum_d(df_value(acc), sh);
   if (threadIdx.x == 0 && red != nullptr) red[(int64_t)c * nblk + blockIdx.x] = s;
-  if (MEASURE && xmax != nullptr) {   // signed extremes [c][blk][2] (f16_col_exp)
+  if (MEASURE && xmax != nullptr) {   // signed extremes [c][blk][2] (split_col_exp)
     const float mx = block_max_f(xhi, shf);
     const float mn = block_max_f(nxlo, shf);
     if (threadIdx.x == 0) {
@@ -469,7 +476,7 @@ __device__ __forceinline__ void gather_D(const float* __restrict__ D, int splits
 }
 
 // Direction-1 finalize (rows = SNPs): val = raw·2^−e1 − gm_j·colsum_c (colsum from the prologue's
-// partials; e1 the FP16 scale of operand column c when xmax1 != nullptr), plus μ·gcorr_j for the
+// partials; e1 the scale of operand column c when xmax1 != nullptr), plus μ·gcorr_j for the
 // mean the prologue removed, times w_j when w != nullptr.  mode 0: out[j,c] = val (j < m).
 // mode 1: val becomes the direction-2 operand (K = SNPs) and red[c][blk] = Σ_j gm_j·stored(val);
 // with V2 != nullptr (FP16 operand) val goes to V2[c][j] in FP32 with its block maxima in xmax2,
@@ -480,7 +487,7 @@ finalize_snp_kernel(const float* __restrict__ D, int splits, int kp1, int64_t m_
                     const float* __restrict__ gm, const float* __restrict__ w, const double* __restrict__ cparts,
                     int nblkc, int mode, float* __restrict__ out, int64_t ldo, int npieces2, int kp2, void* B2,
                     double* __restrict__ red, int nblk, const double* __restrict__ mparts,
-                    const float* __restrict__ gcorr, int64_t n_rows, const double* __restrict__ xmax1,
+                    const float* __restrict__ gcorr, int64_t n_rows, const double* __restrict__ xmax1, int top,
                     float* __restrict__ V2, double* __restrict__ xmax2)
 {
   __shared__ double sh[32];
@@ -497,7 +504,7 @@ finalize_snp_kernel(const float* __restrict__ D, int splits, int kp1, int64_t m_
   block_scalar([&] { return warp_sum_partials(cparts + (int64_t)c * nblkc, nblkc); }, sb, ch, cl);
   if (threadIdx.x < 32) {   // the mean the prologue removed, added back as μ·(pc_j − n·gm_j)
     const float mu_ = mparts != nullptr ? column_mean(mparts, nblkc, c, 1.0 / (double)n_rows) : 0.f;
-    const float isc_ = xmax1 != nullptr ? ldexpf(1.f, -f16_col_exp(xmax1, nblkc, c, mu_)) : 1.f;
+    const float isc_ = xmax1 != nullptr ? ldexpf(1.f, -split_col_exp(xmax1, nblkc, c, mu_, top)) : 1.f;
     if (threadIdx.x == 0) {
       smu = mu_;
       sisc = isc_;
@@ -557,7 +564,7 @@ convert_snp_kernel(const float* __restrict__ V2, int64_t m_pad, int k, int kp2, 
   const int c = blockIdx.y;
   const int64_t j0 = (int64_t)blockIdx.x * kRowsPerBlock, j1 = min64(m_pad, j0 + kRowsPerBlock);
   if (threadIdx.x < 32) {
-    const int e = f16_exp(max_partials(xmax2, nblk, c));
+    const int e = split_exp(max_partials(xmax2, nblk, c), kF16Top);
     if (threadIdx.x == 0) {
       ssc[0] = ldexpf(1.f, e);
       ssc[1] = ldexpf(1.f, -e);
@@ -595,7 +602,7 @@ prologue_snp_kernel(const float* __restrict__ in, int64_t ld, int64_t m, int64_t
   }
   if (F16 && !MEASURE) {
     if (threadIdx.x < 32) {
-      const int e = f16_exp(max_partials(xmax, nblk, c));
+      const int e = split_exp(max_partials(xmax, nblk, c), kF16Top);
       if (threadIdx.x == 0) {
         ssc[0] = ldexpf(1.f, e);
         ssc[1] = ldexpf(1.f, -e);
@@ -634,7 +641,7 @@ __global__ void __launch_bounds__(kRedThreads)
 finalize_indiv_kernel(const float* __restrict__ D, int splits, int kp2, int64_t n_pad, int k,
                       int64_t n, const double* __restrict__ tparts, int nblkt, const float* __restrict__ rr,
                       const float* __restrict__ Vin, int64_t ld_v, float tau0, int nq, float* __restrict__ out,
-                      int64_t ldo, const double* __restrict__ xmax2, const int32_t* __restrict__ map)
+                      int64_t ldo, const double* __restrict__ xmax2, int top, const int32_t* __restrict__ map)
 {
   __shared__ float sb[2];
   __shared__ float sisc;
@@ -642,7 +649,7 @@ finalize_indiv_kernel(const float* __restrict__ D, int splits, int kp2, int64_t 
   float th, tl;
   block_scalar([&] { return warp_sum_partials(tparts + (int64_t)c * nblkt, nblkt); }, sb, th, tl);
   if (threadIdx.x < 32) {
-    const float isc_ = xmax2 != nullptr ? ldexpf(1.f, -f16_exp(max_partials(xmax2, nblkt, c))) : 1.f;
+    const float isc_ = xmax2 != nullptr ? ldexpf(1.f, -split_exp(max_partials(xmax2, nblkt, c), top)) : 1.f;
     if (threadIdx.x == 0) sisc = isc_;
   }
   __syncthreads();
@@ -674,6 +681,196 @@ finalize_indiv_kernel(const float* __restrict__ D, int splits, int kp2, int64_t 
   stv<V>(out + (int64_t)c * ldo + i, val);
 }
 
+// ---- digit operands ---------------------------------------------------------------------------------
+// Writes x[0 … 15] (the rows of one packed word, kidx …) times 2^e = scale as digits into rows p·kp + c, in
+// the counts' decoded order, and adds exactly what the products will see, in the units of x, to
+// acc (weighted by wt when kWeighted).  Every step is exact.
+template <bool kWeighted>
+__device__ __forceinline__ void store_digit_operand(const float (&x)[16], int ndig, uint8_t* __restrict__ B,
+                                                    int64_t K_pad, int kp, int c, int64_t kidx, DF& acc,
+                                                    const float (&wt)[16], float scale, float inv_scale)
+{
+  float r[16];
+#pragma unroll
+  for (int u = 0; u < 16; ++u) r[u] = __fmul_rn(x[u], scale);
+  float last = 1.f;   // 32^−ndig
+#pragma unroll 1
+  for (int p = 0; p < ndig; ++p) {
+    float d[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) {
+      d[u] = rintf(r[u]);
+      r[u] = __fmul_rn(__fsub_rn(r[u], d[u]), 32.f);
+    }
+    *reinterpret_cast<uint4*>(B + piece_row(p, kp, c) * K_pad + kidx) = e4m3_word(d);
+    last *= 0.03125f;
+  }
+  const float back = -last * inv_scale;
+#pragma unroll
+  for (int u = 0; u < 16; ++u) {   // what is stored: x less the digits' remainder
+    if (kWeighted) {
+      df_fma(acc, wt[u], x[u]);
+      df_fma(acc, wt[u], __fmul_rn(r[u], back));
+    } else {
+      df_add(acc, x[u]);
+      df_add(acc, __fmul_rn(r[u], back));
+    }
+  }
+}
+
+// Zeroes operand padding row `row` over the K-elements of this thread's word.
+__device__ __forceinline__ void zero_digit_row(uint8_t* __restrict__ B, int64_t K_pad, int row, int64_t kidx)
+{
+  *reinterpret_cast<uint4*>(B + (int64_t)row * K_pad + kidx) = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// 16 values p[0 … 15] of rows i … i + 15, 0 from row n on; VEC: 16-byte loads (n % 4 == 0)
+template <bool VEC>
+__device__ __forceinline__ void load16(const float* __restrict__ p, int64_t i, int64_t n, float (&x)[16])
+{
+#pragma unroll
+  for (int u = 0; u < 16; u += 4) {
+    if constexpr (VEC) {
+      float t[4] = {};
+      if (i + u < n) ldv<4>(p + u, t);
+      x[u] = t[0], x[u + 1] = t[1], x[u + 2] = t[2], x[u + 3] = t[3];
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) x[u + q] = i + u + q < n ? p[u + q] : 0.f;
+    }
+  }
+}
+
+// proj_dot of the 16 rows i … i + 15 (Q is zero-padded to a multiple of 256 rows): 16-byte loads, the
+// same arithmetic for each row.
+__device__ __forceinline__ void proj_dot16(const float* __restrict__ Q, int64_t ldq, int cq, int64_t i,
+                                           const float2* qt, float (&out)[16])
+{
+  DF a[16];
+  for (int l = 0; l < cq; ++l) {
+    const float2 t = qt[l];
+#pragma unroll
+    for (int u = 0; u < 16; u += 4) {
+      float q[4];
+      ldv<4>(Q + (int64_t)l * ldq + i + u, q);
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        df_fma(a[u + w], q[w], t.x);
+        a[u + w].lo = __fmaf_rn(q[w], t.y, a[u + w].lo);
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 16; ++u) out[u] = __fadd_rn(a[u].hi, a[u].lo);
+}
+
+// prologue_indiv_kernel's store pass with digits: the same values in the same order of operations.  One
+// packed word of 16 individuals per thread: a word's digits are 16 contiguous bytes of each operand
+// row, where four individuals' would be single bytes.
+template <bool VEC>
+__global__ void __launch_bounds__(kRedThreads)
+prologue_indiv_digits_kernel(const float* __restrict__ in, int64_t ld, int64_t n, int64_t n_pad, int k, int kp,
+                             const float* __restrict__ Q, int64_t ldq, int cq, const double* __restrict__ qparts,
+                             int nblkq, int nq, const float* __restrict__ rr, int ndig, uint8_t* __restrict__ B,
+                             double* __restrict__ red, int nblk, const double* __restrict__ mparts,
+                             const double* __restrict__ xrange, const int32_t* __restrict__ inv)
+{
+  __shared__ double sh[32];
+  __shared__ float2 qt[SLEMM_MAX_COVARIATES];
+  __shared__ float smu, ssc[2];
+  const int c = blockIdx.y;
+  const int64_t i = ((int64_t)blockIdx.x * kRedThreads + threadIdx.x) * 16;   // kRowsPerBlock rows per block
+  if (c >= k) {
+    if (i < n_pad) zero_digit_row(B, n_pad, pad_row(c - k, k, kp, ndig), i);
+    return;
+  }
+  const bool proj = qparts != nullptr && c < nq;
+  if (proj) load_qt(qparts, nblkq, cq, nq, c, qt);
+  if (threadIdx.x < 32) {
+    const float mu_ = mparts != nullptr ? column_mean(mparts, nblk, c, 1.0 / (double)n) : 0.f;
+    const int e = split_col_exp(xrange, nblk, c, mu_, kDigitTop);
+    if (threadIdx.x == 0) {
+      smu = mu_;
+      ssc[0] = ldexpf(1.f, e);
+      ssc[1] = ldexpf(1.f, -e);
+    }
+  }
+  __syncthreads();
+  const float mu = smu;
+  DF acc;
+  if (i < n_pad) {
+    float x[16];
+    if (inv != nullptr) {
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        const int64_t rv = inv[i + u];
+        x[u] = 0.f;
+        if (rv >= 0) {
+          x[u] = in[(int64_t)c * ld + rv];
+          if (proj) x[u] = __fsub_rn(x[u], proj_dot(Q, ldq, cq, rv, qt));
+          if (rr) x[u] = __fmul_rn(x[u], rr[rv]);
+          x[u] = __fsub_rn(x[u], mu);
+        }
+      }
+    } else {
+      load16<VEC>(in + (int64_t)c * ld + i, i, n, x);
+      if (proj) {
+        float pd[16];
+        proj_dot16(Q, ldq, cq, i, qt, pd);
+#pragma unroll
+        for (int u = 0; u < 16; ++u) x[u] = __fsub_rn(x[u], pd[u]);
+      }
+      if (rr) {
+        float r[16];
+        load16<true>(rr + i, i, n_pad, r);   // rr is zero-padded to n_pad
+#pragma unroll
+        for (int u = 0; u < 16; ++u) x[u] = __fmul_rn(x[u], r[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < 16; ++u) x[u] = i + u < n ? __fsub_rn(x[u], mu) : 0.f;
+    }
+    const float none[16] = {};
+    store_digit_operand<false>(x, ndig, B, n_pad, kp, c, i, acc, none, ssc[0], ssc[1]);
+  }
+  const double s = block_sum_d(df_value(acc), sh);
+  if (threadIdx.x == 0) red[(int64_t)c * nblk + blockIdx.x] = s;
+}
+
+// Direction-2 operand as digits from FP32 values `in` (rows j < m, column stride ld) with block maxima
+// xmax, and red[c][blk] = Σ_j gm_j·stored; blocks with c ≥ k zero the padding rows.
+template <bool VEC>
+__global__ void __launch_bounds__(kRedThreads)
+snp_digits_kernel(const float* __restrict__ in, int64_t ld, int64_t m, int64_t m_pad, int k, int kp,
+                  const float* __restrict__ gm, int ndig, uint8_t* __restrict__ B, double* __restrict__ red, int nblk,
+                  const double* __restrict__ xmax)
+{
+  __shared__ double sh[32];
+  __shared__ float ssc[2];
+  const int c = blockIdx.y;
+  const int64_t j = ((int64_t)blockIdx.x * kRedThreads + threadIdx.x) * 16;
+  if (c >= k) {
+    if (j < m_pad) zero_digit_row(B, m_pad, pad_row(c - k, k, kp, ndig), j);
+    return;
+  }
+  if (threadIdx.x < 32) {
+    const int e = split_exp(max_partials(xmax, nblk, c), kDigitTop);
+    if (threadIdx.x == 0) {
+      ssc[0] = ldexpf(1.f, e);
+      ssc[1] = ldexpf(1.f, -e);
+    }
+  }
+  __syncthreads();
+  DF acc;
+  if (j < m_pad) {
+    float x[16], g[16];
+    load16<VEC>(in + (int64_t)c * ld + j, j, m, x);
+    load16<true>(gm + j, j, m_pad, g);   // gm is zero-padded to m_pad
+    store_digit_operand<true>(x, ndig, B, m_pad, kp, c, j, acc, g, ssc[0], ssc[1]);
+  }
+  const double s = block_sum_d(df_value(acc), sh);
+  if (threadIdx.x == 0) red[(int64_t)c * nblk + blockIdx.x] = s;
+}
+
 // ---- one packed pass ---------------------------------------------------------------------------------
 struct PassPlan {
   bool tc;
@@ -683,7 +880,17 @@ struct PassPlan {
   int N;        // columns of the product
   int splits;
   int plan = 0; // tensor-core ring plan (GemmArgs::plan)
+  bool digits() const { return plan == 2; }   // the operand is 8-bit digits (f16 then: digits or FP16 pieces)
+  size_t operand_bytes(int64_t K_pad, int k) const
+  {
+    return tc ? (size_t)N * K_pad * (digits() ? 1 : 2) : (size_t)k * K_pad * 4;
+  }
 };
+
+// Columns up to which FP16X2 passes take digits.  Five digits of k columns are an N = 5·kp E4M3 MMA per
+// 32 K-elements against two N = 2·kp FP16 ones; below N = 96 an MMA costs the same 48 cycles.
+constexpr int kDigitCols = 32;
+constexpr int kDigits = 5;
 
 // Fewest splits of a tensor-core pass.  Once the dense operand (K_pad·N BF16) is larger than half
 // the L2, CTAs with long K ranges run slower per K-tile — co-running CTAs drift apart along K and
@@ -738,12 +945,13 @@ static void near_splits(int rule, int64_t ctas, int per_sm, int64_t K_tiles, int
   for (size_t i = 0; i < near.size() && i + 1 < most; ++i) cand.push_back({plan, near[i].second});
 }
 
-// Tunes p.splits and p.plan in place.
-static void tune_pass(slemm_geno* g, PassPlan& p, const uint8_t* A, int64_t M_pad, int64_t K_pad)
+// Tunes p.splits and p.plan in place (a digit plan among its split counts alone: its operand is another);
+// returns the chosen plan's milliseconds per launch, 0 when nothing was timed.
+static double tune_pass(slemm_geno* g, PassPlan& p, const uint8_t* A, int64_t M_pad, int64_t K_pad)
 {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   CUDA_TRY(cudaStreamIsCapturing(g->stream, &cs));
-  if (cs != cudaStreamCaptureStatusNone) return;
+  if (cs != cudaStreamCaptureStatusNone) return 0.0;
   const int64_t K_tiles = K_pad / kTileK;
   const TuneKey key{g->device, p.N, p.pieces, K_tiles, M_pad};
   {
@@ -752,14 +960,14 @@ static void tune_pass(slemm_geno* g, PassPlan& p, const uint8_t* A, int64_t M_pa
     if (it != g_tune.end()) {
       p.splits = it->second.best;
       p.plan = it->second.plan;
-      return;
+      return it->second.ms_best;
     }
   }
   // candidates: the rule's count, then counts near it with a well-filled last wave; for N ≤ 64 the
   // same around the two-CTAs-per-SM plan's rule
   std::vector<std::pair<int, int>> cand;   // (plan, splits)
-  near_splits(p.splits, M_pad / gemm_tc_rows_per_cta(p.N, 0), 1, K_tiles, 0, 6, cand);
-  if (p.N <= 64) {
+  near_splits(p.splits, M_pad / gemm_tc_rows_per_cta(p.N, p.plan), 1, K_tiles, p.plan, 6, cand);
+  if (p.N <= 64 && !p.digits()) {
     const int64_t ctas1 = M_pad / gemm_tc_rows_per_cta(p.N, 1);
     const int rule1 = choose_splits(ctas1, K_tiles, 2, num_sms(), tc_min_splits(K_tiles, p.N));
     near_splits(rule1, ctas1, 2, K_tiles, 1, 3, cand);
@@ -794,6 +1002,7 @@ static void tune_pass(slemm_geno* g, PassPlan& p, const uint8_t* A, int64_t M_pa
   g_tune[key] = {p.splits, cand[b].second, cand[b].first, (int)cand.size(), ms[0], ms[b]};
   p.plan = cand[b].first;
   p.splits = cand[b].second;
+  return ms[b];
 }
 
 static PassPlan plan_pass(slemm_geno* g, int k, int64_t M_pad, int64_t K_pad, const uint8_t* A)
@@ -805,15 +1014,28 @@ static PassPlan plan_pass(slemm_geno* g, int k, int64_t M_pad, int64_t K_pad, co
   p.kp = p.tc ? (int)round_up(k, 8) : k;
   p.N = p.tc ? (int)round_up((int64_t)p.pieces * p.kp, 16) : k;
   const int64_t M_tiles = M_pad / kTileM, K_tiles = K_pad / kTileK;
-  p.splits = p.tc ? choose_splits(M_pad / gemm_tc_rows_per_cta(p.N, 0), K_tiles, 1, num_sms(),
-                                  tc_min_splits(K_tiles, p.N))
-                  : choose_splits(M_tiles, K_tiles, 8, num_sms());
-  if (p.tc && g->autotune == 2 && p.N <= 64) {
-    p.plan = 1;
-    p.splits = choose_splits(M_pad / gemm_tc_rows_per_cta(p.N, 1), K_tiles, 2, num_sms(),
-                             tc_min_splits(K_tiles, p.N));
+  auto rule = [&](const PassPlan& q, int per_sm) {
+    return choose_splits(M_pad / gemm_tc_rows_per_cta(q.N, q.plan), K_tiles, per_sm, num_sms(),
+                         tc_min_splits(K_tiles, q.N));
+  };
+  if (!p.tc) {
+    p.splits = choose_splits(M_tiles, K_tiles, 8, num_sms());
+    return p;
   }
-  if (p.tc && g->autotune == 1 && A) tune_pass(g, p, A, M_pad, K_pad);
+  if (g->autotune == 2 && p.N <= 64) p.plan = 1;
+  p.splits = rule(p, p.plan == 1 ? 2 : 1);
+  const bool tune = g->autotune == 1 && A;
+  double ms = 0.0, ms8 = 0.0;
+  if (tune) ms = tune_pass(g, p, A, M_pad, K_pad);
+  if (p.f16 && k <= kDigitCols && p.plan != 1) {
+    PassPlan d = p;
+    d.plan = 2;
+    d.pieces = kDigits;
+    d.N = (int)round_up((int64_t)kDigits * d.kp, 16);
+    d.splits = rule(d, 1);
+    if (tune) ms8 = tune_pass(g, d, A, M_pad, K_pad);
+    if (!(ms > 0.0 && ms8 > ms)) p = d;
+  }
   return p;
 }
 
@@ -899,8 +1121,9 @@ static void op_group(slemm_geno* g, int kind, float tau0, const float* in, int64
   const int pad1 = p1.tc ? p1.N - p1.pieces * k : 0;                   // padding rows of the operands
   const int pad2 = p2.tc ? p2.N - p2.pieces * k : 0;
   const bool f16 = p1.f16;
-  const size_t b1 = dir1 ? (p1.tc ? (size_t)p1.N * g->n_pad * 2 : (size_t)k * g->n_pad * 4) : 0;
-  const size_t b2 = dir2 ? (p2.tc ? (size_t)p2.N * g->m_pad * 2 : (size_t)k * g->m_pad * 4) : 0;
+  const size_t b1 = dir1 ? p1.operand_bytes(g->n_pad, k) : 0;
+  const size_t b2 = dir2 ? p2.operand_bytes(g->m_pad, k) : 0;
+  const int top1 = p1.digits() ? kDigitTop : kF16Top, top2 = p2.digits() ? kDigitTop : kF16Top;
   // FP16: the direction-2 values in FP32 before they are scaled and split
   const size_t bv2 = (dir1 && dir2 && f16) ? (size_t)k * g->m_pad * 4 : 0;
   uint8_t* Bbuf = (uint8_t*)g->ws_B.ensure(b1 + b2 + bv2);
@@ -957,7 +1180,16 @@ static void op_group(slemm_geno* g, int kind, float tau0, const float* in, int64
             x_max1, inv_ind);
       LAUNCH_CHECK();
     }
-    if (f16) {
+    if (p1.digits()) {
+      if (vin)
+        prologue_indiv_digits_kernel<true><<<grid, kRedThreads, 0, st>>>(
+            in, ld_in, g->n, g->n_pad, k, p1.kp, Qp, g->n_pad, cq, qp, nblk_q, nq, rr, np1, (uint8_t*)B1, r_col, nblk_n,
+            mu, x_max1, inv_ind);
+      else
+        prologue_indiv_digits_kernel<false><<<grid, kRedThreads, 0, st>>>(
+            in, ld_in, g->n, g->n_pad, k, p1.kp, Qp, g->n_pad, cq, qp, nblk_q, nq, rr, np1, (uint8_t*)B1, r_col, nblk_n,
+            mu, x_max1, inv_ind);
+    } else if (f16) {
       if (vin)
         prologue_indiv_kernel<4, false, true><<<grid, kRedThreads, 0, st>>>(
             in, ld_in, g->n, g->n_pad, k, p1.kp, Qp, g->n_pad, cq, qp, nblk_q, nq, rr, np1, B1, r_col, nblk_n, mu,
@@ -982,11 +1214,15 @@ static void op_group(slemm_geno* g, int kind, float tau0, const float* in, int64
     // ---- finalize 1 ----
     const float* wsc = (kind == SLEMM_OP_RMATVEC) ? nullptr : g->w.as<float>();
     if (h0) {
-      finalize_snp_kernel<4><<<dim3(nblk_m, k + pad2), kRedThreads, 0, st>>>(
+      finalize_snp_kernel<4><<<dim3(nblk_m, k + (p2.digits() ? 0 : pad2)), kRedThreads, 0, st>>>(
           D, p1.splits, p1.kp, g->m_pad, k, g->m, g->gm.as<float>(), wsc, r_col, nblk_n, 1, nullptr, 0, np2, p2.kp,
-          B2, r_t, nblk_m, mu, g->gcorr.as<float>(), g->n, x_max1, V2, x_max2);
+          B2, r_t, nblk_m, mu, g->gcorr.as<float>(), g->n, x_max1, top1, V2, x_max2);
       LAUNCH_CHECK();
-      if (f16) {
+      if (p2.digits()) {
+        snp_digits_kernel<true><<<dim3(nblk_m, k + pad2), kRedThreads, 0, st>>>(
+            V2, g->m_pad, g->m_pad, g->m_pad, k, p2.kp, g->gm.as<float>(), np2, (uint8_t*)B2, r_t, nblk_m, x_max2);
+        LAUNCH_CHECK();
+      } else if (f16) {
         convert_snp_kernel<4><<<dim3(nblk_m, k), kRedThreads, 0, st>>>(V2, g->m_pad, k, p2.kp, g->gm.as<float>(),
                                                                         np2, B2, r_t, nblk_m, x_max2);
         LAUNCH_CHECK();
@@ -995,11 +1231,11 @@ static void op_group(slemm_geno* g, int kind, float tau0, const float* in, int64
       if (vec4_ok(g->m, ld_out, out))
         finalize_snp_kernel<4><<<dim3(nblk_m, k), kRedThreads, 0, st>>>(
             D, p1.splits, p1.kp, g->m_pad, k, g->m, g->gm.as<float>(), wsc, r_col, nblk_n, 0, out, ld_out, 0, 8,
-            nullptr, nullptr, 0, mu, g->gcorr.as<float>(), g->n, x_max1, nullptr, nullptr);
+            nullptr, nullptr, 0, mu, g->gcorr.as<float>(), g->n, x_max1, top1, nullptr, nullptr);
       else
         finalize_snp_kernel<1><<<dim3(nblk_m, k), kRedThreads, 0, st>>>(
             D, p1.splits, p1.kp, g->m_pad, k, g->m, g->gm.as<float>(), wsc, r_col, nblk_n, 0, out, ld_out, 0, 8,
-            nullptr, nullptr, 0, mu, g->gcorr.as<float>(), g->n, x_max1, nullptr, nullptr);
+            nullptr, nullptr, 0, mu, g->gcorr.as<float>(), g->n, x_max1, top1, nullptr, nullptr);
       LAUNCH_CHECK();
       return;
     }
@@ -1012,14 +1248,20 @@ static void op_group(slemm_geno* g, int kind, float tau0, const float* in, int64
         prologue_snp_kernel<4, true, true><<<dim3(nblk_m, k), kRedThreads, 0, st>>>(
             in, ld_in, g->m, g->m_pad, k, p2.kp, g->gm.as<float>(), np2, B2, r_t, nblk_m, x_max2);
         LAUNCH_CHECK();
-        prologue_snp_kernel<4, false, true><<<gridm, kRedThreads, 0, st>>>(in, ld_in, g->m, g->m_pad, k, p2.kp,
+        if (p2.digits())
+          snp_digits_kernel<true><<<gridm, kRedThreads, 0, st>>>(in, ld_in, g->m, g->m_pad, k, p2.kp, g->gm.as<float>(),
+                                                                 np2, (uint8_t*)B2, r_t, nblk_m, x_max2);
+        else prologue_snp_kernel<4, false, true><<<gridm, kRedThreads, 0, st>>>(in, ld_in, g->m, g->m_pad, k, p2.kp,
                                                                            g->gm.as<float>(), np2, B2, r_t, nblk_m,
                                                                            x_max2);
       } else {
         prologue_snp_kernel<1, true, true><<<dim3(nblk_m, k), kRedThreads, 0, st>>>(
             in, ld_in, g->m, g->m_pad, k, p2.kp, g->gm.as<float>(), np2, B2, r_t, nblk_m, x_max2);
         LAUNCH_CHECK();
-        prologue_snp_kernel<1, false, true><<<gridm, kRedThreads, 0, st>>>(in, ld_in, g->m, g->m_pad, k, p2.kp,
+        if (p2.digits())
+          snp_digits_kernel<false><<<gridm, kRedThreads, 0, st>>>(in, ld_in, g->m, g->m_pad, k, p2.kp, g->gm.as<float>(),
+                                                                  np2, (uint8_t*)B2, r_t, nblk_m, x_max2);
+        else prologue_snp_kernel<1, false, true><<<gridm, kRedThreads, 0, st>>>(in, ld_in, g->m, g->m_pad, k, p2.kp,
                                                                            g->gm.as<float>(), np2, B2, r_t, nblk_m,
                                                                            x_max2);
       }
@@ -1043,11 +1285,11 @@ static void op_group(slemm_geno* g, int kind, float tau0, const float* in, int64
   if (vec4_ok(g->n, ld_out, out) && (!v2 || vin)) {
     dim3 grid((unsigned)ceil_div(g->n, 4 * kRedThreads), k);
     finalize_indiv_kernel<4><<<grid, kRedThreads, 0, st>>>(D, p2.splits, p2.kp, g->n_pad, k, g->n, r_t, nblk_m, rr2,
-                                                           v2, ld_in, tau0, nq2, out, ld_out, x_max2, map_ind);
+                                                           v2, ld_in, tau0, nq2, out, ld_out, x_max2, top2, map_ind);
   } else {
     dim3 grid((unsigned)ceil_div(g->n, kRedThreads), k);
     finalize_indiv_kernel<1><<<grid, kRedThreads, 0, st>>>(D, p2.splits, p2.kp, g->n_pad, k, g->n, r_t, nblk_m, rr2,
-                                                           v2, ld_in, tau0, nq2, out, ld_out, x_max2, map_ind);
+                                                           v2, ld_in, tau0, nq2, out, ld_out, x_max2, top2, map_ind);
   }
   LAUNCH_CHECK();
   // quadform columns 0 … nq−1: out = T + τ0 v − QQᵀT
@@ -1136,11 +1378,11 @@ void rows_product(slemm_geno* g, int64_t r0, int64_t rows, const float* U, int64
     if (vec4_ok(m_valid, ldo, o))
       finalize_snp_kernel<4><<<dim3(nblk_m, kc), kRedThreads, 0, st>>>(
           D, p.splits, p.kp, rows, kc, m_valid, g->gm.as<float>() + r0, nullptr, r_col, nblk_n, 0, o, ldo, 0, 8,
-          nullptr, nullptr, 0, mu, mu ? g->gcorr.as<float>() + r0 : nullptr, g->n, x_rng, nullptr, nullptr);
+          nullptr, nullptr, 0, mu, mu ? g->gcorr.as<float>() + r0 : nullptr, g->n, x_rng, kF16Top, nullptr, nullptr);
     else
       finalize_snp_kernel<1><<<dim3(nblk_m, kc), kRedThreads, 0, st>>>(
           D, p.splits, p.kp, rows, kc, m_valid, g->gm.as<float>() + r0, nullptr, r_col, nblk_n, 0, o, ldo, 0, 8,
-          nullptr, nullptr, 0, mu, mu ? g->gcorr.as<float>() + r0 : nullptr, g->n, x_rng, nullptr, nullptr);
+          nullptr, nullptr, 0, mu, mu ? g->gcorr.as<float>() + r0 : nullptr, g->n, x_rng, kF16Top, nullptr, nullptr);
     LAUNCH_CHECK();
   }
 }
