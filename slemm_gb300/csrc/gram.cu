@@ -6,11 +6,12 @@
 // h and t come from one exact pass over the packed matrix (gram_stats), so a Gram block is one
 // packed product of SNP rows with columns that are read straight from the packed rows, and no
 // dense FP32 column of n individuals is ever formed.  In general the columns are rr²∘z_k,
-// column-scaled FP16 hi+lo; with every rr 1 they are the counts themselves, one FP16 piece whose
+// column-scaled FP16 hi+lo; with every rr 1 they are the counts themselves, one E4M3 byte each, whose
 // product is an exact integer, and Σ_i x_ij·z_ik = Σ_i x_ij·x_ik − p_j·gm_k with p_j = Σ_i x_ij.  Forming U = rr∘P(rr∘z) as FP32
 // columns instead (centre, project, scale, measure, split: nine passes over n × columns floats)
 // took 38 of the 82 ms of slemm_gwa at n = 50,021 with 20,011 variants and 4,000 model SNPs, and
-// 31 of the 73 ms of --lmm with 30 windows of 1,000 SNPs at n = 50,000.
+// 31 of the 73 ms of --lmm with 30 windows of 1,000 SNPs at n = 50,000; the two calls now take 5.8
+// and 8.1 ms (7.3 and 9.5 with the counts as FP16).
 #include "gram.h"
 #include "decode.cuh"
 #include "reduce.cuh"
@@ -94,11 +95,38 @@ void gram_stats_gather(const GramStats& src, const int64_t* d_idx, int64_t cnt, 
 
 // ---- Gram blocks ----------------------------------------------------------------------------------
 // Operand of the columns SNP j0 … j0 + ncols − 1, group by group: column c is row c % kc of group
-// c / kc, a group's rows kc … kp − 1 are zero.  UNIT: N = kp rows of counts per group.  Otherwise
-// N = 2·kp rows, pieces hi and lo of rr²·z·2^e.  Each value is stored times the 2^−2s of its K position
-// (f16sub_pair_of).  A thread writes 8 K-elements (half of a packed word): 16-byte stores, 512
+// c / kc, a group's rows kc … kp − 1 are zero.
+//
+// Every rr 1: N = kp rows of counts as E4M3 bytes in the decoded order of the matrix's own words
+// (decode.cuh), so the product takes one MMA per 32 individuals and its sums are exact integers.  One
+// word (16 individuals) per thread; a count x ∈ {0, 1, 2} in a byte is x·0x38 − [x = 2]·0x30 (E4M3 0, 1,
+// 2), or x·0x28 − [x = 2]·0x20 times 2^−2, four at a time.  Bound by the bytes it writes.
+__global__ void __launch_bounds__(256)
+gram_counts_kernel(const uint32_t* __restrict__ G, int64_t K_tiles, int64_t j0, int64_t ncols, int kc, int kp,
+                   uint8_t* __restrict__ B)
+{
+  const int64_t q = (int64_t)blockIdx.x * 256 + threadIdx.x;   // word of the row
+  if (q >= K_tiles * 4) return;
+  const int grp = blockIdx.z, r = blockIdx.y;
+  const int64_t c = (int64_t)grp * kc + r;
+  uint4 o = make_uint4(0u, 0u, 0u, 0u);
+  if (r < kc && c < ncols) {
+    const int64_t j = j0 + c;
+    const uint32_t w = G[((j / 128 * K_tiles + (q >> 2)) * 128 + j % 128) * 4 + (q & 3)];
+    uint32_t v[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const uint32_t x = (w >> (2 * p)) & 0x03030303u, two = (x >> 1) & 0x01010101u;
+      v[p] = (p & 1) ? x * 0x28u - two * 0x20u : x * 0x38u - two * 0x30u;
+    }
+    o = make_uint4(v[0], v[1], v[2], v[3]);
+  }
+  *reinterpret_cast<uint4*>(B + ((int64_t)grp * kp + r) * K_tiles * kTileK + q * 16) = o;
+}
+
+// With residual weights: N = 2·kp rows, FP16 pieces hi and lo of rr²·z·2^e, each times the 2^−2s of its K
+// position (f16sub_pair_of).  A thread writes 8 K-elements (half of a packed word): 16-byte stores, 512
 // contiguous bytes per warp.  Bound by the 16-bit operand it writes.
-template <bool UNIT>
 __global__ void __launch_bounds__(256)
 gram_operand_kernel(const uint32_t* __restrict__ G, int64_t K_tiles, int64_t j0, int64_t ncols, int kc, int kp,
                     const float* __restrict__ gm, const float* __restrict__ rr, float scale, __half* __restrict__ B)
@@ -107,8 +135,7 @@ gram_operand_kernel(const uint32_t* __restrict__ G, int64_t K_tiles, int64_t j0,
   const int64_t K_pad = K_tiles * kTileK;
   if (q8 * 8 >= K_pad) return;
   const int grp = blockIdx.z, r = blockIdx.y;
-  const int N = UNIT ? kp : 2 * kp;
-  __half* dst = B + ((int64_t)grp * N + r) * K_pad + q8 * 8;
+  __half* dst = B + ((int64_t)grp * 2 * kp + r) * K_pad + q8 * 8;
   const int64_t c = (int64_t)grp * kc + r;
   uint4 hi = make_uint4(0u, 0u, 0u, 0u), lo = hi;
   if (r < kc && c < ncols) {
@@ -116,43 +143,35 @@ gram_operand_kernel(const uint32_t* __restrict__ G, int64_t K_tiles, int64_t j0,
     const int w = (int)(q8 & 7) >> 1, h = (int)(q8 & 1);
     const uint32_t word = G[((j / 128 * K_tiles + kt) * 128 + j % 128) * 4 + w];
     float zv[3], rv[8];
-    if constexpr (!UNIT) {
-      const float g = gm[j];
+    const float g = gm[j];
 #pragma unroll
-      for (int x = 0; x < 3; ++x) zv[x] = __fsub_rn((float)x, g);
-      const float4 r0 = *reinterpret_cast<const float4*>(rr + q8 * 8);
-      const float4 r1 = *reinterpret_cast<const float4*>(rr + q8 * 8 + 4);
-      rv[0] = r0.x, rv[1] = r0.y, rv[2] = r0.z, rv[3] = r0.w;
-      rv[4] = r1.x, rv[5] = r1.y, rv[6] = r1.z, rv[7] = r1.w;
-    }
+    for (int x = 0; x < 3; ++x) zv[x] = __fsub_rn((float)x, g);
+    const float4 r0 = *reinterpret_cast<const float4*>(rr + q8 * 8);
+    const float4 r1 = *reinterpret_cast<const float4*>(rr + q8 * 8 + 4);
+    rv[0] = r0.x, rv[1] = r0.y, rv[2] = r0.z, rv[3] = r0.w;
+    rv[4] = r1.x, rv[5] = r1.y, rv[6] = r1.z, rv[7] = r1.w;
     uint32_t ph[4], pl[4];
 #pragma unroll
     for (int p = 0; p < 4; ++p) {   // element pair q = 4h + p of the word
       const int q = 4 * h + p, s = f16sub_shift(q);
       const uint32_t xe = (word >> (2 * q)) & 3u, xo = (word >> (16 + 2 * q)) & 3u;
-      if constexpr (UNIT) {
-        // x·2^−2s in FP16: exponent field 14 + x − 2s (x = 1, 2), or zero
-        const uint32_t be = xe ? (14u + xe - 2u * s) << 10 : 0u, bo = xo ? (14u + xo - 2u * s) << 10 : 0u;
-        ph[p] = be | (bo << 16);
-      } else {
-        const float ks = __uint_as_float((uint32_t)(127 - 2 * s) << 23);
-        const float ve = __fmul_rn(__fmul_rn(__fmul_rn(rv[2 * p], rv[2 * p]), xe == 0 ? zv[0] : xe == 1 ? zv[1] : zv[2]),
-                                   scale);
-        const float vo = __fmul_rn(__fmul_rn(__fmul_rn(rv[2 * p + 1], rv[2 * p + 1]),
-                                             xo == 0 ? zv[0] : xo == 1 ? zv[1] : zv[2]),
-                                   scale);
-        const float he = rintf(ve), ho = rintf(vo);
-        ph[p] = (uint32_t)__half_as_ushort(__float2half_rn(__fmul_rn(he, ks))) |
-                ((uint32_t)__half_as_ushort(__float2half_rn(__fmul_rn(ho, ks))) << 16);
-        pl[p] = (uint32_t)__half_as_ushort(__float2half_rn(__fmul_rn(__fsub_rn(ve, he), ks))) |
-                ((uint32_t)__half_as_ushort(__float2half_rn(__fmul_rn(__fsub_rn(vo, ho), ks))) << 16);
-      }
+      const float ks = __uint_as_float((uint32_t)(127 - 2 * s) << 23);
+      const float ve = __fmul_rn(__fmul_rn(__fmul_rn(rv[2 * p], rv[2 * p]), xe == 0 ? zv[0] : xe == 1 ? zv[1] : zv[2]),
+                                 scale);
+      const float vo = __fmul_rn(__fmul_rn(__fmul_rn(rv[2 * p + 1], rv[2 * p + 1]),
+                                           xo == 0 ? zv[0] : xo == 1 ? zv[1] : zv[2]),
+                                 scale);
+      const float he = rintf(ve), ho = rintf(vo);
+      ph[p] = (uint32_t)__half_as_ushort(__float2half_rn(__fmul_rn(he, ks))) |
+              ((uint32_t)__half_as_ushort(__float2half_rn(__fmul_rn(ho, ks))) << 16);
+      pl[p] = (uint32_t)__half_as_ushort(__float2half_rn(__fmul_rn(__fsub_rn(ve, he), ks))) |
+              ((uint32_t)__half_as_ushort(__float2half_rn(__fmul_rn(__fsub_rn(vo, ho), ks))) << 16);
     }
     hi = make_uint4(ph[0], ph[1], ph[2], ph[3]);
-    if constexpr (!UNIT) lo = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+    lo = make_uint4(pl[0], pl[1], pl[2], pl[3]);
   }
   *reinterpret_cast<uint4*>(dst) = hi;
-  if constexpr (!UNIT) *reinterpret_cast<uint4*>(dst + (int64_t)kp * K_pad) = lo;
+  *reinterpret_cast<uint4*>(dst + (int64_t)kp * K_pad) = lo;
 }
 
 // out[c·ldo + i] = Σ_splits D·isc − gm_row·h_c − p_row·gm_c − t_rowᵀt_c for product row i (SNP r0 + i)
@@ -203,7 +222,7 @@ void gram_block(slemm_geno* g, const GramSide& R, int64_t r0, int64_t rows, cons
   cudaStream_t st = g->stream;
   const int64_t K_pad = g->n_pad, K_tiles = K_pad / kTileK;
   const bool unit = rr == nullptr;
-  // |rr²·z| ≤ 2·max rr²: the bound lies in [2^10, 2^11) after scaling (ops.cu, f16_exp)
+  // |rr²·z| ≤ 2·max rr²: the bound lies in [2^10, 2^11) after scaling (ops.cu, split_exp)
   int e = 0;
   if (!unit) {
     int E = 0;
@@ -217,9 +236,11 @@ void gram_block(slemm_geno* g, const GramSide& R, int64_t r0, int64_t rows, cons
   const int kp = (int)round_up(kc, unit ? 16 : 8);
   const int N = unit ? kp : 2 * kp;
   // as many groups per launch as 256 MB of operand and 512 MB of a split's partials hold (at least one)
-  const int64_t per = std::max<int64_t>(1, std::min({groups, ((int64_t)256 << 20) / ((int64_t)N * K_pad * 2),
+  const int64_t group_bytes = (int64_t)N * K_pad * (unit ? 1 : 2);
+  const int64_t per = std::max<int64_t>(1, std::min({groups, ((int64_t)256 << 20) / group_bytes,
                                                      ((int64_t)512 << 20) / ((int64_t)kp * rows * 4)}));
-  const int64_t rctas = rows / gemm_tc_rows_per_cta(N, 0);
+  const int plan = unit ? 2 : 0;
+  const int64_t rctas = rows / gemm_tc_rows_per_cta(N, plan);
   const int64_t nrows = std::min(rows, R.m - r0);
   const uint8_t* A = R.G + (size_t)(r0 / kTileM) * K_tiles * kTileBytes;
   for (int64_t g0 = 0; g0 < groups; g0 += per) {
@@ -227,17 +248,17 @@ void gram_block(slemm_geno* g, const GramSide& R, int64_t r0, int64_t rows, cons
     const int64_t first = g0 * kc, nc = std::min<int64_t>((int64_t)ng * kc, ncols - first);
     // an integer partial sum of 2^22 elements is at most 2^24: exact in FP32
     const int splits = gram_splits(rctas * ng, K_tiles, ceil_div(K_pad, (int64_t)1 << 22));
-    __half* B = (__half*)g->ws_B.ensure((size_t)ng * N * K_pad * sizeof(__half));
+    void* B = g->ws_B.ensure((size_t)ng * group_bytes);
     float* D = (float*)g->ws_D.ensure((size_t)ng * splits * kp * rows * sizeof(float));
-    const dim3 og((unsigned)ceil_div(K_pad / 8, 256), kp, ng);
     const uint32_t* Gc = reinterpret_cast<const uint32_t*>(C.G);
     if (unit)
-      gram_operand_kernel<true><<<og, 256, 0, st>>>(Gc, K_tiles, c0 + first, nc, kc, kp, nullptr, nullptr, 1.f, B);
+      gram_counts_kernel<<<dim3((unsigned)ceil_div(K_pad / 16, 256), kp, ng), 256, 0, st>>>(Gc, K_tiles, c0 + first, nc,
+                                                                                            kc, kp, (uint8_t*)B);
     else
-      gram_operand_kernel<false><<<og, 256, 0, st>>>(Gc, K_tiles, c0 + first, nc, kc, kp, C.stats.gm, rr,
-                                                     (float)std::ldexp(1.0, e), B);
+      gram_operand_kernel<<<dim3((unsigned)ceil_div(K_pad / 8, 256), kp, ng), 256, 0, st>>>(
+          Gc, K_tiles, c0 + first, nc, kc, kp, C.stats.gm, rr, (float)std::ldexp(1.0, e), (__half*)B);
     LAUNCH_CHECK();
-    GemmArgs a{A, rows, K_pad, B, N, D, splits, g->err.as<int>(), kp, unit ? 1 : 2, true};
+    GemmArgs a{A, rows, K_pad, B, N, D, splits, g->err.as<int>(), kp, unit ? 1 : 2, !unit, plan};
     a.groups = ng;
     gemm_tc(a, st);
     gram_finish_kernel<<<dim3((unsigned)ceil_div(nrows, 256), (unsigned)nc), 256, 0, st>>>(
