@@ -8,7 +8,7 @@
 // accumulators are exact whatever their order.  K is therefore split every 8,192 K-tiles at the
 // latest, the partials are added as 64-bit integers, and only the last combination of the digits
 // rounds (in FP64).  Bound by the narrow tensor-core pass.  GB300's FP64 pipe ran the same sums by an
-// FMA per genotype and column: at n = 100,000, m = 50,000 the GEBV took 18,988 µs and takes 593 µs, the
+// FMA per genotype and column: at n = 100,000, m = 50,000 the GEBV took 18,988 µs and takes 556 µs, the
 // score terms with three covariates and residual weights 112,698 µs and 697 µs, with the same or a
 // smaller error against 64-bit sums.
 #include "internal.h"
@@ -71,10 +71,12 @@ __device__ __forceinline__ double gather_digits(const float* __restrict__ D, int
 }
 
 // GEBV operand: rows 0 … 12 the digits of alpha (0 past m), rows 13 … 15 zero; 16 K-elements per thread
-__global__ void __launch_bounds__(kXThreads)
+// (32 threads a block: the FP64 steps of 16 effects are ~1,300 instructions on a pipe of two lanes per
+// clock and SM, so the blocks spread over all SMs)
+__global__ void __launch_bounds__(32)
 gebv_operand_kernel(const double* __restrict__ alpha, int64_t m, int64_t m_pad, int e, uint8_t* __restrict__ B)
 {
-  const int64_t j = ((int64_t)blockIdx.x * kXThreads + threadIdx.x) * 16;
+  const int64_t j = ((int64_t)blockIdx.x * 32 + threadIdx.x) * 16;
   if (j >= m_pad) return;
   double v[16];
 #pragma unroll
@@ -193,7 +195,7 @@ void exact_gebv(slemm_geno* g, const double* d_alpha, double amax, double shift,
   const int splits = exact_splits(g->n_pad, g->m_pad / kTileK, N);
   uint8_t* B = (uint8_t*)g->ws_B.ensure((size_t)N * g->m_pad);
   float* D = (float*)g->ws_D.ensure((size_t)splits * kp * g->n_pad * sizeof(float));
-  gebv_operand_kernel<<<(unsigned)ceil_div(g->m_pad, 16 * kXThreads), kXThreads, 0, st>>>(d_alpha, g->m, g->m_pad, e, B);
+  gebv_operand_kernel<<<(unsigned)ceil_div(g->m_pad, 16 * 32), 32, 0, st>>>(d_alpha, g->m, g->m_pad, e, B);
   LAUNCH_CHECK();
   gemm_tc({g->GT.as<uint8_t>(), g->n_pad, g->m_pad, B, N, D, splits, g->err.as<int>(), kp, 1, false, 2}, st);
   gebv_finish_kernel<<<(unsigned)ceil_div(g->n, kXThreads), kXThreads, 0, st>>>(D, splits, kp, g->n_pad, g->n, e, shift,
