@@ -91,6 +91,13 @@ __device__ __forceinline__ uint4 e4m3_word(const float (&d)[16])
                     e4m3x4(d[4], d[12], d[5], d[13], 1.f), e4m3x4(d[6], d[14], d[7], d[15], 0.25f));
 }
 
+// The 8 K positions 8h … 8h + 7 of a word: digits of its elements 4h … 4h + 3 (d[0 … 3]) and
+// 8 + 4h … 11 + 4h (d[4 … 7]).
+__device__ __forceinline__ uint2 e4m3_half(const float (&d)[8])
+{
+  return make_uint2(e4m3x4(d[0], d[4], d[1], d[5], 1.f), e4m3x4(d[2], d[6], d[3], d[7], 0.25f));
+}
+
 // Exact FP32 counts of element pair q.
 __device__ __forceinline__ void f32pair_of(uint32_t word, int q, float& even, float& odd)
 {

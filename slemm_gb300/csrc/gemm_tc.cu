@@ -356,6 +356,9 @@ gemm_tc_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMa
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t acol = P.acol();
+  // the set-up above overlaps the end of the kernel that writes B (and reads D)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == 0) {
     // ---------------- packed-tile producer (DRAM) ----------------
@@ -633,8 +636,18 @@ static void launch_tc(const GemmArgs& a, cudaStream_t st)
   // 512 / TM CTAs are resident per SM, so no allocation ever has to wait for another CTA's release.
   const size_t smem = std::max<size_t>(P.total, TM == 512 ? 120 * 1024 : 80 * 1024);
   dim3 grid((unsigned)Mc, (unsigned)a.splits, (unsigned)a.groups);
-  gemm_tc_kernel<PK, S, SB, KT, FMT, TM, TWOS><<<grid, P.threads(), smem, st>>>(
-      a.A, map, a.D, a.M_pad, K_tiles, tps, a.N, P.sub, a.kp, a.pieces, a.err, g_withhold_b.exchange(-1));
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)P.threads());
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_tc_kernel<PK, S, SB, KT, FMT, TM, TWOS>, a.A, map, a.D, a.M_pad, K_tiles, tps,
+                              a.N, P.sub, a.kp, a.pieces, a.err, g_withhold_b.exchange(-1)));
   LAUNCH_CHECK();
 }
 

@@ -91,6 +91,13 @@ void op_device(slemm_geno* g, int kind, float tau0, const float* in, int64_t ld_
 void op_device_mixed(slemm_geno* g, int kind, float tau0, const float* in, int64_t ld_in, int k,
                      float* out, int64_t ld_out, int nq);
 
+// The same operator on U (n×k, ld = n) with the rest of a Lanczos step on its result (lanczos.cu): FP16X2
+// handles only, false (and nothing done) otherwise.  tmp: n×k scratch.  Uprev (nullptr at the first step)
+// and Unext: n×k.  beta[k] (device, hi+lo): β of the step before, replaced by this step's.  scal[c],
+// scal[stride + c], scal[2·stride + c] (host-mapped): δ, ‖·‖², ‖U_next‖²; scal_err: the error word.
+bool op_lanczos_step(slemm_geno* g, int kind, float tau0, const float* U, int k, float* tmp, int nq, const float* Uprev,
+                     float* Unext, float2* beta, double* scal, int stride, double* scal_err);
+
 // Centred Z_cᵀU over SNP rows [r0, r0 + rows) (multiples of 256) on the tensor cores at precision
 // prec (SLEMM_PREC_FP16X2, BF16X2 or BF16X3; ops.cu).
 void rows_product(slemm_geno* g, int64_t r0, int64_t rows, const float* U, int64_t ldu, int k, float* out,

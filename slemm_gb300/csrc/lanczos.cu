@@ -4,10 +4,11 @@
 // ops.cu.  The basis vectors are FP32 in HBM like the reference's std::vector<MatrixXf>; the
 // vector updates run in FP32 (with the FP64 scalars applied as double-float pairs) and every
 // scalar of the three-term recurrence (δ = uᵀAu, β = ‖·‖, the CG coefficients γ, ω, ρ and the
-// residual test) is accumulated to FP64 accuracy (reduce.cuh) and kept in FP64.  One step is
-// three vector kernels whose block partials the next kernel sums itself in a fixed order, and one
-// small kernel that writes the step's scalars into mapped host memory: one synchronisation per
-// step, no copies.
+// residual test) is accumulated to FP64 accuracy (reduce.cuh) and kept in FP64.  At FP16X2 the
+// operator's last kernel finishes the step too (columns.cuh) and writes its scalars into mapped host
+// memory.  Otherwise, and with reorthogonalisation, a step is three vector kernels whose block partials
+// the next kernel sums itself in a fixed order, and one small kernel that writes the scalars: one
+// synchronisation per step, no copies, either way.
 //
 // L_Solve (src/reml.cpp:369-431): the reference rebuilds CG on (A + σI) from the stored basis
 // step by step.  Unrolling its recurrences (P_0 = B, P_j = ρ_j U_j + ω_{j−1} P_{j−1},
@@ -401,19 +402,24 @@ slemm_lseed* lanczos_seed_device(slemm_geno* g, int kind, float tau0, const floa
     const bool v4 = (n % 4) == 0;
     const dim3 gr(nblk, t);
     const int* err = g->err.as<int>();
+    DevBuf betab(st);   // β per column of the fused steps
+    float2* s_beta = (float2*)betab.ensure((size_t)t * sizeof(float2));
     // Waits for the step's scalars of columns lo … t−1 in the mapped buffer (h[c], h[t + c],
     // h[2t + c]) and checks the kernels' error word (h[3t]).
-    auto fetch = [&](const double* dot, int lo) {
-      const size_t offr = (size_t)lo * nblk;
-      lz_final_kernel<<<(unsigned)(t - lo), 96, 0, st>>>(dot ? dot + offr : nullptr, r_nrm + offr, r_un + offr, t,
-                                                        nblk, err, d_out + lo, d_out + 3 * t);
-      LAUNCH_CHECK();
+    auto wait = [&] {
       CUDA_TRY(cudaStreamSynchronize(st));
       if (h[3 * t] != 0.0) {
         CUDA_TRY(cudaMemsetAsync(g->err.p, 0, sizeof(int), st));
         SLEMM_THROW(SLEMM_ERR_CUDA, "a tensor-core kernel gave up a bounded wait (code " +
                                         std::to_string((int)h[3 * t]) + ")");
       }
+    };
+    auto fetch = [&](const double* dot, int lo) {
+      const size_t offr = (size_t)lo * nblk;
+      lz_final_kernel<<<(unsigned)(t - lo), 96, 0, st>>>(dot ? dot + offr : nullptr, r_nrm + offr, r_un + offr, t,
+                                                        nblk, err, d_out + lo, d_out + 3 * t);
+      LAUNCH_CHECK();
+      wait();
     };
 
     S->mode = g->lanczos_mode;
@@ -491,8 +497,15 @@ slemm_lseed* lanczos_seed_device(slemm_geno* g, int kind, float tau0, const floa
       float* Un = S->block(j + 1) + off;
       float* tmpa = tmp + off;
       const dim3 gra(nblk, ta);
-      op_device_mixed(g, kind, tau0, Uj, n, ta, tmpa, n, std::max(0, nq_eff - lo));
-      if (v4) {
+      const int nqa = std::max(0, nq_eff - lo);
+      // one kernel for the operator's last pass and the recurrence; reorthogonalisation goes between
+      // the recurrence's own passes, so it keeps them apart
+      const bool fused = !reorth && op_lanczos_step(g, kind, tau0, Uj, ta, tmpa, nqa, Uprev, Un, s_beta + lo, d_out + lo, t,
+                                                    d_out + 3 * t);
+      if (!fused) op_device_mixed(g, kind, tau0, Uj, n, ta, tmpa, n, nqa);
+      if (fused) {
+        wait();
+      } else if (v4) {
         lz_dot_kernel<4><<<gra, kLzThreads, 0, st>>>(tmpa, Uj, Uprev, r_nrm + offr, n, r_dot + offr, nblk);
         LAUNCH_CHECK();
         lz_orth_kernel<4><<<gra, kLzThreads, 0, st>>>(tmpa, Uj, r_dot + offr, n, r_nrm + offr, nblk);
@@ -509,7 +522,7 @@ slemm_lseed* lanczos_seed_device(slemm_geno* g, int kind, float tau0, const floa
         lz_scale_kernel<1><<<gra, kLzThreads, 0, st>>>(Un, tmpa, r_nrm + offr, n, r_un + offr, nblk);
         LAUNCH_CHECK();
       }
-      fetch(r_dot, lo);
+      if (!fused) fetch(r_dot, lo);
       double res = 0.0;
       for (int c = 0; c < t; ++c) {
         if (c < lo) {   // a finished group: placeholders, never read

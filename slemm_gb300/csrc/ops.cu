@@ -30,7 +30,6 @@ namespace slemm {
 constexpr int kRedThreads = 256;
 static_assert(SLEMM_MAX_COVARIATES <= kRedThreads, "load_qt gives one covariate per thread");
 constexpr int kRowsPerBlock = 4096;   // rows handled by one block of the row-wise kernels
-static_assert(kRowsPerBlock == 16 * kRedThreads, "the digit kernels give each thread one packed word");
 
 // 4-wide accesses need rows % 4 == 0 (a vector never straddles the end), ld % 4 == 0 and a
 // 16-byte aligned base.
@@ -234,12 +233,6 @@ __device__ __forceinline__ int split_exp(double bound, int top)
   int E;
   frexp(bound, &E);                        // bound = f·2^E, f ∈ [0.5, 1)
   return max(-120, min(120, top - E));
-}
-
-// max_b parts[c·nblk + b] by the 32 lanes of the calling warp (0 for no partials)
-__device__ __forceinline__ double max_partials(const double* __restrict__ parts, int nblk, int c)
-{
-  return warp_max_partials(parts + (int64_t)c * nblk, nblk);
 }
 
 // Block maximum of one float per thread (valid in thread 0; −∞ when every thread holds −∞);
@@ -478,20 +471,17 @@ __device__ __forceinline__ void gather_D(const float* __restrict__ D, int splits
 // Direction-1 finalize (rows = SNPs): val = raw·2^−e1 − gm_j·colsum_c (colsum from the prologue's
 // partials; e1 the scale of operand column c when xmax1 != nullptr), plus μ·gcorr_j for the
 // mean the prologue removed, times w_j when w != nullptr.  mode 0: out[j,c] = val (j < m).
-// mode 1: val becomes the direction-2 operand (K = SNPs) and red[c][blk] = Σ_j gm_j·stored(val);
-// with V2 != nullptr (FP16 operand) val goes to V2[c][j] in FP32 with its block maxima in xmax2,
-// for convert_snp_kernel to scale and split.  Blocks with c ≥ k zero the operand's padding rows.
+// mode 1: val becomes the direction-2 operand (K = SNPs) and red[c][blk] = Σ_j gm_j·stored(val).
+// Blocks with c ≥ k zero the operand's padding rows.
 template <int V>
 __global__ void __launch_bounds__(kRedThreads)
 finalize_snp_kernel(const float* __restrict__ D, int splits, int kp1, int64_t m_pad, int k, int64_t m,
                     const float* __restrict__ gm, const float* __restrict__ w, const double* __restrict__ cparts,
                     int nblkc, int mode, float* __restrict__ out, int64_t ldo, int npieces2, int kp2, void* B2,
                     double* __restrict__ red, int nblk, const double* __restrict__ mparts,
-                    const float* __restrict__ gcorr, int64_t n_rows, const double* __restrict__ xmax1, int top,
-                    float* __restrict__ V2, double* __restrict__ xmax2)
+                    const float* __restrict__ gcorr, int64_t n_rows, const double* __restrict__ xmax1)
 {
   __shared__ double sh[32];
-  __shared__ float shf[32];
   __shared__ float sb[2];
   __shared__ float smu, sisc;
   const int c = blockIdx.y;
@@ -504,7 +494,7 @@ finalize_snp_kernel(const float* __restrict__ D, int splits, int kp1, int64_t m_
   block_scalar([&] { return warp_sum_partials(cparts + (int64_t)c * nblkc, nblkc); }, sb, ch, cl);
   if (threadIdx.x < 32) {   // the mean the prologue removed, added back as μ·(pc_j − n·gm_j)
     const float mu_ = mparts != nullptr ? column_mean(mparts, nblkc, c, 1.0 / (double)n_rows) : 0.f;
-    const float isc_ = xmax1 != nullptr ? ldexpf(1.f, -split_col_exp(xmax1, nblkc, c, mu_, top)) : 1.f;
+    const float isc_ = xmax1 != nullptr ? ldexpf(1.f, -split_col_exp(xmax1, nblkc, c, mu_, kF16Top)) : 1.f;
     if (threadIdx.x == 0) {
       smu = mu_;
       sisc = isc_;
@@ -514,7 +504,6 @@ finalize_snp_kernel(const float* __restrict__ D, int splits, int kp1, int64_t m_
   const float mu = mparts != nullptr ? smu : 0.f;
   const float isc = sisc;
   DF acc;
-  float amax = 0.f;
   for (int64_t j = j0 + threadIdx.x * V; j < j1; j += kRedThreads * V) {
     float val[V] = {}, g[V], e[V] = {};
     ldv<V>(gm + j, g);   // gm is zero-padded to m_pad
@@ -533,127 +522,80 @@ finalize_snp_kernel(const float* __restrict__ D, int splits, int kp1, int64_t m_
     }
     if (mode == 0) {
       if (j < m) stv<V>(out + (int64_t)c * ldo + j, val);
-    } else if (V2 != nullptr) {
-      stv<V>(V2 + (int64_t)c * m_pad + j, val);
-#pragma unroll
-      for (int u = 0; u < V; ++u) amax = fmaxf(amax, fabsf(val[u]));
     } else {
       store_operand<V, true>(val, npieces2, B2, m_pad, kp2, c, j, acc, g);
     }
   }
   if (mode == 1) {
-    if (V2 != nullptr) {
-      const float mx = block_max_f(amax, shf);
-      if (threadIdx.x == 0) xmax2[(int64_t)c * nblk + blockIdx.x] = (double)mx;
-    } else {
-      const double s = block_sum_d(df_value(acc), sh);
-      if (threadIdx.x == 0) red[(int64_t)c * nblk + blockIdx.x] = s;
-    }
+    const double s = block_sum_d(df_value(acc), sh);
+    if (threadIdx.x == 0) red[(int64_t)c * nblk + blockIdx.x] = s;
   }
 }
 
-// FP16 direction-2 operand from the FP32 values V2[c][j] (finalize_snp_kernel, mode 1): pieces of
-// V2·2^e2, e2 from the block maxima xmax2, and red[c][blk] = Σ_j gm_j·stored(val).
+// Results of the first product alone (Z_cᵀU; FP16X2), the column's scalars given: out[j, c] =
+// raw·2^−e1 − gm_j·colsum_c + μ_c·gcorr_j, times w_j when w != nullptr.  V rows per thread.
 template <int V>
 __global__ void __launch_bounds__(kRedThreads)
-convert_snp_kernel(const float* __restrict__ V2, int64_t m_pad, int k, int kp2, const float* __restrict__ gm,
-                   int npieces, void* B, double* __restrict__ red, int nblk, const double* __restrict__ xmax2)
+snp_out_kernel(const float* __restrict__ D, int splits, int kp1, int64_t m_pad, int64_t m, const float* __restrict__ gm,
+               const float* __restrict__ w, const float4* __restrict__ sums, const float* __restrict__ gcorr,
+               float* __restrict__ out, int64_t ldo)
 {
-  __shared__ double sh[32];
-  __shared__ float ssc[2];
   const int c = blockIdx.y;
-  const int64_t j0 = (int64_t)blockIdx.x * kRowsPerBlock, j1 = min64(m_pad, j0 + kRowsPerBlock);
-  if (threadIdx.x < 32) {
-    const int e = split_exp(max_partials(xmax2, nblk, c), kF16Top);
-    if (threadIdx.x == 0) {
-      ssc[0] = ldexpf(1.f, e);
-      ssc[1] = ldexpf(1.f, -e);
-    }
+  const int64_t j = ((int64_t)blockIdx.x * kRedThreads + threadIdx.x) * V;
+  if (j >= m) return;
+  const float4 s1 = sums[c];   // the mean, 2^−e1, Σ stored as hi + lo (columns.cuh)
+  const float mu = s1.x, isc = s1.y, ch = s1.z, cl = s1.w;
+  float val[V], g[V], e[V], ws[V];
+  gather_D<V>(D, splits, kp1, m_pad, c, j, isc, val);
+  ldv<V>(gm + j, g);
+  ldv<V>(gcorr + j, e);
+  if (w) ldv<V>(w + j, ws);
+#pragma unroll
+  for (int u = 0; u < V; ++u) {
+    val[u] = __fmaf_rn(mu, e[u], __fmaf_rn(-g[u], cl, __fmaf_rn(-g[u], ch, val[u])));
+    if (w) val[u] = __fmul_rn(val[u], ws[u]);
   }
-  __syncthreads();
-  DF acc;
-  for (int64_t j = j0 + threadIdx.x * V; j < j1; j += kRedThreads * V) {
-    float x[V], g[V];
-    ldv<V>(V2 + (int64_t)c * m_pad + j, x);
-    ldv<V>(gm + j, g);
-    store_operand<V, true, true>(x, npieces, B, m_pad, kp2, c, j, acc, g, ssc[0], ssc[1]);
-  }
-  const double s = block_sum_d(df_value(acc), sh);
-  if (threadIdx.x == 0) red[(int64_t)c * nblk + blockIdx.x] = s;
+  stv<V>(out + (int64_t)c * ldo + j, val);
 }
 
 // Direction-2 operand straight from an m×k input (matvec): stored(in) and red = Σ gm·stored;
-// blocks with c ≥ k zero the padding rows.  F16: MEASURE writes the block maxima of |in| to
-// xmax, and the store pass scales each column by 2^e from them.
-template <int V, bool MEASURE = false, bool F16 = false>
+// blocks with c ≥ k zero the padding rows.
+template <int V>
 __global__ void __launch_bounds__(kRedThreads)
 prologue_snp_kernel(const float* __restrict__ in, int64_t ld, int64_t m, int64_t m_pad, int k, int kp,
-                    const float* __restrict__ gm, int npieces, void* B, double* __restrict__ red, int nblk,
-                    double* __restrict__ xmax)
+                    const float* __restrict__ gm, int npieces, void* B, double* __restrict__ red, int nblk)
 {
   __shared__ double sh[32];
-  __shared__ float shf[32];
-  __shared__ float ssc[2];
   const int c = blockIdx.y;
   const int64_t j0 = (int64_t)blockIdx.x * kRowsPerBlock, j1 = min64(m_pad, j0 + kRowsPerBlock);
   if (c >= k) {
-    if (!MEASURE) zero_pad_row(B, m_pad, pad_row(c - k, k, kp, npieces), j0, j1);
+    zero_pad_row(B, m_pad, pad_row(c - k, k, kp, npieces), j0, j1);
     return;
   }
-  if (F16 && !MEASURE) {
-    if (threadIdx.x < 32) {
-      const int e = split_exp(max_partials(xmax, nblk, c), kF16Top);
-      if (threadIdx.x == 0) {
-        ssc[0] = ldexpf(1.f, e);
-        ssc[1] = ldexpf(1.f, -e);
-      }
-    }
-    __syncthreads();
-  }
   DF acc;
-  float amax = 0.f;
   for (int64_t j = j0 + threadIdx.x * V; j < j1; j += kRedThreads * V) {
     float x[V] = {}, g[V];
     if (j < m) ldv<V>(in + (int64_t)c * ld + j, x);
-    if (MEASURE) {
-#pragma unroll
-      for (int u = 0; u < V; ++u) amax = fmaxf(amax, fabsf(x[u]));
-      continue;
-    }
     ldv<V>(gm + j, g);
-    if (F16) store_operand<V, true, true>(x, npieces, B, m_pad, kp, c, j, acc, g, ssc[0], ssc[1]);
-    else store_operand<V, true>(x, npieces, B, m_pad, kp, c, j, acc, g);
-  }
-  if (MEASURE) {
-    const float mx = block_max_f(amax, shf);
-    if (threadIdx.x == 0) xmax[(int64_t)c * nblk + blockIdx.x] = (double)mx;
-    return;
+    store_operand<V, true>(x, npieces, B, m_pad, kp, c, j, acc, g);
   }
   const double s = block_sum_d(df_value(acc), sh);
   if (threadIdx.x == 0) red[(int64_t)c * nblk + blockIdx.x] = s;
 }
 
-// Direction-2 finalize (rows = individuals): val = raw·2^−e2 − t_c (t from the direction-1
-// partials; e2 the FP16 scale of operand column c when xmax2 != nullptr), times rr_i when
-// rr != nullptr, plus tau0·Vin for columns c ≥ nq when Vin != nullptr.
+// Direction-2 finalize (rows = individuals): val = raw − t_c (t from the direction-1 partials), times
+// rr_i when rr != nullptr, plus tau0·Vin for columns c ≥ nq when Vin != nullptr.
 template <int V>
 __global__ void __launch_bounds__(kRedThreads)
 finalize_indiv_kernel(const float* __restrict__ D, int splits, int kp2, int64_t n_pad, int k,
                       int64_t n, const double* __restrict__ tparts, int nblkt, const float* __restrict__ rr,
                       const float* __restrict__ Vin, int64_t ld_v, float tau0, int nq, float* __restrict__ out,
-                      int64_t ldo, const double* __restrict__ xmax2, int top, const int32_t* __restrict__ map)
+                      int64_t ldo, const int32_t* __restrict__ map)
 {
   __shared__ float sb[2];
-  __shared__ float sisc;
   const int c = blockIdx.y;
   float th, tl;
   block_scalar([&] { return warp_sum_partials(tparts + (int64_t)c * nblkt, nblkt); }, sb, th, tl);
-  if (threadIdx.x < 32) {
-    const float isc_ = xmax2 != nullptr ? ldexpf(1.f, -split_exp(max_partials(xmax2, nblkt, c), top)) : 1.f;
-    if (threadIdx.x == 0) sisc = isc_;
-  }
-  __syncthreads();
-  const float isc = sisc;
   const int64_t i = ((int64_t)blockIdx.x * kRedThreads + threadIdx.x) * V;
   if (i >= n) return;
   float val[V];
@@ -661,11 +603,11 @@ finalize_indiv_kernel(const float* __restrict__ D, int splits, int kp2, int64_t 
 #pragma unroll
     for (int u = 0; u < V; ++u) {
       float t[1];
-      gather_D<1>(D, splits, kp2, n_pad, c, map[i + u], isc, t);
+      gather_D<1>(D, splits, kp2, n_pad, c, map[i + u], 1.f, t);
       val[u] = t[0];
     }
   } else {
-    gather_D<V>(D, splits, kp2, n_pad, c, i, isc, val);
+    gather_D<V>(D, splits, kp2, n_pad, c, i, 1.f, val);
   }
   float r[V], v[V];
   if (rr) ldv<V>(rr + i, r);
@@ -681,195 +623,9 @@ finalize_indiv_kernel(const float* __restrict__ D, int splits, int kp2, int64_t 
   stv<V>(out + (int64_t)c * ldo + i, val);
 }
 
-// ---- digit operands ---------------------------------------------------------------------------------
-// Writes x[0 … 15] (the rows of one packed word, kidx …) times 2^e = scale as digits into rows p·kp + c, in
-// the counts' decoded order, and adds exactly what the products will see, in the units of x, to
-// acc (weighted by wt when kWeighted).  Every step is exact.
-template <bool kWeighted>
-__device__ __forceinline__ void store_digit_operand(const float (&x)[16], int ndig, uint8_t* __restrict__ B,
-                                                    int64_t K_pad, int kp, int c, int64_t kidx, DF& acc,
-                                                    const float (&wt)[16], float scale, float inv_scale)
-{
-  float r[16];
-#pragma unroll
-  for (int u = 0; u < 16; ++u) r[u] = __fmul_rn(x[u], scale);
-  float last = 1.f;   // 32^−ndig
-#pragma unroll 1
-  for (int p = 0; p < ndig; ++p) {
-    float d[16];
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      d[u] = rintf(r[u]);
-      r[u] = __fmul_rn(__fsub_rn(r[u], d[u]), 32.f);
-    }
-    *reinterpret_cast<uint4*>(B + piece_row(p, kp, c) * K_pad + kidx) = e4m3_word(d);
-    last *= 0.03125f;
-  }
-  const float back = -last * inv_scale;
-#pragma unroll
-  for (int u = 0; u < 16; ++u) {   // what is stored: x less the digits' remainder
-    if (kWeighted) {
-      df_fma(acc, wt[u], x[u]);
-      df_fma(acc, wt[u], __fmul_rn(r[u], back));
-    } else {
-      df_add(acc, x[u]);
-      df_add(acc, __fmul_rn(r[u], back));
-    }
-  }
-}
-
-// Zeroes operand padding row `row` over the K-elements of this thread's word.
-__device__ __forceinline__ void zero_digit_row(uint8_t* __restrict__ B, int64_t K_pad, int row, int64_t kidx)
-{
-  *reinterpret_cast<uint4*>(B + (int64_t)row * K_pad + kidx) = make_uint4(0u, 0u, 0u, 0u);
-}
-
-// 16 values p[0 … 15] of rows i … i + 15, 0 from row n on; VEC: 16-byte loads (n % 4 == 0)
-template <bool VEC>
-__device__ __forceinline__ void load16(const float* __restrict__ p, int64_t i, int64_t n, float (&x)[16])
-{
-#pragma unroll
-  for (int u = 0; u < 16; u += 4) {
-    if constexpr (VEC) {
-      float t[4] = {};
-      if (i + u < n) ldv<4>(p + u, t);
-      x[u] = t[0], x[u + 1] = t[1], x[u + 2] = t[2], x[u + 3] = t[3];
-    } else {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) x[u + q] = i + u + q < n ? p[u + q] : 0.f;
-    }
-  }
-}
-
-// proj_dot of the 16 rows i … i + 15 (Q is zero-padded to a multiple of 256 rows): 16-byte loads, the
-// same arithmetic for each row.
-__device__ __forceinline__ void proj_dot16(const float* __restrict__ Q, int64_t ldq, int cq, int64_t i,
-                                           const float2* qt, float (&out)[16])
-{
-  DF a[16];
-  for (int l = 0; l < cq; ++l) {
-    const float2 t = qt[l];
-#pragma unroll
-    for (int u = 0; u < 16; u += 4) {
-      float q[4];
-      ldv<4>(Q + (int64_t)l * ldq + i + u, q);
-#pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        df_fma(a[u + w], q[w], t.x);
-        a[u + w].lo = __fmaf_rn(q[w], t.y, a[u + w].lo);
-      }
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < 16; ++u) out[u] = __fadd_rn(a[u].hi, a[u].lo);
-}
-
-// prologue_indiv_kernel's store pass with digits: the same values in the same order of operations.  One
-// packed word of 16 individuals per thread: a word's digits are 16 contiguous bytes of each operand
-// row, where four individuals' would be single bytes.
-template <bool VEC>
-__global__ void __launch_bounds__(kRedThreads)
-prologue_indiv_digits_kernel(const float* __restrict__ in, int64_t ld, int64_t n, int64_t n_pad, int k, int kp,
-                             const float* __restrict__ Q, int64_t ldq, int cq, const double* __restrict__ qparts,
-                             int nblkq, int nq, const float* __restrict__ rr, int ndig, uint8_t* __restrict__ B,
-                             double* __restrict__ red, int nblk, const double* __restrict__ mparts,
-                             const double* __restrict__ xrange, const int32_t* __restrict__ inv)
-{
-  __shared__ double sh[32];
-  __shared__ float2 qt[SLEMM_MAX_COVARIATES];
-  __shared__ float smu, ssc[2];
-  const int c = blockIdx.y;
-  const int64_t i = ((int64_t)blockIdx.x * kRedThreads + threadIdx.x) * 16;   // kRowsPerBlock rows per block
-  if (c >= k) {
-    if (i < n_pad) zero_digit_row(B, n_pad, pad_row(c - k, k, kp, ndig), i);
-    return;
-  }
-  const bool proj = qparts != nullptr && c < nq;
-  if (proj) load_qt(qparts, nblkq, cq, nq, c, qt);
-  if (threadIdx.x < 32) {
-    const float mu_ = mparts != nullptr ? column_mean(mparts, nblk, c, 1.0 / (double)n) : 0.f;
-    const int e = split_col_exp(xrange, nblk, c, mu_, kDigitTop);
-    if (threadIdx.x == 0) {
-      smu = mu_;
-      ssc[0] = ldexpf(1.f, e);
-      ssc[1] = ldexpf(1.f, -e);
-    }
-  }
-  __syncthreads();
-  const float mu = smu;
-  DF acc;
-  if (i < n_pad) {
-    float x[16];
-    if (inv != nullptr) {
-#pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        const int64_t rv = inv[i + u];
-        x[u] = 0.f;
-        if (rv >= 0) {
-          x[u] = in[(int64_t)c * ld + rv];
-          if (proj) x[u] = __fsub_rn(x[u], proj_dot(Q, ldq, cq, rv, qt));
-          if (rr) x[u] = __fmul_rn(x[u], rr[rv]);
-          x[u] = __fsub_rn(x[u], mu);
-        }
-      }
-    } else {
-      load16<VEC>(in + (int64_t)c * ld + i, i, n, x);
-      if (proj) {
-        float pd[16];
-        proj_dot16(Q, ldq, cq, i, qt, pd);
-#pragma unroll
-        for (int u = 0; u < 16; ++u) x[u] = __fsub_rn(x[u], pd[u]);
-      }
-      if (rr) {
-        float r[16];
-        load16<true>(rr + i, i, n_pad, r);   // rr is zero-padded to n_pad
-#pragma unroll
-        for (int u = 0; u < 16; ++u) x[u] = __fmul_rn(x[u], r[u]);
-      }
-#pragma unroll
-      for (int u = 0; u < 16; ++u) x[u] = i + u < n ? __fsub_rn(x[u], mu) : 0.f;
-    }
-    const float none[16] = {};
-    store_digit_operand<false>(x, ndig, B, n_pad, kp, c, i, acc, none, ssc[0], ssc[1]);
-  }
-  const double s = block_sum_d(df_value(acc), sh);
-  if (threadIdx.x == 0) red[(int64_t)c * nblk + blockIdx.x] = s;
-}
-
-// Direction-2 operand as digits from FP32 values `in` (rows j < m, column stride ld) with block maxima
-// xmax, and red[c][blk] = Σ_j gm_j·stored; blocks with c ≥ k zero the padding rows.
-template <bool VEC>
-__global__ void __launch_bounds__(kRedThreads)
-snp_digits_kernel(const float* __restrict__ in, int64_t ld, int64_t m, int64_t m_pad, int k, int kp,
-                  const float* __restrict__ gm, int ndig, uint8_t* __restrict__ B, double* __restrict__ red, int nblk,
-                  const double* __restrict__ xmax)
-{
-  __shared__ double sh[32];
-  __shared__ float ssc[2];
-  const int c = blockIdx.y;
-  const int64_t j = ((int64_t)blockIdx.x * kRedThreads + threadIdx.x) * 16;
-  if (c >= k) {
-    if (j < m_pad) zero_digit_row(B, m_pad, pad_row(c - k, k, kp, ndig), j);
-    return;
-  }
-  if (threadIdx.x < 32) {
-    const int e = split_exp(max_partials(xmax, nblk, c), kDigitTop);
-    if (threadIdx.x == 0) {
-      ssc[0] = ldexpf(1.f, e);
-      ssc[1] = ldexpf(1.f, -e);
-    }
-  }
-  __syncthreads();
-  DF acc;
-  if (j < m_pad) {
-    float x[16], g[16];
-    load16<VEC>(in + (int64_t)c * ld + j, j, m, x);
-    load16<true>(gm + j, j, m_pad, g);   // gm is zero-padded to m_pad
-    store_digit_operand<true>(x, ndig, B, m_pad, kp, c, j, acc, g, ssc[0], ssc[1]);
-  }
-  const double s = block_sum_d(df_value(acc), sh);
-  if (threadIdx.x == 0) red[(int64_t)c * nblk + blockIdx.x] = s;
-}
+}  // namespace slemm
+#include "columns.cuh"
+namespace slemm {
 
 // ---- one packed pass ---------------------------------------------------------------------------------
 struct PassPlan {
@@ -1100,36 +856,97 @@ static void run_gemm(slemm_geno* g, const PassPlan& p, const uint8_t* A, int64_t
   }
 }
 
+// FP16X2: three cluster kernels around the two products (columns.cuh), the last with the rest of a
+// Lanczos step when lz is given.
+static void op_group_f16(slemm_geno* g, int kind, float tau0, const float* in, int64_t ld_in, int k, float* out,
+                         int64_t ld_out, int nq, const PassPlan& p1, const PassPlan& p2, const LzColumn* lz)
+{
+  cudaStream_t st = g->stream;
+  const bool dir1 = kind != SLEMM_OP_MATVEC, h0 = kind == SLEMM_OP_LDET, dir2 = h0 || !dir1;
+  const int64_t n = g->n, n_pad = g->n_pad, m = g->m, m_pad = g->m_pad;
+  const int cq = g->c;
+  const size_t b1 = dir1 ? p1.operand_bytes(n_pad, k) : 0, b2 = dir2 ? p2.operand_bytes(m_pad, k) : 0;
+  const size_t bv2 = h0 ? (size_t)k * m_pad * sizeof(float) : 0;
+  uint8_t* B1 = (uint8_t*)g->ws_B.ensure(b1 + b2 + bv2);
+  uint8_t* B2 = B1 + b1;
+  float* V2 = reinterpret_cast<float*>(B2 + b2);
+  const size_t d1 = dir1 ? (size_t)p1.splits * p1.kp * m_pad : 0, d2 = dir2 ? (size_t)p2.splits * p2.kp * n_pad : 0;
+  float* D = (float*)g->ws_D.ensure(std::max(d1, d2) * sizeof(float));
+  float4* sums = (float4*)g->ws_red.ensure((size_t)2 * k * sizeof(float4));
+  float4* tsums = sums + k;
+  const int pad1 = p1.N - p1.pieces * k, pad2 = p2.N - p2.pieces * k;
+  const int32_t* inv = g->is_view ? g->ind_inv.as<int32_t>() : nullptr;
+  const int32_t* map = g->is_view ? g->ind_map.as<int32_t>() : nullptr;
+  const float *rr = kind == SLEMM_OP_LDET ? g->rr.as<float>() : nullptr, *Q = g->Q.as<float>();
+  const float *gm = g->gm.as<float>(), *gcorr = g->gcorr.as<float>();
+  const float* w = kind == SLEMM_OP_RMATVEC ? nullptr : g->w.as<float>();
+  int* err = g->err.as<int>();
+  if (dir1) {
+    const bool vec = vec4_ok(n, ld_in, in);
+    auto kernel = p1.digits() ? (vec ? col_operand_kernel<true, true> : col_operand_kernel<true, false>)
+                              : (vec ? col_operand_kernel<false, true> : col_operand_kernel<false, false>);
+    launch_columns(kernel, n_pad / kColRows, k + pad1, st, in, ld_in, n, n_pad, k, p1.kp, Q, n_pad, cq, h0 ? nq : 0, rr,
+                   p1.pieces, B1, sums, inv);
+    run_gemm(g, p1, g->G.as<uint8_t>(), m_pad, n_pad, B1, D, err, k, 1);
+    if (!h0) {
+      const bool v4 = vec4_ok(m, ld_out, out);
+      const dim3 grid((unsigned)ceil_div(m, (v4 ? 4 : 1) * kRedThreads), k);
+      if (v4)
+        snp_out_kernel<4><<<grid, kRedThreads, 0, st>>>(D, p1.splits, p1.kp, m_pad, m, gm, w, sums, gcorr, out, ld_out);
+      else
+        snp_out_kernel<1><<<grid, kRedThreads, 0, st>>>(D, p1.splits, p1.kp, m_pad, m, gm, w, sums, gcorr, out, ld_out);
+      LAUNCH_CHECK();
+      return;
+    }
+    launch_columns(p2.digits() ? col_snp_kernel<true, true, true> : col_snp_kernel<false, true, true>, m_pad / kColRows,
+                   k + pad2, st, D, p1.splits, p1.kp, w, sums, gcorr, V2, nullptr, (int64_t)0, m, m_pad, k, p2.kp, gm,
+                   p2.pieces, B2, tsums);
+  } else {
+    const bool vec = vec4_ok(m, ld_in, in);
+    auto kernel = p2.digits() ? (vec ? col_snp_kernel<true, false, true> : col_snp_kernel<true, false, false>)
+                              : (vec ? col_snp_kernel<false, false, true> : col_snp_kernel<false, false, false>);
+    launch_columns(kernel, m_pad / kColRows, k + pad2, st, nullptr, 0, 0, nullptr, nullptr, nullptr, nullptr, in, ld_in, m,
+                   m_pad, k, p2.kp, gm, p2.pieces, B2, tsums);
+  }
+  run_gemm(g, p2, g->GT.as<uint8_t>(), n_pad, m_pad, B2, D, err, k, 2);
+  const float* vin = h0 ? in : nullptr;
+  const bool vec = vec4_ok(n, ld_out, out) && (!vin || vec4_ok(n, ld_in, vin));
+  auto kernel = lz ? (vec ? col_out_kernel<true, true> : col_out_kernel<false, true>)
+                   : (vec ? col_out_kernel<true, false> : col_out_kernel<false, false>);
+  launch_columns(kernel, ceil_div(n, 16) * 2, k, st, D, p2.splits, p2.kp, n_pad, n, tsums, rr, vin, ld_in, tau0,
+                 h0 ? nq : 0, Q, n_pad, cq, out, ld_out, map, lz ? *lz : LzColumn{});
+}
+
 // One operator application on a column group (k ≤ max_group).  For the H0 operators (kind
 // LDET, or QUADFORM) the first nq columns get the projections of H0_quadform_mv and the others
 // are plain H0_ldet_mv columns, so one block can carry both kinds of seed systems.
 //
-// Launches: [QᵀV partials] → prologue (operand 1 + its column sums) → packed pass 1 → finalize 1
-// (operand 2 + its centring sums) → packed pass 2 → finalize 2 → [QᵀT partials → projection].
-// Each kernel sums the partials it needs itself, in a fixed order.
+// Launches (BF16 and FP32; FP16X2: op_group_f16): [QᵀV partials] → prologue (operand 1 + its column
+// sums) → packed pass 1 → finalize 1 (operand 2 + its centring sums) → packed pass 2 → finalize 2 →
+// [QᵀT partials → projection].  Each kernel sums the partials it needs itself, in a fixed order.
 static void op_group(slemm_geno* g, int kind, float tau0, const float* in, int64_t ld_in, int k,
-                     float* out, int64_t ld_out, int nq)
+                     float* out, int64_t ld_out, int nq, const LzColumn* lz)
 {
   if (kind == SLEMM_OP_QUADFORM) kind = SLEMM_OP_LDET;   // nq carries the projected columns
   cudaStream_t st = g->stream;
   const bool dir1 = kind != SLEMM_OP_MATVEC;                          // needs Zᵀ pass
-  const bool dir2 = kind == SLEMM_OP_QUADFORM || kind == SLEMM_OP_LDET || kind == SLEMM_OP_MATVEC;
+  const bool dir2 = kind == SLEMM_OP_LDET || kind == SLEMM_OP_MATVEC;
   // (the tuner times only the directions this operator runs)
   const PassPlan p1 = plan_pass(g, k, g->m_pad, g->n_pad, dir1 ? g->G.as<uint8_t>() : nullptr);    // M = SNPs, K = indiv
   const PassPlan p2 = plan_pass(g, k, g->n_pad, g->m_pad, dir2 ? g->GT.as<uint8_t>() : nullptr);   // M = indiv, K = SNPs
+  CHECK_ARG(g->c <= SLEMM_MAX_COVARIATES, "too many covariates");
+  if (p1.f16) {
+    op_group_f16(g, kind, tau0, in, ld_in, k, out, ld_out, nq, p1, p2, lz);
+    return;
+  }
   const int np1 = p1.tc ? p1.pieces : 0, np2 = p2.tc ? p2.pieces : 0;
   const int pad1 = p1.tc ? p1.N - p1.pieces * k : 0;                   // padding rows of the operands
   const int pad2 = p2.tc ? p2.N - p2.pieces * k : 0;
-  const bool f16 = p1.f16;
   const size_t b1 = dir1 ? p1.operand_bytes(g->n_pad, k) : 0;
   const size_t b2 = dir2 ? p2.operand_bytes(g->m_pad, k) : 0;
-  const int top1 = p1.digits() ? kDigitTop : kF16Top, top2 = p2.digits() ? kDigitTop : kF16Top;
-  // FP16: the direction-2 values in FP32 before they are scaled and split
-  const size_t bv2 = (dir1 && dir2 && f16) ? (size_t)k * g->m_pad * 4 : 0;
-  uint8_t* Bbuf = (uint8_t*)g->ws_B.ensure(b1 + b2 + bv2);
+  uint8_t* Bbuf = (uint8_t*)g->ws_B.ensure(b1 + b2);
   void* B1 = Bbuf;
   void* B2 = Bbuf + b1;
-  float* V2 = bv2 ? (float*)(Bbuf + b1 + b2) : nullptr;
   const size_t d1 = dir1 ? (size_t)p1.splits * p1.kp * g->m_pad : 0;
   const size_t d2 = dir2 ? (size_t)p2.splits * p2.kp * g->n_pad : 0;
   float* D = (float*)g->ws_D.ensure(std::max(d1, d2) * sizeof(float));
@@ -1137,23 +954,18 @@ static void op_group(slemm_geno* g, int kind, float tau0, const float* in, int64
   const int nblk_m = (int)ceil_div(g->m_pad, kRowsPerBlock);
   const int nblk_q = (int)ceil_div(g->n, kRowsPerBlock);
   // partials: colsum [k][nblk_n] | tsum [k][nblk_m] | QᵀV [c·nq][nblk_q] | QᵀT [c·nq][nblk_q] |
-  // column sums for the means [k][nblk_n] | FP16 ranges: operand 1 signed extremes [k][nblk_n][2],
-  // operand 2 maxima of |x| [k][nblk_m]
+  // column sums for the means [k][nblk_n]
   const int cq = g->c;
-  CHECK_ARG(cq <= SLEMM_MAX_COVARIATES, "too many covariates");
-  const size_t nred = 2 * (size_t)k * nblk_n + (size_t)k * nblk_m + 2 * (size_t)std::max(cq, 1) * k * nblk_q +
-                      (f16 ? (size_t)k * (2 * nblk_n + nblk_m) : 0);
+  const size_t nred = 2 * (size_t)k * nblk_n + (size_t)k * nblk_m + 2 * (size_t)std::max(cq, 1) * k * nblk_q;
   double* r_col = (double*)g->ws_red.ensure(nred * sizeof(double));
   double* r_t = r_col + (size_t)k * nblk_n;
   double* r_qv = r_t + (size_t)k * nblk_m;
   double* r_qt = r_qv + (size_t)std::max(cq, 1) * k * nblk_q;
   double* r_mu = r_qt + (size_t)std::max(cq, 1) * k * nblk_q;   // column sums for the means [k][nblk_n]
-  double* x_max1 = f16 ? r_mu + (size_t)k * nblk_n : nullptr;        // [k][nblk_n][2]
-  double* x_max2 = f16 ? x_max1 + 2 * (size_t)k * nblk_n : nullptr;  // [k][nblk_m]
   int* err = g->err.as<int>();
 
   // H0 operators: the first nq columns are projected (H0_quadform_mv), the rest are not (H0_ldet_mv)
-  const bool h0 = kind == SLEMM_OP_QUADFORM || kind == SLEMM_OP_LDET;
+  const bool h0 = kind == SLEMM_OP_LDET;
   const bool vin = vec4_ok(g->n, ld_in, in);
   // a trait view reads its inputs and writes its outputs through its individual map
   const int32_t* inv_ind = g->is_view ? g->ind_inv.as<int32_t>() : nullptr;
@@ -1168,111 +980,57 @@ static void op_group(slemm_geno* g, int kind, float tau0, const float* in, int64
     const float* Qp = g->Q.as<float>();
     const double* qp = proj ? r_qv : nullptr;
     double* const mu = g->gcorr.p ? r_mu : nullptr;   // mean removal needs Z_cᵀ1 (set with the weights)
-    if (mu || f16) {
-      // measure pass: column sums (for the means) and, for FP16 operands, the column maxima
+    if (mu) {
+      // measure pass: column sums for the means
       if (vin)
         prologue_indiv_kernel<4, true><<<dim3(nblk_n, k), kRedThreads, 0, st>>>(
             in, ld_in, g->n, g->n_pad, k, p1.kp, Qp, g->n_pad, cq, qp, nblk_q, nq, rr, np1, B1, mu, nblk_n, nullptr,
-            x_max1, inv_ind);
+            nullptr, inv_ind);
       else
         prologue_indiv_kernel<1, true><<<dim3(nblk_n, k), kRedThreads, 0, st>>>(
             in, ld_in, g->n, g->n_pad, k, p1.kp, Qp, g->n_pad, cq, qp, nblk_q, nq, rr, np1, B1, mu, nblk_n, nullptr,
-            x_max1, inv_ind);
+            nullptr, inv_ind);
       LAUNCH_CHECK();
     }
-    if (p1.digits()) {
-      if (vin)
-        prologue_indiv_digits_kernel<true><<<grid, kRedThreads, 0, st>>>(
-            in, ld_in, g->n, g->n_pad, k, p1.kp, Qp, g->n_pad, cq, qp, nblk_q, nq, rr, np1, (uint8_t*)B1, r_col, nblk_n,
-            mu, x_max1, inv_ind);
-      else
-        prologue_indiv_digits_kernel<false><<<grid, kRedThreads, 0, st>>>(
-            in, ld_in, g->n, g->n_pad, k, p1.kp, Qp, g->n_pad, cq, qp, nblk_q, nq, rr, np1, (uint8_t*)B1, r_col, nblk_n,
-            mu, x_max1, inv_ind);
-    } else if (f16) {
-      if (vin)
-        prologue_indiv_kernel<4, false, true><<<grid, kRedThreads, 0, st>>>(
-            in, ld_in, g->n, g->n_pad, k, p1.kp, Qp, g->n_pad, cq, qp, nblk_q, nq, rr, np1, B1, r_col, nblk_n, mu,
-            x_max1, inv_ind);
-      else
-        prologue_indiv_kernel<1, false, true><<<grid, kRedThreads, 0, st>>>(
-            in, ld_in, g->n, g->n_pad, k, p1.kp, Qp, g->n_pad, cq, qp, nblk_q, nq, rr, np1, B1, r_col, nblk_n, mu,
-            x_max1, inv_ind);
-    } else {
-      if (vin)
-        prologue_indiv_kernel<4, false><<<grid, kRedThreads, 0, st>>>(
-            in, ld_in, g->n, g->n_pad, k, p1.kp, Qp, g->n_pad, cq, qp, nblk_q, nq, rr, np1, B1, r_col, nblk_n, mu,
-            nullptr, inv_ind);
-      else
-        prologue_indiv_kernel<1, false><<<grid, kRedThreads, 0, st>>>(
-            in, ld_in, g->n, g->n_pad, k, p1.kp, Qp, g->n_pad, cq, qp, nblk_q, nq, rr, np1, B1, r_col, nblk_n, mu,
-            nullptr, inv_ind);
-    }
+    if (vin)
+      prologue_indiv_kernel<4, false><<<grid, kRedThreads, 0, st>>>(
+          in, ld_in, g->n, g->n_pad, k, p1.kp, Qp, g->n_pad, cq, qp, nblk_q, nq, rr, np1, B1, r_col, nblk_n, mu,
+          nullptr, inv_ind);
+    else
+      prologue_indiv_kernel<1, false><<<grid, kRedThreads, 0, st>>>(
+          in, ld_in, g->n, g->n_pad, k, p1.kp, Qp, g->n_pad, cq, qp, nblk_q, nq, rr, np1, B1, r_col, nblk_n, mu,
+          nullptr, inv_ind);
     LAUNCH_CHECK();
     // ---- pass 1: Cntᵀ over individuals ----
     run_gemm(g, p1, g->G.as<uint8_t>(), g->m_pad, g->n_pad, B1, D, err, k, 1);
     // ---- finalize 1 ----
     const float* wsc = (kind == SLEMM_OP_RMATVEC) ? nullptr : g->w.as<float>();
     if (h0) {
-      finalize_snp_kernel<4><<<dim3(nblk_m, k + (p2.digits() ? 0 : pad2)), kRedThreads, 0, st>>>(
+      finalize_snp_kernel<4><<<dim3(nblk_m, k + pad2), kRedThreads, 0, st>>>(
           D, p1.splits, p1.kp, g->m_pad, k, g->m, g->gm.as<float>(), wsc, r_col, nblk_n, 1, nullptr, 0, np2, p2.kp,
-          B2, r_t, nblk_m, mu, g->gcorr.as<float>(), g->n, x_max1, top1, V2, x_max2);
+          B2, r_t, nblk_m, mu, g->gcorr.as<float>(), g->n, nullptr);
       LAUNCH_CHECK();
-      if (p2.digits()) {
-        snp_digits_kernel<true><<<dim3(nblk_m, k + pad2), kRedThreads, 0, st>>>(
-            V2, g->m_pad, g->m_pad, g->m_pad, k, p2.kp, g->gm.as<float>(), np2, (uint8_t*)B2, r_t, nblk_m, x_max2);
-        LAUNCH_CHECK();
-      } else if (f16) {
-        convert_snp_kernel<4><<<dim3(nblk_m, k), kRedThreads, 0, st>>>(V2, g->m_pad, k, p2.kp, g->gm.as<float>(),
-                                                                        np2, B2, r_t, nblk_m, x_max2);
-        LAUNCH_CHECK();
-      }
     } else {
       if (vec4_ok(g->m, ld_out, out))
         finalize_snp_kernel<4><<<dim3(nblk_m, k), kRedThreads, 0, st>>>(
             D, p1.splits, p1.kp, g->m_pad, k, g->m, g->gm.as<float>(), wsc, r_col, nblk_n, 0, out, ld_out, 0, 8,
-            nullptr, nullptr, 0, mu, g->gcorr.as<float>(), g->n, x_max1, top1, nullptr, nullptr);
+            nullptr, nullptr, 0, mu, g->gcorr.as<float>(), g->n, nullptr);
       else
         finalize_snp_kernel<1><<<dim3(nblk_m, k), kRedThreads, 0, st>>>(
             D, p1.splits, p1.kp, g->m_pad, k, g->m, g->gm.as<float>(), wsc, r_col, nblk_n, 0, out, ld_out, 0, 8,
-            nullptr, nullptr, 0, mu, g->gcorr.as<float>(), g->n, x_max1, top1, nullptr, nullptr);
+            nullptr, nullptr, 0, mu, g->gcorr.as<float>(), g->n, nullptr);
       LAUNCH_CHECK();
       return;
     }
   } else {
     // matvec: operand straight from the m×k input
     dim3 gridm(nblk_m, k + pad2);
-    const bool v4 = vec4_ok(g->m, ld_in, in);
-    if (f16) {
-      if (v4) {
-        prologue_snp_kernel<4, true, true><<<dim3(nblk_m, k), kRedThreads, 0, st>>>(
-            in, ld_in, g->m, g->m_pad, k, p2.kp, g->gm.as<float>(), np2, B2, r_t, nblk_m, x_max2);
-        LAUNCH_CHECK();
-        if (p2.digits())
-          snp_digits_kernel<true><<<gridm, kRedThreads, 0, st>>>(in, ld_in, g->m, g->m_pad, k, p2.kp, g->gm.as<float>(),
-                                                                 np2, (uint8_t*)B2, r_t, nblk_m, x_max2);
-        else prologue_snp_kernel<4, false, true><<<gridm, kRedThreads, 0, st>>>(in, ld_in, g->m, g->m_pad, k, p2.kp,
-                                                                           g->gm.as<float>(), np2, B2, r_t, nblk_m,
-                                                                           x_max2);
-      } else {
-        prologue_snp_kernel<1, true, true><<<dim3(nblk_m, k), kRedThreads, 0, st>>>(
-            in, ld_in, g->m, g->m_pad, k, p2.kp, g->gm.as<float>(), np2, B2, r_t, nblk_m, x_max2);
-        LAUNCH_CHECK();
-        if (p2.digits())
-          snp_digits_kernel<false><<<gridm, kRedThreads, 0, st>>>(in, ld_in, g->m, g->m_pad, k, p2.kp, g->gm.as<float>(),
-                                                                  np2, (uint8_t*)B2, r_t, nblk_m, x_max2);
-        else prologue_snp_kernel<1, false, true><<<gridm, kRedThreads, 0, st>>>(in, ld_in, g->m, g->m_pad, k, p2.kp,
-                                                                           g->gm.as<float>(), np2, B2, r_t, nblk_m,
-                                                                           x_max2);
-      }
-    } else {
-      if (v4)
-        prologue_snp_kernel<4><<<gridm, kRedThreads, 0, st>>>(in, ld_in, g->m, g->m_pad, k, p2.kp, g->gm.as<float>(),
-                                                              np2, B2, r_t, nblk_m, nullptr);
-      else
-        prologue_snp_kernel<1><<<gridm, kRedThreads, 0, st>>>(in, ld_in, g->m, g->m_pad, k, p2.kp, g->gm.as<float>(),
-                                                              np2, B2, r_t, nblk_m, nullptr);
-    }
+    if (vec4_ok(g->m, ld_in, in))
+      prologue_snp_kernel<4><<<gridm, kRedThreads, 0, st>>>(in, ld_in, g->m, g->m_pad, k, p2.kp, g->gm.as<float>(),
+                                                            np2, B2, r_t, nblk_m);
+    else
+      prologue_snp_kernel<1><<<gridm, kRedThreads, 0, st>>>(in, ld_in, g->m, g->m_pad, k, p2.kp, g->gm.as<float>(),
+                                                            np2, B2, r_t, nblk_m);
     LAUNCH_CHECK();
   }
   // ---- pass 2: Cnt over SNPs ----
@@ -1285,11 +1043,11 @@ static void op_group(slemm_geno* g, int kind, float tau0, const float* in, int64
   if (vec4_ok(g->n, ld_out, out) && (!v2 || vin)) {
     dim3 grid((unsigned)ceil_div(g->n, 4 * kRedThreads), k);
     finalize_indiv_kernel<4><<<grid, kRedThreads, 0, st>>>(D, p2.splits, p2.kp, g->n_pad, k, g->n, r_t, nblk_m, rr2,
-                                                           v2, ld_in, tau0, nq2, out, ld_out, x_max2, top2, map_ind);
+                                                           v2, ld_in, tau0, nq2, out, ld_out, map_ind);
   } else {
     dim3 grid((unsigned)ceil_div(g->n, kRedThreads), k);
     finalize_indiv_kernel<1><<<grid, kRedThreads, 0, st>>>(D, p2.splits, p2.kp, g->n_pad, k, g->n, r_t, nblk_m, rr2,
-                                                           v2, ld_in, tau0, nq2, out, ld_out, x_max2, top2, map_ind);
+                                                           v2, ld_in, tau0, nq2, out, ld_out, map_ind);
   }
   LAUNCH_CHECK();
   // quadform columns 0 … nq−1: out = T + τ0 v − QQᵀT
@@ -1378,17 +1136,17 @@ void rows_product(slemm_geno* g, int64_t r0, int64_t rows, const float* U, int64
     if (vec4_ok(m_valid, ldo, o))
       finalize_snp_kernel<4><<<dim3(nblk_m, kc), kRedThreads, 0, st>>>(
           D, p.splits, p.kp, rows, kc, m_valid, g->gm.as<float>() + r0, nullptr, r_col, nblk_n, 0, o, ldo, 0, 8,
-          nullptr, nullptr, 0, mu, mu ? g->gcorr.as<float>() + r0 : nullptr, g->n, x_rng, kF16Top, nullptr, nullptr);
+          nullptr, nullptr, 0, mu, mu ? g->gcorr.as<float>() + r0 : nullptr, g->n, x_rng);
     else
       finalize_snp_kernel<1><<<dim3(nblk_m, kc), kRedThreads, 0, st>>>(
           D, p.splits, p.kp, rows, kc, m_valid, g->gm.as<float>() + r0, nullptr, r_col, nblk_n, 0, o, ldo, 0, 8,
-          nullptr, nullptr, 0, mu, mu ? g->gcorr.as<float>() + r0 : nullptr, g->n, x_rng, kF16Top, nullptr, nullptr);
+          nullptr, nullptr, 0, mu, mu ? g->gcorr.as<float>() + r0 : nullptr, g->n, x_rng);
     LAUNCH_CHECK();
   }
 }
 
-void op_device_mixed(slemm_geno* g, int kind, float tau0, const float* in, int64_t ld_in, int k,
-                     float* out, int64_t ld_out, int nq)
+static void op_columns(slemm_geno* g, int kind, float tau0, const float* in, int64_t ld_in, int k, float* out,
+                       int64_t ld_out, int nq, const LzColumn* lz)
 {
   if (!g->weights_set) SLEMM_THROW(SLEMM_ERR_STATE, "set_weights must be called before operators");
   CHECK_ARG(kind >= SLEMM_OP_QUADFORM && kind <= SLEMM_OP_WRMATVEC, "unknown operator kind");
@@ -1401,8 +1159,32 @@ void op_device_mixed(slemm_geno* g, int kind, float tau0, const float* in, int64
   for (int c0 = 0; c0 < k; c0 += grp) {
     const int kc = std::min(grp, k - c0);
     const int nqg = std::max(0, std::min(kc, nq - c0));
-    op_group(g, kind, tau0, in + (int64_t)c0 * ld_in, ld_in, kc, out + (int64_t)c0 * ld_out, ld_out, nqg);
+    LzColumn z;
+    if (lz) {
+      z = *lz;
+      if (z.Uprev) z.Uprev += (int64_t)c0 * g->n;
+      z.Unext += (int64_t)c0 * g->n;
+      z.beta += c0;
+      z.scal += c0;
+    }
+    op_group(g, kind, tau0, in + (int64_t)c0 * ld_in, ld_in, kc, out + (int64_t)c0 * ld_out, ld_out, nqg,
+             lz ? &z : nullptr);
   }
+}
+
+void op_device_mixed(slemm_geno* g, int kind, float tau0, const float* in, int64_t ld_in, int k,
+                     float* out, int64_t ld_out, int nq)
+{
+  op_columns(g, kind, tau0, in, ld_in, k, out, ld_out, nq, nullptr);
+}
+
+bool op_lanczos_step(slemm_geno* g, int kind, float tau0, const float* U, int k, float* tmp, int nq, const float* Uprev,
+                     float* Unext, float2* beta, double* scal, int stride, double* scal_err)
+{
+  if (g->prec != SLEMM_PREC_FP16X2) return false;
+  const LzColumn lz{Uprev, Unext, beta, scal, stride, scal_err, g->err.as<int>()};
+  op_columns(g, kind, tau0, U, g->n, k, tmp, g->n, nq, &lz);
+  return true;
 }
 
 void op_device(slemm_geno* g, int kind, float tau0, const float* in, int64_t ld_in, int k,
