@@ -153,34 +153,44 @@ __device__ __forceinline__ float warp_max_f(float v)
   return v;
 }
 
+// Σ (or maximum) of one double per lane over the warp, the same in every lane: a fixed butterfly.
+__device__ __forceinline__ double warp_all(double v, bool mx)
+{
+  for (int o = 16; o; o >>= 1) {
+    const double t = __shfl_xor_sync(0xffffffffu, v, o);
+    v = mx ? fmax(v, t) : v + t;
+  }
+  return v;
+}
+
 // Combines S.warp[·][q], q < NV, over the column's warps (sum, or maximum where bit q of MAX is set) into
 // S.total; then thread 0 of every block runs done(S.total), which leaves what all threads need in S.f.
+// One warp does it, a lane per warp and then per block: walking them one after another took 2 µs.
 template <int NV, unsigned MAX, class F>
 __device__ __forceinline__ void col_combine(ColShared& S, int& turn, F&& done)
 {
   namespace cg = cooperative_groups;
-  const int nw = blockDim.x >> 5;
+  const int nw = blockDim.x >> 5, lane = threadIdx.x & 31;
   __syncthreads();
   cg::cluster_group cl = cg::this_cluster();
-  if (threadIdx.x < NV) {
-    const int q = threadIdx.x;
-    double r = S.warp[0][q];
-    for (int w = 1; w < nw; ++w) r = ((MAX >> q) & 1u) ? fmax(r, S.warp[w][q]) : r + S.warp[w][q];
-    S.block[turn][q] = r;
+  if (threadIdx.x < 32) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      const bool mx = (MAX >> q) & 1u;
+      const double r = warp_all(lane < nw ? S.warp[lane][q] : (mx ? -INFINITY : 0.0), mx);
+      if (lane == 0) S.block[turn][q] = r;
+    }
   }
   cl.sync();
   if (threadIdx.x < 32) {
-    if (threadIdx.x < NV) {
-      const int q = threadIdx.x;
-      double r = *cl.map_shared_rank(&S.block[turn][q], 0);
-      for (unsigned b = 1; b < cl.num_blocks(); ++b) {
-        const double t = *cl.map_shared_rank(&S.block[turn][q], b);
-        r = ((MAX >> q) & 1u) ? fmax(r, t) : r + t;
-      }
-      S.total[q] = r;
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      const bool mx = (MAX >> q) & 1u;
+      const bool has = lane < (int)cl.num_blocks();
+      const double r = warp_all(has ? *cl.map_shared_rank(&S.block[turn][q], has ? lane : 0) : (mx ? -INFINITY : 0.0), mx);
+      if (lane == 0) S.total[q] = r;
     }
-    __syncwarp();
-    if (threadIdx.x == 0) done(S.total);
+    if (lane == 0) done(S.total);
   }
   __syncthreads();
   turn ^= 1;
@@ -239,21 +249,23 @@ __device__ __forceinline__ void col_project(const float* __restrict__ Q, int64_t
       }
     }
     __syncthreads();
-    if ((int)threadIdx.x < nl) {
-      double r = 0.0;
-      for (int w = 0; w < nw; ++w) r += S.warp[w][threadIdx.x];
-      S.block[turn][l0 + threadIdx.x] = r;
+    if (threadIdx.x < 32) {
+#pragma unroll
+      for (int l = 0; l < L; ++l) {
+        if (l < nl) {
+          const double r = warp_all(lane < nw ? S.warp[lane][l] : 0.0, false);
+          if (lane == 0) S.block[turn][l0 + l] = r;
+        }
+      }
     }
     __syncthreads();
   }
   cg::cluster_group cl = cg::this_cluster();
   cl.sync();
-  for (int l = threadIdx.x; l < cq; l += blockDim.x) {
-    double r = 0.0;
-    for (unsigned b = 0; b < cl.num_blocks(); ++b) r += *cl.map_shared_rank(&S.block[turn][l], b);
-    float h, lo;
-    split_double(r, h, lo);
-    qt[l] = make_float2(h, lo);
+  for (int l = warp; l < cq; l += nw) {
+    const bool has = lane < (int)cl.num_blocks();
+    const double r = warp_all(has ? *cl.map_shared_rank(&S.block[turn][l], has ? lane : 0) : 0.0, false);
+    if (lane == 0) split_double(r, qt[l].x, qt[l].y);
   }
   __syncthreads();
   turn ^= 1;
