@@ -731,12 +731,10 @@ int slemm_gpu_set_projection(slemm_geno* g, const float* Q, int64_t ldq, int c)
     g->c = c;
     if (c == 0) return;
     CHECK_ARG(Q != nullptr && ldq >= g->n, "bad Q");
-    std::vector<float> hq((size_t)g->n_pad * c, 0.f);
-    for (int l = 0; l < c; ++l)
-      for (int64_t i = 0; i < g->n; ++i) hq[(size_t)l * g->n_pad + i] = Q[(size_t)l * ldq + i];
-    g->Q.ensure(hq.size() * sizeof(float));
-    CUDA_TRY(cudaMemcpyAsync(g->Q.p, hq.data(), hq.size() * sizeof(float), cudaMemcpyHostToDevice,
-                             g->stream));
+    g->Q.ensure((size_t)g->n_pad * c * sizeof(float));
+    CUDA_TRY(cudaMemsetAsync(g->Q.p, 0, (size_t)g->n_pad * c * sizeof(float), g->stream));   // rows n … n_pad − 1
+    CUDA_TRY(cudaMemcpy2DAsync(g->Q.p, g->n_pad * sizeof(float), Q, ldq * sizeof(float), g->n * sizeof(float), c,
+                               cudaMemcpyHostToDevice, g->stream));
     CUDA_TRY(cudaStreamSynchronize(g->stream));
   });
 }

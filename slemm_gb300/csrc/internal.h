@@ -158,6 +158,24 @@ void lseed_free(slemm_lseed* S);
 // probes.cu — the reference's normalised Rademacher block (n×n_V, ld) on the device.
 void rademacher_device(int seed, int64_t n, int n_V, float* dV, int64_t ld, cudaStream_t st);
 
+// The first nA + nB samples of std::normal_distribution<float>(0, 1) over std::mt19937(seed + 54321), the
+// first nA into dA, the others into dB (device).  The constructor queues them; finish() waits and checks
+// that enough draws were made (and makes more if not): the samples may be used after it.
+class NormalDraws {
+ public:
+  NormalDraws(int seed, int64_t nA, float* dA, int64_t nB, float* dB, cudaStream_t st);
+  void finish();
+
+ private:
+  void launch();
+  uint32_t seed_;
+  int64_t nA_, total_, pairs_ = 0;
+  float *dA_, *dB_;
+  cudaStream_t st_;
+  int blocks_ = 0;
+  DevBuf words_, offs_;
+};
+
 // geno.cu — per-SNP popcounts (missing = 1) and class counts n1 (fields 01), n2 (fields 10).
 void row_counts_device(slemm_geno* g, int64_t* pc, int32_t* c1, int32_t* c2);
 

@@ -2,15 +2,14 @@
 // MC-REML (LMC_REML, src/reml.cpp:730-883).
 //
 // All vectors of length n or m stay in HBM; the host keeps the FP64 scalars (Lanczos/CG
-// coefficients, golden-section and secant state, c×c covariate algebra).  Probe draws come
-// from libstdc++'s std::mt19937 with the reference's distributions and draw order, so the GPU
-// engine sees the reference's probes.
+// coefficients, golden-section and secant state, c×c covariate algebra).  Probes and samples follow
+// libstdc++'s std::mt19937 with the reference's distributions and draw order (probes.cu), so the GPU
+// engine sees the reference's.
 #include "internal.h"
 #include "reduce.cuh"
 
 #include <chrono>
 #include <memory>
-#include <random>
 
 namespace slemm {
 
@@ -18,6 +17,26 @@ namespace slemm {
 // Column-pivoted Householder QR of an n×c column-major matrix (the reference uses Eigen's
 // ColPivHouseholderQR, src/reml.cpp:583-588).  Returns Q (n×rank), R·Pᵀ (rank×c) and the rank
 // under Eigen's rule |R_ii| > eps_f32·min(n,c)·|R_00|.
+// aᵀb in FP64 with eight running sums (one sum is a chain of additions, four cycles each).
+static double dot8(const double* a, const double* b, int64_t n)
+{
+  double s[8] = {};
+  int64_t i = 0;
+  for (; i + 8 <= n; i += 8)
+    for (int q = 0; q < 8; ++q) s[q] += a[i + q] * b[i + q];
+  for (; i < n; ++i) s[0] += a[i] * b[i];
+  return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+}
+static double dot8(const float* a, const float* b, int64_t n)
+{
+  double s[8] = {};
+  int64_t i = 0;
+  for (; i + 8 <= n; i += 8)
+    for (int q = 0; q < 8; ++q) s[q] += (double)a[i + q] * (double)b[i + q];
+  for (; i < n; ++i) s[0] += (double)a[i] * (double)b[i];
+  return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+}
+
 struct QRHost {
   std::vector<double> Q;     // n×rank
   std::vector<double> RPt;   // rank×c (column-major)
@@ -37,9 +56,7 @@ static QRHost qr_colpiv(const std::vector<double>& A0, int64_t n, int c)
     int p = k;
     double best = -1.0;
     for (int j = k; j < c; ++j) {
-      double s = 0.0;
-      const double* a = col(j);
-      for (int64_t i = k; i < n; ++i) s += a[i] * a[i];
+      const double s = dot8(col(j) + k, col(j) + k, n - k);
       if (s > best) {
         best = s;
         p = j;
@@ -59,15 +76,11 @@ static QRHost qr_colpiv(const std::vector<double>& A0, int64_t n, int c)
     const double v0 = a[k] - alpha;
     // v = [1, a[k+1..]/v0], tau = (alpha - a_k)/alpha ... use explicit 2/(vᵀv)
     for (int64_t i = k + 1; i < n; ++i) a[i] /= v0;
-    double vtv = 1.0;
-    for (int64_t i = k + 1; i < n; ++i) vtv += a[i] * a[i];
-    tau[k] = 2.0 / vtv;
+    tau[k] = 2.0 / (1.0 + dot8(a + k + 1, a + k + 1, n - k - 1));
     a[k] = alpha;
     for (int j = k + 1; j < c; ++j) {
       double* b = col(j);
-      double s = b[k];
-      for (int64_t i = k + 1; i < n; ++i) s += a[i] * b[i];
-      s *= tau[k];
+      const double s = (b[k] + dot8(a + k + 1, b + k + 1, n - k - 1)) * tau[k];
       b[k] -= s;
       for (int64_t i = k + 1; i < n; ++i) b[i] -= s * a[i];
     }
@@ -87,9 +100,7 @@ static QRHost qr_colpiv(const std::vector<double>& A0, int64_t n, int c)
     for (int k = kmax - 1; k >= 0; --k) {
       if (tau[k] == 0.0) continue;
       const double* v = col(k);
-      double s = q[k];
-      for (int64_t i = k + 1; i < n; ++i) s += v[i] * q[i];
-      s *= tau[k];
+      const double s = (q[k] + dot8(v + k + 1, q + k + 1, n - k - 1)) * tau[k];
       q[k] -= s;
       for (int64_t i = k + 1; i < n; ++i) q[i] -= s * v[i];
     }
@@ -339,8 +350,7 @@ void reml_sldf(slemm_geno* g, const float* rvec, const float* X, int64_t ldx, in
     for (int64_t i = 0; i < n; ++i) ry[i] = (double)(S.rr[i] * y[i]);
     for (int l = 0; l < c; ++l) {
       const double* q = S.qr.Q.data() + (size_t)l * n;
-      double s = 0.0;
-      for (int64_t i = 0; i < n; ++i) s += q[i] * ry[i];
+      const double s = dot8(q, ry.data(), n);
       for (int64_t i = 0; i < n; ++i) ry[i] -= s * q[i];
     }
     for (int64_t i = 0; i < n; ++i) yproj[i] = (float)ry[i];
@@ -555,28 +565,24 @@ void reml_lmc(slemm_geno* g, const float* rvec, const float* X, int64_t ldx, int
   const int64_t n = g->n, m = g->m;
   const bool verbose = o.verbose != 0;
   if (verbose) printf("\nStarted Lanczos MC-REML.\n");
-  Setup S = reml_setup(g, rvec, X, ldx, c, persnp);
   cudaStream_t st = g->stream;
   const int n_MC = o.n_V;
   CHECK_ARG(n_MC >= 1, "n_MC must be >= 1");
   const int tV = 1 + 2 * n_MC;
-  // draws: u (m×n_MC) then e (n×n_MC) from one generator (src/reml.cpp:795-809)
-  std::vector<float> u((size_t)m * n_MC), V((size_t)n * tV);
-  {
-    if (verbose) printf("Generating %d MC samples for genetic effects.\n", n_MC);
-    std::mt19937 rng(o.seed + 54321);
-    std::normal_distribution<float> rnorm(0.0, 1.0);
-    for (int j = 0; j < n_MC; ++j)
-      for (int64_t i = 0; i < m; ++i) u[(size_t)j * m + i] = rnorm(rng);
-    if (verbose) printf("Generating %d MC samples for residuals.\n", n_MC);
-    for (int j = 1 + n_MC; j < tV; ++j)
-      for (int64_t i = 0; i < n; ++i) V[(size_t)j * n + i] = rnorm(rng);
-  }
-  for (int64_t i = 0; i < n; ++i) V[i] = y[i];
   DevBuf d_V(g->stream), d_u(g->stream), d_PV(g->stream), d_Py(g->stream), d_ub(g->stream),
       d_tmp(g->stream), d_aux(g->stream);
   d_V.ensure((size_t)n * tV * sizeof(float));
   d_u.ensure((size_t)m * n_MC * sizeof(float));
+  // draws: u (m×n_MC) then e (n×n_MC) from one generator (src/reml.cpp:795-809), on the GPU while the host
+  // set-up below runs
+  if (verbose) {
+    printf("Generating %d MC samples for genetic effects.\n", n_MC);
+    printf("Generating %d MC samples for residuals.\n", n_MC);
+  }
+  NormalDraws draws(o.seed, (int64_t)m * n_MC, d_u.as<float>(), (int64_t)n * n_MC, d_V.as<float>() + (size_t)(1 + n_MC) * n,
+                    st);
+  Setup S = reml_setup(g, rvec, X, ldx, c, persnp);
+  draws.finish();
   d_PV.ensure((size_t)n * tV * sizeof(float));
   d_Py.ensure((size_t)n * (1 + n_MC) * sizeof(float));
   d_ub.ensure((size_t)m * (1 + n_MC) * sizeof(float));
@@ -584,8 +590,7 @@ void reml_lmc(slemm_geno* g, const float* rvec, const float* X, int64_t ldx, int
   const size_t scal_off = (size_t)c * tV;
   d_tmp.ensure((scal_off + 4 * (size_t)tV) * sizeof(double));
   double* d_scal = d_tmp.as<double>();
-  upload(g, d_V.as<float>(), V.data(), (size_t)n * tV);
-  upload(g, d_u.as<float>(), u.data(), (size_t)m * n_MC);
+  upload(g, d_V.as<float>(), y, n);
   // u *= sqrt(gw); V[:,1:1+n_MC] = Z_c u   (src/reml.cpp:801-802)
   scale_rows(g, d_u.as<float>(), m, m, n_MC, g->w.as<float>(), true);
   op_device(g, SLEMM_OP_MATVEC, 0.f, d_u.as<float>(), m, n_MC, d_V.as<float>() + n, n);
@@ -690,13 +695,9 @@ void reml_lmc(slemm_geno* g, const float* rvec, const float* X, int64_t ldx, int
       const float* xa = X + (size_t)a * ldx;
       for (int b = 0; b <= a; ++b) {
         const float* xb = X + (size_t)b * ldx;
-        double s = 0.0;
-        for (int64_t i = 0; i < n; ++i) s += (double)xa[i] * xb[i];
-        XtX[(size_t)b * c + a] = XtX[(size_t)a * c + b] = s;
+        XtX[(size_t)b * c + a] = XtX[(size_t)a * c + b] = dot8(xa, xb, n);
       }
-      double s = 0.0;
-      for (int64_t i = 0; i < n; ++i) s += (double)xa[i] * resid[i];
-      Xtr[a] = s;
+      Xtr[a] = dot8(xa, resid.data(), n);
     }
     std::vector<double> blue = spd_solve(XtX, c, Xtr);
     for (int a = 0; a < c; ++a) blue_out[a] = (float)blue[a];
@@ -853,8 +854,7 @@ void reml_grad(slemm_geno* g, const float* rvec, const float* X, int64_t ldx, in
     for (int64_t i = 0; i < n; ++i) ry[i] = (double)(S.rr[i] * y[i]);
     for (int l = 0; l < c; ++l) {
       const double* q = S.qr.Q.data() + (size_t)l * n;
-      double sum = 0.0;
-      for (int64_t i = 0; i < n; ++i) sum += q[i] * ry[i];
+      const double sum = dot8(q, ry.data(), n);
       for (int64_t i = 0; i < n; ++i) ry[i] -= sum * q[i];
     }
     for (int64_t i = 0; i < n; ++i) yproj[i] = (float)ry[i];
