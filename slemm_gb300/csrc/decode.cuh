@@ -98,12 +98,4 @@ __device__ __forceinline__ uint2 e4m3_half(const float (&d)[8])
   return make_uint2(e4m3x4(d[0], d[4], d[1], d[5], 1.f), e4m3x4(d[2], d[6], d[3], d[7], 0.25f));
 }
 
-// Exact FP32 counts of element pair q.
-__device__ __forceinline__ void f32pair_of(uint32_t word, int q, float& even, float& odd)
-{
-  const uint32_t p = bf16pair_of(word, q);
-  even = __uint_as_float(p << 16);
-  odd = __uint_as_float(p & 0xFFFF0000u);
-}
-
 }  // namespace slemm
