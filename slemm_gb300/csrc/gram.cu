@@ -354,7 +354,12 @@ spd_panel_kernel(SpdRows S, const float* __restrict__ ridge, int k0, float* __re
       __syncthreads();
       const float d = scol[buf][j];
       bad = bad || !(d > 0.f);
-      const float piv = sqrtf(fmaxf(d, 1e-30f)), inv = 1.f / piv;
+      // 1/√d to about one unit in the last place: the pivot's chain is in every step's way, and a square
+      // root and a division (IEEE) are some 40 instructions of it
+      const float dc = fmaxf(d, 1e-30f);
+      float inv = rsqrtf(dc);
+      inv = fmaf(inv * 0.5f, fmaf(-dc * inv, inv, 1.f), inv);
+      const float piv = dc * inv;
       float lk[8];
 #pragma unroll
       for (int q = jb; q < 8; ++q) lk[q] = scol[buf][tx + 16 * q] * inv;
@@ -399,13 +404,16 @@ spd_panel_kernel(SpdRows S, const float* __restrict__ ridge, int k0, float* __re
 }
 
 // Trailing update after panel k0: C[I, J] −= P_I·P_Jᵀ over the panel's tk columns, for A's row tiles
-// (J ≤ I, the lower triangle alone) and Z's (every J).  128×128 per CTA, 8×8 per thread, the panels
-// through shared memory 32 columns at a time (stride 129: no bank conflicts either way).  Bound by FP32
-// FMA issue.
-__global__ void __launch_bounds__(256)
+// (J ≤ I, the lower triangle alone) and Z's (every J).  128×128 per CTA, 8×8 per thread (rows 4ty … and
+// 64 + 4ty …, columns alike), the panels through shared memory 16 columns at a time, the next 16 loaded
+// into registers meanwhile.  Operands are read four at a time: single words cost as many shared-memory
+// cycles as the 64 FMAs they feed.  Bound by FP32 FMA issue.
+constexpr int kUD = 16;          // panel columns of one stage
+constexpr int kUS = kPT + 4;     // row stride of a staged column
+__global__ void __launch_bounds__(256, 2)
 spd_update_kernel(SpdRows S, int k0)
 {
-  __shared__ float Pa[32][kPT + 1], Pb[32][kPT + 1];
+  __shared__ __align__(16) float Pa[kUD][kUS], Pb[kUD][kUS];
   const int b = blockIdx.y;
   const int tk = min(kPT, S.s - k0), c0 = k0 + tk;
   const int nA = (S.s - c0 + kPT - 1) / kPT;
@@ -424,40 +432,57 @@ spd_update_kernel(SpdRows S, int k0)
     tj = (q - tri) % nA;
   }
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  // loads: panel column lu of rows lr, lr + 16, …
+  const int lu = threadIdx.x & 15, lr = threadIdx.x >> 4;
+  const float *base_a = S.row(b, c0, ti, 0), *base_b = S.row(b, c0, tj, 0);   // a tile has a first row
+  const int rows_a = ti < nA ? min(kPT, S.s - c0 - ti * kPT) : min(kPT, S.t[b] - (ti - nA) * kPT);
+  const int rows_b = min(kPT, S.s - c0 - tj * kPT);
+  float na[8], nb[8];
+  auto fetch = [&](int u0) {
+    const bool cu = u0 + lu < tk;
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+      const int r = lr + 16 * v;
+      na[v] = (cu && r < rows_a) ? base_a[(int64_t)r * S.ld + k0 + u0 + lu] : 0.f;
+      nb[v] = (cu && r < rows_b) ? base_b[(int64_t)r * S.ld + k0 + u0 + lu] : 0.f;
+    }
+  };
   float acc[8][8] = {};
-  for (int u0 = 0; u0 < tk; u0 += 32) {
-    for (int e = threadIdx.x; e < 32 * kPT; e += 256) {
-      const int u = e & 31, r = e >> 5;
-      const bool cu = u0 + u < tk;
-      const float* ra = S.row(b, c0, ti, r);
-      const float* rb = S.row(b, c0, tj, r);
-      Pa[u][r] = (cu && ra) ? ra[k0 + u0 + u] : 0.f;
-      Pb[u][r] = (cu && rb) ? rb[k0 + u0 + u] : 0.f;
+  fetch(0);
+  for (int u0 = 0; u0 < tk; u0 += kUD) {
+    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+      Pa[lu][lr + 16 * v] = na[v];
+      Pb[lu][lr + 16 * v] = nb[v];
     }
     __syncthreads();
-#pragma unroll 8
-    for (int u = 0; u < 32; ++u) {
+    if (u0 + kUD < tk) fetch(u0 + kUD);
+#pragma unroll
+    for (int u = 0; u < kUD; ++u) {
       float x[8], y[8];
 #pragma unroll
-      for (int v = 0; v < 8; ++v) {
-        x[v] = Pa[u][ty + 16 * v];
-        y[v] = Pb[u][tx + 16 * v];
+      for (int h = 0; h < 2; ++h) {
+        const float4 fx = *reinterpret_cast<const float4*>(&Pa[u][64 * h + 4 * ty]);
+        const float4 fy = *reinterpret_cast<const float4*>(&Pb[u][64 * h + 4 * tx]);
+        x[4 * h] = fx.x, x[4 * h + 1] = fx.y, x[4 * h + 2] = fx.z, x[4 * h + 3] = fx.w;
+        y[4 * h] = fy.x, y[4 * h + 1] = fy.y, y[4 * h + 2] = fy.z, y[4 * h + 3] = fy.w;
       }
 #pragma unroll
       for (int v = 0; v < 8; ++v)
 #pragma unroll
         for (int w = 0; w < 8; ++w) acc[v][w] = fmaf(x[v], y[w], acc[v][w]);
     }
-    __syncthreads();
   }
 #pragma unroll
   for (int v = 0; v < 8; ++v) {
-    float* row = S.row(b, c0, ti, ty + 16 * v);
-    if (!row) continue;
+    const int i = 64 * (v >> 2) + 4 * ty + (v & 3);
+    if (i >= rows_a) continue;
+    float* row = const_cast<float*>(base_a) + (int64_t)i * S.ld + c0 + tj * kPT;
 #pragma unroll
     for (int w = 0; w < 8; ++w) {
-      const int j = tj * kPT + tx + 16 * w;   // column c0 + j
-      if (c0 + j < S.s && (ti >= nA || j <= ti * kPT + ty + 16 * v)) row[c0 + j] -= acc[v][w];
+      const int j = 64 * (w >> 2) + 4 * tx + (w & 3);   // column c0 + tj·128 + j
+      if (j < rows_b && (ti != tj || j <= i)) row[j] -= acc[v][w];
     }
   }
 }
