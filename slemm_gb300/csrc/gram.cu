@@ -278,7 +278,7 @@ void gram_block(slemm_geno* g, const GramSide& R, int64_t r0, int64_t rows, cons
 // to Ld (a panel's CTAs all read the tile, so it stays as it was); the upper triangle of A keeps the
 // matrix.  One CTA per system factoring alone (a chain of 1,000 columns on one SM) took 20.4 ms for 7
 // systems of 1,000 and its triangular solves another 13.4 ms.
-constexpr int kPT = 128;   // panel width and row-tile height
+constexpr int kPT = 128;   // panel width and row-tile height of the update
 
 struct SpdRows {
   float* A;
@@ -303,53 +303,62 @@ struct SpdRows {
   }
 };
 
-// Panel k0: every CTA factors the diagonal tile (tk ≤ 128 columns) and solves its own 128 rows
-// against it in the same sweep: thread (tx, ty) holds elements (ty + 16a, tx + 16b) of both tiles, and a
-// column is published through shared memory, one barrier per column.  Bound by that chain of 128
-// steps (about 20 µs), not by its arithmetic: so the rows ride along instead of a launch of
-// their own.
-__global__ void __launch_bounds__(256)
+// Panel k0: every CTA factors the diagonal tile (tk ≤ 128 columns) and solves its own 256 rows against it
+// in the same sweep: the values wait in shared memory, thread (tx, ty) keeps the sums of products of
+// its rows' elements tx + 16q in both tiles, and a column, less its sums, is published through shared
+// memory, one barrier per column.  Bound by that chain of 128 steps, not by its arithmetic: so the rows
+// ride along instead of a launch of their own, and 512 threads on 256 rows (all of the SM's registers)
+// halve the CTAs that repeat the diagonal tile and keep the panel in one wave (129 µs for 210 CTAs of 128
+// rows and twice the instructions a step, 84 µs now).
+constexpr int kPR = 256;   // rows of one CTA
+constexpr size_t kPanelSmem = (size_t)(kPT + kPR) * kPT * sizeof(float);
+__global__ void __launch_bounds__(512, 1)
 spd_panel_kernel(SpdRows S, const float* __restrict__ ridge, int k0, float* __restrict__ Ld, int* __restrict__ status)
 {
-  __shared__ float scol[2][kPT], srow[2][kPT];
+  extern __shared__ float tiles[];
+  __shared__ __align__(16) float scol[2][kPT], srow[2][kPR];
+  float* sD = tiles;               // [128][128]
+  float* sR = tiles + kPT * kPT;   // [256][128]
   const int b = blockIdx.y, tile = blockIdx.x;
   const int tk = min(kPT, S.s - k0), c0 = k0 + tk;
-  const int nA = (S.s - c0 + kPT - 1) / kPT;
-  const int ntiles = nA + (S.t[b] + kPT - 1) / kPT;
+  const int nA = (S.s - c0 + kPR - 1) / kPR;
+  const int ntiles = nA + (S.t[b] + kPR - 1) / kPR;
   if (tile >= ntiles && tile > 0) return;
+  // this CTA's rows: nrow of them from row0, S.ld apart
+  const float* Ab = S.A + (int64_t)b * S.strideA + S.offA[b];
+  const bool inA = tile < nA;
+  const int i0 = inA ? c0 + tile * kPR : (tile - nA) * kPR;
+  const int nrow = tile < ntiles ? min(kPR, (inA ? S.s : S.t[b]) - i0) : 0;
+  float* row0 = (inA ? S.A + (int64_t)b * S.strideA : S.Z + S.offZ[b] * S.ld) + S.offA[b] + (int64_t)i0 * S.ld + k0;
+#pragma unroll 16
+  for (int e = threadIdx.x; e < kPT * kPT; e += 512) {
+    const int i = e / kPT, j = e % kPT;
+    float v = (i < tk && j <= i) ? Ab[(int64_t)(k0 + i) * S.ld + k0 + j] : 0.f;
+    if (i == j) v = i < tk ? v + ridge[(int64_t)b * S.s + k0 + i] : 1.f;
+    sD[e] = v;
+  }
+#pragma unroll 16
+  for (int e = threadIdx.x; e < kPR * kPT; e += 512) {
+    const int i = e / kPT, j = e % kPT;
+    sR[e] = (i < nrow && j < tk) ? row0[(int64_t)i * S.ld + j] : 0.f;
+  }
+  __syncthreads();
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  // D, R: Σ l·l over the columns done so far; a column's own value is subtracted from once, when its
-  // turn comes (Dv, Rv: the values of the next 16 columns, loaded a block ahead)
-  float D[8][8] = {}, R[8][8] = {}, Dv[8], Rv[8];
-  auto load = [&](int jb) {
-    const int j = tx + 16 * jb;
-#pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      const int i = ty + 16 * a;
-      const float* rrow = tile < ntiles ? S.row(b, c0, tile, i) : nullptr;
-      float v = 0.f;
-      if (i < tk && j <= i) v = S.A[(int64_t)b * S.strideA + (int64_t)(k0 + i) * S.ld + S.offA[b] + k0 + j];
-      if (i == j) v = i < tk ? v + ridge[(int64_t)b * S.s + k0 + i] : 1.f;
-      Dv[a] = v;
-      Rv[a] = (rrow && j < tk) ? rrow[k0 + j] : 0.f;
-    }
-  };
-  load(0);
+  // Σ l·l over the columns done so far; afterwards l itself.  Rows 4ty + a of D, rows 4ty + a and
+  // 128 + 4ty + a of R: a column's values are read four rows at a time
+  float D[4][8] = {}, R[8][8] = {};
+  auto rrow = [&](int a) { return 4 * ty + (a & 3) + 128 * (a >> 2); };
   bool bad = false;
 #pragma unroll
   for (int jb = 0; jb < 8; ++jb) {
-    float dv[8], rv[8];
-#pragma unroll
-    for (int a = 0; a < 8; ++a) dv[a] = Dv[a], rv[a] = Rv[a];
-    if (jb < 7) load(jb + 1);
+    const bool below = 4 * ty + 3 >= 16 * jb;   // some of this thread's rows of D are not done
     for (int jj = 0; jj < 16; ++jj) {
       const int j = 16 * jb + jj, buf = jj & 1;
       if (tx == jj) {
 #pragma unroll
-        for (int a = 0; a < 8; ++a) {
-          scol[buf][ty + 16 * a] = dv[a] - D[a][jb];
-          srow[buf][ty + 16 * a] = rv[a] - R[a][jb];
-        }
+        for (int a = 0; a < 4; ++a) scol[buf][4 * ty + a] = sD[(4 * ty + a) * kPT + j] - D[a][jb];
+#pragma unroll
+        for (int a = 0; a < 8; ++a) srow[buf][rrow(a)] = sR[rrow(a) * kPT + j] - R[a][jb];
       }
       __syncthreads();
       const float d = scol[buf][j];
@@ -359,47 +368,50 @@ spd_panel_kernel(SpdRows S, const float* __restrict__ ridge, int k0, float* __re
       const float dc = fmaxf(d, 1e-30f);
       float inv = rsqrtf(dc);
       inv = fmaf(inv * 0.5f, fmaf(-dc * inv, inv, 1.f), inv);
-      const float piv = dc * inv;
+      const float inv2 = inv * inv;   // l_i·l_k = v_i·(v_k·inv²) of the published values
       float lk[8];
 #pragma unroll
-      for (int q = jb; q < 8; ++q) lk[q] = scol[buf][tx + 16 * q] * inv;
+      for (int q = jb; q < 8; ++q) lk[q] = scol[buf][tx + 16 * q] * inv2;
       const bool own = tx == jj;
-      const bool right = tx > jj;   // column tx + 16·jb lies right of j
+      lk[jb] = tx > jj ? lk[jb] : 0.f;   // column tx + 16·jb lies right of j
 #pragma unroll
-      for (int a = 0; a < 8; ++a) {
-        const float rl = srow[buf][ty + 16 * a] * inv;
-        if (own) R[a][jb] = rl;
-        else if (right) R[a][jb] = fmaf(rl, lk[jb], R[a][jb]);
+      for (int h = 0; h < 2; ++h) {
+        const float4 v4 = *reinterpret_cast<const float4*>(&srow[buf][128 * h + 4 * ty]);
+        const float v[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
-        for (int q = jb + 1; q < 8; ++q) R[a][q] = fmaf(rl, lk[q], R[a][q]);
+        for (int a = 0; a < 4; ++a) {
+#pragma unroll
+          for (int q = jb; q < 8; ++q) R[4 * h + a][q] = fmaf(v[a], lk[q], R[4 * h + a][q]);
+          R[4 * h + a][jb] = own ? v[a] * inv : R[4 * h + a][jb];
+        }
       }
+      if (below) {
+        const float4 v4 = *reinterpret_cast<const float4*>(&scol[buf][4 * ty]);
+        const float v[4] = {v4.x, v4.y, v4.z, v4.w};
 #pragma unroll
-      for (int a = jb; a < 8; ++a) {
-        const float li = scol[buf][ty + 16 * a] * inv;
-        if (own) D[a][jb] = (ty + 16 * a == j) ? piv : li;
-        else if (right) D[a][jb] = fmaf(li, lk[jb], D[a][jb]);
+        for (int a = 0; a < 4; ++a) {
 #pragma unroll
-        for (int q = jb + 1; q < 8; ++q) D[a][q] = fmaf(li, lk[q], D[a][q]);
+          for (int q = jb; q < 8; ++q) D[a][q] = fmaf(v[a], lk[q], D[a][q]);
+          D[a][jb] = own ? v[a] * inv : D[a][jb];   // v = d on the diagonal: d/√d
+        }
       }
     }
   }
-  if (tile < ntiles) {
 #pragma unroll
-    for (int a = 0; a < 8; ++a) {
-      float* rrow = S.row(b, c0, tile, ty + 16 * a);
-      if (!rrow) continue;
+  for (int a = 0; a < 8; ++a) {
+    if (rrow(a) >= nrow) continue;
+    float* r = row0 + (int64_t)rrow(a) * S.ld;
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
-        if (tx + 16 * q < tk) rrow[k0 + tx + 16 * q] = R[a][q];
-    }
+    for (int q = 0; q < 8; ++q)
+      if (tx + 16 * q < tk) r[tx + 16 * q] = R[a][q];
   }
   if (tile == 0) {
     if (bad && threadIdx.x == 0) atomicOr(status, 1);
     float* L = Ld + ((int64_t)b * ((S.s + kPT - 1) / kPT) + k0 / kPT) * kPT * kPT;
 #pragma unroll
-    for (int a = 0; a < 8; ++a)
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
-      for (int q = 0; q < 8; ++q) L[(ty + 16 * a) * kPT + tx + 16 * q] = (tx + 16 * q <= ty + 16 * a) ? D[a][q] : 0.f;
+      for (int q = 0; q < 8; ++q) L[(4 * ty + a) * kPT + tx + 16 * q] = (tx + 16 * q <= 4 * ty + a) ? D[a][q] : 0.f;
   }
 }
 
@@ -607,10 +619,12 @@ static void spd_panels(const SpdBatch& B, const float* ridge, float* Ld, int* st
 {
   const SpdRows S = rows_of(B);
   const int nZ = (B.t_max + kPT - 1) / kPT;
+  CUDA_TRY(cudaFuncSetAttribute(spd_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmem));
   for (int k0 = 0; k0 < B.s; k0 += kPT) {
     const int c0 = std::min(k0 + kPT, B.s);
     const int nA = (B.s - c0 + kPT - 1) / kPT;
-    spd_panel_kernel<<<dim3(std::max(1, nA + nZ), B.nb), 256, 0, st>>>(S, ridge, k0, Ld, status);
+    const int pr = (B.s - c0 + kPR - 1) / kPR + (B.t_max + kPR - 1) / kPR;
+    spd_panel_kernel<<<dim3(std::max(1, pr), B.nb), 512, kPanelSmem, st>>>(S, ridge, k0, Ld, status);
     LAUNCH_CHECK();
     const int tiles = nA * (nA + 1) / 2 + nA * nZ;
     if (tiles == 0) continue;
