@@ -108,8 +108,9 @@ __device__ __forceinline__ DF hwe_ratio(int h, int rare, int n, bool down)
   return down ? df_div(den, num) : df_div(num, den);
 }
 
-// hwe_exact_p in double-float pairs; false when the case is out of its range.
-__device__ bool hwe_exact_df(int64_t het64, int64_t hom1, int64_t hom2, int midp, float* out)
+// hwe_exact_p in double-float pairs by two neighbouring lanes, one per side of the mode (lane bit 0; `pair`:
+// their mask); both return the same.  False when the case is out of its range.
+__device__ bool hwe_exact_df(int64_t het64, int64_t hom1, int64_t hom2, int midp, bool down, unsigned pair, float* out)
 {
   const int64_t n64 = het64 + hom1 + hom2;
   if (n64 == 0 || n64 >= (1 << 22)) return false;
@@ -136,26 +137,36 @@ __device__ bool hwe_exact_df(int64_t het64, int64_t hom1, int64_t hom2, int midp
   if (!(pobs.hi >= kLeast)) return false;
   const DF cut = df_norm(pobs.hi, __fmaf_rn(pobs.hi, 1e-7f, pobs.lo));
   const float stop = fminf(pobs.hi, 1.f) * 1e-18f;
-  DF tot = one, tail;
-  if (df_le(one, cut)) tail = one;
+  // this lane's side of the mode, four terms at a time: their ratios do not depend on one another, so only
+  // the products are a chain (terms past the end have ratio 0)
+  DF tot, tail, p = one;
   auto add = [](DF& s, const DF& v) {
     df_add(s, v.hi);
     s.lo = __fadd_rn(s.lo, v.lo);
   };
-  DF p = one;
-  for (int k = mode; k + 2 <= hmax; k += 2) {
-    p = df_mul(p, hwe_ratio(k, rare, n, false));
-    add(tot, p);
-    if (df_le(p, cut)) add(tail, p);
+  const int terms = down ? mode / 2 : (hmax - mode) / 2;
+  for (int t = 0; t < terms; t += 4) {
+    DF r[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (t + q < terms) r[q] = hwe_ratio(down ? mode - 2 * (t + q) - 2 : mode + 2 * (t + q), rare, n, down);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      p = df_mul(p, r[q]);
+      add(tot, p);
+      if (df_le(p, cut)) add(tail, p);
+    }
     if (p.hi < stop) break;
   }
-  p = one;
-  for (int k = mode; k >= 2; k -= 2) {
-    p = df_mul(p, hwe_ratio(k - 2, rare, n, true));
-    add(tot, p);
-    if (df_le(p, cut)) add(tail, p);
-    if (p.hi < stop) break;
+  // both sides and the mode's own term
+  for (DF* s : {&tot, &tail}) {
+    DF o;
+    o.hi = __shfl_xor_sync(pair, s->hi, 1);
+    o.lo = __shfl_xor_sync(pair, s->lo, 1);
+    add(*s, o);
   }
+  add(tot, one);
+  if (df_le(one, cut)) add(tail, one);
   if (midp) {
     df_add(tail, -0.5f * pobs.hi);
     tail.lo = __fmaf_rn(-0.5f, pobs.lo, tail.lo);
@@ -171,18 +182,21 @@ __global__ void hwe_kernel(const int32_t* __restrict__ het, const int32_t* __res
   if (j < m) p[j] = hwe_exact_p(het[j], hom1[j], hom2[j], midp);
 }
 
-// From the per-row counts of the G copy: maf (FP32, reference formula) and the HWE p-value.
+// From the per-row counts of the G copy: maf (FP32, reference formula) and the HWE p-value; two lanes per
+// SNP.
 __global__ void marker_qc_kernel(const int64_t* __restrict__ pc, const int32_t* __restrict__ c1,
                                  const int32_t* __restrict__ c2, int64_t m, int64_t n, int midp,
                                  float* __restrict__ maf, float* __restrict__ hwep)
 {
-  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= m) return;
-  const float f = (float)(int)pc[j] / (float)(2 * n);
-  maf[j] = fabsf((f > 0.5f ? 1.0f : 0.0f) - f);
+  const int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 1;
+  if (j >= m) return;   // both lanes of a pair
   const int64_t n1 = c1[j], n2 = c2[j], n0 = n - n1 - n2;
   float p;
-  hwep[j] = hwe_exact_df(n1, n0, n2, midp, &p) ? p : (float)hwe_exact_p(n1, n0, n2, midp);
+  const bool fine = hwe_exact_df(n1, n0, n2, midp, threadIdx.x & 1, 3u << (threadIdx.x & 30), &p);
+  if (threadIdx.x & 1) return;
+  const float f = (float)(int)pc[j] / (float)(2 * n);
+  maf[j] = fabsf((f > 0.5f ? 1.0f : 0.0f) - f);
+  hwep[j] = fine ? p : (float)hwe_exact_p(n1, n0, n2, midp);
 }
 
 // out[c·ld + i] = count of SNP rows[c] for kept individual i (i < n), from the G copy (at packed
@@ -242,7 +256,7 @@ int slemm_gpu_marker_qc(slemm_geno* g, int midp, float* maf, float* hwep)
     float* d_maf = reinterpret_cast<float*>(d_c2 + m);
     float* d_hwe = d_maf + m;
     row_counts_device(g, d_pc, d_c1, d_c2);
-    marker_qc_kernel<<<(unsigned)ceil_div(m, 128), 128, 0, g->stream>>>(d_pc, d_c1, d_c2, m, g->n, midp ? 1 : 0,
+    marker_qc_kernel<<<(unsigned)ceil_div(2 * m, 128), 128, 0, g->stream>>>(d_pc, d_c1, d_c2, m, g->n, midp ? 1 : 0,
                                                                         d_maf, d_hwe);
     LAUNCH_CHECK();
     CUDA_TRY(cudaMemcpyAsync(maf, d_maf, m * sizeof(float), cudaMemcpyDeviceToHost, g->stream));
