@@ -5,20 +5,25 @@
 // next element-wise pass reads.  As separate kernels that is a launch, a preamble that re-reduces the
 // previous kernel's block partials and a pass over the column for each number: 13 kernels of 4–16 µs
 // per Lanczos step at n = 50,000 with 7 columns, where the two products take 134 of 254 µs.  Here a
-// cluster of up to 8 blocks owns a column: the numbers go through distributed shared memory (one cluster
+// cluster of up to 16 blocks owns a column: the numbers go through distributed shared memory (one cluster
 // barrier each), a thread keeps its first 8 rows in registers from pass to pass, and the others are
 // re-read from L2, where a column (2 MB at n = 500,000) stays.  So an operator takes three of these
 // kernels and a Lanczos step no more.  Bound by the latency of their four to six cluster-wide reductions
 // for short columns, by L2 and HBM for long ones.  One projected operator at n = 2,000, m = 10,000 with 31
 // columns takes 63 µs (102 with ten kernels), the REML gradient at n = 50,000, m = 25,000 with 30
 // probes 5.6 ms (6.0), an MC-REML fit at n = 50,000, m = 20,000 7.3 ms (7.8); at n = 500,000 with 66 columns,
-// where the products are 95 %, nothing changes.
+// where the products are 95 %, nothing changes.  Clusters of 16 where 8 columns or fewer leave half of the
+// GPU idle with 8: that gradient 5.24 → 5.16 ms, the fit (its samples now drawn on the GPU) 4.58 → 4.52 ms.
 //
 // A thread works on half of a packed word, elements 4h … 4h + 3 and 8 + 4h … 11 + 4h: two 4-wide loads,
 // and its digits are 8 contiguous bytes of each operand row (four neighbours' would be single bytes).
 // Whole words (16 rows) took twice the registers, one block per SM, and were slower than the separate
-// kernels from 31 columns on (76 and 98 µs for the operand and the step at n = 50,000).  All sums are double-float per thread and FP64 above, in a fixed
-// order (warps, then blocks by rank), so results are bit-reproducible.
+// kernels from 31 columns on (76 and 98 µs for the operand and the step at n = 50,000).  All sums are
+// double-float per thread and FP64 above, in a fixed order (warps, then blocks by rank), so results are
+// bit-reproducible.
+//
+// The operand's padding rows (from k to kp in each piece, and up to N) are left as they are: they only
+// reach product columns that nobody reads (66 columns at n = 100,000, m = 50,000: 1,554 → 1,534 µs).
 //
 // Included by ops.cu (its operand helpers).  Every kernel waits for the one before it
 // (griddepcontrol.wait) and lets the next one be set up meanwhile.
@@ -29,7 +34,8 @@
 namespace slemm {
 
 constexpr int kColThreads = 512;   // most threads of a block (two blocks per SM: 64 registers each)
-constexpr int kColCluster = 8;     // most blocks of a column (the portable cluster size)
+constexpr int kColCluster = 16;    // most blocks of a column; more than 8, the portable size, only where
+constexpr int kColFew = 8;         // there are at most this many columns
 constexpr int kColRows = 8;        // rows of one thread and sweep
 
 struct ColPlan {
@@ -41,7 +47,7 @@ struct ColPlan {
 static ColPlan col_plan(int64_t units, int columns)
 {
   int cs = 1;
-  while (cs < kColCluster && units >= (int64_t)cs * 2 * 64 && (int64_t)columns * cs * 2 <= 2 * num_sms() * 7 / 8) cs *= 2;
+  while (cs < (columns <= kColFew ? kColCluster : 8) && units >= (int64_t)cs * 2 * 64 && (int64_t)columns * cs * 2 <= 2 * num_sms() * 7 / 8) cs *= 2;
   return {cs, (int)std::min<int64_t>(kColThreads, round_up(ceil_div(units, cs), 32))};
 }
 
@@ -61,6 +67,7 @@ static void launch_columns(void (*kernel)(P...), int64_t units, int columns, cud
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = 2;
+  if (p.cluster > 8) CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
   LAUNCH_CHECK();
 }
@@ -335,23 +342,12 @@ __device__ __forceinline__ void store_unit(const float (&x)[8], int np, void* B,
 // Units of x per unit of a remainder after kDigits digits: 32^−5·2^−e
 __device__ __forceinline__ float rest_scale(float inv_scale) { return __fmul_rn(inv_scale, 2.98023223876953125e-8f); }
 
-// Columns past k: operand padding row `row`, zeroed by its cluster.
-template <bool DIGITS>
-__device__ __forceinline__ void zero_column(void* B, int64_t K_pad, int row, int64_t units, int64_t w0, int64_t step)
-{
-  for (int64_t w = w0; w < units; w += step) {
-    uint8_t* d = static_cast<uint8_t*>(B) + ((int64_t)row * K_pad + w * 8) * (DIGITS ? 1 : 2);
-    if (DIGITS) *reinterpret_cast<uint2*>(d) = make_uint2(0u, 0u);
-    else *reinterpret_cast<uint4*>(d) = make_uint4(0u, 0u, 0u, 0u);
-  }
-}
-
 // Direction-1 operand (K = individuals) of column c: x = in − Q(Qᵀin) for c < nq, times rr, less its mean,
 // scaled to its range and split; rows that hold no individual are 0.  sums[c] = {the mean, 2^−e, and the sum
 // of what is stored as a hi+lo pair}.
 template <bool DIGITS, bool VEC>
 __global__ void __launch_bounds__(kColThreads, 2)
-col_operand_kernel(const float* __restrict__ in, int64_t ld, int64_t n, int64_t n_pad, int k, int kp,
+col_operand_kernel(const float* __restrict__ in, int64_t ld, int64_t n, int64_t n_pad, int kp,
                    const float* __restrict__ Q, int64_t ldq, int cq, int nq, const float* __restrict__ rr, int np,
                    void* B, float4* __restrict__ sums, const int32_t* __restrict__ inv)
 {
@@ -361,10 +357,6 @@ col_operand_kernel(const float* __restrict__ in, int64_t ld, int64_t n, int64_t 
   const int c = blockIdx.y;
   const int64_t units = n_pad / kColRows, w0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
-  if (c >= k) {
-    zero_column<DIGITS>(B, n_pad, pad_row(c - k, k, kp, np), units, w0, step);
-    return;
-  }
   int turn = 0;
   const float* col = in + (int64_t)c * ld;
   auto raw = [&](int64_t w, float (&x)[8]) {
@@ -478,7 +470,7 @@ template <bool DIGITS, bool FROM_D, bool VEC>
 __global__ void __launch_bounds__(kColThreads, 2)
 col_snp_kernel(const float* __restrict__ D, int splits, int kp1, const float* __restrict__ w_,
                const float4* __restrict__ sums, const float* __restrict__ gcorr, float* __restrict__ V2, const float* __restrict__ in, int64_t ld,
-               int64_t m, int64_t m_pad, int k, int kp, const float* __restrict__ gm, int np, void* B,
+               int64_t m, int64_t m_pad, int kp, const float* __restrict__ gm, int np, void* B,
                float4* __restrict__ tsums)
 {
   __shared__ ColShared S;
@@ -486,10 +478,6 @@ col_snp_kernel(const float* __restrict__ D, int splits, int kp1, const float* __
   const int c = blockIdx.y;
   const int64_t units = m_pad / kColRows, w0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
-  if (c >= k) {
-    zero_column<DIGITS>(B, m_pad, pad_row(c - k, k, kp, np), units, w0, step);
-    return;
-  }
   int turn = 0;
   const float4 s1 = FROM_D ? sums[c] : make_float4(0.f, 1.f, 0.f, 0.f);
   const float mu = s1.x, isc1 = s1.y, ch = s1.z, cl = s1.w;

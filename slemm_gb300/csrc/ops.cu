@@ -874,7 +874,6 @@ static void op_group_f16(slemm_geno* g, int kind, float tau0, const float* in, i
   float* D = (float*)g->ws_D.ensure(std::max(d1, d2) * sizeof(float));
   float4* sums = (float4*)g->ws_red.ensure((size_t)2 * k * sizeof(float4));
   float4* tsums = sums + k;
-  const int pad1 = p1.N - p1.pieces * k, pad2 = p2.N - p2.pieces * k;
   const int32_t* inv = g->is_view ? g->ind_inv.as<int32_t>() : nullptr;
   const int32_t* map = g->is_view ? g->ind_map.as<int32_t>() : nullptr;
   const float *rr = kind == SLEMM_OP_LDET ? g->rr.as<float>() : nullptr, *Q = g->Q.as<float>();
@@ -885,7 +884,7 @@ static void op_group_f16(slemm_geno* g, int kind, float tau0, const float* in, i
     const bool vec = vec4_ok(n, ld_in, in);
     auto kernel = p1.digits() ? (vec ? col_operand_kernel<true, true> : col_operand_kernel<true, false>)
                               : (vec ? col_operand_kernel<false, true> : col_operand_kernel<false, false>);
-    launch_columns(kernel, n_pad / kColRows, k + pad1, st, in, ld_in, n, n_pad, k, p1.kp, Q, n_pad, cq, h0 ? nq : 0, rr,
+    launch_columns(kernel, n_pad / kColRows, k, st, in, ld_in, n, n_pad, p1.kp, Q, n_pad, cq, h0 ? nq : 0, rr,
                    p1.pieces, B1, sums, inv);
     run_gemm(g, p1, g->G.as<uint8_t>(), m_pad, n_pad, B1, D, err, k, 1);
     if (!h0) {
@@ -899,14 +898,14 @@ static void op_group_f16(slemm_geno* g, int kind, float tau0, const float* in, i
       return;
     }
     launch_columns(p2.digits() ? col_snp_kernel<true, true, true> : col_snp_kernel<false, true, true>, m_pad / kColRows,
-                   k + pad2, st, D, p1.splits, p1.kp, w, sums, gcorr, V2, nullptr, (int64_t)0, m, m_pad, k, p2.kp, gm,
+                   k, st, D, p1.splits, p1.kp, w, sums, gcorr, V2, nullptr, (int64_t)0, m, m_pad, p2.kp, gm,
                    p2.pieces, B2, tsums);
   } else {
     const bool vec = vec4_ok(m, ld_in, in);
     auto kernel = p2.digits() ? (vec ? col_snp_kernel<true, false, true> : col_snp_kernel<true, false, false>)
                               : (vec ? col_snp_kernel<false, false, true> : col_snp_kernel<false, false, false>);
-    launch_columns(kernel, m_pad / kColRows, k + pad2, st, nullptr, 0, 0, nullptr, nullptr, nullptr, nullptr, in, ld_in, m,
-                   m_pad, k, p2.kp, gm, p2.pieces, B2, tsums);
+    launch_columns(kernel, m_pad / kColRows, k, st, nullptr, 0, 0, nullptr, nullptr, nullptr, nullptr, in, ld_in, m,
+                   m_pad, p2.kp, gm, p2.pieces, B2, tsums);
   }
   run_gemm(g, p2, g->GT.as<uint8_t>(), n_pad, m_pad, B2, D, err, k, 2);
   const float* vin = h0 ? in : nullptr;
