@@ -1,6 +1,8 @@
 """The projected Gram blocks and their batched systems (--lmm windows, slemm_gwa blocks) against the
 oracle, at the edges of the 128-column panels, of the 160- and 80-column operand groups and of the
 256-row product tiles, with and without residual weights."""
+import math
+
 import numpy as np
 import pytest
 
@@ -53,3 +55,26 @@ def test_gwa_blocks_at_panel_edges(gpu, weighted, block, n, c):
     # the oracle is the script's float32: a few hundred FP32 products and sums per entry on both sides
     for a, b in zip(got[:3], ref[:3]):
         assert np.allclose(a[ok], b[ok], rtol=1e-3, atol=1e-5 * np.abs(b[ok]).max())
+
+
+@pytest.mark.parametrize("ntest,mac", [(9, 0), (127, 60), (128, 60), (129, 200), (384, 60), (385, 10 ** 6)])
+def test_gwa_statistics_of_the_tested_range(gpu, ntest, mac):
+    """The last step of slemm_gwa: which variants are dropped, and β, se, χ² and p of the others from each
+    other, for ranges at the edges of a block of 128 variants that do not start at SNP 0."""
+    n, m, begin = 300, 400, 7
+    counts, rows, y, _, X = _data(n, m, 2, False, seed=ntest)
+    model = np.arange(begin, begin + ntest, max(1, ntest // 60))
+    cfactor, snp_var = np.float32(0.9), np.float32(0.4)
+    with api.Genotypes(rows, n) as g:
+        beta, se, chisq, p = g.gwa_windows(y, None, X, model, begin, begin + ntest - 1, 40, 1.5, model.size, cfactor,
+                                           snp_var, mac)
+    s2 = counts[begin:begin + ntest].sum(1, dtype=np.int64)
+    drop = np.minimum(s2, 2 * n - s2) <= mac
+    for v in (beta, se, chisq, p):
+        assert v.shape == (ntest,) and np.array_equal(np.isnan(v), drop)
+    ok = ~drop
+    z = beta[ok] / se[ok]   # IEEE FP32 on both sides
+    assert np.array_equal(chisq[ok], z * z)
+    # two complementary error functions (CUDA's and the C library's) of at most 5 units in the last place each
+    want = np.array([math.erfc(math.sqrt(float(x) / 2)) for x in chisq[ok]])
+    assert np.allclose(p[ok], want, rtol=10 * 2.0 ** -52, atol=0)
