@@ -20,6 +20,7 @@
 // norms are the quadratic forms (gram.cu).
 #include "internal.h"
 #include "gram.h"
+#include "qr.h"
 
 #include <algorithm>
 #include <cmath>
@@ -127,11 +128,7 @@ extern "C" int slemm_gpu_gwa_windows(slemm_geno* g, const float* y, const float*
       rr_one = rr_one && rr[i] == 1.0f;
       rr_max = std::max(rr_max, rr[i]);
     }
-    std::vector<double> A((size_t)n * c), Qd;
-    for (int j = 0; j < c; ++j)
-      for (int64_t i = 0; i < n; ++i) A[(size_t)j * n + i] = (double)(covar[(size_t)j * ldc + i] * rr[i]);
-    const int rank = orthonormal_columns(A, n, c, Qd);
-    CHECK_ARG(rank == c, "covariate matrix is not of full rank");
+    DesignQr qr(covar, ldc, rr.data(), n, c, st);
     // per-SNP means (allele-2) of the whole handle
     std::vector<float> mean(g->m_pad, 0.f);
     DevBuf d_counts(st);
@@ -143,6 +140,8 @@ extern "C" int slemm_gpu_gwa_windows(slemm_geno* g, const float* y, const float*
       CUDA_TRY(cudaStreamSynchronize(st));
       for (int64_t j = 0; j < m; ++j) mean[j] = (float)pc[j] / (float)n;
     }
+    qr.finish();
+    CHECK_ARG(qr.rank == c, "covariate matrix is not of full rank");
     // packed copy of the model SNPs, and every variant's statistics
     const int64_t K_tiles = g->n_pad / kTileK;
     const int64_t model_rows = round_up(n_model, kPadRows);
@@ -154,10 +153,8 @@ extern "C" int slemm_gpu_gwa_windows(slemm_geno* g, const float* y, const float*
     gather_rows_kernel<<<(unsigned)ceil_div(total, 256), 256, 0, st>>>(g->G.as<uint4>(), K_tiles, didx, n_model, total,
                                                                        reinterpret_cast<uint4*>(Gm));
     LAUNCH_CHECK();
-    std::vector<float> Qf((size_t)g->n_pad * c, 0.f);
-    for (int j = 0; j < c; ++j)
-      for (int64_t i = 0; i < n; ++i) Qf[(size_t)j * g->n_pad + i] = (float)Qd[(size_t)j * n + i];
-    float* dQ = (float*)d_Q.ensure(Qf.size() * sizeof(float));
+    float* dQ = (float*)d_Q.ensure((size_t)g->n_pad * c * sizeof(float));
+    qr.store(dQ, g->n_pad, g->n_pad);
     float* dmean = (float*)d_mean.ensure(mean.size() * sizeof(float));
     float* dy = (float*)d_y.ensure(n * sizeof(float));
     float* drr = nullptr;
@@ -165,7 +162,6 @@ extern "C" int slemm_gpu_gwa_windows(slemm_geno* g, const float* y, const float*
       drr = (float*)d_rr.ensure(rr.size() * sizeof(float));
       CUDA_TRY(cudaMemcpyAsync(drr, rr.data(), rr.size() * sizeof(float), cudaMemcpyHostToDevice, st));
     }
-    CUDA_TRY(cudaMemcpyAsync(dQ, Qf.data(), Qf.size() * sizeof(float), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(dmean, mean.data(), mean.size() * sizeof(float), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(dy, y, n * sizeof(float), cudaMemcpyHostToDevice, st));
     GramStatsBuf all_stats, model_stats;

@@ -121,9 +121,6 @@ struct ExactCols {
 // twos[j] = 2·Σ_i rr_i²·[count_ij = 2].  Device pointers; at least one column.
 void exact_dots(slemm_geno* g, const ExactCols& a, double* dots, double* tot, double* twos);
 
-// reml.cu — orthonormal basis (FP64 column-pivoted QR) of an n×c matrix; returns the rank.
-int orthonormal_columns(const std::vector<double>& A, int64_t n, int c, std::vector<double>& Q);
-
 // Column reductions with FP64 accumulation, deterministic two-stage (ops.cu).
 // dots[c] = Σ_i a[i,c]·b[i,c] over i < n for c < k (b == nullptr → Σ a²).  Result on device.
 void col_dots(slemm_geno* g, const float* a, int64_t lda, const float* b, int64_t ldb,

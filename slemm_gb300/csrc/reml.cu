@@ -6,6 +6,7 @@
 // libstdc++'s std::mt19937 with the reference's distributions and draw order (probes.cu), so the GPU
 // engine sees the reference's.
 #include "internal.h"
+#include "qr.h"
 #include "reduce.cuh"
 
 #include <chrono>
@@ -14,19 +15,7 @@
 namespace slemm {
 
 // ---- host dense helpers (FP64) ---------------------------------------------------------------
-// Column-pivoted Householder QR of an n×c column-major matrix (the reference uses Eigen's
-// ColPivHouseholderQR, src/reml.cpp:583-588).  Returns Q (n×rank), R·Pᵀ (rank×c) and the rank
-// under Eigen's rule |R_ii| > eps_f32·min(n,c)·|R_00|.
 // aᵀb in FP64 with eight running sums (one sum is a chain of additions, four cycles each).
-static double dot8(const double* a, const double* b, int64_t n)
-{
-  double s[8] = {};
-  int64_t i = 0;
-  for (; i + 8 <= n; i += 8)
-    for (int q = 0; q < 8; ++q) s[q] += a[i + q] * b[i + q];
-  for (; i < n; ++i) s[0] += a[i] * b[i];
-  return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
-}
 static double dot8(const float* a, const float* b, int64_t n)
 {
   double s[8] = {};
@@ -35,81 +24,6 @@ static double dot8(const float* a, const float* b, int64_t n)
     for (int q = 0; q < 8; ++q) s[q] += (double)a[i + q] * (double)b[i + q];
   for (; i < n; ++i) s[0] += (double)a[i] * (double)b[i];
   return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
-}
-
-struct QRHost {
-  std::vector<double> Q;     // n×rank
-  std::vector<double> RPt;   // rank×c (column-major)
-  int rank = 0;
-};
-
-static QRHost qr_colpiv(const std::vector<double>& A0, int64_t n, int c)
-{
-  std::vector<double> A(A0);
-  std::vector<int> perm(c);
-  std::vector<double> tau(c, 0.0);
-  for (int j = 0; j < c; ++j) perm[j] = j;
-  auto col = [&](int j) { return A.data() + (size_t)j * n; };
-  const int kmax = (int)std::min<int64_t>(n, c);
-  for (int k = 0; k < kmax; ++k) {
-    // pivot: largest remaining column norm
-    int p = k;
-    double best = -1.0;
-    for (int j = k; j < c; ++j) {
-      const double s = dot8(col(j) + k, col(j) + k, n - k);
-      if (s > best) {
-        best = s;
-        p = j;
-      }
-    }
-    if (p != k) {
-      std::swap_ranges(col(k), col(k) + n, col(p));
-      std::swap(perm[k], perm[p]);
-    }
-    double* a = col(k);
-    const double nrm = std::sqrt(best);
-    if (nrm == 0.0) {
-      tau[k] = 0.0;
-      continue;
-    }
-    const double alpha = a[k] >= 0 ? -nrm : nrm;
-    const double v0 = a[k] - alpha;
-    // v = [1, a[k+1..]/v0], tau = (alpha - a_k)/alpha ... use explicit 2/(vᵀv)
-    for (int64_t i = k + 1; i < n; ++i) a[i] /= v0;
-    tau[k] = 2.0 / (1.0 + dot8(a + k + 1, a + k + 1, n - k - 1));
-    a[k] = alpha;
-    for (int j = k + 1; j < c; ++j) {
-      double* b = col(j);
-      const double s = (b[k] + dot8(a + k + 1, b + k + 1, n - k - 1)) * tau[k];
-      b[k] -= s;
-      for (int64_t i = k + 1; i < n; ++i) b[i] -= s * a[i];
-    }
-  }
-  QRHost r;
-  const double maxpiv = kmax ? std::fabs(A[0]) : 0.0;
-  const double thr = 1.1920928955078125e-07 * kmax * maxpiv;
-  int rank = 0;
-  for (int k = 0; k < kmax; ++k)
-    if (std::fabs(A[(size_t)k * n + k]) > thr) ++rank;
-  r.rank = rank;
-  // Q = H_0 … H_{kmax−1} · I[:, :rank]
-  r.Q.assign((size_t)n * rank, 0.0);
-  for (int j = 0; j < rank; ++j) {
-    double* q = r.Q.data() + (size_t)j * n;
-    q[j] = 1.0;
-    for (int k = kmax - 1; k >= 0; --k) {
-      if (tau[k] == 0.0) continue;
-      const double* v = col(k);
-      const double s = (q[k] + dot8(v + k + 1, q + k + 1, n - k - 1)) * tau[k];
-      q[k] -= s;
-      for (int64_t i = k + 1; i < n; ++i) q[i] -= s * v[i];
-    }
-  }
-  // R·Pᵀ: column perm[j] of the result = column j of R (upper triangle)
-  r.RPt.assign((size_t)rank * c, 0.0);
-  for (int j = 0; j < c; ++j)
-    for (int i = 0; i < rank && i <= j; ++i) r.RPt[(size_t)perm[j] * rank + i] = A[(size_t)j * n + i];
-  return r;
 }
 
 // log|det M| and M^{-1} for a small c×c matrix (partial-pivot LU), column-major.
@@ -224,17 +138,16 @@ static std::vector<double> d2h(slemm_geno* g, const double* d, size_t cnt)
   return h;
 }
 
-// Common set-up of both drivers: rr, Q (rank check), gm, gw (src/reml.cpp:574-622, 757-781).
+// Common set-up of the drivers: rr, Q (rank check), gm, gw (src/reml.cpp:574-622, 757-781).
 struct Setup {
   std::vector<float> rr, gm, gw;
-  QRHost qr;
-  int c = 0;
+  std::unique_ptr<DesignQr> qr;
 };
 
-static Setup reml_setup(slemm_geno* g, const float* rvec, const float* X, int64_t ldx, int c,
-                        const float* persnp)
+// First part: rr, and the QR of rr∘X under way on the GPU.
+static Setup reml_begin(slemm_geno* g, const float* rvec, const float* X, int64_t ldx, int c)
 {
-  const int64_t n = g->n, m = g->m;
+  const int64_t n = g->n;
   CHECK_ARG(c >= 1 && c <= SLEMM_MAX_COVARIATES, "number of covariates must be in [1, SLEMM_MAX_COVARIATES]");
   Setup S;
   S.rr.resize(n);
@@ -243,16 +156,14 @@ static Setup reml_setup(slemm_geno* g, const float* rvec, const float* X, int64_
     if (!(r > 0.f) || !std::isfinite(r)) SLEMM_THROW(SLEMM_ERR_NUMERIC, "error variance weight must be > 0");
     S.rr[i] = 1.0f / std::sqrt(r);   // Eigen rsqrt
   }
-  std::vector<double> A((size_t)n * c);
-  for (int j = 0; j < c; ++j)
-    for (int64_t i = 0; i < n; ++i) {
-      const float xv = X[(size_t)j * ldx + i];
-      if (!std::isfinite(xv)) SLEMM_THROW(SLEMM_ERR_NUMERIC, "non-finite covariate");
-      A[(size_t)j * n + i] = (double)(S.rr[i] * xv);
-    }
-  S.qr = qr_colpiv(A, n, c);
-  if (S.qr.rank != c) SLEMM_THROW(SLEMM_ERR_RANK, "Fixed-effects design matrix is not of full rank.");
-  S.c = c;
+  S.qr.reset(new DesignQr(X, ldx, S.rr.data(), n, c, g->stream));
+  return S;
+}
+
+// Second part: gm and gw while the GPU factors, then the handle's projection and, if `weights`, its weights.
+static void reml_setup(Setup& S, slemm_geno* g, int c, const float* persnp, bool weights = true)
+{
+  const int64_t n = g->n, m = g->m;
   // gm = nz_bits/float(n) from the GPU popcounts (bit-exact integers)
   std::vector<int64_t> pc(m);
   {
@@ -266,28 +177,21 @@ static Setup reml_setup(slemm_geno* g, const float* rvec, const float* X, int64_
   for (int64_t j = 0; j < m; ++j) psum += persnp[j];
   const float pmean = psum / (float)m;
   S.gw.resize(m);
+  int64_t mono = m;
   for (int64_t j = 0; j < m; ++j) {
     const float v = S.gm[j] * (2.0f - S.gm[j]) / 2.0f;
     S.gw[j] = (1.0f / v) / (float)m * (persnp[j] / pmean);
-    if (!std::isfinite(S.gw[j]))
-      SLEMM_THROW(SLEMM_ERR_NUMERIC, "monomorphic SNP " + std::to_string(j) + " gives an infinite weight");
+    if (!std::isfinite(S.gw[j])) mono = std::min(mono, j);
   }
+  S.qr->finish();
+  if (!S.qr->finite) SLEMM_THROW(SLEMM_ERR_NUMERIC, "non-finite covariate");
+  if (S.qr->rank != c) SLEMM_THROW(SLEMM_ERR_RANK, "Fixed-effects design matrix is not of full rank.");
+  if (mono < m)
+    SLEMM_THROW(SLEMM_ERR_NUMERIC, "monomorphic SNP " + std::to_string(mono) + " gives an infinite weight");
+  set_projection_qr(g, *S.qr, c);
+  if (!weights) return;
   int st = slemm_gpu_set_weights(g, S.gm.data(), S.gw.data(), S.rr.data());
   if (st != SLEMM_OK) SLEMM_THROW(st, "set_weights failed");
-  std::vector<float> Qf((size_t)n * c);
-  for (size_t i = 0; i < Qf.size(); ++i) Qf[i] = (float)S.qr.Q[i];
-  st = slemm_gpu_set_projection(g, Qf.data(), n, c);
-  if (st != SLEMM_OK) SLEMM_THROW(st, "set_projection failed");
-  return S;
-}
-
-// Orthonormal basis of the columns of an n×c matrix (column-pivoted Householder QR, FP64); returns
-// the numerical rank and Q (n×rank).
-int orthonormal_columns(const std::vector<double>& A, int64_t n, int c, std::vector<double>& Q)
-{
-  QRHost r = qr_colpiv(A, n, c);
-  Q = std::move(r.Q);
-  return r.rank;
 }
 
 static void upload(slemm_geno* g, float* d, const float* h, size_t cnt)
@@ -339,28 +243,17 @@ void reml_sldf(slemm_geno* g, const float* rvec, const float* X, int64_t ldx, in
   d_X.ensure((size_t)n * tQV * sizeof(float));
   // scalars: projection coefficients (up to c×c) first, one more value from offset c·c
   d_tmp.ensure((size_t)std::max<int64_t>(n, m) * 4 * sizeof(double) + ((size_t)c * c + 64) * sizeof(double));
-  // Rademacher probes (src/reml.cpp:597-605), the reference's mt19937 draws generated on the GPU;
-  // launched first so that the host set-up below runs while they are drawn
+  Setup S = reml_begin(g, rvec, X, ldx, c);
+  // Rademacher probes (src/reml.cpp:597-605), the reference's mt19937 draws generated on the GPU while the
+  // host set-up below runs
   rademacher_device(o.seed, n, n_V, d_QV.as<float>() + (size_t)(1 + c) * n, n, g->stream);
-  Setup S = reml_setup(g, rvec, X, ldx, c, persnp);
-  // y_proj = (I − QQᵀ)(rr∘y)   (src/reml.cpp:591-592), FP64 on the host
-  std::vector<float> yproj(n);
-  {
-    std::vector<double> ry(n);
-    for (int64_t i = 0; i < n; ++i) ry[i] = (double)(S.rr[i] * y[i]);
-    for (int l = 0; l < c; ++l) {
-      const double* q = S.qr.Q.data() + (size_t)l * n;
-      const double s = dot8(q, ry.data(), n);
-      for (int64_t i = 0; i < n; ++i) ry[i] -= s * q[i];
-    }
-    for (int64_t i = 0; i < n; ++i) yproj[i] = (float)ry[i];
-  }
+  reml_setup(S, g, c, persnp);
+  // y_proj = (I − QQᵀ)(rr∘y)   (src/reml.cpp:591-592), in FP64
+  upload(g, d_y.as<float>(), y, n);
+  S.qr->project(d_y.as<float>(), d_QV.as<float>(), false);
+  S.qr->store(d_QV.as<float>() + n, n, n);
+  CUDA_TRY(cudaMemcpyAsync(d_y.p, d_QV.p, (size_t)n * sizeof(float), cudaMemcpyDeviceToDevice, st));
   if (verbose) printf("Projected covariates out of phenotypes.\nGenerating %d Rademacher probing vectors.\n", n_V);
-  std::vector<float> QV((size_t)n * (1 + c));
-  std::copy(yproj.begin(), yproj.end(), QV.begin());
-  for (size_t i = 0; i < (size_t)n * c; ++i) QV[(size_t)n + i] = (float)S.qr.Q[i];
-  upload(g, d_y.as<float>(), yproj.data(), n);
-  upload(g, d_QV.as<float>(), QV.data(), (size_t)n * (1 + c));
   const double t_a = stamp();
   double* d_scal = d_tmp.as<double>();
 
@@ -496,7 +389,7 @@ void reml_sldf(slemm_geno* g, const float* rvec, const float* X, int64_t ldx, in
     col_dots(g, d_S + (size_t)l * n, n, d_y.as<float>(), n, n, 1, d_scal + (size_t)c * c);
     Sty[l] = d2h(g, d_scal + (size_t)c * c, 1)[0];
   }
-  const std::vector<double>& R = S.qr.RPt;   // c×c
+  const std::vector<double>& R = S.qr->RPt;   // c×c
   std::vector<double> XtHX((size_t)c * c, 0.0), rhs(c, 0.0), T((size_t)c * c, 0.0);
   for (int i = 0; i < c; ++i)          // T = (QᵀS)·R
     for (int j = 0; j < c; ++j) {
@@ -579,9 +472,10 @@ void reml_lmc(slemm_geno* g, const float* rvec, const float* X, int64_t ldx, int
     printf("Generating %d MC samples for genetic effects.\n", n_MC);
     printf("Generating %d MC samples for residuals.\n", n_MC);
   }
+  Setup S = reml_begin(g, rvec, X, ldx, c);
   NormalDraws draws(o.seed, (int64_t)m * n_MC, d_u.as<float>(), (int64_t)n * n_MC, d_V.as<float>() + (size_t)(1 + n_MC) * n,
                     st);
-  Setup S = reml_setup(g, rvec, X, ldx, c, persnp);
+  reml_setup(S, g, c, persnp);
   draws.finish();
   d_PV.ensure((size_t)n * tV * sizeof(float));
   d_Py.ensure((size_t)n * (1 + n_MC) * sizeof(float));
@@ -838,28 +732,20 @@ void reml_grad(slemm_geno* g, const float* rvec, const float* X, int64_t ldx, in
   const int t = 1 + n_V, k = 1 + 2 * n_V;
   DevBuf d_B(st), d_X(st), d_U(st), d_T(st), d_s(st);
   d_B.ensure((size_t)n * t * sizeof(float));
+  Setup S = reml_begin(g, rvec, X, ldx, c);
   // probes straight into the block, drawn while the host set-up runs
   rademacher_device(seed, n, n_V, d_B.as<float>() + n, n, st);
-  Setup S = reml_setup(g, rvec, X, ldx, c, persnp);
+  reml_setup(S, g, c, persnp, false);
   std::vector<float> W(m);
   for (int64_t j = 0; j < m; ++j) W[j] = S.gw[j] * ((window && window[j] >= 0) ? wwin[window[j]] : 1.0f);
   {
     const int s2 = slemm_gpu_set_weights(g, S.gm.data(), W.data(), S.rr.data());
     if (s2 != SLEMM_OK) SLEMM_THROW(s2, "set_weights failed");
   }
-  // ỹ_proj = (I − QQᵀ)(rr∘y) on the host in FP64, as the DF-REML path
-  std::vector<float> yproj(n);
-  {
-    std::vector<double> ry(n);
-    for (int64_t i = 0; i < n; ++i) ry[i] = (double)(S.rr[i] * y[i]);
-    for (int l = 0; l < c; ++l) {
-      const double* q = S.qr.Q.data() + (size_t)l * n;
-      const double sum = dot8(q, ry.data(), n);
-      for (int64_t i = 0; i < n; ++i) ry[i] -= sum * q[i];
-    }
-    for (int64_t i = 0; i < n; ++i) yproj[i] = (float)ry[i];
-  }
-  upload(g, d_B.as<float>(), yproj.data(), n);
+  // ỹ_proj = (I − QQᵀ)(rr∘y) in FP64, as the DF-REML path
+  d_X.ensure((size_t)n * t * sizeof(float));
+  upload(g, d_X.as<float>(), y, n);
+  S.qr->project(d_X.as<float>(), d_B.as<float>(), false);
   // U's last n_V columns keep the raw probes; the block's get projected
   d_U.ensure((size_t)n * k * sizeof(float));
   CUDA_TRY(cudaMemcpyAsync(d_U.as<float>() + (size_t)(1 + n_V) * n, d_B.as<float>() + n, (size_t)n * n_V * sizeof(float),
@@ -873,7 +759,6 @@ void reml_grad(slemm_geno* g, const float* rvec, const float* X, int64_t ldx, in
   const float tau = (float)(se2 / sg2);
   slemm_lseed* sd = lanczos_seed_device(g, SLEMM_OP_QUADFORM, tau, d_B.as<float>(), t, tol, 600, false, {1, n_V}, 5, t);
   std::unique_ptr<slemm_lseed, void (*)(slemm_lseed*)> hold(sd, lseed_free);
-  d_X.ensure((size_t)n * t * sizeof(float));
   lanczos_solve_device(sd, 0.0, 1e-6, d_X.as<float>(), n, 0);
   lanczos_solve_device(sd, 0.0, 1e-6, d_X.as<float>() + n, n, 1);
   proj_coeffs(g, d_X.as<float>(), n, t, d_scal);

@@ -12,6 +12,7 @@
 // diagonal tile, one CTA per tile below solves the panel, and a shared-memory tiled FP32
 // SYRK/GEMM updates the trailing lower triangle; the triangular solves are blocked the same way.
 #include "internal.h"
+#include "qr.h"
 #include "reduce.cuh"
 #include "dense.cuh"
 
@@ -185,42 +186,32 @@ extern "C" int slemm_gpu_wls(slemm_geno* g, const float* rvec, const float* X, i
     const int64_t n = g->n, m = g->m;
     CHECK_ARG(c >= 1 && c <= SLEMM_MAX_COVARIATES && ldx >= n, "bad covariate matrix");
     cudaStream_t st = g->stream;
-    // rr, Q, y_proj on the host (FP64 QR); gm from the exact popcounts
+    // rr; Q and y_proj in FP64 on the GPU (qr.cu); gm from the exact popcounts
     std::vector<float> rr(n);
     for (int64_t i = 0; i < n; ++i) {
       const float r = rvec ? rvec[i] : 1.0f;
       CHECK_ARG(r > 0.f && std::isfinite(r), "error variance weight must be > 0");
       rr[i] = 1.0f / std::sqrt(r);
     }
-    std::vector<double> A((size_t)n * c), Qd;
-    for (int j = 0; j < c; ++j)
-      for (int64_t i = 0; i < n; ++i) A[(size_t)j * n + i] = (double)(X[(size_t)j * ldx + i] * rr[i]);
-    CHECK_ARG(orthonormal_columns(A, n, c, Qd) == c, "Fixed-effects design matrix is not of full rank.");
-    std::vector<float> yp(n);
-    {
-      std::vector<double> v(n);
-      for (int64_t i = 0; i < n; ++i) v[i] = (double)(rr[i] * y[i]);
-      for (int l = 0; l < c; ++l) {
-        const double* q = Qd.data() + (size_t)l * n;
-        double s = 0.0;
-        for (int64_t i = 0; i < n; ++i) s += q[i] * v[i];
-        for (int64_t i = 0; i < n; ++i) v[i] -= s * q[i];
-      }
-      for (int64_t i = 0; i < n; ++i) yp[i] = (float)(rr[i] * (float)v[i]);   // rr∘y_proj
-    }
+    DesignQr qr(X, ldx, rr.data(), n, c, st);
+    qr.finish();
+    CHECK_ARG(qr.rank == c, "Fixed-effects design matrix is not of full rank.");
+    DevBuf d_yraw(st), d_y(st);
+    float* yraw = (float*)d_yraw.ensure(n * sizeof(float));
+    float* dy = (float*)d_y.ensure(n * sizeof(float));   // rr∘y_proj
+    CUDA_TRY(cudaMemcpyAsync(yraw, y, n * sizeof(float), cudaMemcpyHostToDevice, st));
+    qr.project(yraw, dy, true);
     std::vector<int64_t> pc(m);
     int stc = slemm_gpu_genotype_counts(g, pc.data(), nullptr, nullptr, nullptr);
     if (stc != SLEMM_OK) SLEMM_THROW(stc, "genotype counts failed");
-    std::vector<float> gm(m), ones(m, 1.0f), Qf((size_t)n * c);
+    std::vector<float> gm(m), ones(m, 1.0f);
     for (int64_t j = 0; j < m; ++j) gm[j] = (int)pc[j] / (float)n;
-    for (size_t i = 0; i < Qf.size(); ++i) Qf[i] = (float)Qd[i];
     stc = slemm_gpu_set_weights(g, gm.data(), ones.data(), rr.data());
     if (stc != SLEMM_OK) SLEMM_THROW(stc, "set_weights failed");
-    stc = slemm_gpu_set_projection(g, Qf.data(), n, c);
-    if (stc != SLEMM_OK) SLEMM_THROW(stc, "set_projection failed");
+    set_projection_qr(g, qr, c);
     // Z̃ᵀZ̃ (lower part) and Z̃ᵀy_proj
     const int64_t lda = m;
-    DevBuf d_A(st), d_U(st), d_qt(st), d_y(st), d_b(st), d_d(st), d_st(st), d_x(st);
+    DevBuf d_A(st), d_U(st), d_qt(st), d_b(st), d_d(st), d_st(st), d_x(st);
     float* Am = (float*)d_A.ensure((size_t)lda * m * sizeof(float));
     const int kc = 1024;
     float* U = (float*)d_U.ensure((size_t)n * kc * sizeof(float));
@@ -238,9 +229,7 @@ extern "C" int slemm_gpu_wls(slemm_geno* g, const float* rvec, const float* X, i
       const int64_t r0 = j0 / kPadRows * kPadRows;
       rows_product(g, r0, g->m_pad - r0, U, n, k, Am + j0 * lda + r0, lda, SLEMM_PREC_FP16X2);
     }
-    float* dy = (float*)d_y.ensure(n * sizeof(float));
     float* b = (float*)d_b.ensure(g->m_pad * sizeof(float));
-    CUDA_TRY(cudaMemcpyAsync(dy, yp.data(), n * sizeof(float), cudaMemcpyHostToDevice, st));
     rows_product(g, 0, g->m_pad, dy, n, 1, b, g->m_pad, SLEMM_PREC_FP16X2);
     check_device_error(g);
     // ridge: 1e-4·mean(diag) (src/wls.cpp:123)
