@@ -174,8 +174,26 @@ gram_operand_kernel(const uint32_t* __restrict__ G, int64_t K_tiles, int64_t j0,
   *reinterpret_cast<uint4*>(dst + (int64_t)kp * K_pad) = lo;
 }
 
-// out[c·ldo + i] = Σ_splits D·isc − gm_row·h_c − p_row·gm_c − t_rowᵀt_c for product row i (SNP r0 + i)
-// and column c (SNP c0 + c); double-float sums.  Rows past the matrix are left alone.
+// Σ_splits D·isc − gm_row·h_c − p_row·gm_c − t_rowᵀt_c of product row i (SNP r) and column cc of group grp
+// (SNP c); double-float sums.
+__device__ __forceinline__ float gram_entry(const float* __restrict__ D, int splits, int kp, int64_t rows, int64_t i, int grp,
+                                            int cc, float isc, const GramStats& rs, int64_t r, const GramStats& cs, int64_t c,
+                                            int cq)
+{
+  const float* Dc = D + ((int64_t)grp * splits * kp + cc) * rows + i;
+  DF a;
+#pragma unroll 4
+  for (int s = 0; s < splits; ++s) df_add(a, __fmul_rn(Dc[(int64_t)s * kp * rows], isc));
+  const float2 h = cs.h[c], p = rs.p[r];
+  const float gr = rs.gm[r], gc = cs.gm[c];
+  df_fma(a, -gr, h.x);
+  df_fma(a, -p.x, gc);
+  a.lo = __fmaf_rn(-gr, h.y, __fmaf_rn(-p.y, gc, a.lo));
+  for (int l = 0; l < cq; ++l) df_fma(a, -rs.t[(int64_t)l * rs.ld + r], cs.t[(int64_t)l * cs.ld + c]);
+  return __fadd_rn(a.hi, a.lo);
+}
+
+// out[c·ldo + i] of every product row i (SNP r0 + i) and column c (SNP c0 + c).  Rows past the matrix are left alone.
 __global__ void __launch_bounds__(256)
 gram_finish_kernel(const float* __restrict__ D, int splits, int kp, int64_t rows, int64_t nrows, int kc, float isc,
                    GramStats rs, int64_t r0, GramStats cs, int64_t c0, int cq, float* __restrict__ out, int64_t ldo)
@@ -183,45 +201,68 @@ gram_finish_kernel(const float* __restrict__ D, int splits, int kp, int64_t rows
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= nrows) return;
   const int64_t c = blockIdx.y;
-  const int grp = (int)(c / kc), cc = (int)(c % kc);
-  const float* Dc = D + ((int64_t)grp * splits * kp + cc) * rows + i;
-  DF a;
-  for (int s = 0; s < splits; ++s) df_add(a, __fmul_rn(Dc[(int64_t)s * kp * rows], isc));
-  const float2 h = cs.h[c0 + c], p = rs.p[r0 + i];
-  const float gr = rs.gm[r0 + i], gc = cs.gm[c0 + c];
-  df_fma(a, -gr, h.x);
-  df_fma(a, -p.x, gc);
-  a.lo = __fmaf_rn(-gr, h.y, __fmaf_rn(-p.y, gc, a.lo));
-  for (int l = 0; l < cq; ++l) df_fma(a, -rs.t[(int64_t)l * rs.ld + r0 + i], cs.t[(int64_t)l * cs.ld + c0 + c]);
-  out[c * ldo + i] = __fadd_rn(a.hi, a.lo);
+  out[c * ldo + i] = gram_entry(D, splits, kp, rows, i, (int)(c / kc), (int)(c % kc), isc, rs, r0 + i, cs, c0 + c, cq);
 }
 
-// Split-K count of a product of `ctas` CTAs without splits: the count whose CTAs fill the last wave
-// best, each with at least 48 K-tiles (a CTA's ramp and epilogue cost about eight).
+// The same of a block of a symmetric product, for its entries with r0 + i ≤ c0 + c; with `mirror` each of
+// them also at the other half's place, product row c0 + c − r0 and column r0 + i − c0 (where that is one of the
+// ncols columns from c00), through shared memory so that both writes are whole lines.  Columns c0 … c0 + nc − 1
+// are those from c0 − c00 of out.
+__global__ void __launch_bounds__(256)
+gram_finish_sym_kernel(const float* __restrict__ D, int splits, int kp, int64_t rows, int64_t nrows, int kc, float isc,
+                       GramStats st, int64_t r0, int64_t c0, int64_t nc, int64_t c00, int64_t ncols, int cq,
+                       float* __restrict__ out, int64_t ldo, int mirror)
+{
+  __shared__ float tile[32][33];
+  const int64_t i0 = (int64_t)blockIdx.x * 32, ct = (int64_t)blockIdx.y * 32;
+  if (r0 + i0 > c0 + min64(ct + 31, nc - 1)) return;   // past every column's SNP
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  const int64_t i = i0 + x;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int64_t c = ct + y + 8 * q;
+    if (i >= nrows || c >= nc || r0 + i > c0 + c) continue;
+    const float v = gram_entry(D, splits, kp, rows, i, (int)(c / kc), (int)(c % kc), isc, st, r0 + i, st, c0 + c, cq);
+    out[(c0 - c00 + c) * ldo + i] = v;
+    tile[y + 8 * q][x] = v;
+  }
+  if (!mirror) return;
+  __syncthreads();
+  const int64_t c = ct + x;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int64_t k = i0 + y + 8 * q, col = r0 + k - c00;   // product row k becomes column col
+    if (k < nrows && c < nc && r0 + k < c0 + c && col >= 0 && col < ncols) out[col * ldo + c0 + c - r0] = tile[x][y + 8 * q];
+  }
+}
+
+// Split-K count of a product of `ctas` CTAs without splits: the least time in K-tiles of a CTA, its waves
+// times their K-tiles and what each split costs beside them (ramp, epilogue, and its partial sums written and
+// read again by the finishing kernel).  Anything from 24 to 64 is within a percent at n = 7,000 to 50,000; 8,
+// the ramp and epilogue alone, took 1 to 3 % more of the calls.
+constexpr int64_t kSplitTiles = 32;
 static int gram_splits(int64_t ctas, int64_t K_tiles, int64_t min_splits)
 {
-  int best = (int)min_splits;
-  double best_eff = -1.0;
-  for (int64_t s = min_splits; s == min_splits || K_tiles / s >= 48; ++s) {
-    const double waves = (double)(ctas * s) / num_sms();
-    const double eff = waves / std::ceil(waves) * (1.0 - 8.0 / (8.0 + (double)K_tiles / s));
-    if (eff > best_eff + 1e-9) {
-      best_eff = eff;
-      best = (int)s;
+  int64_t best = min_splits, best_cost = INT64_MAX;
+  for (int64_t s = min_splits; s == min_splits || (K_tiles / s >= 48 && s <= 64); ++s) {
+    const int64_t cost = ceil_div(ctas * s, num_sms()) * (ceil_div(K_tiles, s) + kSplitTiles);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = s;
     }
-    if (s > 64) break;
   }
-  return best;
+  return (int)best;
 }
 
 void gram_block(slemm_geno* g, const GramSide& R, int64_t r0, int64_t rows, const GramSide& C, int64_t c0, int64_t ncols,
-                int cq, const float* rr, float rr_max, float* out, int64_t ldo)
+                int cq, const float* rr, float rr_max, float* out, int64_t ldo, GramHalf half)
 {
   CHECK_ARG(r0 % kPadRows == 0 && rows % kPadRows == 0 && r0 + rows <= round_up(R.m, kPadRows), "row range not aligned");
   if (ncols <= 0) return;
   cudaStream_t st = g->stream;
   const int64_t K_pad = g->n_pad, K_tiles = K_pad / kTileK;
   const bool unit = rr == nullptr;
+  CHECK_ARG(half == GramHalf::all || (R.G == C.G && c0 >= r0 && c0 + ncols <= r0 + rows), "not a symmetric block");
   // |rr²·z| ≤ 2·max rr²: the bound lies in [2^10, 2^11) after scaling (ops.cu, split_exp)
   int e = 0;
   if (!unit) {
@@ -246,8 +287,13 @@ void gram_block(slemm_geno* g, const GramSide& R, int64_t r0, int64_t rows, cons
   for (int64_t g0 = 0; g0 < groups; g0 += per) {
     const int ng = (int)std::min(per, groups - g0);
     const int64_t first = g0 * kc, nc = std::min<int64_t>((int64_t)ng * kc, ncols - first);
+    // CTAs with work: half of them or so where only one half is wanted
+    const int64_t diag = c0 + first - r0;
+    int64_t live = 0;
+    for (int z = 0; z < ng; ++z)
+      live += half == GramHalf::all ? rctas : std::min(rctas, ceil_div(diag + (int64_t)(z + 1) * kc, rows / rctas));
     // an integer partial sum of 2^22 elements is at most 2^24: exact in FP32
-    const int splits = gram_splits(rctas * ng, K_tiles, ceil_div(K_pad, (int64_t)1 << 22));
+    const int splits = gram_splits(live, K_tiles, ceil_div(K_pad, (int64_t)1 << 22));
     void* B = g->ws_B.ensure((size_t)ng * group_bytes);
     float* D = (float*)g->ws_D.ensure((size_t)ng * splits * kp * rows * sizeof(float));
     const uint32_t* Gc = reinterpret_cast<const uint32_t*>(C.G);
@@ -260,7 +306,18 @@ void gram_block(slemm_geno* g, const GramSide& R, int64_t r0, int64_t rows, cons
     LAUNCH_CHECK();
     GemmArgs a{A, rows, K_pad, B, N, D, splits, g->err.as<int>(), kp, unit ? 1 : 2, !unit, plan};
     a.groups = ng;
+    if (half != GramHalf::all) {
+      a.diag = diag;
+      a.diag_step = kc;
+    }
     gemm_tc(a, st);
+    if (half != GramHalf::all) {
+      gram_finish_sym_kernel<<<dim3((unsigned)ceil_div(nrows, 32), (unsigned)ceil_div(nc, 32)), 256, 0, st>>>(
+          D, splits, kp, rows, nrows, kc, (float)std::ldexp(1.0, -e), R.stats, r0, c0 + first, nc, c0, ncols, cq, out, ldo,
+          half == GramHalf::mirrored ? 1 : 0);
+      LAUNCH_CHECK();
+      continue;
+    }
     gram_finish_kernel<<<dim3((unsigned)ceil_div(nrows, 256), (unsigned)nc), 256, 0, st>>>(
         D, splits, kp, rows, nrows, kc, (float)std::ldexp(1.0, -e), R.stats, r0, C.stats, c0 + first, cq,
         out + first * ldo, ldo);

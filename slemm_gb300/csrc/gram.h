@@ -49,8 +49,11 @@ struct GramSide {
 // out[c·ldo + i] = (P(rr∘z_{r0+i}))ᵀ(P(rr∘z_{c0+c})) for product rows r0 … r0 + rows − 1 of R (multiples
 // of 256; rows past R.m are not written) and columns c0 … c0 + ncols − 1 of C.  g gives the stream,
 // the work buffers and the individuals; rr (n_pad) == nullptr: all 1, else rr_max ≥ max|rr|.
+// With R and C the same side: `lower` wants the rows up to each column's own SNP alone (out's others are
+// left alone or hold sums of their own), `mirrored` has the columns' SNPs from the other half as well.
+enum class GramHalf { all, lower, mirrored };
 void gram_block(slemm_geno* g, const GramSide& R, int64_t r0, int64_t rows, const GramSide& C, int64_t c0, int64_t ncols,
-                int cq, const float* rr, float rr_max, float* out, int64_t ldo);
+                int cq, const float* rr, float rr_max, float* out, int64_t ldo, GramHalf half = GramHalf::all);
 
 // A batch of nb systems of s unknowns (layout in gram.cu); offA, offZ and t are device arrays.
 struct SpdBatch {

@@ -198,7 +198,8 @@ extern "C" int slemm_gpu_gwa_windows(slemm_geno* g, const float* y, const float*
         off[bn + bi] = lo[b0 + bi] - lo[b0];
         tb[bi] = (int)(hi[b0 + bi] - lo[b0 + bi]);
         t_max = std::max(t_max, tb[bi]);
-        gram_block(g, model, r0, r1 - r0, model, s0, bs, c, drr, rr_max, gram + (size_t)bi * stride, rows_max);
+        gram_block(g, model, r0, r1 - r0, model, s0, bs, c, drr, rr_max, gram + (size_t)bi * stride, rows_max,
+                   GramHalf::lower);
         gram_block(g, model, r0, r1 - r0, all, lo[b0 + bi], tb[bi], c, drr, rr_max, Z + off[bn + bi] * rows_max, rows_max);
       }
       float* dr = (float*)d_ridge.ensure(ridge.size() * sizeof(float));

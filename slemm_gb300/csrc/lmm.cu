@@ -150,7 +150,8 @@ extern "C" int slemm_gpu_lmm_quadforms(slemm_geno* g, const float* Py, float tau
       for (int t = 0; t < ws; ++t) dd[(size_t)c * ws + t] = tau1 / gw[wds + t];
       const int64_t r0 = wds / kPadRows * kPadRows;
       const int64_t r1 = std::min<int64_t>(round_up(wds + ws, kPadRows), g->m_pad);
-      gram_block(g, side, r0, r1 - r0, side, wds, ws, g->c, rr, g->rr_max, gram + (size_t)c * stride, rows_max);
+      gram_block(g, side, r0, r1 - r0, side, wds, ws, g->c, rr, g->rr_max, gram + (size_t)c * stride, rows_max,
+                 GramHalf::mirrored);
       idx[c] = wds - r0;   // this window's Gram starts at row wds − r0 of its block
       idx[k + c] = (int64_t)c * (ws + 1);
       idx[2 * k + c] = j - wds;
