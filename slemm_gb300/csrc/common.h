@@ -200,8 +200,8 @@ struct GemmArgs {
   bool twos = false;    // TC, plan 2: the matrix is 2·[count = 2] instead of the count
   int groups = 1;       // TC: products of as many operands B[grp] (N rows each, one after the other) with
                         // the same matrix, partials [groups][splits][kp][M_pad]
-  int64_t diag = 0;     // TC, with diag_step > 0: only row i ≤ diag + c of column c of group grp is wanted, c
-  int diag_step = 0;    // counted from grp·diag_step (a group's columns): blocks past all of theirs write nothing
+  const int2* table = nullptr;   // TC: group grp takes the row tiles from table[grp].x of A on, and only those
+                        // below table[grp].y of its own (blocks past them write nothing); device memory
 };
 
 void gemm_simt(const GemmArgs& a, cudaStream_t st);

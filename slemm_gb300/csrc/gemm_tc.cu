@@ -297,10 +297,10 @@ template <int PK, int S, int SB, int KT, Fmt FMT, int TM, bool TWOS>
 __global__ void __launch_bounds__(tc_max_threads(TM), tc_min_blocks(TM))
 gemm_tc_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMap tmapB,
                float* __restrict__ D, int64_t M_pad, int K_tiles, int tiles_per_split, int N, int sub,
-               int kp, int pieces, int* __restrict__ err, int withhold, int64_t diag, int diag_step)
+               int kp, int pieces, int* __restrict__ err, int withhold, const int2* __restrict__ table)
 {
-  // a symmetric product's block whose rows all lie past its columns
-  if (diag_step > 0 && (int64_t)blockIdx.x * sub * kTileM >= diag + (int64_t)(blockIdx.z + 1) * diag_step) return;
+  const int2 where = table != nullptr ? table[blockIdx.z] : make_int2(0, INT_MAX);
+  if ((int)blockIdx.x * sub >= where.y) return;   // rows that nobody wants
   extern __shared__ uint8_t smem_raw[];
   // 1024-byte alignment of the shared-window address (SWIZZLE_128B tiles need it)
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -378,7 +378,7 @@ gemm_tc_kernel(const uint8_t* __restrict__ A, const __grid_constant__ CUtensorMa
         const int kt = kt0 + j * kPkg;
         uint8_t* dst = sPk + (size_t)s * sub * kPkg * kTileBytes;
         for (int t = 0; t < sub; ++t)
-          bulk_copy_g2s(dst + (size_t)t * kPkg * kTileBytes, A + ((size_t)(mt0 + t) * K_tiles + kt) * kTileBytes, bytes,
+          bulk_copy_g2s(dst + (size_t)t * kPkg * kTileBytes, A + ((size_t)(where.x + mt0 + t) * K_tiles + kt) * kTileBytes, bytes,
                         &pk_full[s]);
         ++issued;
       }
@@ -649,7 +649,7 @@ static void launch_tc(const GemmArgs& a, cudaStream_t st)
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_tc_kernel<PK, S, SB, KT, FMT, TM, TWOS>, a.A, map, a.D, a.M_pad, K_tiles, tps,
-                              a.N, P.sub, a.kp, a.pieces, a.err, g_withhold_b.exchange(-1), a.diag, a.diag_step));
+                              a.N, P.sub, a.kp, a.pieces, a.err, g_withhold_b.exchange(-1), a.table));
   LAUNCH_CHECK();
 }
 

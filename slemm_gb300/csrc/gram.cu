@@ -10,8 +10,8 @@
 // product is an exact integer, and Σ_i x_ij·z_ik = Σ_i x_ij·x_ik − p_j·gm_k with p_j = Σ_i x_ij.  Forming U = rr∘P(rr∘z) as FP32
 // columns instead (centre, project, scale, measure, split: nine passes over n × columns floats)
 // took 38 of the 82 ms of slemm_gwa at n = 50,021 with 20,011 variants and 4,000 model SNPs, and
-// 31 of the 73 ms of --lmm with 30 windows of 1,000 SNPs at n = 50,000; the two calls now take 5.8
-// and 8.1 ms (7.3 and 9.5 with the counts as FP16).
+// 31 of the 73 ms of --lmm with 30 windows of 1,000 SNPs at n = 50,000; the two calls now take 3.3
+// and 6.1 ms.
 #include "gram.h"
 #include "decode.cuh"
 #include "reduce.cuh"
@@ -94,52 +94,55 @@ void gram_stats_gather(const GramStats& src, const int64_t* d_idx, int64_t cnt, 
 }
 
 // ---- Gram blocks ----------------------------------------------------------------------------------
-// Operand of the columns SNP j0 … j0 + ncols − 1, group by group: column c is row c % kc of group
-// c / kc, a group's rows kc … kp − 1 are zero.
+// A block's columns go in groups of at most kp; a launch takes groups of several blocks.  The operand of a
+// group are the columns SNP c0 … c0 + nc − 1, row c of kp each; rows nc … kp − 1 only reach sums that
+// nobody reads and stay as they are.
+struct GramGroup {
+  int64_t r0, nrows;   // SNP of the product's first row, rows that exist
+  int64_t c0, nc;      // SNP of the group's first column, columns
+  int64_t b0, bc;      // the block's first column's SNP and columns
+  float* out;          // the block's first column
+};
 //
 // Every rr 1: N = kp rows of counts as E4M3 bytes in the decoded order of the matrix's own words
 // (decode.cuh), so the product takes one MMA per 32 individuals and its sums are exact integers.  One
 // word (16 individuals) per thread; a count x ∈ {0, 1, 2} in a byte is x·0x38 − [x = 2]·0x30 (E4M3 0, 1,
 // 2), or x·0x28 − [x = 2]·0x20 times 2^−2, four at a time.  Bound by the bytes it writes.
 __global__ void __launch_bounds__(256)
-gram_counts_kernel(const uint32_t* __restrict__ G, int64_t K_tiles, int64_t j0, int64_t ncols, int kc, int kp,
+gram_counts_kernel(const uint32_t* __restrict__ G, int64_t K_tiles, const GramGroup* __restrict__ groups, int kp,
                    uint8_t* __restrict__ B)
 {
   const int64_t q = (int64_t)blockIdx.x * 256 + threadIdx.x;   // word of the row
   if (q >= K_tiles * 4) return;
   const int grp = blockIdx.z, r = blockIdx.y;
-  const int64_t c = (int64_t)grp * kc + r;
-  uint4 o = make_uint4(0u, 0u, 0u, 0u);
-  if (r < kc && c < ncols) {
-    const int64_t j = j0 + c;
-    const uint32_t w = G[((j / 128 * K_tiles + (q >> 2)) * 128 + j % 128) * 4 + (q & 3)];
-    uint32_t v[4];
+  if (r >= groups[grp].nc) return;
+  const int64_t j = groups[grp].c0 + r;
+  const uint32_t w = G[((j / 128 * K_tiles + (q >> 2)) * 128 + j % 128) * 4 + (q & 3)];
+  uint32_t v[4];
 #pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      const uint32_t x = (w >> (2 * p)) & 0x03030303u, two = (x >> 1) & 0x01010101u;
-      v[p] = (p & 1) ? x * 0x28u - two * 0x20u : x * 0x38u - two * 0x30u;
-    }
-    o = make_uint4(v[0], v[1], v[2], v[3]);
+  for (int p = 0; p < 4; ++p) {
+    const uint32_t x = (w >> (2 * p)) & 0x03030303u, two = (x >> 1) & 0x01010101u;
+    v[p] = (p & 1) ? x * 0x28u - two * 0x20u : x * 0x38u - two * 0x30u;
   }
-  *reinterpret_cast<uint4*>(B + ((int64_t)grp * kp + r) * K_tiles * kTileK + q * 16) = o;
+  *reinterpret_cast<uint4*>(B + ((int64_t)grp * kp + r) * K_tiles * kTileK + q * 16) = make_uint4(v[0], v[1], v[2], v[3]);
 }
 
 // With residual weights: N = 2·kp rows, FP16 pieces hi and lo of rr²·z·2^e, each times the 2^−2s of its K
 // position (f16sub_pair_of).  A thread writes 8 K-elements (half of a packed word): 16-byte stores, 512
 // contiguous bytes per warp.  Bound by the 16-bit operand it writes.
 __global__ void __launch_bounds__(256)
-gram_operand_kernel(const uint32_t* __restrict__ G, int64_t K_tiles, int64_t j0, int64_t ncols, int kc, int kp,
+gram_operand_kernel(const uint32_t* __restrict__ G, int64_t K_tiles, const GramGroup* __restrict__ groups, int kp,
                     const float* __restrict__ gm, const float* __restrict__ rr, float scale, __half* __restrict__ B)
 {
   const int64_t q8 = (int64_t)blockIdx.x * 256 + threadIdx.x;   // K-elements 8·q8 …
   const int64_t K_pad = K_tiles * kTileK;
   if (q8 * 8 >= K_pad) return;
   const int grp = blockIdx.z, r = blockIdx.y;
+  if (r >= groups[grp].nc) return;
   __half* dst = B + ((int64_t)grp * 2 * kp + r) * K_pad + q8 * 8;
-  const int64_t c = (int64_t)grp * kc + r;
-  uint4 hi = make_uint4(0u, 0u, 0u, 0u), lo = hi;
-  if (r < kc && c < ncols) {
-    const int64_t j = j0 + c, kt = q8 >> 3;
+  uint4 hi, lo;
+  {
+    const int64_t j = groups[grp].c0 + r, kt = q8 >> 3;
     const int w = (int)(q8 & 7) >> 1, h = (int)(q8 & 1);
     const uint32_t word = G[((j / 128 * K_tiles + kt) * 128 + j % 128) * 4 + w];
     float zv[3], rv[8];
@@ -193,37 +196,37 @@ __device__ __forceinline__ float gram_entry(const float* __restrict__ D, int spl
   return __fadd_rn(a.hi, a.lo);
 }
 
-// out[c·ldo + i] of every product row i (SNP r0 + i) and column c (SNP c0 + c).  Rows past the matrix are left alone.
+// out[c·ldo + i] of every product row i and column c of the groups (blockIdx.z).
 __global__ void __launch_bounds__(256)
-gram_finish_kernel(const float* __restrict__ D, int splits, int kp, int64_t rows, int64_t nrows, int kc, float isc,
-                   GramStats rs, int64_t r0, GramStats cs, int64_t c0, int cq, float* __restrict__ out, int64_t ldo)
+gram_finish_kernel(const float* __restrict__ D, int splits, int kp, int64_t rows, float isc, GramStats rs, GramStats cs,
+                   const GramGroup* __restrict__ groups, int cq, int64_t ldo)
 {
-  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (i >= nrows) return;
-  const int64_t c = blockIdx.y;
-  out[c * ldo + i] = gram_entry(D, splits, kp, rows, i, (int)(c / kc), (int)(c % kc), isc, rs, r0 + i, cs, c0 + c, cq);
+  const GramGroup G = groups[blockIdx.z];
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x, c = blockIdx.y;
+  if (i >= G.nrows || c >= G.nc) return;
+  G.out[(G.c0 - G.b0 + c) * ldo + i] = gram_entry(D, splits, kp, rows, i, blockIdx.z, (int)c, isc, rs, G.r0 + i, cs, G.c0 + c, cq);
 }
 
-// The same of a block of a symmetric product, for its entries with r0 + i ≤ c0 + c; with `mirror` each of
-// them also at the other half's place, product row c0 + c − r0 and column r0 + i − c0 (where that is one of the
-// ncols columns from c00), through shared memory so that both writes are whole lines.  Columns c0 … c0 + nc − 1
-// are those from c0 − c00 of out.
+// The same of blocks of a symmetric product, for the entries with r0 + i ≤ c0 + c; with `mirror` each of them
+// also at the other half's place, product row c0 + c − r0 and column r0 + i − b0 (where that is one of the
+// block's columns), through shared memory so that both writes are whole lines.
 __global__ void __launch_bounds__(256)
-gram_finish_sym_kernel(const float* __restrict__ D, int splits, int kp, int64_t rows, int64_t nrows, int kc, float isc,
-                       GramStats st, int64_t r0, int64_t c0, int64_t nc, int64_t c00, int64_t ncols, int cq,
-                       float* __restrict__ out, int64_t ldo, int mirror)
+gram_finish_sym_kernel(const float* __restrict__ D, int splits, int kp, int64_t rows, float isc, GramStats st,
+                       const GramGroup* __restrict__ groups, int cq, int64_t ldo, int mirror)
 {
   __shared__ float tile[32][33];
+  const GramGroup G = groups[blockIdx.z];
   const int64_t i0 = (int64_t)blockIdx.x * 32, ct = (int64_t)blockIdx.y * 32;
-  if (r0 + i0 > c0 + min64(ct + 31, nc - 1)) return;   // past every column's SNP
+  // past the rows, the columns or every column's SNP
+  if (i0 >= G.nrows || ct >= G.nc || G.r0 + i0 > G.c0 + min64(ct + 31, G.nc - 1)) return;
   const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
   const int64_t i = i0 + x;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const int64_t c = ct + y + 8 * q;
-    if (i >= nrows || c >= nc || r0 + i > c0 + c) continue;
-    const float v = gram_entry(D, splits, kp, rows, i, (int)(c / kc), (int)(c % kc), isc, st, r0 + i, st, c0 + c, cq);
-    out[(c0 - c00 + c) * ldo + i] = v;
+    if (i >= G.nrows || c >= G.nc || G.r0 + i > G.c0 + c) continue;
+    const float v = gram_entry(D, splits, kp, rows, i, blockIdx.z, (int)c, isc, st, G.r0 + i, st, G.c0 + c, cq);
+    G.out[(G.c0 - G.b0 + c) * ldo + i] = v;
     tile[y + 8 * q][x] = v;
   }
   if (!mirror) return;
@@ -231,8 +234,9 @@ gram_finish_sym_kernel(const float* __restrict__ D, int splits, int kp, int64_t 
   const int64_t c = ct + x;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const int64_t k = i0 + y + 8 * q, col = r0 + k - c00;   // product row k becomes column col
-    if (k < nrows && c < nc && r0 + k < c0 + c && col >= 0 && col < ncols) out[col * ldo + c0 + c - r0] = tile[x][y + 8 * q];
+    const int64_t k = i0 + y + 8 * q, col = G.r0 + k - G.b0;   // product row k becomes column col
+    if (k < G.nrows && c < G.nc && G.r0 + k < G.c0 + c && col >= 0 && col < G.bc)
+      G.out[col * ldo + G.c0 + c - G.r0] = tile[x][y + 8 * q];
   }
 }
 
@@ -241,6 +245,11 @@ gram_finish_sym_kernel(const float* __restrict__ D, int splits, int kp, int64_t 
 // read again by the finishing kernel).  Anything from 24 to 64 is within a percent at n = 7,000 to 50,000; 8,
 // the ramp and epilogue alone, took 1 to 3 % more of the calls.
 constexpr int64_t kSplitTiles = 32;
+// Operand bytes of one launch.  Launches of many blocks' groups fill the GPU's last wave and take few splits,
+// which is worth more than an operand that stays in L2: at 48, 96, 192 and 512 MB slemm_gwa (50,021 × 20,011, blocks of
+// 1,000) takes 3.81, 3.57, 3.47 and 3.29 ms, with blocks of 100 (46,280 × 16,455) 1.92, 1.57, 1.46 and 1.45 ms
+// (3.70 with a launch for each block), --lmm (50,000, 30 windows of 1,000) 6.81, 6.47, 6.32 and 6.13 ms (6.75).
+constexpr int64_t kGramOperand = (int64_t)512 << 20;
 static int gram_splits(int64_t ctas, int64_t K_tiles, int64_t min_splits)
 {
   int64_t best = min_splits, best_cost = INT64_MAX;
@@ -254,15 +263,24 @@ static int gram_splits(int64_t ctas, int64_t K_tiles, int64_t min_splits)
   return (int)best;
 }
 
-void gram_block(slemm_geno* g, const GramSide& R, int64_t r0, int64_t rows, const GramSide& C, int64_t c0, int64_t ncols,
-                int cq, const float* rr, float rr_max, float* out, int64_t ldo, GramHalf half)
+void gram_rows(const GramSide& R, int64_t s0, int64_t cnt, GramJob& job)
 {
-  CHECK_ARG(r0 % kPadRows == 0 && rows % kPadRows == 0 && r0 + rows <= round_up(R.m, kPadRows), "row range not aligned");
-  if (ncols <= 0) return;
+  const int64_t end = round_up(R.m, kPadRows);
+  job.r0 = s0 / kTileM * kTileM;
+  job.rows = round_up(s0 + cnt - job.r0, kPadRows);
+  job.r0 = std::min(job.r0, end - job.rows);
+  if (job.r0 < 0) {
+    job.r0 = 0;
+    job.rows = end;
+  }
+}
+
+void gram_blocks(slemm_geno* g, const GramSide& R, const GramSide& C, const std::vector<GramJob>& jobs, int cq, const float* rr,
+                 float rr_max, int64_t ldo, GramHalf half)
+{
   cudaStream_t st = g->stream;
   const int64_t K_pad = g->n_pad, K_tiles = K_pad / kTileK;
-  const bool unit = rr == nullptr;
-  CHECK_ARG(half == GramHalf::all || (R.G == C.G && c0 >= r0 && c0 + ncols <= r0 + rows), "not a symmetric block");
+  const bool unit = rr == nullptr, sym = half != GramHalf::all;
   // |rr²·z| ≤ 2·max rr²: the bound lies in [2^10, 2^11) after scaling (ops.cu, split_exp)
   int e = 0;
   if (!unit) {
@@ -272,55 +290,64 @@ void gram_block(slemm_geno* g, const GramSide& R, int64_t r0, int64_t rows, cons
   }
   // N ≤ 160 keeps two row tiles, each with its own MMA-issuing thread, in one CTA
   const int most = unit ? 160 : 80;
-  const int64_t groups = ceil_div(ncols, most);
-  const int kc = (int)ceil_div(ncols, groups);
-  const int kp = (int)round_up(kc, unit ? 16 : 8);
+  std::vector<GramGroup> groups;
+  std::vector<int2> tiles;   // as GemmArgs::table
+  int64_t widest = 0, rows = 0;
+  for (const GramJob& j : jobs) {
+    if (j.ncols <= 0) continue;
+    CHECK_ARG(j.r0 % kTileM == 0 && j.rows % kPadRows == 0 && j.r0 + j.rows <= round_up(R.m, kPadRows), "row range not aligned");
+    CHECK_ARG(!sym || (R.G == C.G && j.c0 >= j.r0 && j.c0 + j.ncols <= j.r0 + j.rows), "not a symmetric block");
+    const int64_t kc = ceil_div(j.ncols, ceil_div(j.ncols, most));
+    for (int64_t f = 0; f < j.ncols; f += kc) {
+      const int64_t nc = std::min(kc, j.ncols - f);
+      groups.push_back({j.r0, std::min(j.rows, R.m - j.r0), j.c0 + f, nc, j.c0, j.ncols, j.out});
+      const int64_t wanted = sym ? std::min(j.rows, j.c0 + f + nc - j.r0) : j.rows;
+      tiles.push_back(make_int2((int)(j.r0 / kTileM), (int)ceil_div(wanted, kTileM)));
+    }
+    widest = std::max(widest, kc);
+    rows = std::max(rows, j.rows);
+  }
+  if (groups.empty()) return;
+  const int kp = (int)round_up(widest, unit ? 16 : 8);
   const int N = unit ? kp : 2 * kp;
-  // as many groups per launch as 256 MB of operand and 512 MB of a split's partials hold (at least one)
-  const int64_t group_bytes = (int64_t)N * K_pad * (unit ? 1 : 2);
-  const int64_t per = std::max<int64_t>(1, std::min({groups, ((int64_t)256 << 20) / group_bytes,
-                                                     ((int64_t)512 << 20) / ((int64_t)kp * rows * 4)}));
   const int plan = unit ? 2 : 0;
-  const int64_t rctas = rows / gemm_tc_rows_per_cta(N, plan);
-  const int64_t nrows = std::min(rows, R.m - r0);
-  const uint8_t* A = R.G + (size_t)(r0 / kTileM) * K_tiles * kTileBytes;
-  for (int64_t g0 = 0; g0 < groups; g0 += per) {
-    const int ng = (int)std::min(per, groups - g0);
-    const int64_t first = g0 * kc, nc = std::min<int64_t>((int64_t)ng * kc, ncols - first);
-    // CTAs with work: half of them or so where only one half is wanted
-    const int64_t diag = c0 + first - r0;
-    int64_t live = 0;
-    for (int z = 0; z < ng; ++z)
-      live += half == GramHalf::all ? rctas : std::min(rctas, ceil_div(diag + (int64_t)(z + 1) * kc, rows / rctas));
+  const int64_t cta_tiles = gemm_tc_rows_per_cta(N, plan) / kTileM;
+  DevBuf d_groups(st), d_tiles(st);
+  GramGroup* dg = (GramGroup*)d_groups.ensure(groups.size() * sizeof(GramGroup));
+  int2* dt = (int2*)d_tiles.ensure(tiles.size() * sizeof(int2));
+  CUDA_TRY(cudaMemcpyAsync(dg, groups.data(), groups.size() * sizeof(GramGroup), cudaMemcpyHostToDevice, st));
+  CUDA_TRY(cudaMemcpyAsync(dt, tiles.data(), tiles.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
+  // As many groups per launch as kGramOperand of operand and 512 MB of a split's partials hold (at least one)
+  const int64_t group_bytes = (int64_t)N * K_pad * (unit ? 1 : 2), total = (int64_t)groups.size();
+  int64_t per = std::max<int64_t>(1, std::min({total, kGramOperand / group_bytes, ((int64_t)512 << 20) / ((int64_t)kp * rows * 4),
+                                               (int64_t)65535}));
+  per = ceil_div(total, ceil_div(total, per));   // launches of about the same size
+  for (int64_t g0 = 0; g0 < total; g0 += per) {
+    const int ng = (int)std::min(per, total - g0);
+    int64_t live = 0;   // CTAs with work
+    for (int z = 0; z < ng; ++z) live += ceil_div(tiles[g0 + z].y, cta_tiles);
     // an integer partial sum of 2^22 elements is at most 2^24: exact in FP32
     const int splits = gram_splits(live, K_tiles, ceil_div(K_pad, (int64_t)1 << 22));
     void* B = g->ws_B.ensure((size_t)ng * group_bytes);
     float* D = (float*)g->ws_D.ensure((size_t)ng * splits * kp * rows * sizeof(float));
     const uint32_t* Gc = reinterpret_cast<const uint32_t*>(C.G);
     if (unit)
-      gram_counts_kernel<<<dim3((unsigned)ceil_div(K_pad / 16, 256), kp, ng), 256, 0, st>>>(Gc, K_tiles, c0 + first, nc,
-                                                                                            kc, kp, (uint8_t*)B);
+      gram_counts_kernel<<<dim3((unsigned)ceil_div(K_pad / 16, 256), kp, ng), 256, 0, st>>>(Gc, K_tiles, dg + g0, kp, (uint8_t*)B);
     else
       gram_operand_kernel<<<dim3((unsigned)ceil_div(K_pad / 8, 256), kp, ng), 256, 0, st>>>(
-          Gc, K_tiles, c0 + first, nc, kc, kp, C.stats.gm, rr, (float)std::ldexp(1.0, e), (__half*)B);
+          Gc, K_tiles, dg + g0, kp, C.stats.gm, rr, (float)std::ldexp(1.0, e), (__half*)B);
     LAUNCH_CHECK();
-    GemmArgs a{A, rows, K_pad, B, N, D, splits, g->err.as<int>(), kp, unit ? 1 : 2, !unit, plan};
+    GemmArgs a{R.G, rows, K_pad, B, N, D, splits, g->err.as<int>(), kp, unit ? 1 : 2, !unit, plan};
     a.groups = ng;
-    if (half != GramHalf::all) {
-      a.diag = diag;
-      a.diag_step = kc;
-    }
+    a.table = dt + g0;
     gemm_tc(a, st);
-    if (half != GramHalf::all) {
-      gram_finish_sym_kernel<<<dim3((unsigned)ceil_div(nrows, 32), (unsigned)ceil_div(nc, 32)), 256, 0, st>>>(
-          D, splits, kp, rows, nrows, kc, (float)std::ldexp(1.0, -e), R.stats, r0, c0 + first, nc, c0, ncols, cq, out, ldo,
-          half == GramHalf::mirrored ? 1 : 0);
-      LAUNCH_CHECK();
-      continue;
-    }
-    gram_finish_kernel<<<dim3((unsigned)ceil_div(nrows, 256), (unsigned)nc), 256, 0, st>>>(
-        D, splits, kp, rows, nrows, kc, (float)std::ldexp(1.0, -e), R.stats, r0, C.stats, c0 + first, cq,
-        out + first * ldo, ldo);
+    const float isc = (float)std::ldexp(1.0, -e);
+    if (sym)
+      gram_finish_sym_kernel<<<dim3((unsigned)ceil_div(rows, 32), (unsigned)ceil_div(widest, 32), ng), 256, 0, st>>>(
+          D, splits, kp, rows, isc, R.stats, dg + g0, cq, ldo, half == GramHalf::mirrored ? 1 : 0);
+    else
+      gram_finish_kernel<<<dim3((unsigned)ceil_div(rows, 256), (unsigned)widest, ng), 256, 0, st>>>(
+          D, splits, kp, rows, isc, R.stats, C.stats, dg + g0, cq, ldo);
     LAUNCH_CHECK();
   }
 }

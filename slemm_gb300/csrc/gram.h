@@ -3,6 +3,8 @@
 
 #include "internal.h"
 
+#include <vector>
+
 namespace slemm {
 
 // Per-SNP statistics (device) with z = x − gm: h = Σ rr²·z and, when every rr is 1, p = Σ x (else 0), as
@@ -46,14 +48,21 @@ struct GramSide {
   int64_t m;
   GramStats stats;
 };
-// out[c·ldo + i] = (P(rr∘z_{r0+i}))ᵀ(P(rr∘z_{c0+c})) for product rows r0 … r0 + rows − 1 of R (multiples
-// of 256; rows past R.m are not written) and columns c0 … c0 + ncols − 1 of C.  g gives the stream,
-// the work buffers and the individuals; rr (n_pad) == nullptr: all 1, else rr_max ≥ max|rr|.
-// With R and C the same side: `lower` wants the rows up to each column's own SNP alone (out's others are
-// left alone or hold sums of their own), `mirrored` has the columns' SNPs from the other half as well.
+// One block: out[c·ldo + i] = (P(rr∘z_{r0+i}))ᵀ(P(rr∘z_{c0+c})) for product rows r0 … r0 + rows − 1 of R (r0 a
+// multiple of 128, rows of 256; rows past R.m are not written) and columns c0 … c0 + ncols − 1 of C.
+struct GramJob {
+  int64_t r0, rows, c0, ncols;
+  float* out;
+};
+// The rows of a block that has to hold SNPs s0 … s0 + cnt − 1 of R: at most round_up(cnt, 256) + 256.
+void gram_rows(const GramSide& R, int64_t s0, int64_t cnt, GramJob& job);
+// The blocks of one pair of sides.  g gives the stream, the work buffers and the individuals; rr (n_pad) ==
+// nullptr: all 1, else rr_max ≥ max|rr|.  With R and C the same side and a block's columns among its rows: `lower`
+// wants the rows up to each column's own SNP alone (out's others are left alone), `mirrored` has the columns'
+// SNPs from the other half as well.
 enum class GramHalf { all, lower, mirrored };
-void gram_block(slemm_geno* g, const GramSide& R, int64_t r0, int64_t rows, const GramSide& C, int64_t c0, int64_t ncols,
-                int cq, const float* rr, float rr_max, float* out, int64_t ldo, GramHalf half = GramHalf::all);
+void gram_blocks(slemm_geno* g, const GramSide& R, const GramSide& C, const std::vector<GramJob>& jobs, int cq, const float* rr,
+                 float rr_max, int64_t ldo, GramHalf half);
 
 // A batch of nb systems of s unknowns (layout in gram.cu); offA, offZ and t are device arrays.
 struct SpdBatch {

@@ -185,23 +185,28 @@ extern "C" int slemm_gpu_gwa_windows(slemm_geno* g, const float* y, const float*
       std::vector<int64_t> off((size_t)2 * bn);   // offA | offZ
       std::vector<int> tb(bn);
       std::vector<float> ridge((size_t)bn * bs);
+      std::vector<GramJob> own, tested_by;   // the blocks' own Gram, and with the variants each serves
       int t_max = 0;
       for (int bi = 0; bi < bn; ++bi) {
         const int64_t s0 = start[b0 + bi];
-        const int64_t r0 = s0 / kPadRows * kPadRows;
-        const int64_t r1 = std::min<int64_t>(round_up(s0 + bs, kPadRows), model_rows);
+        GramJob job{0, 0, s0, bs, gram + (size_t)bi * stride};
+        gram_rows(model, s0, bs, job);
+        own.push_back(job);
         for (int t = 0; t < bs; ++t) {
           const float mu = mean[model_idx[s0 + t]];
           ridge[(size_t)bi * bs + t] = (float)model_snp_ct * tau * ((2.0f - mu) * mu / 2.0f);
         }
-        off[bi] = s0 - r0;
+        off[bi] = s0 - job.r0;
         off[bn + bi] = lo[b0 + bi] - lo[b0];
         tb[bi] = (int)(hi[b0 + bi] - lo[b0 + bi]);
         t_max = std::max(t_max, tb[bi]);
-        gram_block(g, model, r0, r1 - r0, model, s0, bs, c, drr, rr_max, gram + (size_t)bi * stride, rows_max,
-                   GramHalf::lower);
-        gram_block(g, model, r0, r1 - r0, all, lo[b0 + bi], tb[bi], c, drr, rr_max, Z + off[bn + bi] * rows_max, rows_max);
+        job.c0 = lo[b0 + bi];
+        job.ncols = tb[bi];
+        job.out = Z + off[bn + bi] * rows_max;
+        tested_by.push_back(job);
       }
+      gram_blocks(g, model, model, own, c, drr, rr_max, rows_max, GramHalf::lower);
+      gram_blocks(g, model, all, tested_by, c, drr, rr_max, rows_max, GramHalf::all);
       float* dr = (float*)d_ridge.ensure(ridge.size() * sizeof(float));
       int64_t* doff = (int64_t*)d_off.ensure(off.size() * sizeof(int64_t));
       CUDA_TRY(cudaMemcpyAsync(dr, ridge.data(), ridge.size() * sizeof(float), cudaMemcpyHostToDevice, st));

@@ -140,6 +140,7 @@ extern "C" int slemm_gpu_lmm_quadforms(slemm_geno* g, const float* Py, float tau
     const GramSide side{g->G.as<uint8_t>(), m, stats.s};
     std::vector<int64_t> idx((size_t)3 * k);   // offA | offZ | which
     std::vector<int> one(k, 1);
+    std::vector<GramJob> jobs;
     std::vector<float> dd((size_t)k * ws);
     for (int c = 0; c < k; ++c) {
       const int64_t j = var[c];
@@ -148,14 +149,14 @@ extern "C" int slemm_gpu_lmm_quadforms(slemm_geno* g, const float* Py, float tau
       else if (j > m - ws / 2) wds = m - ws;
       else wds = j - ws / 2;
       for (int t = 0; t < ws; ++t) dd[(size_t)c * ws + t] = tau1 / gw[wds + t];
-      const int64_t r0 = wds / kPadRows * kPadRows;
-      const int64_t r1 = std::min<int64_t>(round_up(wds + ws, kPadRows), g->m_pad);
-      gram_block(g, side, r0, r1 - r0, side, wds, ws, g->c, rr, g->rr_max, gram + (size_t)c * stride, rows_max,
-                 GramHalf::mirrored);
-      idx[c] = wds - r0;   // this window's Gram starts at row wds − r0 of its block
+      GramJob job{0, 0, wds, ws, gram + (size_t)c * stride};
+      gram_rows(side, wds, ws, job);
+      jobs.push_back(job);
+      idx[c] = wds - job.r0;   // this window's Gram starts at row wds − r0 of its block
       idx[k + c] = (int64_t)c * (ws + 1);
       idx[2 * k + c] = j - wds;
     }
+    gram_blocks(g, side, side, jobs, g->c, rr, g->rr_max, rows_max, GramHalf::mirrored);
     check_device_error(g);
     // batched systems: q_c = zᵀ(ZᵀZ + D)⁻¹z
     float* dvec = (float*)d_d.ensure((size_t)k * ws * sizeof(float));
