@@ -121,6 +121,11 @@ struct ExactCols {
 // twos[j] = 2·Σ_i rr_i²·[count_ij = 2].  Device pointers; at least one column.
 void exact_dots(slemm_geno* g, const ExactCols& a, double* dots, double* tot, double* twos);
 
+// MC-REML's criterion terms (ops.cu), device memory: Py = rr∘e and norms[c] = ‖e_c‖², e_0 = P·PV_0 and
+// e_c = P(PV_c + st·PV_{q+c}), c = 1 … q; and X ← √w∘X (m×k), norms[c] = ‖X_c‖².
+void first_order_terms(slemm_geno* g, const float* PV, int q, float st, float* Py, double* norms);
+void weighted_norms(slemm_geno* g, float* X, int k, double* norms);
+
 // Column reductions with FP64 accumulation, deterministic two-stage (ops.cu).
 // dots[c] = Σ_i a[i,c]·b[i,c] over i < n for c < k (b == nullptr → Σ a²).  Result on device.
 void col_dots(slemm_geno* g, const float* a, int64_t lda, const float* b, int64_t ldb,

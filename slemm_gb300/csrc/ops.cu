@@ -1199,6 +1199,21 @@ int64_t workspace_bytes(const slemm_geno* g)
 }
 
 // Checks the device error word of the kernels' bounded waits (synchronises the stream).
+void first_order_terms(slemm_geno* g, const float* PV, int q, float st, float* Py, double* norms)
+{
+  const int64_t n = g->n, units = round_up(n, 16) / kColRows;
+  const bool vec = vec4_ok(n, n, PV) && vec4_ok(n, n, Py);
+  launch_columns(vec ? col_first_kernel<true> : col_first_kernel<false>, units, 1 + q, g->stream, PV, n, units, q, st,
+                 g->Q.as<float>(), g->n_pad, g->c, g->rr.as<float>(), Py, norms);
+}
+
+void weighted_norms(slemm_geno* g, float* X, int k, double* norms)
+{
+  const int64_t m = g->m, units = round_up(m, 16) / kColRows;
+  launch_columns(vec4_ok(m, m, X) ? col_weigh_kernel<true> : col_weigh_kernel<false>, units, k, g->stream, X, m, units,
+                 g->w.as<float>(), norms);
+}
+
 void check_device_error(slemm_geno* g)
 {
   int h = 0;

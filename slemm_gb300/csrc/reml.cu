@@ -108,17 +108,6 @@ static void scale_rows(slemm_geno* g, float* X, int64_t ld, int64_t rows, int k,
   LAUNCH_CHECK();
 }
 
-// Py[:,0] = PV[:,0]; Py[:,c] = PV[:,c] + st·PV[:,n_MC+c]   (src/reml.cpp:716-717)
-__global__ void lmc_combine_kernel(const float* __restrict__ PV, float* __restrict__ Py, int64_t n,
-                                   int n_MC, float st)
-{
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int c = blockIdx.y;
-  if (i >= n) return;
-  if (c == 0) Py[i] = PV[i];
-  else Py[(int64_t)c * n + i] = PV[(int64_t)c * n + i] + st * PV[(int64_t)(n_MC + c) * n + i];
-}
-
 // y_out[i] = r[i]·y[i] − s·rv[i]·p[i]  helper for the LMC BLUE residual (src/reml.cpp:872-874)
 __global__ void lmc_resid_kernel(const float* __restrict__ y, const float* __restrict__ zb,
                                  const float* __restrict__ rvec, const float* __restrict__ Py, float tau1,
@@ -508,16 +497,9 @@ void reml_lmc(slemm_geno* g, const float* rvec, const float* X, int64_t ldx, int
     const float tau = (1 - ss) / ss;
     const float sigma = tau - tau0;
     lanczos_solve_device(seed_V, (double)sigma, 1e-6, d_PV.as<float>(), n, 0);
-    dim3 gr((unsigned)ceil_div(n, 256), 1 + n_MC);
-    lmc_combine_kernel<<<gr, 256, 0, st>>>(d_PV.as<float>(), d_Py.as<float>(), n, n_MC, std::sqrt(tau));
-    LAUNCH_CHECK();
-    proj_coeffs(g, d_Py.as<float>(), n, 1 + n_MC, d_scal);
-    proj_apply(g, d_Py.as<float>(), n, 1 + n_MC, d_scal);
-    col_dots(g, d_Py.as<float>(), n, nullptr, 0, n, 1 + n_MC, d_scal + scal_off);              // ‖e‖²
-    scale_rows(g, d_Py.as<float>(), n, n, 1 + n_MC, g->rr.as<float>());
+    first_order_terms(g, d_PV.as<float>(), n_MC, std::sqrt(tau), d_Py.as<float>(), d_scal + scal_off);   // ‖e‖²
     op_device(g, SLEMM_OP_RMATVEC, 0.f, d_Py.as<float>(), n, 1 + n_MC, d_ub.as<float>(), m);
-    scale_rows(g, d_ub.as<float>(), m, m, 1 + n_MC, g->w.as<float>(), true);
-    col_dots(g, d_ub.as<float>(), m, nullptr, 0, m, 1 + n_MC, d_scal + scal_off + (1 + n_MC));   // ‖u‖²
+    weighted_norms(g, d_ub.as<float>(), 1 + n_MC, d_scal + scal_off + (1 + n_MC));                       // ‖u‖²
     std::vector<double> h = d2h(g, d_scal + scal_off, 2 * (1 + n_MC));
     double e0 = h[0], u0 = h[1 + n_MC], es = 0.0, us = 0.0;
     for (int q = 1; q <= n_MC; ++q) {
