@@ -641,7 +641,10 @@ __device__ __forceinline__ void grad_terms(const float* __restrict__ T, int64_t 
 // blocks from n_runs each reduce a chunk of all m SNPs weighted by W_j (the handle's weights,
 // gw·wwin), glob[2b …] = Σ W_j·(a_j, b_j).  The partials are summed in a fixed order afterwards, so
 // the gradient is bit-reproducible.
-constexpr int kGradChunk = 8192;
+// A chunk is what keeps one SM's FP64 units (two lanes a clock, some 70 operations a SNP at 30 probes) busy
+// for 9 µs: chunks of 8,192 left 25,000 SNPs to 4 SMs for 150 µs (REML gradient at n = 50,000, m = 25,000,
+// 30 probes: 4.70 → 4.42 ms).
+constexpr int kGradChunk = 512;
 __global__ void __launch_bounds__(256)
 grad_window_kernel(const float* __restrict__ T, int64_t m, int n_V, double scale, const float* __restrict__ gw,
                    const float* __restrict__ W, const int64_t* __restrict__ runs, int n_runs,
