@@ -108,23 +108,33 @@ struct GramGroup {
 // (decode.cuh), so the product takes one MMA per 32 individuals and its sums are exact integers.  One
 // word (16 individuals) per thread; a count x ∈ {0, 1, 2} in a byte is x·0x38 − [x = 2]·0x30 (E4M3 0, 1,
 // 2), or x·0x28 − [x = 2]·0x20 times 2^−2, four at a time.  Bound by the bytes it writes.
+constexpr int kCountRows = 8;   // rows of one thread: with one, the turnover of blocks bound it (378 µs for 27,000 columns
+                                // of slemm_gwa at n = 50,021, 244 now, 5.5 TB/s)
 __global__ void __launch_bounds__(256)
 gram_counts_kernel(const uint32_t* __restrict__ G, int64_t K_tiles, const GramGroup* __restrict__ groups, int kp,
                    uint8_t* __restrict__ B)
 {
   const int64_t q = (int64_t)blockIdx.x * 256 + threadIdx.x;   // word of the row
   if (q >= K_tiles * 4) return;
-  const int grp = blockIdx.z, r = blockIdx.y;
-  if (r >= groups[grp].nc) return;
-  const int64_t j = groups[grp].c0 + r;
-  const uint32_t w = G[((j / 128 * K_tiles + (q >> 2)) * 128 + j % 128) * 4 + (q & 3)];
-  uint32_t v[4];
+  const int grp = blockIdx.z, r0 = blockIdx.y * kCountRows;
+  const int64_t nc = groups[grp].nc, c0 = groups[grp].c0;
+  uint32_t w[kCountRows];
 #pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    const uint32_t x = (w >> (2 * p)) & 0x03030303u, two = (x >> 1) & 0x01010101u;
-    v[p] = (p & 1) ? x * 0x28u - two * 0x20u : x * 0x38u - two * 0x30u;
+  for (int e = 0; e < kCountRows; ++e) {
+    const int64_t j = c0 + r0 + e;
+    w[e] = r0 + e < nc ? G[((j / 128 * K_tiles + (q >> 2)) * 128 + j % 128) * 4 + (q & 3)] : 0u;
   }
-  *reinterpret_cast<uint4*>(B + ((int64_t)grp * kp + r) * K_tiles * kTileK + q * 16) = make_uint4(v[0], v[1], v[2], v[3]);
+#pragma unroll
+  for (int e = 0; e < kCountRows; ++e) {
+    if (r0 + e >= nc) return;
+    uint32_t v[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      const uint32_t x = (w[e] >> (2 * p)) & 0x03030303u, two = (x >> 1) & 0x01010101u;
+      v[p] = (p & 1) ? x * 0x28u - two * 0x20u : x * 0x38u - two * 0x30u;
+    }
+    *reinterpret_cast<uint4*>(B + ((int64_t)grp * kp + r0 + e) * K_tiles * kTileK + q * 16) = make_uint4(v[0], v[1], v[2], v[3]);
+  }
 }
 
 // With residual weights: N = 2·kp rows, FP16 pieces hi and lo of rr²·z·2^e, each times the 2^−2s of its K
@@ -332,7 +342,7 @@ void gram_blocks(slemm_geno* g, const GramSide& R, const GramSide& C, const std:
     float* D = (float*)g->ws_D.ensure((size_t)ng * splits * kp * rows * sizeof(float));
     const uint32_t* Gc = reinterpret_cast<const uint32_t*>(C.G);
     if (unit)
-      gram_counts_kernel<<<dim3((unsigned)ceil_div(K_pad / 16, 256), kp, ng), 256, 0, st>>>(Gc, K_tiles, dg + g0, kp, (uint8_t*)B);
+      gram_counts_kernel<<<dim3((unsigned)ceil_div(K_pad / 16, 256), (unsigned)ceil_div(kp, kCountRows), ng), 256, 0, st>>>(Gc, K_tiles, dg + g0, kp, (uint8_t*)B);
     else
       gram_operand_kernel<<<dim3((unsigned)ceil_div(K_pad / 8, 256), kp, ng), 256, 0, st>>>(
           Gc, K_tiles, dg + g0, kp, C.stats.gm, rr, (float)std::ldexp(1.0, e), (__half*)B);
