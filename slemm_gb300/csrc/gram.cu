@@ -10,8 +10,8 @@
 // product is an exact integer, and Σ_i x_ij·z_ik = Σ_i x_ij·x_ik − p_j·gm_k with p_j = Σ_i x_ij.  Forming U = rr∘P(rr∘z) as FP32
 // columns instead (centre, project, scale, measure, split: nine passes over n × columns floats)
 // took 38 of the 82 ms of slemm_gwa at n = 50,021 with 20,011 variants and 4,000 model SNPs, and
-// 31 of the 73 ms of --lmm with 30 windows of 1,000 SNPs at n = 50,000; the two calls now take 3.3
-// and 6.1 ms.
+// 31 of the 73 ms of --lmm with 30 windows of 1,000 SNPs at n = 50,000; the two calls now take 3.2
+// and 6.0 ms.
 #include "gram.h"
 #include "decode.cuh"
 #include "reduce.cuh"

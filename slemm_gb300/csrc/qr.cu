@@ -8,7 +8,7 @@
 // shared memory.  Bound by the FP64 units of its 16 SMs (two lanes a clock each) from some 100,000 rows
 // on, by its 3c cluster-wide reductions below.  On the host the factorisation, the forming of A and
 // of the FP32 copies were 0.75 ms of an MC-REML fit's 4.52 ms at n = 50,000 with 3 covariates and 0.5 of
-// the REML gradient's 5.16 ms with 2, the GPU idle meanwhile; the calls now take 3.95 and 4.63 ms, and
+// the REML gradient's 5.16 ms with 2, the GPU idle meanwhile; the calls took 3.95 and 4.63 ms with it, and
 // slemm_gwa at n = 50,021 with 2 covariates 3.78 (4.00).
 #include "qr.h"
 
