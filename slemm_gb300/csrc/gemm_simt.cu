@@ -12,9 +12,11 @@
 // 2-bit field is already an FP32 number: at bits 2s, 2s + 1 of a word (s ≤ 11) it reads as x·2^(2s−149),
 // a subnormal (bit 23 is the exponent's lowest, and 2^−126 = 2·2^(22−149)), which FMAs take at full
 // rate.  So a count costs one LOP and one FMA, and one shift serves the last four fields of a word.  The
-// staged B carries 2^(100−2s) for its position, and a power of two that brings the stage's largest value
-// into [1, 2): products x·b·2^−49 stay normal down to 2^−77 of that value, all scalings are exact, and the
-// sums are those of x·b.  One column at n = 100,000, m = 20,000, H0_ldet_mv: 652 → 433 µs, the same bits.
+// staged B carries 2^(100−2s) for its position, so that products are x·b·2^−49.  That gives the same bits
+// as x·b where every nonzero |b| of the stage lies in [2^−76, 2^28): the staged value is finite, products are
+// normal, and a sum that cancels below 2^−126 is a multiple of 2^−148 like its terms, so nothing rounds there
+// that would not have.  A stage with any other value (subnormal, non-finite or just far from 1) takes the
+// counts as BF16 pairs instead, at the old cost.  One column at n = 100,000, m = 20,000, H0_ldet_mv: 652 → 433 µs.
 #include "common.h"
 #include "decode.cuh"
 #include "reduce.cuh"
@@ -39,7 +41,6 @@ gemm_simt_kernel(const uint4* __restrict__ A, int64_t M_pad, int64_t K_tiles,
                  float* __restrict__ D, int N, int tiles_per_split)
 {
   __shared__ __align__(16) float sB[kStageK * KC];   // [element][column]
-  __shared__ uint32_t smax[4];
   const int t = threadIdx.x;
   const int64_t mt = blockIdx.x;
   const int s = blockIdx.y;
@@ -58,30 +59,46 @@ gemm_simt_kernel(const uint4* __restrict__ A, int64_t M_pad, int64_t K_tiles,
       pk[u] = u < ntile ? A[((mt * K_tiles + ks + u) * 128 + t)] : make_uint4(0u, 0u, 0u, 0u);
     // stage B[c0 .. c0+KC)[ks*64 .. +ntile*64), element t + 128i of each column
     float raw[KC][kStageK / 128];
-    uint32_t mx = 0;
+    bool near = true;   // 0 or in [2^−76, 2^28)
 #pragma unroll
     for (int c = 0; c < KC; ++c)
 #pragma unroll
       for (int i = 0; i < kStageK / 128; ++i) {
         const int kk = t + 128 * i, col = c0 + c;
         raw[c][i] = (col < k_total && kk < ntile * kTileK) ? B[(int64_t)col * K_pad + ks * kTileK + kk] : 0.f;
-        mx = max(mx, __float_as_uint(raw[c][i]) & 0x7FFFFFFFu);
+        const uint32_t mag = __float_as_uint(raw[c][i]) & 0x7FFFFFFFu;
+        near = near && (mag == 0u || mag - ((127u - 76u) << 23) < (104u << 23));
       }
-    mx = __reduce_max_sync(0xffffffffu, mx);
-    if ((t & 31) == 0) smax[t >> 5] = mx;
-    __syncthreads();   // and every thread is done with the last stage
-    mx = max(max(smax[0], smax[1]), max(smax[2], smax[3]));
-    // the stage's largest value times 2^e lies in [1, 2) (0, subnormal: less; ∞, NaN: e = 0)
-    const int E = (int)(mx >> 23), e = E == 255 ? 0 : (E == 0 ? 126 : 127 - E);
-    const float up = e >= -126 ? __uint_as_float((uint32_t)(e + 127) << 23) : __uint_as_float(0x00400000u);
-    const float down = __uint_as_float((uint32_t)(127 - e) << 23);   // 2^−e, −e ≤ 127
-    const float kscale = __uint_as_float((uint32_t)(127 + 100 - 2 * f32sub_shift(t & 15)) << 23);   // 128 ≡ 0 mod 16
+    near = __syncthreads_and(near);   // and every thread is done with the last stage
+    const float kscale = near ? __uint_as_float((uint32_t)(127 + 100 - 2 * f32sub_shift(t & 15)) << 23) : 1.f;   // 128 ≡ 0 mod 16
 #pragma unroll
     for (int c = 0; c < KC; ++c)
 #pragma unroll
       for (int i = 0; i < kStageK / 128; ++i)
-        sB[(t + 128 * i) * KC + c] = __fmul_rn(__fmul_rn(raw[c][i], up), kscale);
+        sB[(t + 128 * i) * KC + c] = __fmul_rn(raw[c][i], kscale);
     __syncthreads();
+    if (!near) {
+      for (int u = 0; u < ntile; ++u) {
+        const uint4 p4 = A[(mt * K_tiles + ks + u) * 128 + t];
+        const uint32_t words[4] = {p4.x, p4.y, p4.z, p4.w};
+        float part[KC];
+#pragma unroll
+        for (int c = 0; c < KC; ++c) part[c] = 0.f;
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const uint32_t pair = bf16pair_of(words[w], q);   // FP32 in either half
+            const float* b = &sB[(u * kTileK + w * 16 + 2 * q) * KC];
+#pragma unroll
+            for (int c = 0; c < KC; ++c)
+              part[c] = fmaf(__uint_as_float(pair << 16), b[c], fmaf(__uint_as_float(pair & 0xFFFF0000u), b[KC + c], part[c]));
+          }
+#pragma unroll
+        for (int c = 0; c < KC; ++c) df_add(acc[c], part[c]);
+      }
+      continue;
+    }
 #pragma unroll
     for (int u = 0; u < kStageTiles; ++u) {
       if (u >= ntile) break;
@@ -113,7 +130,7 @@ gemm_simt_kernel(const uint4* __restrict__ A, int64_t M_pad, int64_t K_tiles,
         }
       }
 #pragma unroll
-      for (int c = 0; c < KC; ++c) df_add(acc[c], __fmul_rn(__fmul_rn(part[c], 562949953421312.f), down));   // 2^49
+      for (int c = 0; c < KC; ++c) df_add(acc[c], __fmul_rn(part[c], 562949953421312.f));   // 2^49
     }
   }
 #pragma unroll
