@@ -662,19 +662,20 @@ static int tc_min_splits(int64_t K_tiles, int N)
 static cudaEvent_t take_event(slemm_geno* g);
 
 // ---- split-K autotuner ------------------------------------------------------------------------------
-// With a handle's autotune on, the first tensor-core pass of each shape (device, N, pieces, K-tiles,
-// padded rows) times a handful of (plan, split-K) choices with CUDA events on the handle's stream —
+// With a handle's autotune on, the first tensor-core pass of each shape (device, operand format, N, pieces,
+// K-tiles, padded rows) times a handful of (plan, split-K) choices with CUDA events on the handle's stream —
 // the fixed rule's count, and counts near it whose CTAs fill the last wave to ≥ 80 %; for N ≤ 64
 // also the two-CTAs-per-SM plan at its own rule's count and counts near it — each launched once to
 // warm up and twice timed over the real packed copy, and keeps the fastest if it beats the rule's by
 // ≥ 3 % (else the rule's, so close calls do not flip between processes).  Decisions are cached for
 // the life of the process; no tuning happens while the stream is being captured.
 struct TuneKey {
-  int dev, N, pieces;
+  int dev, format, N, pieces;   // format: 0 BF16, 1 FP16, 2 E4M3 digits
   int64_t K_tiles, M_pad;
   bool operator<(const TuneKey& o) const
   {
-    return std::tie(dev, N, pieces, K_tiles, M_pad) < std::tie(o.dev, o.N, o.pieces, o.K_tiles, o.M_pad);
+    return std::tie(dev, format, N, pieces, K_tiles, M_pad) <
+           std::tie(o.dev, o.format, o.N, o.pieces, o.K_tiles, o.M_pad);
   }
 };
 struct TuneEntry {
@@ -709,7 +710,7 @@ static double tune_pass(slemm_geno* g, PassPlan& p, const uint8_t* A, int64_t M_
   CUDA_TRY(cudaStreamIsCapturing(g->stream, &cs));
   if (cs != cudaStreamCaptureStatusNone) return 0.0;
   const int64_t K_tiles = K_pad / kTileK;
-  const TuneKey key{g->device, p.N, p.pieces, K_tiles, M_pad};
+  const TuneKey key{g->device, p.digits() ? 2 : (p.f16 ? 1 : 0), p.N, p.pieces, K_tiles, M_pad};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(key);

@@ -70,3 +70,27 @@ def test_two_cta_plan_matches_oracle(gpu, prec, tol, k):
         got = g.matvec(u)
         want = ref.matvec(u)
         assert np.linalg.norm(got - want) / np.linalg.norm(want) < tol
+
+
+def _tuned_table(precs, ks):
+    """Decisions of passes of k columns on a handle of its own shape (7,936 × 3,584 padded)."""
+    n, m = 7681, 3329
+    rows, _, dec = make_case(n, m, seed=84)
+    gm = orc.genotype_mean(orc.popcounts(dec), n)
+    v = np.random.default_rng(3).standard_normal((n, max(ks))).astype(np.float32)
+    with api.Genotypes(rows, n) as g:
+        g.set_weights(gm, orc.snp_weights(gm, np.ones(m, np.float32)))
+        g.set_autotune(True)
+        for prec in precs:
+            g.set_precision(prec)
+            for k in ks:
+                g.H0_ldet_mv(0.43, v[:, :k])
+    return [t for t in api.autotune_table() if {t["M_pad"], t["K_tiles"] * 64} == {7936, 3584}]
+
+
+def test_tuner_keeps_formats_apart(gpu):
+    """BF16X2 and FP16X2 passes of one shape have their own decisions."""
+    ks = (3, 9, 17, 24, 31)
+    table = _tuned_table((_lib.PREC_BF16X2, _lib.PREC_FP16X2), ks)
+    for N in (16, 32, 48, 64):
+        assert sorted(t["M_pad"] for t in table if t["N"] == N and t["pieces"] == 2) == [3584, 3584, 7936, 7936]
