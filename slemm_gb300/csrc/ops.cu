@@ -784,7 +784,7 @@ static PassPlan plan_pass(slemm_geno* g, int k, int64_t M_pad, int64_t K_pad, co
   const bool tune = g->autotune == 1 && A;
   double ms = 0.0, ms8 = 0.0;
   if (tune) ms = tune_pass(g, p, A, M_pad, K_pad);
-  if (p.f16 && k <= kDigitCols && p.plan != 1) {
+  if (p.f16 && k <= kDigitCols && g->autotune != 2) {   // the fastest of the three plans when all are timed
     PassPlan d = p;
     d.plan = 2;
     d.pieces = kDigits;

@@ -94,3 +94,13 @@ def test_tuner_keeps_formats_apart(gpu):
     table = _tuned_table((_lib.PREC_BF16X2, _lib.PREC_FP16X2), ks)
     for N in (16, 32, 48, 64):
         assert sorted(t["M_pad"] for t in table if t["N"] == N and t["pieces"] == 2) == [3584, 3584, 7936, 7936]
+
+
+def test_tuner_times_digits_whichever_fp16_plan_wins(gpu):
+    """Passes of at most 32 columns at FP16X2 are timed with digits too, in both directions."""
+    ks = (3, 9, 17, 31)
+    table = _tuned_table((_lib.PREC_FP16X2,), ks)
+    for k in ks:
+        N = -(-5 * (-(-k // 8) * 8) // 16) * 16
+        digits = [t for t in table if t["pieces"] == 5 and t["N"] == N]
+        assert {t["M_pad"] for t in digits} == {7936, 3584} and all(t["plan"] == 2 for t in digits)
