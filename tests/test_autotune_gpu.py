@@ -72,35 +72,36 @@ def test_two_cta_plan_matches_oracle(gpu, prec, tol, k):
         assert np.linalg.norm(got - want) / np.linalg.norm(want) < tol
 
 
-def _tuned_table(precs, ks):
-    """Decisions of passes of k columns on a handle of its own shape (7,936 × 3,584 padded)."""
-    n, m = 7681, 3329
+def _tuned_table(n, m, precs, ks):
+    """The decisions of passes of k columns on a handle of its own shape."""
     rows, _, dec = make_case(n, m, seed=84)
-    gm = orc.genotype_mean(orc.popcounts(dec), n)
+    gm = np.ones(m, np.float32)
     v = np.random.default_rng(3).standard_normal((n, max(ks))).astype(np.float32)
     with api.Genotypes(rows, n) as g:
-        g.set_weights(gm, orc.snp_weights(gm, np.ones(m, np.float32)))
+        g.set_weights(gm, gm)
         g.set_autotune(True)
         for prec in precs:
             g.set_precision(prec)
             for k in ks:
                 g.H0_ldet_mv(0.43, v[:, :k])
-    return [t for t in api.autotune_table() if {t["M_pad"], t["K_tiles"] * 64} == {7936, 3584}]
+    pads = {-(-n // 256) * 256, -(-m // 256) * 256}
+    return [t for t in api.autotune_table() if {t["M_pad"], t["K_tiles"] * 64} == pads], pads
 
 
 def test_tuner_keeps_formats_apart(gpu):
     """BF16X2 and FP16X2 passes of one shape have their own decisions."""
-    ks = (3, 9, 17, 24, 31)
-    table = _tuned_table((_lib.PREC_BF16X2, _lib.PREC_FP16X2), ks)
+    table, pads = _tuned_table(7681, 3329, (_lib.PREC_BF16X2, _lib.PREC_FP16X2), (3, 9, 17, 24, 31))
     for N in (16, 32, 48, 64):
-        assert sorted(t["M_pad"] for t in table if t["N"] == N and t["pieces"] == 2) == [3584, 3584, 7936, 7936]
+        assert sorted(t["M_pad"] for t in table if t["N"] == N and t["pieces"] == 2) == sorted([*pads, *pads])
 
 
-def test_tuner_times_digits_whichever_fp16_plan_wins(gpu):
+# 256 rows by 20,224: the FP16 plan with two CTAs per SM beats the default one by an eighth
+@pytest.mark.parametrize("n,m", [(200, 20001), (7681, 3329)])
+def test_tuner_times_digits_whichever_fp16_plan_wins(gpu, n, m):
     """Passes of at most 32 columns at FP16X2 are timed with digits too, in both directions."""
     ks = (3, 9, 17, 31)
-    table = _tuned_table((_lib.PREC_FP16X2,), ks)
+    table, pads = _tuned_table(n, m, (_lib.PREC_FP16X2,), ks)
     for k in ks:
         N = -(-5 * (-(-k // 8) * 8) // 16) * 16
         digits = [t for t in table if t["pieces"] == 5 and t["N"] == N]
-        assert {t["M_pad"] for t in digits} == {7936, 3584} and all(t["plan"] == 2 for t in digits)
+        assert {t["M_pad"] for t in digits} == pads and all(t["plan"] == 2 for t in digits)
