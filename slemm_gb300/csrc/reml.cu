@@ -149,8 +149,9 @@ static Setup reml_begin(slemm_geno* g, const float* rvec, const float* X, int64_
   return S;
 }
 
-// Second part: gm and gw while the GPU factors, then the handle's projection and, if `weights`, its weights.
-static void reml_setup(Setup& S, slemm_geno* g, int c, const float* persnp, bool weights = true)
+// Second part: gm and gw while the GPU factors, then the handle's weights (W_j = gw_j·scale_j when `scale` is
+// given) and, once they are accepted, its projection: a refused call leaves the handle as it was.
+static void reml_setup(Setup& S, slemm_geno* g, int c, const float* persnp, const float* scale = nullptr)
 {
   const int64_t n = g->n, m = g->m;
   // gm = nz_bits/float(n) from the GPU popcounts (bit-exact integers)
@@ -177,10 +178,14 @@ static void reml_setup(Setup& S, slemm_geno* g, int c, const float* persnp, bool
   if (S.qr->rank != c) SLEMM_THROW(SLEMM_ERR_RANK, "Fixed-effects design matrix is not of full rank.");
   if (mono < m)
     SLEMM_THROW(SLEMM_ERR_NUMERIC, "monomorphic SNP " + std::to_string(mono) + " gives an infinite weight");
-  set_projection_qr(g, *S.qr, c);
-  if (!weights) return;
-  int st = slemm_gpu_set_weights(g, S.gm.data(), S.gw.data(), S.rr.data());
+  std::vector<float> W;
+  if (scale) {
+    W.resize(m);
+    for (int64_t j = 0; j < m; ++j) W[j] = S.gw[j] * scale[j];
+  }
+  int st = slemm_gpu_set_weights(g, S.gm.data(), scale ? W.data() : S.gw.data(), S.rr.data());
   if (st != SLEMM_OK) SLEMM_THROW(st, "set_weights failed");
+  set_projection_qr(g, *S.qr, c);
 }
 
 static void upload(slemm_geno* g, float* d, const float* h, size_t cnt)
@@ -720,12 +725,12 @@ void reml_grad(slemm_geno* g, const float* rvec, const float* X, int64_t ldx, in
   Setup S = reml_begin(g, rvec, X, ldx, c);
   // probes straight into the block, drawn while the host set-up runs
   rademacher_device(seed, n, n_V, d_B.as<float>() + n, n, st);
-  reml_setup(S, g, c, persnp, false);
-  std::vector<float> W(m);
-  for (int64_t j = 0; j < m; ++j) W[j] = S.gw[j] * ((window && window[j] >= 0) ? wwin[window[j]] : 1.0f);
   {
-    const int s2 = slemm_gpu_set_weights(g, S.gm.data(), W.data(), S.rr.data());
-    if (s2 != SLEMM_OK) SLEMM_THROW(s2, "set_weights failed");
+    std::vector<float> scale(m, 1.0f);   // the handle's weights are gw·wwin
+    if (window)
+      for (int64_t j = 0; j < m; ++j)
+        if (window[j] >= 0) scale[j] = wwin[window[j]];
+    reml_setup(S, g, c, persnp, scale.data());
   }
   // ỹ_proj = (I − QQᵀ)(rr∘y) in FP64, as the DF-REML path
   d_X.ensure((size_t)n * t * sizeof(float));

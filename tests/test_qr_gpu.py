@@ -61,3 +61,21 @@ def test_designs_that_are_refused(gpu):
                 g.weighted_least_squares(rvec, bad, y)
             assert e.value.code == -1
         assert np.array_equal(before, g.op(_lib.OP_QUADFORM, v, 0.5))   # the handle is as it was
+
+
+def test_refused_gradient_weights_leave_the_handle(gpu):
+    """Window weights whose product with a SNP's own weight overflows are refused, and the handle keeps its
+    weights and its projection."""
+    n = 700
+    rows, X, rvec, y = _problem(n, 3, seed=6)
+    _, X2, rvec2, _ = _problem(n, 4, seed=7)
+    v = np.random.default_rng(1).standard_normal((n, 2)).astype(np.float32)
+    persnp = np.ones(96, np.float32)
+    persnp[0] = 1000
+    with api.Genotypes(rows, n) as g:
+        g.REML_grad(rvec, X, y, np.ones(96, np.float32), None, None, 0.4, 0.6, n_V=2)
+        before = [g.op(_lib.OP_QUADFORM, v, 0.5), g.op(_lib.OP_LDET, v, 0.5)]
+        with pytest.raises(_lib.SlemmError):
+            g.REML_grad(rvec2, X2, y, persnp, np.zeros(96, np.int32), np.full(1, 3e38, np.float32), 0.4, 0.6, n_V=2)
+        for a, kind in zip(before, (_lib.OP_QUADFORM, _lib.OP_LDET)):
+            assert np.array_equal(a, g.op(kind, v, 0.5))
