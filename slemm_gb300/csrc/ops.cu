@@ -231,8 +231,8 @@ __device__ __forceinline__ int split_exp(double bound, int top)
 {
   if (!(bound > 0.0) || !isfinite(bound)) return 0;
   int E;
-  frexp(bound, &E);                        // bound = f·2^E, f ∈ [0.5, 1)
-  return max(-120, min(120, top - E));
+  frexp(bound, &E);                        // bound = f·2^E, f ∈ [0.5, 1), E ≤ 129
+  return min(120, top - E);                // ≥ −125: 2^e and 2^−e are normal
 }
 
 // Block maximum of one float per thread (valid in thread 0; −∞ when every thread holds −∞);

@@ -65,3 +65,24 @@ def test_withheld_digit_copy_times_out_and_handle_recovers(gpu, k):
         assert e.value.code == -2 and "bounded wait" in str(e.value)
         got = g.rmatvec(v)
         assert np.linalg.norm(got - want) / np.linalg.norm(want) < 2e-6
+
+
+@pytest.mark.parametrize("which", ["rmatvec", "matvec"])
+@pytest.mark.parametrize("size", [8.6e37, 1.05e38, 1.7e38])
+def test_columns_near_the_largest_float(gpu, size, which):
+    """One large entry, whose products with the counts are finite, and an ordinary column beside it."""
+    n, m = 300, 260
+    rows, _, dec = make_case(n, m, seed=4)
+    rng = np.random.default_rng(2)
+    gm = orc.genotype_mean(orc.popcounts(dec), n)
+    x = dec.astype(np.float64) - gm[:, None].astype(np.float64)
+    if which == "matvec":
+        x = x.T
+    v = rng.standard_normal((x.shape[1], 2)).astype(np.float32)
+    v[:, 0] = 0
+    v[5, 0] = size
+    with api.Genotypes(rows, n) as g:
+        g.set_weights(gm, np.ones(m, np.float32))
+        got = getattr(g, which)(v)
+    want = x @ v.astype(np.float64)
+    assert np.all(np.linalg.norm(got - want, axis=0) <= 2e-6 * np.linalg.norm(want, axis=0))
