@@ -86,3 +86,30 @@ def test_columns_near_the_largest_float(gpu, size, which):
         got = getattr(g, which)(v)
     want = x @ v.astype(np.float64)
     assert np.all(np.linalg.norm(got - want, axis=0) <= 2e-6 * np.linalg.norm(want, axis=0))
+
+
+def test_odd_sums_just_below_their_bound(gpu):
+    """2^19 SNPs, one partial sum of each digit: the leading digits' sums of most individuals are odd integers
+    between 2^24 − 2^11 and 2^24, which 24 bits just hold."""
+    n, m = 130, 1 << 19
+    odd = np.arange(64) * 8192 + 77                      # SNPs whose counts vary, with odd leading digits
+    rng = np.random.default_rng(8)
+    counts = np.full((odd.size, n), 2, np.uint8)
+    counts[:] = rng.integers(0, 3, counts.shape)
+    rows = np.full((m, (n + 3) // 4), 0xFF, np.uint8)    # every other count is 2
+    rows[odd] = synth.encode_bed(counts)
+    digit = np.full(m, 16.0)
+    digit[odd] = rng.choice([7.0, 9.0, 11.0, 13.0], odd.size)
+    sign = -1.0                                          # −16 is a digit, 16 the one above 15.5
+    alpha = sign * (digit - np.where(digit == 16, 2.0 ** -30 * rng.integers(1, 2 ** 29, m), 0.0))
+    with api.Genotypes(rows, n) as g:
+        got = g.gebv(alpha)
+    lead = (np.rint(-alpha)[odd][:, None] * counts).sum(0) + 2.0 * 16 * (m - odd.size)
+    assert lead.max() <= 2 ** 24 and lead.min() >= 2 ** 24 - 2 ** 11 and (lead % 2 == 1).sum() > n // 4
+    # effects in units of 2^-30: whole numbers, summed exactly
+    a = np.rint(alpha * 2.0 ** 30).astype(np.int64)
+    assert np.array_equal(a / 2.0 ** 30, alpha)
+    rest = np.ones(m, bool)
+    rest[odd] = False
+    total = (a[odd][:, None] * counts.astype(np.int64)).sum(0) + 2 * int(a[rest].sum())
+    assert np.array_equal(got, total.astype(np.longdouble).astype(np.float64) / 2.0 ** 30)
