@@ -204,6 +204,10 @@ struct GemmArgs {
                         // below table[grp].y of its own (blocks past them write nothing); device memory
 };
 
+// K-tiles of one exact digit sum: 2^19 counts of at most 2 by digits of at most 16 are an integer of at most
+// 2^24, which an FP32 accumulator holds in any order.
+constexpr int kDigitKTiles = (1 << 19) / kTileK;
+
 void gemm_simt(const GemmArgs& a, cudaStream_t st);
 // Tensor-core path (tcgen05); N must be a multiple of 16 in [16, 256].
 void gemm_tc(const GemmArgs& a, cudaStream_t st);

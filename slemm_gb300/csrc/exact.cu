@@ -20,7 +20,6 @@ namespace slemm {
 constexpr int kDigitBits = 5;
 constexpr int kDigitsF64 = 13;
 constexpr int kDigitsF32 = 9;
-constexpr int kExactKTiles = (1 << 19) / kTileK;   // K-tiles of one exact FP32 partial sum
 constexpr int kXRows = 2048;                  // K-elements of one block of the operand kernels
 constexpr int kXThreads = 256;
 
@@ -180,11 +179,11 @@ dots_gather_kernel(const float* __restrict__ D, int splits, int kp, int64_t m_pa
   out[(int64_t)blockIdx.y * m + j] = isnan(tot[c]) ? NAN : v;
 }
 
-// Split-K count of an exact product over K_tiles K-tiles: at most kExactKTiles of them each.
+// Split-K count of an exact product over K_tiles K-tiles: at most kDigitKTiles of them each.
 static int exact_splits(int64_t M_pad, int64_t K_tiles, int N)
 {
   return choose_splits(M_pad / gemm_tc_rows_per_cta(N, 2), K_tiles, 1, num_sms(),
-                       (int)ceil_div(K_tiles, kExactKTiles));
+                       (int)ceil_div(K_tiles, kDigitKTiles));
 }
 
 void exact_gebv(slemm_geno* g, const double* d_alpha, double amax, double shift, double* d_tgv)

@@ -225,7 +225,7 @@ void col_dots(slemm_geno* g, const float* a, int64_t lda, const float* b, int64_
 // Digits (the same precision for at most kDigitCols columns) are a fixed-point split too: the column is
 // scaled into [2^3, 2^4) and written as five base-32 digits |d_p| ≤ 16, E4M3 bytes in the decoded
 // order of the counts (decode.cuh).  They resolve 2^−21 of a unit, ≤ 2^−24 of the column's largest
-// value, and every digit's sum is an exact integer.
+// value, and every digit's sum over a split's at most 2^19 K-elements is an exact integer.
 constexpr int kF16Top = 11, kDigitTop = 4;   // a column's bound times 2^e lies in [2^(top−1), 2^top)
 __device__ __forceinline__ int split_exp(double bound, int top)
 {
@@ -653,10 +653,11 @@ constexpr int kDigits = 5;
 // miss on the dense tiles they share.  Measured for Zᵀ over n = 950,000 individuals at N = 144:
 // 4,948 K-tiles per CTA 0.417 µs per K-tile, 1,485 0.356 (8.25 → 6.87 ms per launch), and 0.331
 // at n = 100,000 where the operand stays in L2.  So such passes keep ≤ 1,536 K-tiles per CTA.
-static int tc_min_splits(int64_t K_tiles, int N)
+static int digit_min_splits(int64_t K_tiles) { return (int)ceil_div(K_tiles, kDigitKTiles); }
+static int tc_min_splits(int64_t K_tiles, int N, bool digits)
 {
   const double dense_bytes = (double)K_tiles * kTileK * N * 2.0;
-  return dense_bytes > 64.0 * 1024 * 1024 ? (int)ceil_div(K_tiles, 1536) : 1;
+  return dense_bytes > 64.0 * 1024 * 1024 ? (int)ceil_div(K_tiles, 1536) : digits ? digit_min_splits(K_tiles) : 1;
 }
 
 static cudaEvent_t take_event(slemm_geno* g);
@@ -685,15 +686,15 @@ struct TuneEntry {
 static std::mutex g_tune_mu;
 static std::map<TuneKey, TuneEntry> g_tune;
 
-// Up to `most` split counts near `rule` (rule first) whose CTAs fill the last wave to ≥ 80 %.
-static void near_splits(int rule, int64_t ctas, int per_sm, int64_t K_tiles, int plan, size_t most,
+// Up to `most` split counts of at least `least` near `rule` (rule first) whose CTAs fill the last wave to ≥ 80 %.
+static void near_splits(int rule, int64_t ctas, int per_sm, int64_t K_tiles, int plan, int least, size_t most,
                         std::vector<std::pair<int, int>>& cand)
 {
   const int sms = num_sms() * per_sm;
   cand.push_back({plan, rule});
   std::vector<std::pair<int, int>> near;   // (distance, s)
   const int smax = (int)std::min<int64_t>(std::max(3 * rule + 2, 8), std::max<int64_t>(1, K_tiles / 16));
-  for (int s = std::max(1, rule / 3); s <= smax; ++s) {
+  for (int s = std::max(least, rule / 3); s <= smax; ++s) {
     if (s == rule) continue;
     const double waves = (double)(ctas * s) / sms;
     if (waves / std::ceil(waves) >= 0.8) near.push_back({std::abs(s - rule), s});
@@ -723,11 +724,12 @@ static double tune_pass(slemm_geno* g, PassPlan& p, const uint8_t* A, int64_t M_
   // candidates: the rule's count, then counts near it with a well-filled last wave; for N ≤ 64 the
   // same around the two-CTAs-per-SM plan's rule
   std::vector<std::pair<int, int>> cand;   // (plan, splits)
-  near_splits(p.splits, M_pad / gemm_tc_rows_per_cta(p.N, p.plan), 1, K_tiles, p.plan, 6, cand);
+  near_splits(p.splits, M_pad / gemm_tc_rows_per_cta(p.N, p.plan), 1, K_tiles, p.plan,
+              p.digits() ? digit_min_splits(K_tiles) : 1, 6, cand);
   if (p.N <= 64 && !p.digits()) {
     const int64_t ctas1 = M_pad / gemm_tc_rows_per_cta(p.N, 1);
-    const int rule1 = choose_splits(ctas1, K_tiles, 2, num_sms(), tc_min_splits(K_tiles, p.N));
-    near_splits(rule1, ctas1, 2, K_tiles, 1, 3, cand);
+    const int rule1 = choose_splits(ctas1, K_tiles, 2, num_sms(), tc_min_splits(K_tiles, p.N, false));
+    near_splits(rule1, ctas1, 2, K_tiles, 1, 1, 3, cand);
   }
   int smost = 1;
   for (const auto& c : cand) smost = std::max(smost, c.second);
@@ -773,7 +775,7 @@ static PassPlan plan_pass(slemm_geno* g, int k, int64_t M_pad, int64_t K_pad, co
   const int64_t M_tiles = M_pad / kTileM, K_tiles = K_pad / kTileK;
   auto rule = [&](const PassPlan& q, int per_sm) {
     return choose_splits(M_pad / gemm_tc_rows_per_cta(q.N, q.plan), K_tiles, per_sm, num_sms(),
-                         tc_min_splits(K_tiles, q.N));
+                         tc_min_splits(K_tiles, q.N, q.digits()));
   };
   if (!p.tc) {
     p.splits = choose_splits(M_tiles, K_tiles, 8, num_sms());
@@ -1088,7 +1090,7 @@ void rows_product(slemm_geno* g, int64_t r0, int64_t rows, const float* U, int64
     p.pieces = pieces;
     p.kp = (int)round_up(kc, 8);
     p.N = (int)round_up((int64_t)pieces * p.kp, 16);
-    p.splits = choose_splits(rows / gemm_tc_rows_per_cta(p.N, 0), K_tiles, 1, num_sms(), tc_min_splits(K_tiles, p.N));
+    p.splits = choose_splits(rows / gemm_tc_rows_per_cta(p.N, 0), K_tiles, 1, num_sms(), tc_min_splits(K_tiles, p.N, false));
     const int pad = p.N - pieces * kc;
     void* B1 = g->ws_B.ensure((size_t)p.N * K_pad * 2);
     float* D = (float*)g->ws_D.ensure((size_t)p.splits * p.kp * rows * sizeof(float));

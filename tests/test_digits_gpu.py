@@ -113,3 +113,20 @@ def test_odd_sums_just_below_their_bound(gpu):
     rest[odd] = False
     total = (a[odd][:, None] * counts.astype(np.int64)).sum(0) + 2 * int(a[rest].sum())
     assert np.array_equal(got, total.astype(np.longdouble).astype(np.float64) / 2.0 ** 30)
+
+
+def test_long_digit_sums_are_split(gpu):
+    """More than 2^19 K-elements, whose digit sums pass 2^24 in one accumulator."""
+    n, m = 130, 690000
+    rng = np.random.default_rng(6)
+    rows = np.bitwise_or.reduce([rng.integers(0, 256, (m, (n + 3) // 4), dtype=np.uint8) for _ in range(3)])
+    u = rng.uniform(0.96, 0.999, (m, 1)).astype(np.float32)
+    want = np.zeros(n)
+    for j in range(0, m, 50000):
+        want += orc.bed_decode(rows[j:j + 50000], n).T.astype(np.float64) @ u[j:j + 50000, 0].astype(np.float64)
+    assert want.min() * 16 > 2 ** 24
+    with api.Genotypes(rows, n) as g:
+        g.set_weights(np.zeros(m, np.float32), np.ones(m, np.float32))
+        got = g.matvec(u)[:, 0]
+    # 2^-24 of the largest value per entry, the digits' combination and the FP32 result
+    assert np.all(np.abs(got - want) <= 2.0 ** -22 * want)
