@@ -309,8 +309,8 @@ int slemm_gpu_wls(slemm_geno* g, const float* rvec, const float* X, int64_t ldx,
                   const float* y, float* snp_blup);
 
 /* ---- prediction and GWAS score statistics ------------------------------------------------- */
-/* GEBV: tgv_i = Σ_j (flip_j ? 2−count_ij : count_ij)·alpha_j, summed exactly (alpha to 2^−65 of its
- * largest value) and rounded to FP64 (src/pred.cpp:112-130).  Uses the handle's genotypes (no centring). flip: m
+/* GEBV: tgv_i = Σ_j (flip_j ? 2−count_ij : count_ij)·alpha_j, summed exactly (all bits of every
+ * alpha) and rounded to FP64 (src/pred.cpp:112-130).  Uses the handle's genotypes (no centring). flip: m
  * bytes or NULL.  Host pointers. */
 int slemm_gpu_gebv(slemm_geno* g, const double* alpha, const uint8_t* flip, double* tgv);
 /* GRAMMAR-Gamma per-SNP terms (bin/slemm_gamma.py:302-325), counting allele 1 like pgenlib:

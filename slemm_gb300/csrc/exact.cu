@@ -2,13 +2,14 @@
 //
 // A dense column v is cut into base-32 digits,
 //   v·2^e = d_0 + 2^−5·d_1 + 2^−10·d_2 + …,   d_p integers, |d_p| ≤ 16,
-// with e such that max|v|·2^e lies in [2^3, 2^4): 13 digits hold an FP64 column to 2^−65 of its
-// largest value, nine hold an FP32 one to 2^−45.  Digits are exact in E4M3 and a count is at most 2,
-// so a product row's sum over 2^19 K-elements is an integer of at most 2^24: the tensor cores' FP32
-// accumulators are exact whatever their order.  K is therefore split every 8,192 K-tiles at the
-// latest, the partials are added as 64-bit integers, and only the last combination of the digits
+// with e such that max|v|·2^e lies in [2^3, 2^4).  An FP64 column takes as many digits as reach the last bit
+// of its smallest nonzero value (11 where all are of one size, 15 for a million between the largest and the
+// smallest; up to 420, in passes of 160), an FP32 one nine: 2^−45 of its largest value.  Digits are exact in
+// E4M3 and a count is at most 2, so a product row's sum over 2^19 K-elements is an integer of at most 2^24: the
+// tensor cores' FP32 accumulators are exact whatever their order.  K is therefore split every 8,192 K-tiles at
+// the latest, the partials are added as 64-bit integers, and only the last combination of the digits
 // rounds (in FP64).  Bound by the narrow tensor-core pass.  GB300's FP64 pipe ran the same sums by an
-// FMA per genotype and column: at n = 100,000, m = 50,000 the GEBV took 18,988 µs and takes 556 µs, the
+// FMA per genotype and column: at n = 100,000, m = 50,000 the GEBV took 18,988 µs and takes 425 µs, the
 // score terms with three covariates and residual weights 112,698 µs and 697 µs, with the same or a
 // smaller error against 64-bit sums.
 #include "internal.h"
@@ -18,7 +19,7 @@
 namespace slemm {
 
 constexpr int kDigitBits = 5;
-constexpr int kDigitsF64 = 13;
+constexpr int kDigitRows = 160;   // digits of one pass
 constexpr int kDigitsF32 = 9;
 constexpr int kXRows = 2048;                  // K-elements of one block of the operand kernels
 constexpr int kXThreads = 256;
@@ -32,13 +33,35 @@ __host__ __device__ inline int digit_exp(double amax)
   return 4 - E;
 }
 
-// Digits 0 … S−1 of the 16 values v[·]·2^e of K-elements kidx … kidx + 15 (one packed word) into rows
-// row0 … row0 + S − 1 of the operand.
-template <int S, class T>
-__device__ __forceinline__ void store_digits(const T (&v)[16], int e, uint8_t* __restrict__ B, int64_t K_pad,
-                                             int row0, int64_t kidx)
+// Digits of a column at exponent e that reach the last of the `bits` bits of its smallest nonzero magnitude (at
+// 2^least the lowest bit of the type).
+__host__ __device__ inline int digit_count(int e, double amin, int bits, int least)
 {
-  T r[16];   // every step below is exact in the values' own type
+  if (!(amin > 0.0) || !isfinite(amin)) return 1;
+  int E;
+  frexp(amin, &E);
+  const int low = -((E - bits > least ? E - bits : least) + e);   // the bit is 2^−low of a unit
+  return 1 + (low > 0 ? (low + kDigitBits - 1) / kDigitBits : 0);
+}
+
+// v·2^e = I·2^−5K with integers I and K ≥ 0 (|v·2^e| ≤ 2^4).
+__device__ __forceinline__ void digit_int(double v, int e, long long& I, int& K)
+{
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  const int ex = (int)(b >> 52) & 0x7FF;
+  const long long M = (long long)((b & 0xFFFFFFFFFFFFFull) | (ex ? 0x10000000000000ull : 0ull));
+  const int L = 1075 - max(ex, 1) - e;   // |v·2^e| = M·2^−L
+  K = L > 0 ? (L + kDigitBits - 1) / kDigitBits : 0;
+  I = M << (K * kDigitBits - L);
+  I = (long long)b < 0 ? -I : I;
+}
+
+// Digits 0 … S−1 of the 16 FP32 values v[·]·2^e into rows row0 … row0 + S − 1.
+template <int S>
+__device__ __forceinline__ void store_digits_f32(const float (&v)[16], int e, uint8_t* __restrict__ B, int64_t K_pad,
+                                                 int row0, int64_t kidx)
+{
+  float r[16];   // every step below is exact
 #pragma unroll
   for (int u = 0; u < 16; ++u) r[u] = ldexp(v[u], e);
 #pragma unroll 1
@@ -46,50 +69,81 @@ __device__ __forceinline__ void store_digits(const T (&v)[16], int e, uint8_t* _
     float d[16];
 #pragma unroll
     for (int u = 0; u < 16; ++u) {
-      const T q = rint(r[u]);
-      d[u] = (float)q;
-      r[u] = (r[u] - q) * (T)(1 << kDigitBits);
+      d[u] = rint(r[u]);
+      r[u] = (r[u] - d[u]) * (float)(1 << kDigitBits);
     }
     *reinterpret_cast<uint4*>(B + (int64_t)(row0 + p) * K_pad + kidx) = e4m3_word(d);
   }
 }
 
-// Σ_p 2^−5p·(Σ_splits D[s][row0 + p][r]) — the column's product with row r, in units of 2^−e
-template <int S>
-__device__ __forceinline__ double gather_digits(const float* __restrict__ D, int splits, int kp, int64_t M_pad,
-                                                int row0, int64_t r)
+// Digits p0 … p0 + cnt − 1, of `digits` that hold every bit, of the 16 values v[·]·2^e of K-elements kidx …
+// kidx + 15 (one packed word) into rows row0 … row0 + cnt − 1 of the operand.  From the last digit up: the low five
+// bits of I as −16 … 15 in each step, and what is left as the first; in integers, since GB300's FP64 pipe has two
+// lanes (50,000 effects: 7 µs; the same digits by FP64 rounding and differences took 45 µs more).
+template <class T, class Int>
+__device__ __forceinline__ void store_digits(const T (&v)[16], int e, uint8_t* __restrict__ B, int64_t K_pad,
+                                             int row0, int digits, int p0, int cnt, int64_t kidx)
 {
-  long long sum[S] = {};
-  for (int s = 0; s < splits; ++s)
+  Int I[16];
+  int K[16];
 #pragma unroll
-    for (int p = 0; p < S; ++p) sum[p] += (long long)D[((int64_t)s * kp + row0 + p) * M_pad + r];
-  double v = 0.0;
+  for (int u = 0; u < 16; ++u) digit_int(v[u], e, I[u], K[u]);
+#pragma unroll 1
+  for (int p = digits - 1; p >= p0; --p) {
+    float d[16];
 #pragma unroll
-  for (int p = S - 1; p >= 0; --p) v = v * (1.0 / (1 << kDigitBits)) + (double)sum[p];
+    for (int u = 0; u < 16; ++u) {
+      int q = p > 0 ? (((int)I[u] + 16) & 31) - 16 : (int)I[u];
+      if (p > K[u]) q = 0;
+      d[u] = (float)q;
+      I[u] = p > K[u] ? I[u] : (I[u] - q) >> kDigitBits;
+    }
+    if (p < p0 + cnt) *reinterpret_cast<uint4*>(B + (int64_t)(row0 + p - p0) * K_pad + kidx) = e4m3_word(d);
+  }
+}
+
+// 2^−5cnt·v + Σ_p 2^−5p·(Σ_splits D[s][row0 + p][r]), p < cnt — the column's product with row r, in units of 2^−e,
+// with v what the digits after these gave.
+__device__ __forceinline__ double gather_digits(const float* __restrict__ D, int splits, int kp, int64_t M_pad,
+                                                int row0, int cnt, int64_t r, double v)
+{
+  constexpr int G = 8;   // digits read at a time, the last first
+  for (int p = cnt - 1; p >= 0; p -= G) {
+    long long sum[G] = {};
+    for (int s = 0; s < splits; ++s)
+#pragma unroll
+      for (int q = 0; q < G; ++q)
+        if (p >= q) sum[q] += (long long)D[((int64_t)s * kp + row0 + p - q) * M_pad + r];
+#pragma unroll
+    for (int q = 0; q < G; ++q)
+      if (p >= q) v = v * (1.0 / (1 << kDigitBits)) + (double)sum[q];
+  }
   return v;
 }
 
-// GEBV operand: rows 0 … 12 the digits of alpha (0 past m), rows 13 … 15 zero; 16 K-elements per thread
-// (32 threads a block: the FP64 steps of 16 effects are ~1,300 instructions on a pipe of two lanes per
-// clock and SM, so the blocks spread over all SMs)
+// GEBV operand: digits p0 … p0 + cnt − 1 of alpha (0 past m); 16 K-elements per thread
+// (32 threads a block, so that the blocks spread over all SMs)
 __global__ void __launch_bounds__(32)
-gebv_operand_kernel(const double* __restrict__ alpha, int64_t m, int64_t m_pad, int e, uint8_t* __restrict__ B)
+gebv_operand_kernel(const double* __restrict__ alpha, int64_t m, int64_t m_pad, int e, int digits, int p0, int cnt,
+                    uint8_t* __restrict__ B)
 {
   const int64_t j = ((int64_t)blockIdx.x * 32 + threadIdx.x) * 16;
   if (j >= m_pad) return;
   double v[16];
 #pragma unroll
   for (int u = 0; u < 16; ++u) v[u] = j + u < m ? alpha[j + u] : 0.0;
-  store_digits<kDigitsF64>(v, e, B, m_pad, 0, j);
-  for (int q = kDigitsF64; q < 16; ++q) *reinterpret_cast<uint4*>(B + (int64_t)q * m_pad + j) = make_uint4(0u, 0u, 0u, 0u);
+  store_digits<double, long long>(v, e, B, m_pad, 0, digits, p0, cnt, j);
 }
 
+// tgv = the digits' sums and, if `more`, the later digits' in tgv before; the first pass's result is shift + 2^−e·it.
 __global__ void __launch_bounds__(kXThreads)
-gebv_finish_kernel(const float* __restrict__ D, int splits, int kp, int64_t n_pad, int64_t n, int e, double shift,
-                   double* __restrict__ tgv)
+gebv_finish_kernel(const float* __restrict__ D, int splits, int kp, int64_t n_pad, int64_t n, int cnt, int more, int first,
+                   int e, double shift, double* __restrict__ tgv)
 {
   const int64_t i = (int64_t)blockIdx.x * kXThreads + threadIdx.x;
-  if (i < n) tgv[i] = shift + ldexp(gather_digits<kDigitsF64>(D, splits, kp, n_pad, 0, i), -e);
+  if (i >= n) return;
+  const double v = gather_digits(D, splits, kp, n_pad, 0, cnt, i, more ? tgv[i] : 0.0);
+  tgv[i] = first ? shift + ldexp(v, -e) : v;
 }
 
 // The columns of exact_dots (FP32 values), i < n.
@@ -164,7 +218,7 @@ dots_operand_kernel(ExactCols a, int64_t n, int64_t n_pad, int c0, int nc, const
   float v[16];
 #pragma unroll
   for (int u = 0; u < 16; ++u) v[u] = (i + u < n && fine) ? dot_column(a, c, i + u) : 0.f;
-  store_digits<kDigitsF32>(v, e, B, n_pad, kDigitsF32 * b, i);
+  store_digits_f32<kDigitsF32>(v, e, B, n_pad, kDigitsF32 * b, i);
 }
 
 // out[c0 + c][j] of the pass over columns c0 …; grid (rows, columns)
@@ -175,7 +229,7 @@ dots_gather_kernel(const float* __restrict__ D, int splits, int kp, int64_t m_pa
   const int64_t j = (int64_t)blockIdx.x * kXThreads + threadIdx.x;
   if (j >= m) return;
   const int c = c0 + blockIdx.y;
-  const double v = ldexp(gather_digits<kDigitsF32>(D, splits, kp, m_pad, kDigitsF32 * blockIdx.y, j), -exps[c]);
+  const double v = ldexp(gather_digits(D, splits, kp, m_pad, kDigitsF32 * blockIdx.y, kDigitsF32, j, 0.0), -exps[c]);
   out[(int64_t)blockIdx.y * m + j] = isnan(tot[c]) ? NAN : v;
 }
 
@@ -186,20 +240,24 @@ static int exact_splits(int64_t M_pad, int64_t K_tiles, int N)
                        (int)ceil_div(K_tiles, kDigitKTiles));
 }
 
-void exact_gebv(slemm_geno* g, const double* d_alpha, double amax, double shift, double* d_tgv)
+void exact_gebv(slemm_geno* g, const double* d_alpha, double amax, double amin, double shift, double* d_tgv)
 {
   cudaStream_t st = g->stream;
-  const int e = digit_exp(amax);
-  const int N = 16, kp = 16;
-  const int splits = exact_splits(g->n_pad, g->m_pad / kTileK, N);
-  uint8_t* B = (uint8_t*)g->ws_B.ensure((size_t)N * g->m_pad);
-  float* D = (float*)g->ws_D.ensure((size_t)splits * kp * g->n_pad * sizeof(float));
-  gebv_operand_kernel<<<(unsigned)ceil_div(g->m_pad, 16 * 32), 32, 0, st>>>(d_alpha, g->m, g->m_pad, e, B);
-  LAUNCH_CHECK();
-  gemm_tc({g->GT.as<uint8_t>(), g->n_pad, g->m_pad, B, N, D, splits, g->err.as<int>(), kp, 1, false, 2}, st);
-  gebv_finish_kernel<<<(unsigned)ceil_div(g->n, kXThreads), kXThreads, 0, st>>>(D, splits, kp, g->n_pad, g->n, e, shift,
-                                                                               d_tgv);
-  LAUNCH_CHECK();
+  const int e = digit_exp(amax), digits = digit_count(e, amin, 53, -1074);
+  for (int p0 = (digits - 1) / kDigitRows * kDigitRows; p0 >= 0; p0 -= kDigitRows) {   // the last digits first
+    const int cnt = std::min(kDigitRows, digits - p0);
+    const int kp = (int)round_up(cnt, 8), N = (int)round_up(kp, 16);
+    const int splits = exact_splits(g->n_pad, g->m_pad / kTileK, N);
+    uint8_t* B = (uint8_t*)g->ws_B.ensure((size_t)N * g->m_pad);
+    float* D = (float*)g->ws_D.ensure((size_t)splits * kp * g->n_pad * sizeof(float));
+    gebv_operand_kernel<<<(unsigned)ceil_div(g->m_pad, 16 * 32), 32, 0, st>>>(d_alpha, g->m, g->m_pad, e, digits, p0, cnt,
+                                                                                B);
+    LAUNCH_CHECK();
+    gemm_tc({g->GT.as<uint8_t>(), g->n_pad, g->m_pad, B, N, D, splits, g->err.as<int>(), kp, 1, false, 2}, st);
+    gebv_finish_kernel<<<(unsigned)ceil_div(g->n, kXThreads), kXThreads, 0, st>>>(
+        D, splits, kp, g->n_pad, g->n, cnt, p0 + cnt < digits, p0 == 0, e, shift, d_tgv);
+    LAUNCH_CHECK();
+  }
 }
 
 void exact_dots(slemm_geno* g, const ExactCols& a, double* dots, double* tot, double* twos)

@@ -104,8 +104,9 @@ void rows_product(slemm_geno* g, int64_t r0, int64_t rows, const float* U, int64
                   int64_t ldo, int prec);
 
 // exact.cu — exact products of the packed counts with dense columns.
-// d_tgv[i] = shift + Σ_j count_ij·d_alpha[j] (FP64 effects, largest magnitude amax).
-void exact_gebv(slemm_geno* g, const double* d_alpha, double amax, double shift, double* d_tgv);
+// d_tgv[i] = shift + Σ_j count_ij·d_alpha[j] (FP64 effects, largest magnitude amax, smallest nonzero one amin: ∞
+// if there is none).
+void exact_gebv(slemm_geno* g, const double* d_alpha, double amax, double amin, double shift, double* d_tgv);
 // The columns of exact_dots over individuals i < n, FP32 values in this order: y (when given), rr·Q_l
 // for l < cq, rr² (when rr is given; rr == nullptr means every rr is 1).
 struct ExactCols {

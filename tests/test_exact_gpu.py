@@ -65,3 +65,52 @@ def test_score_terms_exact_products(gpu, n, m, c, unit):
     assert np.all(np.abs(xy - want_xy) <= 2.0 ** -23 * np.abs(want_xy) + 1e-12 * np.abs(y).sum())
     assert np.all(np.abs(xx - want_xx) <= 2.0 ** -23 * np.abs(want_xx) + 1e-12 * r2.sum())
     assert np.all(np.isnan(nan_xy)) and np.array_equal(same_xx, xx)
+
+
+@pytest.mark.parametrize("small", [1e-6, 1e-14, 1e-40, 1e-300])
+def test_gebv_small_effects_beside_a_large_one(gpu, small):
+    """Individuals without a copy of the SNP of the large effect: their sum of small effects is as accurate as
+    without it."""
+    from slemm_gb300 import api
+    n, m = 700, 300
+    rows, _, dec = make_case(n, m, seed=9)
+    rng = np.random.default_rng(5)
+    alpha = rng.uniform(0.5, 1.0, m) * small
+    alpha[7] = 1.0
+    alpha[11] = 0.0
+    assert (dec[7] == 0).sum() > 10
+    with api.Genotypes(rows, n) as g:
+        got = g.gebv(alpha)
+    want = (dec.astype(np.longdouble) * alpha.astype(np.longdouble)[:, None]).sum(0)
+    # exact sums of positive terms, rounded a few times at the end
+    assert np.all(np.abs(got - want) <= 2.0 ** -51 * want)
+
+
+@pytest.mark.parametrize("n,m,c", [(700, 300, 2), (8200, 257, 14)])
+def test_score_terms_with_far_smaller_weights(gpu, n, m, c):
+    """Rare variants carried by individuals of small weight alone: what is left of xx after the centring terms
+    of the large weights has FP64's accuracy."""
+    from slemm_gb300 import api
+    rng = np.random.default_rng(n)
+    rr = np.where(np.arange(n) < 40, 1.0, rng.uniform(0.5, 1.0, n) * 1e-12).astype(np.float32)
+    dec = rng.binomial(2, 0.3, (m, n)).astype(np.uint8)
+    dec[:, :40] = 0
+    y = (rng.standard_normal(n) * 10.0 ** rng.uniform(-12, 12, n)).astype(np.float32)
+    y[:40] = 0
+    Q = np.zeros((n, c), np.float32)
+    Q[np.arange(c), np.arange(c)] = 1                     # the projection takes the first c individuals out
+    x = dec.astype(np.float64)
+    gm = x.mean(1)
+    with api.Genotypes(synth.encode_bed(dec), n) as g:
+        g.set_weights(gm.astype(np.float32), np.ones(m, np.float32), rr)
+        g.set_projection(Q)
+        xy, xx = g.score_terms(y, 0)
+    z = (x - gm[:, None]).astype(np.longdouble)
+    want_xy = -(z @ y.astype(np.longdouble))
+    r2 = (rr * rr).astype(np.longdouble)
+    rq = (rr[:, None] * Q).astype(np.longdouble)
+    want_xx = (z * z) @ r2 - ((z @ rq) ** 2).sum(1)
+    # FP64 sums of the terms, then FP32
+    size = (z * z) @ r2 + ((np.abs(z) @ np.abs(rq)) ** 2).sum(1)
+    assert np.all(np.abs(xy - want_xy) <= 2.0 ** -23 * np.abs(want_xy) + 2.0 ** -50 * (np.abs(z) @ np.abs(y).astype(np.longdouble)))
+    assert np.all(np.abs(xx - want_xx) <= 2.0 ** -23 * np.abs(want_xx) + 2.0 ** -50 * size)
