@@ -4,13 +4,13 @@
 //   v·2^e = d_0 + 2^−5·d_1 + 2^−10·d_2 + …,   d_p integers, |d_p| ≤ 16,
 // with e such that max|v|·2^e lies in [2^3, 2^4).  An FP64 column takes as many digits as reach the last bit
 // of its smallest nonzero value (11 where all are of one size, 15 for a million between the largest and the
-// smallest; up to 420, in passes of 160), an FP32 one nine: 2^−45 of its largest value.  Digits are exact in
-// E4M3 and a count is at most 2, so a product row's sum over 2^19 K-elements is an integer of at most 2^24: the
+// smallest; up to 420, in passes of 160), an FP32 one likewise (five to 56; the device finds their number, and the host
+// waits for it to lay out the passes).  Digits are exact in E4M3 and a count is at most 2, so a product row's sum over 2^19 K-elements is an integer of at most 2^24: the
 // tensor cores' FP32 accumulators are exact whatever their order.  K is therefore split every 8,192 K-tiles at
 // the latest, the partials are added as 64-bit integers, and only the last combination of the digits
 // rounds (in FP64).  Bound by the narrow tensor-core pass.  GB300's FP64 pipe ran the same sums by an
-// FMA per genotype and column: at n = 100,000, m = 50,000 the GEBV took 18,988 µs and takes 425 µs, the
-// score terms with three covariates and residual weights 112,698 µs and 697 µs, with the same or a
+// FMA per genotype and column: at n = 100,000, m = 50,000 the GEBV took 18,988 µs and takes 415 µs, the
+// score terms with three covariates and residual weights 112,698 µs and 694 µs, with the same or a
 // smaller error against 64-bit sums.
 #include "internal.h"
 #include "decode.cuh"
@@ -20,7 +20,7 @@ namespace slemm {
 
 constexpr int kDigitBits = 5;
 constexpr int kDigitRows = 160;   // digits of one pass
-constexpr int kDigitsF32 = 9;
+constexpr int kDigitCols = 32;    // most columns of one pass (an FP32 value has five digits at least)
 constexpr int kXRows = 2048;                  // K-elements of one block of the operand kernels
 constexpr int kXThreads = 256;
 
@@ -55,25 +55,15 @@ __device__ __forceinline__ void digit_int(double v, int e, long long& I, int& K)
   I = M << (K * kDigitBits - L);
   I = (long long)b < 0 ? -I : I;
 }
-
-// Digits 0 … S−1 of the 16 FP32 values v[·]·2^e into rows row0 … row0 + S − 1.
-template <int S>
-__device__ __forceinline__ void store_digits_f32(const float (&v)[16], int e, uint8_t* __restrict__ B, int64_t K_pad,
-                                                 int row0, int64_t kidx)
+__device__ __forceinline__ void digit_int(float v, int e, int& I, int& K)
 {
-  float r[16];   // every step below is exact
-#pragma unroll
-  for (int u = 0; u < 16; ++u) r[u] = ldexp(v[u], e);
-#pragma unroll 1
-  for (int p = 0; p < S; ++p) {
-    float d[16];
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      d[u] = rint(r[u]);
-      r[u] = (r[u] - d[u]) * (float)(1 << kDigitBits);
-    }
-    *reinterpret_cast<uint4*>(B + (int64_t)(row0 + p) * K_pad + kidx) = e4m3_word(d);
-  }
+  const unsigned b = __float_as_uint(v);
+  const int ex = (int)(b >> 23) & 0xFF;
+  const int M = (int)((b & 0x7FFFFFu) | (ex ? 0x800000u : 0u));
+  const int L = 150 - max(ex, 1) - e;
+  K = L > 0 ? (L + kDigitBits - 1) / kDigitBits : 0;
+  I = M << (K * kDigitBits - L);
+  I = (int)b < 0 ? -I : I;
 }
 
 // Digits p0 … p0 + cnt − 1, of `digits` that hold every bit, of the 16 values v[·]·2^e of K-elements kidx …
@@ -103,22 +93,29 @@ __device__ __forceinline__ void store_digits(const T (&v)[16], int e, uint8_t* _
 }
 
 // 2^−5cnt·v + Σ_p 2^−5p·(Σ_splits D[s][row0 + p][r]), p < cnt — the column's product with row r, in units of 2^−e,
-// with v what the digits after these gave.
+// with v what the digits after these gave.  Six digits at a time are one integer (a digit's sum is below 2^31 up to
+// 2^26 K-elements), so that they take one conversion and one FMA of the FP64 pipe instead of six.
 __device__ __forceinline__ double gather_digits(const float* __restrict__ D, int splits, int kp, int64_t M_pad,
                                                 int row0, int cnt, int64_t r, double v)
 {
-  constexpr int G = 8;   // digits read at a time, the last first
-  for (int p = cnt - 1; p >= 0; p -= G) {
+  constexpr int G = 6;
+  const float* Dr = D + (int64_t)row0 * M_pad + r;
+  v *= (double)(1 << kDigitBits * ((cnt + G - 1) / G * G - cnt));   // to the unit of the last group
+  for (int p = (cnt - 1) / G * G; p >= 0; p -= G) {
     long long sum[G] = {};
+#pragma unroll 4
     for (int s = 0; s < splits; ++s)
 #pragma unroll
       for (int q = 0; q < G; ++q)
-        if (p >= q) sum[q] += (long long)D[((int64_t)s * kp + row0 + p - q) * M_pad + r];
+        if (p + q < cnt) sum[q] += (long long)__float2int_rn(Dr[((int64_t)s * kp + p + q) * M_pad]);
+    long long I = sum[0];
 #pragma unroll
-    for (int q = 0; q < G; ++q)
-      if (p >= q) v = v * (1.0 / (1 << kDigitBits)) + (double)sum[q];
+    for (int q = 1; q < G; ++q) I = I * (1 << kDigitBits) + sum[q];
+    // v counts 2^−5 of the group's last digit
+    v = fma(v, 1.0 / (1 << kDigitBits), (double)I);
+    if (p > 0) v *= 1.0 / (1 << kDigitBits * (G - 1));
   }
-  return v;
+  return v * (1.0 / (1 << kDigitBits * (G - 1)));
 }
 
 // GEBV operand: digits p0 … p0 + cnt − 1 of alpha (0 past m); 16 K-elements per thread
@@ -157,80 +154,89 @@ __device__ __forceinline__ float dot_column(const ExactCols& a, int c, int64_t i
   return __fmul_rn(r, c < a.cq ? a.Q[(int64_t)c * a.ldq + i] : r);
 }
 
-// Block partials of each column's sum and largest magnitude (∞ for a non-finite value):
-// sums[c][blk], amax[c][blk]; grid (blocks, C).
+// Block partials of each column's sum and largest magnitude (∞ for a non-finite value), and of its smallest
+// nonzero magnitude negated (−∞: none): sums[c][blk], amax[c][blk], namin[c][blk]; grid (blocks, C).
 __global__ void __launch_bounds__(kXThreads)
-dots_stats_kernel(ExactCols a, int64_t n, double* __restrict__ sums, double* __restrict__ amax, int nblk)
+dots_stats_kernel(ExactCols a, int64_t n, double* __restrict__ sums, double* __restrict__ amax, double* __restrict__ namin,
+                  int nblk)
 {
   __shared__ double sh[32];
+  __shared__ float ext[2][kXThreads / 32];
   const int c = blockIdx.y;
   const int64_t i0 = (int64_t)blockIdx.x * kXRows, i1 = min64(n, i0 + kXRows);
-  DF acc;
-  float mx = 0.f;
+  double acc = 0.0;
+  float mx = 0.f, nmn = -INFINITY;
   for (int64_t i = i0 + threadIdx.x; i < i1; i += kXThreads) {
-    const float v = dot_column(a, c, i);
-    df_add(acc, v);
-    mx = fmaxf(mx, isfinite(v) ? fabsf(v) : INFINITY);
+    const float v = dot_column(a, c, i), mag = isfinite(v) ? fabsf(v) : INFINITY;
+    acc += (double)v;
+    mx = fmaxf(mx, mag);
+    nmn = fmaxf(nmn, mag > 0.f ? -mag : -INFINITY);
   }
-  const double s = block_sum_d(df_value(acc), sh);
-  __syncthreads();
-  double w = mx;
-  for (int o = 16; o; o >>= 1) w = fmax(w, __shfl_down_sync(0xffffffffu, w, o));
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = w;
+  const double s = block_sum_d(acc, sh);
+  for (int o = 16; o; o >>= 1) {
+    mx = fmaxf(mx, __shfl_down_sync(0xffffffffu, mx, o));
+    nmn = fmaxf(nmn, __shfl_down_sync(0xffffffffu, nmn, o));
+  }
+  if ((threadIdx.x & 31) == 0) ext[0][threadIdx.x >> 5] = mx, ext[1][threadIdx.x >> 5] = nmn;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int q = 1; q < kXThreads / 32; ++q) w = fmax(w, sh[q]);
+    for (int q = 1; q < kXThreads / 32; ++q) mx = fmaxf(mx, ext[0][q]), nmn = fmaxf(nmn, ext[1][q]);
     sums[(int64_t)c * nblk + blockIdx.x] = s;
-    amax[(int64_t)c * nblk + blockIdx.x] = w;
+    amax[(int64_t)c * nblk + blockIdx.x] = mx;
+    namin[(int64_t)c * nblk + blockIdx.x] = nmn;
   }
 }
 
-// Column c's total (NaN when it holds a non-finite value) and digit exponent, one warp each.
-__global__ void dots_scale_kernel(const double* __restrict__ sums, const double* __restrict__ amax, int nblk, int C,
-                                  double* __restrict__ tot, int* __restrict__ exps)
+// Column c's total (NaN when it holds a non-finite value), digit exponent and number of digits (host-mapped), one
+// warp each.
+__global__ void dots_scale_kernel(const double* __restrict__ sums, const double* __restrict__ amax,
+                                  const double* __restrict__ namin, int nblk, int C, double* __restrict__ tot,
+                                  int* __restrict__ exps, double* __restrict__ digits)
 {
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (c >= C) return;
   const double s = warp_sum_partials(sums + (int64_t)c * nblk, nblk);
   const double a = warp_max_partials(amax + (int64_t)c * nblk, nblk);
+  const double mn = -warp_max_partials(namin + (int64_t)c * nblk, nblk, 1, -INFINITY);
   if ((threadIdx.x & 31) == 0) {
     tot[c] = isfinite(a) ? s : NAN;
     exps[c] = digit_exp(a);
+    digits[c] = isfinite(a) ? digit_count(digit_exp(a), mn, 24, -149) : 1;
   }
 }
 
-// Operand of columns c0 … c0 + nc − 1: column c's digits in rows 9(c − c0) …, rows up to N zero.
-// Blocks y < nc write a column, y ≥ nc one zero row each.  A non-finite column is stored as zeros (its
-// products come out NaN through its total).
+// The columns c0 … c0 + count − 1 of one pass: column c0 + b has the operand rows off[b] … off[b + 1] − 1, its digits.
+struct DotsPass {
+  int c0, count;
+  int off[kDigitCols + 1];
+};
+
+// Their operand.  A non-finite column is stored as zeros (its products come out NaN through its total).
 __global__ void __launch_bounds__(kXThreads)
-dots_operand_kernel(ExactCols a, int64_t n, int64_t n_pad, int c0, int nc, const double* __restrict__ tot,
+dots_operand_kernel(ExactCols a, int64_t n, int64_t n_pad, const __grid_constant__ DotsPass P, const double* __restrict__ tot,
                     const int* __restrict__ exps, uint8_t* __restrict__ B)
 {
-  const int b = blockIdx.y;
+  const int b = blockIdx.y, c = P.c0 + b;
   const int64_t i = ((int64_t)blockIdx.x * kXThreads + threadIdx.x) * 16;
   if (i >= n_pad) return;
-  if (b >= nc) {
-    *reinterpret_cast<uint4*>(B + (int64_t)(kDigitsF32 * nc + b - nc) * n_pad + i) = make_uint4(0u, 0u, 0u, 0u);
-    return;
-  }
-  const int c = c0 + b, e = exps[c];
   const bool fine = !isnan(tot[c]);
   float v[16];
 #pragma unroll
   for (int u = 0; u < 16; ++u) v[u] = (i + u < n && fine) ? dot_column(a, c, i + u) : 0.f;
-  store_digits_f32<kDigitsF32>(v, e, B, n_pad, kDigitsF32 * b, i);
+  const int digits = P.off[b + 1] - P.off[b];
+  store_digits<float, int>(v, exps[c], B, n_pad, P.off[b], digits, 0, digits, i);
 }
 
-// out[c0 + c][j] of the pass over columns c0 …; grid (rows, columns)
+// out[b][j] of the pass; grid (rows, columns)
 __global__ void __launch_bounds__(kXThreads)
-dots_gather_kernel(const float* __restrict__ D, int splits, int kp, int64_t m_pad, int64_t m, int c0,
+dots_gather_kernel(const float* __restrict__ D, int splits, int kp, int64_t m_pad, int64_t m, const __grid_constant__ DotsPass P,
                    const double* __restrict__ tot, const int* __restrict__ exps, double* __restrict__ out)
 {
   const int64_t j = (int64_t)blockIdx.x * kXThreads + threadIdx.x;
   if (j >= m) return;
-  const int c = c0 + blockIdx.y;
-  const double v = ldexp(gather_digits(D, splits, kp, m_pad, kDigitsF32 * blockIdx.y, kDigitsF32, j, 0.0), -exps[c]);
-  out[(int64_t)blockIdx.y * m + j] = isnan(tot[c]) ? NAN : v;
+  const int b = blockIdx.y, c = P.c0 + b;
+  const double v = gather_digits(D, splits, kp, m_pad, P.off[b], P.off[b + 1] - P.off[b], j, 0.0);
+  out[(int64_t)b * m + j] = isnan(tot[c]) ? NAN : ldexp(v, -exps[c]);
 }
 
 // Split-K count of an exact product over K_tiles K-tiles: at most kDigitKTiles of them each.
@@ -264,42 +270,42 @@ void exact_dots(slemm_geno* g, const ExactCols& a, double* dots, double* tot, do
 {
   cudaStream_t st = g->stream;
   const int C = a.count();
-  const int64_t n_pad = g->n_pad, K_tiles = n_pad / kTileK;
+  const int64_t n_pad = g->n_pad, m_pad = g->m_pad, K_tiles = n_pad / kTileK;
   const int nblk = (int)ceil_div(n_pad, kXRows);
-  // up to 17 columns of nine digits fill one pass (N = 160)
-  const int grp = (int)ceil_div(C, ceil_div(C, 17));
-  const int kp = (int)round_up(kDigitsF32 * grp, 8), N = (int)round_up(kp, 16);
-  const int splits = exact_splits(g->m_pad, K_tiles, N), splits2 = exact_splits(g->m_pad, K_tiles, 16);
   DevBuf dst(st);
-  double* sums = (double*)dst.ensure((size_t)2 * C * nblk * sizeof(double) + C * sizeof(int));
-  double* amax = sums + (size_t)C * nblk;
-  int* exps = reinterpret_cast<int*>(amax + (size_t)C * nblk);
-  uint8_t* B = (uint8_t*)g->ws_B.ensure((size_t)N * n_pad);
-  float* D = (float*)g->ws_D.ensure(std::max((size_t)splits * kp, (size_t)splits2 * 16) * g->m_pad * sizeof(float));
-  const uint8_t* G = g->G.as<uint8_t>();
-  int* err = g->err.as<int>();
+  double* sums = (double*)dst.ensure((size_t)3 * C * nblk * sizeof(double) + C * sizeof(int));
+  double *amax = sums + (size_t)C * nblk, *namin = amax + (size_t)C * nblk;
+  int* exps = reinterpret_cast<int*>(namin + (size_t)C * nblk);
   const unsigned rows = (unsigned)ceil_div(g->m, kXThreads), oblk = (unsigned)ceil_div(n_pad, 16 * kXThreads);
-  dots_stats_kernel<<<dim3(nblk, C), kXThreads, 0, st>>>(a, g->n, sums, amax, nblk);
+  dots_stats_kernel<<<dim3(nblk, C), kXThreads, 0, st>>>(a, g->n, sums, amax, namin, nblk);
   LAUNCH_CHECK();
-  dots_scale_kernel<<<(unsigned)ceil_div(C * 32, 128), 128, 0, st>>>(sums, amax, nblk, C, tot, exps);
+  dots_scale_kernel<<<(unsigned)ceil_div(C * 32, 128), 128, 0, st>>>(sums, amax, namin, nblk, C, tot, exps,
+                                                                     g->scal.ensure(C));
   LAUNCH_CHECK();
-  for (int c0 = 0; c0 < C; c0 += grp) {
-    const int nc = std::min(grp, C - c0);
-    const int kpc = (int)round_up(kDigitsF32 * nc, 8), Nc = (int)round_up(kpc, 16);
-    dots_operand_kernel<<<dim3(oblk, nc + Nc - kDigitsF32 * nc), kXThreads, 0, st>>>(a, g->n, n_pad, c0, nc, tot, exps, B);
+  CUDA_TRY(cudaStreamSynchronize(st));   // the columns' numbers of digits
+  auto run = [&](const DotsPass& P, double* out, bool high) {
+    const int kp = (int)round_up(P.off[P.count], 8), N = (int)round_up(kp, 16);
+    const int splits = exact_splits(m_pad, K_tiles, N);
+    uint8_t* B = (uint8_t*)g->ws_B.ensure((size_t)N * n_pad);
+    float* D = (float*)g->ws_D.ensure((size_t)splits * kp * m_pad * sizeof(float));
+    dots_operand_kernel<<<dim3(oblk, P.count), kXThreads, 0, st>>>(a, g->n, n_pad, P, tot, exps, B);
     LAUNCH_CHECK();
-    gemm_tc({G, g->m_pad, n_pad, B, Nc, D, splits, err, kpc, 1, false, 2}, st);
-    dots_gather_kernel<<<dim3(rows, nc), kXThreads, 0, st>>>(D, splits, kpc, g->m_pad, g->m, c0, tot, exps,
-                                                              dots + (size_t)c0 * g->m);
+    gemm_tc({g->G.as<uint8_t>(), m_pad, n_pad, B, N, D, splits, g->err.as<int>(), kp, 1, false, 2, high}, st);
+    dots_gather_kernel<<<dim3(rows, P.count), kXThreads, 0, st>>>(D, splits, kp, m_pad, g->m, P, tot, exps, out);
     LAUNCH_CHECK();
+  };
+  const std::vector<double> digits(g->scal.h, g->scal.h + C);
+  for (int c = 0; c < C;) {   // as many columns per pass as fit
+    DotsPass P{c, 0, {0}};
+    while (c < C && P.count < kDigitCols && P.off[P.count] + (int)digits[c] <= kDigitRows) {
+      P.off[P.count + 1] = P.off[P.count] + (int)digits[c];
+      ++P.count;
+      ++c;
+    }
+    run(P, dots + (size_t)P.c0 * g->m, false);
   }
-  if (twos != nullptr) {   // 2·Σ rr²·[count = 2]: the last column (rr²) against the high bits
-    dots_operand_kernel<<<dim3(oblk, 1 + 16 - kDigitsF32), kXThreads, 0, st>>>(a, g->n, n_pad, C - 1, 1, tot, exps, B);
-    LAUNCH_CHECK();
-    gemm_tc({G, g->m_pad, n_pad, B, 16, D, splits2, err, 16, 1, false, 2, true}, st);
-    dots_gather_kernel<<<dim3(rows, 1), kXThreads, 0, st>>>(D, splits2, 16, g->m_pad, g->m, C - 1, tot, exps, twos);
-    LAUNCH_CHECK();
-  }
+  if (twos != nullptr)   // 2·Σ rr²·[count = 2]: the last column (rr²) against the high bits
+    run({C - 1, 1, {0, (int)digits[C - 1]}}, twos, true);
 }
 
 }  // namespace slemm

@@ -114,3 +114,25 @@ def test_score_terms_with_far_smaller_weights(gpu, n, m, c):
     size = (z * z) @ r2 + ((np.abs(z) @ np.abs(rq)) ** 2).sum(1)
     assert np.all(np.abs(xy - want_xy) <= 2.0 ** -23 * np.abs(want_xy) + 2.0 ** -50 * (np.abs(z) @ np.abs(y).astype(np.longdouble)))
     assert np.all(np.abs(xx - want_xx) <= 2.0 ** -23 * np.abs(want_xx) + 2.0 ** -50 * size)
+
+
+def test_score_terms_of_rare_variants_with_small_weights(gpu):
+    """Variants carried by individuals of small weight alone, in a sample whose weight is one individual's: the
+    carriers' part of xx, 2^-46 of the largest weight each, is comparable with the centring terms."""
+    from slemm_gb300 import api
+    n, m = 100003, 40
+    rng = np.random.default_rng(3)
+    rr = (rng.uniform(0.5, 1.0, n) * 2.0 ** -23).astype(np.float32)
+    rr[77] = 1
+    dec = np.zeros((m, n), np.uint8)
+    for j in range(m):
+        dec[j, rng.choice(np.arange(100, n), 25, replace=False)] = 1
+    y = rng.standard_normal(n).astype(np.float32)
+    with api.Genotypes(synth.encode_bed(dec), n) as g:
+        g.set_weights(dec.mean(1).astype(np.float32), np.ones(m, np.float32), rr)
+        g.set_projection(np.zeros((n, 0), np.float32))
+        _, xx = g.score_terms(y, 0)
+    z = (dec - dec.mean(1, dtype=np.float64)[:, None]).astype(np.longdouble)
+    want = (z * z) @ (rr * rr).astype(np.longdouble)
+    # FP64 sums of positive terms, then FP32
+    assert np.all(np.abs(xx - want) <= 2.0 ** -23 * want)
