@@ -78,3 +78,37 @@ def test_gwa_statistics_of_the_tested_range(gpu, ntest, mac):
     # two complementary error functions (CUDA's and the C library's) of at most 5 units in the last place each
     want = np.array([math.erfc(math.sqrt(float(x) / 2)) for x in chisq[ok]])
     assert np.allclose(p[ok], want, rtol=10 * 2.0 ** -52, atol=0)
+
+
+def _gwa_fp64(a2, y, R, X, model, block, tau, model_ct):
+    """β (times 1/cfactor) and xx/τ of every variant in FP64; rr and the variants' means as FP32 values."""
+    m, n = a2.shape
+    rr = (np.float32(1) / np.sqrt(R)).astype(np.float64)
+    Q = np.linalg.qr(rr[:, None] * X.astype(np.float64))[0]
+    mean = (a2.sum(1, dtype=np.int64).astype(np.float32) / np.float32(n)).astype(np.float64)
+    z = a2 - mean[:, None]
+    Z = z * rr
+    Z -= (Z @ Q) @ Q.T
+    xx = np.empty(m)
+    blocks, bounds, _ = orc.gwa_blocks(model, block, 0, m - 1)
+    for blk, (lo, hi) in zip(blocks, bounds):
+        B, mu = Z[blk], mean[blk]
+        H = B @ B.T + np.diag(model_ct * tau * (2 - mu) * mu / 2)
+        W = Z[lo:hi] @ B.T
+        xx[lo:hi] = (Z[lo:hi] ** 2).sum(1) - np.einsum("ij,ij->i", W, np.linalg.solve(H, W.T).T)
+    xx /= tau
+    return -(z @ y.astype(np.float64)) / xx, xx
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("block,n,c", [(4, 300, 1), (128, 1025, 2), (130, 700, 17), (322, 700, 2)])
+def test_gwa_blocks_vs_fp64(gpu, weighted, block, n, c):
+    m, n_model = 1200, 500
+    counts, rows, y, R, X = _data(n, m, c, weighted, seed=block + n)
+    model = np.sort(np.random.default_rng(block).permutation(m)[:n_model])
+    beta64, xx64 = _gwa_fp64(counts, y, R, X, model, block, 1.5, n_model)
+    with api.Genotypes(rows, n) as g:
+        beta, se, _, _ = g.gwa_windows(y, R, X, model, 0, m - 1, block, 1.5, n_model, 1.0, 1.0, -1)
+    # FP32 Gram entries (2^-22 of the diagonal) in well-conditioned systems of up to 322 unknowns: xx to 1e-5
+    assert np.allclose(1 / se.astype(np.float64) ** 2, xx64, rtol=1e-5, atol=0)
+    assert np.allclose(beta, beta64, rtol=1e-5, atol=1e-5 * np.abs(beta64).max())
