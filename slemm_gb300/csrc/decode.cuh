@@ -62,6 +62,21 @@ __device__ __forceinline__ uint32_t pair_of(uint32_t word, int q)
   else return bf16pair_of(word, q);
 }
 
+// Half the bit position s of element j (0 … 15) of a word read as an FP32 subnormal (x·2^(2s−149), gemm_simt.cu): even elements 2q at bits 2q, odd ones at 16 + 2q, the odd ones
+// from q = 4 on read from the word shifted right by 24.
+__host__ __device__ constexpr int f32sub_shift(int j)
+{
+  const int q = j >> 1;
+  return (j & 1) == 0 ? q : (q < 4 ? 8 + q : q - 4);
+}
+
+// Those bits: top is the word shifted right by 24.
+__device__ __forceinline__ float f32sub_of(uint32_t word, uint32_t top, int j)
+{
+  const int q = j >> 1;
+  return __uint_as_float((j & 1) == 0 ? word & (3u << (2 * q)) : q < 4 ? word & (3u << (16 + 2 * q)) : top & (3u << (2 * q - 8)));
+}
+
 // Four counts of a word as E4M3 bytes, by masking alone: a byte whose low two bits hold x is the
 // subnormal x·2^−9, and one whose bits 2, 3 hold x (mantissa and exponent zero elsewhere) reads as
 // x·2^−7 — x = 1 is the subnormal 4·2^−9, x = 2 the exponent field 1, 2^−6.  Group p = 0 … 3 of a

@@ -26,14 +26,6 @@ namespace slemm {
 constexpr int kStageTiles = 8;                 // 512 K elements per shared-memory stage
 constexpr int kStageK = kStageTiles * kTileK;
 
-// Shift s of element j (0 … 15) of a word: even elements 2q at bits 2q, odd ones at 16 + 2q, the odd ones
-// from q = 4 on read from the word shifted right by 24.
-__host__ __device__ constexpr int f32sub_shift(int j)
-{
-  const int q = j >> 1;
-  return (j & 1) == 0 ? q : (q < 4 ? 8 + q : q - 4);
-}
-
 template <int KC>
 __global__ void __launch_bounds__(128)
 gemm_simt_kernel(const uint4* __restrict__ A, int64_t M_pad, int64_t K_tiles,
@@ -121,8 +113,7 @@ gemm_simt_kernel(const uint4* __restrict__ A, int64_t M_pad, int64_t K_tiles,
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int qq = q + h;
-            const float xe = __uint_as_float(words[w] & (3u << (2 * qq)));
-            const float xo = __uint_as_float(qq < 4 ? words[w] & (3u << (16 + 2 * qq)) : top & (3u << (2 * qq - 8)));
+            const float xe = f32sub_of(words[w], top, 2 * qq), xo = f32sub_of(words[w], top, 2 * qq + 1);
 #pragma unroll
             for (int c = 0; c < KC; ++c)
               part[c] = fmaf(xe, bb[2 * h * KC + c], fmaf(xo, bb[(2 * h + 1) * KC + c], part[c]));

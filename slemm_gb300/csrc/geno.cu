@@ -689,12 +689,10 @@ int slemm_gpu_set_weights(slemm_geno* g, const float* gm, const float* w, const 
       hw[j] = w[j];
     }
     bool rr_one = true;
-    float rr_max = 0.f;
     for (int64_t i = 0; i < g->n; ++i) {
       hrr[i] = rr ? rr[i] : 1.0f;
       CHECK_ARG(std::isfinite(hrr[i]), "non-finite rr");
       rr_one = rr_one && hrr[i] == 1.0f;
-      rr_max = std::max(rr_max, std::fabs(hrr[i]));
     }
     // Z_cᵀ1 = Σ_i (x_ij − gm_j) = pc_j − n·gm_j, from the exact integer popcounts
     std::vector<int64_t> pc(g->m);
@@ -719,7 +717,6 @@ int slemm_gpu_set_weights(slemm_geno* g, const float* gm, const float* w, const 
     CUDA_TRY(cudaStreamSynchronize(g->stream));
     g->weights_set = true;
     g->rr_one = rr_one;
-    g->rr_max = rr_max;
   });
 }
 

@@ -1,17 +1,20 @@
 // gram.cu — projected Gram blocks of SNP rows, and the batched factorisation of their systems
 // (the windows of --lmm and the blocks of slemm_gwa).
 //
-// With P = I − QQᵀ, z_j = x_j − gm_j the centred counts of SNP j and t_j = Qᵀ(rr∘z_j),
-//   G_jk = (P(rr∘z_j))ᵀ(P(rr∘z_k)) = Σ_i rr_i²·x_ij·z_ik − gm_j·h_k − t_jᵀt_k,   h_k = Σ_i rr_i²·z_ik.
+// With P = I − QQᵀ, z_j = x_j − a_j the centred counts of SNP j and t_j = Qᵀ(rr∘z_j),
+//   G_jk = (P(rr∘z_j))ᵀ(P(rr∘z_k)) = Σ_i rr_i²·x_ij·z_ik − a_j·h_k − t_jᵀt_k,   h_k = Σ_i rr_i²·z_ik.
 // h and t come from one exact pass over the packed matrix (gram_stats), so a Gram block is one
 // packed product of SNP rows with columns that are read straight from the packed rows, and no
-// dense FP32 column of n individuals is ever formed.  In general the columns are rr²∘z_k,
-// column-scaled FP16 hi+lo; with every rr 1 they are the counts themselves, one E4M3 byte each, whose
-// product is an exact integer, and Σ_i x_ij·z_ik = Σ_i x_ij·x_ik − p_j·gm_k with p_j = Σ_i x_ij.  Forming U = rr∘P(rr∘z) as FP32
-// columns instead (centre, project, scale, measure, split: nine passes over n × columns floats)
-// took 38 of the 82 ms of slemm_gwa at n = 50,021 with 20,011 variants and 4,000 model SNPs, and
-// 31 of the 73 ms of --lmm with 30 windows of 1,000 SNPs at n = 50,000; the two calls now take 3.2
-// and 6.0 ms.
+// dense FP32 column of n individuals is ever formed.  With residual weights the columns are rr²∘z_k − f_k
+// in FP16 hi+lo at each column's own scale, f_k = 0 or their mean h_k/n where that is large, and
+//   Σ_i rr_i²·x_ij·z_ik = Σ_i x_ij·(rr_i²·z_ik − f_k) + p_j·f_k,   p_j = Σ_i x_ij;
+// with every rr 1 they are the counts themselves, one E4M3 byte each, whose product is an exact integer, and
+// f_k = −a_k.  Forming U = rr∘P(rr∘z) as FP32 columns instead (centre, project, scale, measure, split: nine
+// passes over n × columns floats) took 38 of the 82 ms of slemm_gwa at n = 50,021 with 20,011 variants and 4,000
+// model SNPs, and 31 of the 73 ms of --lmm with 30 windows of 1,000 SNPs at n = 50,000; the two calls now
+// take 3.2 and 6.0 ms (7.2 and 9.7 with residual weights).  With 600 variants in 20,000 individuals of weights 1 and
+// 1/100, half of them in the light individuals alone, the median error of slemm_gwa's xx is 1.3e-7 (3.5e-6 with
+// one scale for all columns, a = gm and t as single floats; 1.2e-6 with the dense columns).
 #include "gram.h"
 #include "decode.cuh"
 #include "reduce.cuh"
@@ -19,34 +22,109 @@
 namespace slemm {
 
 // ---- per-SNP statistics ------------------------------------------------------------------------
+// bound[j] = max_i rr_i²·|x_ij − a_j| (as the bits of a float, to a few units in the last place), zero at first: the
+// range of SNP j's column.  One thread per row of a tile and a share of the K-tiles; a count is the subnormal
+// x·2^(2s−149) of its masked bits (gemm_simt.cu), so an individual costs a LOP, an FMA, a product and half of a
+// three-way maximum.  A single bound 2·max rr² for all columns cost rare variants in individuals of small weight the
+// bits that lie between.
+constexpr int kBoundTiles = 8;
+__global__ void __launch_bounds__(kTileM)
+gram_bound_kernel(const uint4* __restrict__ G, int64_t K_tiles, const float* __restrict__ a, const float* __restrict__ rr,
+                  int64_t m, int tiles_per_block, unsigned* __restrict__ bound)
+{
+  __shared__ __align__(16) float r2[kBoundTiles * kTileK];   // rr²·2^49
+  const int64_t j = (int64_t)blockIdx.x * kTileM + threadIdx.x;
+  const float na = j < m ? __fmul_rn(-a[j], 1.7763568394002505e-15f) : 0.f;   // −a·2^−49
+  const int64_t kt0 = (int64_t)blockIdx.y * tiles_per_block, kt1 = min64(K_tiles, kt0 + tiles_per_block);
+  float most = 0.f;
+  for (int64_t ks = kt0; ks < kt1; ks += kBoundTiles) {
+    const int nt = (int)min64(kBoundTiles, kt1 - ks);
+    __syncthreads();
+    for (int q = threadIdx.x; q < nt * kTileK; q += kTileM) {
+      const float r = rr[ks * kTileK + q];
+      r2[q] = __fmul_rn(__fmul_rn(r, r), 562949953421312.f);
+    }
+    __syncthreads();
+    for (int u = 0; u < nt; ++u) {
+      const uint4 pk = G[((int64_t)blockIdx.x * K_tiles + ks + u) * kTileM + threadIdx.x];
+      const uint32_t words[4] = {pk.x, pk.y, pk.z, pk.w};
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const uint32_t top = words[w] >> 24;
+#pragma unroll
+        for (int e = 0; e < 16; e += 4) {
+          const float4 r4 = *reinterpret_cast<const float4*>(&r2[u * kTileK + w * 16 + e]);
+          const float r[4] = {r4.x, r4.y, r4.z, r4.w};
+          float v[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float k = __uint_as_float((uint32_t)(127 + 100 - 2 * f32sub_shift(e + q)) << 23);   // (x − a)·2^−49
+            v[q] = __fmul_rn(r[q], __fmaf_rn(f32sub_of(words[w], top, e + q), k, na));
+          }
+          most = fmaxf(fmaxf(most, fabsf(v[0])), fabsf(v[1]));
+          most = fmaxf(fmaxf(most, fabsf(v[2])), fabsf(v[3]));
+        }
+      }
+    }
+  }
+  if (j < m) atomicMax(bound + j, __float_as_uint(most));
+}
+
+// sc of every SNP: |rr²·z − f|·2^e below 2^11 (ops.cu, split_exp); an infinite bound stands for 2^128
+__global__ void __launch_bounds__(256)
+gram_scale_kernel(const unsigned* __restrict__ bound, int64_t m, GramStats s)
+{
+  const int64_t j = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (j >= m) return;
+  const double range = fmin((double)__uint_as_float(bound[j]), 3.4e38) * (1.0 + 1e-6) + fabs((double)s.f[j]);
+  int E = 11;
+  if (range > 0.0) frexp(range, &E);
+  const int e = max(-120, min(120, 11 - E));
+  s.sc[j] = make_float2(ldexpf(1.f, e), ldexpf(1.f, -e));
+}
+
 __global__ void __launch_bounds__(256)
 gram_stats_kernel(const double* __restrict__ dots, const double* __restrict__ twos, const double* __restrict__ tot,
                   int64_t m, int64_t n, const int64_t* __restrict__ pc, const int32_t* __restrict__ n2,
                   const float* __restrict__ gmf, int yb, int cq, GramStats s)
 {
   const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  // ‖P(rr∘1)‖² = Σ rr² − Σ_l (Q_lᵀrr)² to FP32's rounding of Q: the projection takes the intercept out
+  __shared__ bool intercept;
+  const double R = twos != nullptr ? tot[yb + cq] : (double)n;   // the last column is rr²
+  if (threadIdx.x < 32) {
+    double v = 0.0;
+    for (int l = threadIdx.x; l < cq; l += 32) v = fma(tot[yb + l], tot[yb + l], v);
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (threadIdx.x == 0) intercept = fabs(R - v) <= 0x1p-22 * R;
+  }
+  __syncthreads();
   if (j >= m) return;
   const double p = (double)pc[j], gm = (double)gmf[j];
-  double h, xx;
-  if (twos != nullptr) {   // the last column is rr²
-    const double S1 = dots[(int64_t)(yb + cq) * m + j], R = tot[yb + cq];
-    h = S1 - gm * R;
-    xx = (S1 + twos[j]) - 2.0 * gm * S1 + gm * gm * R;
-  } else {
-    h = p - gm * (double)n;
-    xx = (p + 2.0 * (double)n2[j]) - 2.0 * gm * p + gm * gm * (double)n;
-  }
+  const double S1 = twos != nullptr ? dots[(int64_t)(yb + cq) * m + j] : p;
+  const double S2 = twos != nullptr ? twos[j] : 2.0 * (double)n2[j];
+  // With the intercept projected out any constant may be taken off a count.  The weighted mean leaves the projection
+  // nothing to cancel (with gm it took h²/R of ‖rr∘z‖², more than half where genotypes go with the weights), and as
+  // a multiple of 2^−23 it has exact FP32 differences 1 − a and 2 − a.  Else a is gm, and a large mean of rr²∘z (h²/R
+  // over a fifth of ‖rr∘z‖²) is taken off the stored columns.
+  const double h0 = S1 - gm * R, zz0 = (S1 + S2) - 2.0 * gm * S1 + gm * gm * R;
+  const float af = intercept ? (float)(rint(S1 / R * 0x1p23) * 0x1p-23) : gmf[j];
+  const double a = (double)af, h = S1 - a * R;
+  double xx = (S1 + S2) - 2.0 * a * S1 + a * a * R;
+  float x, y;
   for (int l = 0; l < cq; ++l) {
-    const double t = dots[(int64_t)(yb + l) * m + j] - gm * tot[yb + l];
-    s.t[(int64_t)l * s.ld + j] = (float)t;
+    const double t = dots[(int64_t)(yb + l) * m + j] - a * tot[yb + l];
+    split_double(t, x, y);
+    s.t[(int64_t)l * s.ld + j] = make_float2(x, y);
     xx -= t * t;
   }
-  float a, b;
-  split_double(h, a, b);
-  s.h[j] = make_float2(a, b);
-  split_double(twos != nullptr ? 0.0 : p, a, b);
-  s.p[j] = make_float2(a, b);
-  s.gm[j] = gmf[j];
+  split_double(h, x, y);
+  s.h[j] = make_float2(x, y);
+  split_double(p, x, y);
+  s.p[j] = make_float2(x, y);
+  s.a[j] = af;
+  s.f[j] = twos == nullptr ? -af : !intercept && 5.0 * h0 * h0 > R * zz0 ? (float)(h / (double)n) : 0.f;
+  s.sc[j] = make_float2(1.f, 1.f);
   s.xy[j] = yb ? dots[j] - gm * tot[0] : 0.0;
   s.xx[j] = xx;
 }
@@ -70,6 +148,19 @@ void gram_stats(slemm_geno* g, const float* gm, const float* y, const float* rr,
   gram_stats_kernel<<<(unsigned)ceil_div(m, 256), 256, 0, st>>>(dots, twos, tot, m, g->n, pc, n1 + m, gm, y ? 1 : 0, cq,
                                                                  s);
   LAUNCH_CHECK();
+  if (rr == nullptr) return;
+  DevBuf db(st);
+  unsigned* bound = (unsigned*)db.ensure((size_t)m * sizeof(unsigned));
+  CUDA_TRY(cudaMemsetAsync(bound, 0, (size_t)m * sizeof(unsigned), st));
+  const int64_t K_tiles = g->n_pad / kTileK, M_tiles = g->m_pad / kTileM;
+  // twelve blocks an SM run at once; shares of whole stages
+  const int64_t stages = ceil_div(K_tiles, kBoundTiles), shares = std::min(stages, ceil_div(12 * num_sms(), M_tiles));
+  const int per = (int)ceil_div(stages, shares) * kBoundTiles;
+  gram_bound_kernel<<<dim3((unsigned)M_tiles, (unsigned)ceil_div(K_tiles, per)), kTileM, 0, st>>>(
+      g->G.as<uint4>(), K_tiles, s.a, rr, m, per, bound);
+  LAUNCH_CHECK();
+  gram_scale_kernel<<<(unsigned)ceil_div(m, 256), 256, 0, st>>>(bound, m, s);
+  LAUNCH_CHECK();
 }
 
 // dst SNP k = src SNP idx[k]
@@ -78,9 +169,11 @@ __global__ void gram_stats_gather_kernel(GramStats src, const int64_t* __restric
   const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= cnt) return;
   const int64_t j = idx[k];
-  dst.gm[k] = src.gm[j];
+  dst.a[k] = src.a[j];
   dst.h[k] = src.h[j];
   dst.p[k] = src.p[j];
+  dst.f[k] = src.f[j];
+  dst.sc[k] = src.sc[j];
   dst.xy[k] = src.xy[j];
   dst.xx[k] = src.xx[j];
   for (int l = 0; l < cq; ++l) dst.t[(int64_t)l * dst.ld + k] = src.t[(int64_t)l * src.ld + j];
@@ -137,12 +230,12 @@ gram_counts_kernel(const uint32_t* __restrict__ G, int64_t K_tiles, const GramGr
   }
 }
 
-// With residual weights: N = 2·kp rows, FP16 pieces hi and lo of rr²·z·2^e, each times the 2^−2s of its K
+// With residual weights: N = 2·kp rows, FP16 pieces hi and lo of (rr²·z − f)·2^e, each times the 2^−2s of its K
 // position (f16sub_pair_of).  A thread writes 8 K-elements (half of a packed word): 16-byte stores, 512
 // contiguous bytes per warp.  Bound by the 16-bit operand it writes.
 __global__ void __launch_bounds__(256)
 gram_operand_kernel(const uint32_t* __restrict__ G, int64_t K_tiles, const GramGroup* __restrict__ groups, int kp,
-                    const float* __restrict__ gm, const float* __restrict__ rr, float scale, __half* __restrict__ B)
+                    GramStats cs, const float* __restrict__ rr, __half* __restrict__ B)
 {
   const int64_t q8 = (int64_t)blockIdx.x * 256 + threadIdx.x;   // K-elements 8·q8 …
   const int64_t K_pad = K_tiles * kTileK;
@@ -156,9 +249,9 @@ gram_operand_kernel(const uint32_t* __restrict__ G, int64_t K_tiles, const GramG
     const int w = (int)(q8 & 7) >> 1, h = (int)(q8 & 1);
     const uint32_t word = G[((j / 128 * K_tiles + kt) * 128 + j % 128) * 4 + w];
     float zv[3], rv[8];
-    const float g = gm[j];
+    const float a = cs.a[j], f = cs.f[j], scale = cs.sc[j].x;
 #pragma unroll
-    for (int x = 0; x < 3; ++x) zv[x] = __fsub_rn((float)x, g);
+    for (int x = 0; x < 3; ++x) zv[x] = __fsub_rn((float)x, a);
     const float4 r0 = *reinterpret_cast<const float4*>(rr + q8 * 8);
     const float4 r1 = *reinterpret_cast<const float4*>(rr + q8 * 8 + 4);
     rv[0] = r0.x, rv[1] = r0.y, rv[2] = r0.z, rv[3] = r0.w;
@@ -169,11 +262,9 @@ gram_operand_kernel(const uint32_t* __restrict__ G, int64_t K_tiles, const GramG
       const int q = 4 * h + p, s = f16sub_shift(q);
       const uint32_t xe = (word >> (2 * q)) & 3u, xo = (word >> (16 + 2 * q)) & 3u;
       const float ks = __uint_as_float((uint32_t)(127 - 2 * s) << 23);
-      const float ve = __fmul_rn(__fmul_rn(__fmul_rn(rv[2 * p], rv[2 * p]), xe == 0 ? zv[0] : xe == 1 ? zv[1] : zv[2]),
-                                 scale);
-      const float vo = __fmul_rn(__fmul_rn(__fmul_rn(rv[2 * p + 1], rv[2 * p + 1]),
-                                           xo == 0 ? zv[0] : xo == 1 ? zv[1] : zv[2]),
-                                 scale);
+      const float ze = xe == 0 ? zv[0] : xe == 1 ? zv[1] : zv[2], zo = xo == 0 ? zv[0] : xo == 1 ? zv[1] : zv[2];
+      const float ve = __fmul_rn(__fmaf_rn(__fmul_rn(rv[2 * p], rv[2 * p]), ze, -f), scale);
+      const float vo = __fmul_rn(__fmaf_rn(__fmul_rn(rv[2 * p + 1], rv[2 * p + 1]), zo, -f), scale);
       const float he = rintf(ve), ho = rintf(vo);
       ph[p] = (uint32_t)__half_as_ushort(__float2half_rn(__fmul_rn(he, ks))) |
               ((uint32_t)__half_as_ushort(__float2half_rn(__fmul_rn(ho, ks))) << 16);
@@ -187,41 +278,46 @@ gram_operand_kernel(const uint32_t* __restrict__ G, int64_t K_tiles, const GramG
   *reinterpret_cast<uint4*>(dst + (int64_t)kp * K_pad) = lo;
 }
 
-// Σ_splits D·isc − gm_row·h_c − p_row·gm_c − t_rowᵀt_c of product row i (SNP r) and column cc of group grp
+// 2^−e_c·Σ_splits D − a_row·h_c + p_row·f_c − t_rowᵀt_c of product row i (SNP r) and column cc of group grp
 // (SNP c); double-float sums.
 __device__ __forceinline__ float gram_entry(const float* __restrict__ D, int splits, int kp, int64_t rows, int64_t i, int grp,
-                                            int cc, float isc, const GramStats& rs, int64_t r, const GramStats& cs, int64_t c,
+                                            int cc, const GramStats& rs, int64_t r, const GramStats& cs, int64_t c,
                                             int cq)
 {
   const float* Dc = D + ((int64_t)grp * splits * kp + cc) * rows + i;
   DF a;
+  const float isc = cs.sc[c].y;
 #pragma unroll 4
   for (int s = 0; s < splits; ++s) df_add(a, __fmul_rn(Dc[(int64_t)s * kp * rows], isc));
   const float2 h = cs.h[c], p = rs.p[r];
-  const float gr = rs.gm[r], gc = cs.gm[c];
-  df_fma(a, -gr, h.x);
-  df_fma(a, -p.x, gc);
-  a.lo = __fmaf_rn(-gr, h.y, __fmaf_rn(-p.y, gc, a.lo));
-  for (int l = 0; l < cq; ++l) df_fma(a, -rs.t[(int64_t)l * rs.ld + r], cs.t[(int64_t)l * cs.ld + c]);
+  const float ar = rs.a[r], f = cs.f[c];
+  df_fma(a, -ar, h.x);
+  df_fma(a, p.x, f);
+  a.lo = __fmaf_rn(-ar, h.y, __fmaf_rn(p.y, f, a.lo));
+  for (int l = 0; l < cq; ++l) {
+    const float2 tr = rs.t[(int64_t)l * rs.ld + r], tc = cs.t[(int64_t)l * cs.ld + c];
+    df_fma(a, -tr.x, tc.x);
+    a.lo = __fmaf_rn(-tr.x, tc.y, __fmaf_rn(-tr.y, tc.x, a.lo));
+  }
   return __fadd_rn(a.hi, a.lo);
 }
 
 // out[c·ldo + i] of every product row i and column c of the groups (blockIdx.z).
 __global__ void __launch_bounds__(256)
-gram_finish_kernel(const float* __restrict__ D, int splits, int kp, int64_t rows, float isc, GramStats rs, GramStats cs,
+gram_finish_kernel(const float* __restrict__ D, int splits, int kp, int64_t rows, GramStats rs, GramStats cs,
                    const GramGroup* __restrict__ groups, int cq, int64_t ldo)
 {
   const GramGroup G = groups[blockIdx.z];
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x, c = blockIdx.y;
   if (i >= G.nrows || c >= G.nc) return;
-  G.out[(G.c0 - G.b0 + c) * ldo + i] = gram_entry(D, splits, kp, rows, i, blockIdx.z, (int)c, isc, rs, G.r0 + i, cs, G.c0 + c, cq);
+  G.out[(G.c0 - G.b0 + c) * ldo + i] = gram_entry(D, splits, kp, rows, i, blockIdx.z, (int)c, rs, G.r0 + i, cs, G.c0 + c, cq);
 }
 
 // The same of blocks of a symmetric product, for the entries with r0 + i ≤ c0 + c; with `mirror` each of them
 // also at the other half's place, product row c0 + c − r0 and column r0 + i − b0 (where that is one of the
 // block's columns), through shared memory so that both writes are whole lines.
 __global__ void __launch_bounds__(256)
-gram_finish_sym_kernel(const float* __restrict__ D, int splits, int kp, int64_t rows, float isc, GramStats st,
+gram_finish_sym_kernel(const float* __restrict__ D, int splits, int kp, int64_t rows, GramStats st,
                        const GramGroup* __restrict__ groups, int cq, int64_t ldo, int mirror)
 {
   __shared__ float tile[32][33];
@@ -235,7 +331,7 @@ gram_finish_sym_kernel(const float* __restrict__ D, int splits, int kp, int64_t 
   for (int q = 0; q < 4; ++q) {
     const int64_t c = ct + y + 8 * q;
     if (i >= G.nrows || c >= G.nc || G.r0 + i > G.c0 + c) continue;
-    const float v = gram_entry(D, splits, kp, rows, i, blockIdx.z, (int)c, isc, st, G.r0 + i, st, G.c0 + c, cq);
+    const float v = gram_entry(D, splits, kp, rows, i, blockIdx.z, (int)c, st, G.r0 + i, st, G.c0 + c, cq);
     G.out[(G.c0 - G.b0 + c) * ldo + i] = v;
     tile[y + 8 * q][x] = v;
   }
@@ -286,18 +382,11 @@ void gram_rows(const GramSide& R, int64_t s0, int64_t cnt, GramJob& job)
 }
 
 void gram_blocks(slemm_geno* g, const GramSide& R, const GramSide& C, const std::vector<GramJob>& jobs, int cq, const float* rr,
-                 float rr_max, int64_t ldo, GramHalf half)
+                 int64_t ldo, GramHalf half)
 {
   cudaStream_t st = g->stream;
   const int64_t K_pad = g->n_pad, K_tiles = K_pad / kTileK;
   const bool unit = rr == nullptr, sym = half != GramHalf::all;
-  // |rr²·z| ≤ 2·max rr²: the bound lies in [2^10, 2^11) after scaling (ops.cu, split_exp)
-  int e = 0;
-  if (!unit) {
-    int E = 0;
-    std::frexp(2.0 * (double)rr_max * (double)rr_max, &E);
-    e = std::max(-120, std::min(120, 11 - E));
-  }
   // N ≤ 160 keeps two row tiles, each with its own MMA-issuing thread, in one CTA
   const int most = unit ? 160 : 80;
   std::vector<GramGroup> groups;
@@ -345,19 +434,18 @@ void gram_blocks(slemm_geno* g, const GramSide& R, const GramSide& C, const std:
       gram_counts_kernel<<<dim3((unsigned)ceil_div(K_pad / 16, 256), (unsigned)ceil_div(kp, kCountRows), ng), 256, 0, st>>>(Gc, K_tiles, dg + g0, kp, (uint8_t*)B);
     else
       gram_operand_kernel<<<dim3((unsigned)ceil_div(K_pad / 8, 256), kp, ng), 256, 0, st>>>(
-          Gc, K_tiles, dg + g0, kp, C.stats.gm, rr, (float)std::ldexp(1.0, e), (__half*)B);
+          Gc, K_tiles, dg + g0, kp, C.stats, rr, (__half*)B);
     LAUNCH_CHECK();
     GemmArgs a{R.G, rows, K_pad, B, N, D, splits, g->err.as<int>(), kp, unit ? 1 : 2, !unit, plan};
     a.groups = ng;
     a.table = dt + g0;
     gemm_tc(a, st);
-    const float isc = (float)std::ldexp(1.0, -e);
     if (sym)
       gram_finish_sym_kernel<<<dim3((unsigned)ceil_div(rows, 32), (unsigned)ceil_div(widest, 32), ng), 256, 0, st>>>(
-          D, splits, kp, rows, isc, R.stats, dg + g0, cq, ldo, half == GramHalf::mirrored ? 1 : 0);
+          D, splits, kp, rows, R.stats, dg + g0, cq, ldo, half == GramHalf::mirrored ? 1 : 0);
     else
       gram_finish_kernel<<<dim3((unsigned)ceil_div(rows, 256), (unsigned)widest, ng), 256, 0, st>>>(
-          D, splits, kp, rows, isc, R.stats, C.stats, dg + g0, cq, ldo);
+          D, splits, kp, rows, R.stats, C.stats, dg + g0, cq, ldo);
     LAUNCH_CHECK();
   }
 }

@@ -7,13 +7,18 @@
 
 namespace slemm {
 
-// Per-SNP statistics (device) with z = x − gm: h = Σ rr²·z and, when every rr is 1, p = Σ x (else 0), as
-// hi+lo FP32 pairs; t = Qᵀ(rr∘z) (cq × ld), xy = zᵀy (0 without y) and xx = ‖(I − QQᵀ)(rr∘z)‖².
+// Per-SNP statistics (device) with z = x − a: h = Σ rr²·z, p = Σ x and t = Qᵀ(rr∘z) (cq × ld) as hi+lo FP32
+// pairs, xx = ‖(I − QQᵀ)(rr∘z)‖², and xy = (x − gm)ᵀy (0 without y).  a is the mean weighted by rr² where the
+// projection takes the intercept out, else gm.  As a column of a Gram block a SNP is stored as (rr²∘z − f)·sc.x with
+// residual weights, f = h/n where gm is far from the weighted mean and has to stay, else 0, and sc = {2^e, 2^−e} of
+// its range; and as its counts x = z − f, f = −a, without.
 struct GramStats {
-  float* gm;
+  float* a;
+  float* f;
+  float2* sc;
   float2* h;
   float2* p;
-  float* t;
+  float2* t;
   double* xy;
   double* xx;
   int64_t ld;
@@ -26,12 +31,14 @@ struct GramStatsBuf {
     buf.stream = st;
     buf.ordered = true;
     s.ld = m;
-    s.xy = (double*)buf.ensure((size_t)m * (2 * sizeof(double) + 2 * sizeof(float2) + ((size_t)cq + 1) * sizeof(float)));
+    s.xy = (double*)buf.ensure((size_t)m * (2 * sizeof(double) + ((size_t)cq + 3) * sizeof(float2) + 2 * sizeof(float)));
     s.xx = s.xy + m;
     s.h = reinterpret_cast<float2*>(s.xx + m);
     s.p = s.h + m;
-    s.gm = reinterpret_cast<float*>(s.p + m);
-    s.t = s.gm + m;
+    s.sc = s.p + m;
+    s.t = s.sc + m;
+    s.a = reinterpret_cast<float*>(s.t + (size_t)cq * m);
+    s.f = s.a + m;
     return s;
   }
 };
@@ -57,12 +64,12 @@ struct GramJob {
 // The rows of a block that has to hold SNPs s0 … s0 + cnt − 1 of R: at most round_up(cnt, 256) + 256.
 void gram_rows(const GramSide& R, int64_t s0, int64_t cnt, GramJob& job);
 // The blocks of one pair of sides.  g gives the stream, the work buffers and the individuals; rr (n_pad) ==
-// nullptr: all 1, else rr_max ≥ max|rr|.  With R and C the same side and a block's columns among its rows: `lower`
+// nullptr: all 1.  With R and C the same side and a block's columns among its rows: `lower`
 // wants the rows up to each column's own SNP alone (out's others are left alone), `mirrored` has the columns'
 // SNPs from the other half as well.
 enum class GramHalf { all, lower, mirrored };
 void gram_blocks(slemm_geno* g, const GramSide& R, const GramSide& C, const std::vector<GramJob>& jobs, int cq, const float* rr,
-                 float rr_max, int64_t ldo, GramHalf half);
+                 int64_t ldo, GramHalf half);
 
 // A batch of nb systems of s unknowns (layout in gram.cu); offA, offZ and t are device arrays.
 struct SpdBatch {

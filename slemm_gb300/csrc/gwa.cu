@@ -120,13 +120,11 @@ extern "C" int slemm_gpu_gwa_windows(slemm_geno* g, const float* y, const float*
     // same projection)
     std::vector<float> rr(g->n_pad, 0.f);
     bool rr_one = true;
-    float rr_max = 0.f;
     for (int64_t i = 0; i < n; ++i) {
       const float r = R ? R[i] : 1.0f;
       CHECK_ARG(r > 0.f && std::isfinite(r), "R must be positive");
       rr[i] = 1.0f / std::sqrt(r);
       rr_one = rr_one && rr[i] == 1.0f;
-      rr_max = std::max(rr_max, rr[i]);
     }
     DesignQr qr(covar, ldc, rr.data(), n, c, st);
     // per-SNP means (allele-2) of the whole handle
@@ -205,8 +203,8 @@ extern "C" int slemm_gpu_gwa_windows(slemm_geno* g, const float* y, const float*
         job.out = Z + off[bn + bi] * rows_max;
         tested_by.push_back(job);
       }
-      gram_blocks(g, model, model, own, c, drr, rr_max, rows_max, GramHalf::lower);
-      gram_blocks(g, model, all, tested_by, c, drr, rr_max, rows_max, GramHalf::all);
+      gram_blocks(g, model, model, own, c, drr, rows_max, GramHalf::lower);
+      gram_blocks(g, model, all, tested_by, c, drr, rows_max, GramHalf::all);
       float* dr = (float*)d_ridge.ensure(ridge.size() * sizeof(float));
       int64_t* doff = (int64_t*)d_off.ensure(off.size() * sizeof(int64_t));
       CUDA_TRY(cudaMemcpyAsync(dr, ridge.data(), ridge.size() * sizeof(float), cudaMemcpyHostToDevice, st));

@@ -16,7 +16,6 @@ struct slemm_geno {
   int c = 0;
   bool weights_set = false;
   bool rr_one = false;            // every rr of set_weights is 1
-  float rr_max = 0.f;             // its largest |rr|
   int prec = SLEMM_PREC_FP16X2;
   int per_vector = 0;
   int lanczos_mode = 0;           // SLEMM_LANCZOS_* bits of the seeds run on this handle

@@ -156,7 +156,7 @@ extern "C" int slemm_gpu_lmm_quadforms(slemm_geno* g, const float* Py, float tau
       idx[k + c] = (int64_t)c * (ws + 1);
       idx[2 * k + c] = j - wds;
     }
-    gram_blocks(g, side, side, jobs, g->c, rr, g->rr_max, rows_max, GramHalf::mirrored);
+    gram_blocks(g, side, side, jobs, g->c, rr, rows_max, GramHalf::mirrored);
     check_device_error(g);
     // batched systems: q_c = zᵀ(ZᵀZ + D)⁻¹z
     float* dvec = (float*)d_d.ensure((size_t)k * ws * sizeof(float));
@@ -170,7 +170,11 @@ extern "C" int slemm_gpu_lmm_quadforms(slemm_geno* g, const float* Py, float tau
     CUDA_TRY(cudaMemcpyAsync(status + 1, one.data(), (size_t)k * sizeof(int), cudaMemcpyHostToDevice, st));
     spd_quadforms({gram, stride, gram + (size_t)ws * rows_max, didx, didx + k, status + 1, rows_max, ws, k, 1}, dvec,
                   didx + 2 * k, q, status, st);
-    std::vector<double> h(3 * k), hq((size_t)k * nq);
+    // ‖v‖² as the Gram blocks have it: xBx is its difference from q
+    GramStatsBuf own;
+    gram_stats_gather(stats.s, d_rows.as<int64_t>(), k, g->c, own, st);
+    std::vector<double> h(3 * k), hq((size_t)k * nq), hxx(k);
+    CUDA_TRY(cudaMemcpyAsync(hxx.data(), own.s.xx, k * sizeof(double), cudaMemcpyDeviceToHost, st));
     int hs = 0;
     CUDA_TRY(cudaMemcpyAsync(h.data(), sc, 3 * k * sizeof(double), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(cudaMemcpyAsync(hq.data(), q, hq.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -183,7 +187,7 @@ extern "C" int slemm_gpu_lmm_quadforms(slemm_geno* g, const float* Py, float tau
       xPy[c] = (float)h[c];
       xPx[c] = (float)h[k + c];
       xSx[c] = (float)h[2 * k + c];
-      xBx[c] = (float)((h[2 * k + c] - qc) / (double)tau1);
+      xBx[c] = (float)((hxx[c] - qc) / (double)tau1);
     }
   });
 }

@@ -112,3 +112,23 @@ def test_gwa_blocks_vs_fp64(gpu, weighted, block, n, c):
     # FP32 Gram entries (2^-22 of the diagonal) in well-conditioned systems of up to 322 unknowns: xx to 1e-5
     assert np.allclose(1 / se.astype(np.float64) ** 2, xx64, rtol=1e-5, atol=0)
     assert np.allclose(beta, beta64, rtol=1e-5, atol=1e-5 * np.abs(beta64).max())
+
+
+# weights over a factor of 100 of every size, and of two sizes; half of the variants in the individuals of small weight alone
+@pytest.mark.parametrize("n", [2000, 20000])
+@pytest.mark.parametrize("two", [False, True])
+def test_gwa_rare_variants_of_small_weights(gpu, n, two):
+    m, n_model = 600, 300
+    rng = np.random.default_rng(3)
+    counts = rng.binomial(2, rng.uniform(0.05, 0.5, m)[:, None], (m, n)).astype(np.uint8)
+    R = (np.where(np.arange(n) % 2, 1.0, 100.0) if two else 10.0 ** rng.uniform(-2, 2, n)).astype(np.float32)
+    counts[::2] *= R > np.median(R) if not two else R > 50
+    y = rng.standard_normal(n).astype(np.float32)
+    X = np.column_stack([np.ones(n), rng.standard_normal(n)]).astype(np.float32)
+    model = np.sort(rng.permutation(m)[:n_model])
+    _, xx64 = _gwa_fp64(counts, y, R, X, model, 100, 1.5, n_model)
+    with api.Genotypes(synth.encode_bed(counts), n) as g:
+        _, se, _, _ = g.gwa_windows(y, R, X, model, 0, m - 1, 100, 1.5, n_model, 1.0, 1.0, -1)
+    # half of the variants are none of the model's, and their xx no small difference: FP32 entries and products, 2^-23 each,
+    # give its relative error of a few of them
+    assert np.median(np.abs(1 / se.astype(np.float64) ** 2 - xx64) / xx64) <= 4 * 2.0 ** -23
