@@ -19,6 +19,8 @@
 #include "decode.cuh"
 #include "reduce.cuh"
 
+#include <cfloat>
+
 namespace slemm {
 
 // ---- per-SNP statistics ------------------------------------------------------------------------
@@ -545,11 +547,12 @@ spd_panel_kernel(SpdRows S, const float* __restrict__ ridge, int k0, float* __re
       __syncthreads();
       const float d = scol[buf][j];
       bad = bad || !(d > 0.f);
-      // 1/√d to about one unit in the last place: the pivot's chain is in every step's way, and a square
-      // root and a division (IEEE) are some 40 instructions of it
-      const float dc = fmaxf(d, 1e-30f);
-      float inv = rsqrtf(dc);
-      inv = fmaf(inv * 0.5f, fmaf(-dc * inv, inv, 1.f), inv);
+      // 1/√d to half a unit in the last place, by one Newton step with the residual 1 − d·inv² in two pieces (0 for an
+      // infinite pivot, whose row the ridge takes out): the pivot's chain is in every step's way, and a square root and
+      // a division (IEEE) are some 40 instructions of it
+      float inv = rsqrtf(d);
+      const float hi = d * inv, rest = fmaf(-fmaf(d, inv, -hi), inv, fmaf(-hi, inv, 1.f));
+      inv = d <= FLT_MAX ? fmaf(inv * 0.5f, rest, inv) : inv;
       const float inv2 = inv * inv;   // l_i·l_k = v_i·(v_k·inv²) of the published values
       float lk[8];
 #pragma unroll

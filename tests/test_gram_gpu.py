@@ -132,3 +132,25 @@ def test_gwa_rare_variants_of_small_weights(gpu, n, two):
     # half of the variants are none of the model's, and their xx no small difference: FP32 entries and products, 2^-23 each,
     # give its relative error of a few of them
     assert np.median(np.abs(1 / se.astype(np.float64) ** 2 - xx64) / xx64) <= 4 * 2.0 ** -23
+
+
+def test_lmm_windows_with_a_zero_weight(gpu):
+    """A SNP of weight 0 has an infinite ridge: the markers whose windows hold it have no xBx, the others are as
+    without it."""
+    n, m, ws = 700, 600, 130
+    counts, rows, Py, _, _ = _data(n, m, 1, False, seed=4)
+    gm = orc.genotype_mean(orc.popcounts(counts), n)
+    gw = orc.snp_weights(gm, np.ones(m, np.float32))
+    got = []
+    with api.Genotypes(rows, n) as g:
+        g.set_projection(np.full((n, 1), 1 / np.sqrt(n), np.float32))
+        for at in (None, 300):
+            if at is not None:
+                gw[at] = 0
+            g.set_weights(gm, gw)
+            got.append(g.LMM_quadforms(Py, 1.7, num_qf=20, window_size=ws))
+    start = np.clip(np.array(got[0]["variants"]) - ws // 2, 0, m - ws)
+    holds = (start <= 300) & (300 < start + ws)
+    assert 0 < holds.sum() < holds.size
+    a, b = got[0]["xBx"], got[1]["xBx"]
+    assert np.array_equal(np.isnan(b), holds) and np.array_equal(a[~holds], b[~holds])
