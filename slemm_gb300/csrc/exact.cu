@@ -5,7 +5,7 @@
 // with e such that max|v|·2^e lies in [2^3, 2^4).  An FP64 column takes as many digits as reach the last bit
 // of its smallest nonzero value (11 where all are of one size, 15 for a million between the largest and the
 // smallest; up to 420, in passes of 160), an FP32 one likewise (five to 56; the device finds their number, and the host
-// waits for it to lay out the passes).  Digits are exact in E4M3 and a count is at most 2, so a product row's sum over 2^19 K-elements is an integer of at most 2^24: the
+// waits for it to lay out the passes, or guesses it).  Digits are exact in E4M3 and a count is at most 2, so a product row's sum over 2^19 K-elements is an integer of at most 2^24: the
 // tensor cores' FP32 accumulators are exact whatever their order.  K is therefore split every 8,192 K-tiles at
 // the latest, the partials are added as 64-bit integers, and only the last combination of the digits
 // rounds (in FP64).  Bound by the narrow tensor-core pass.  GB300's FP64 pipe ran the same sums by an
@@ -163,12 +163,15 @@ dots_stats_kernel(ExactCols a, int64_t n, double* __restrict__ sums, double* __r
   __shared__ double sh[32];
   __shared__ float ext[2][kXThreads / 32];
   const int c = blockIdx.y;
-  const int64_t i0 = (int64_t)blockIdx.x * kXRows, i1 = min64(n, i0 + kXRows);
+  const int64_t i0 = (int64_t)blockIdx.x * kXRows + threadIdx.x;
   double acc = 0.0;
-  float mx = 0.f, nmn = -INFINITY;
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += kXThreads) {
-    const float v = dot_column(a, c, i), mag = isfinite(v) ? fabsf(v) : INFINITY;
-    acc += (double)v;
+  float mx = 0.f, nmn = -INFINITY, v[kXRows / kXThreads];
+#pragma unroll
+  for (int u = 0; u < kXRows / kXThreads; ++u) v[u] = i0 + u * kXThreads < n ? dot_column(a, c, i0 + u * kXThreads) : 0.f;
+#pragma unroll
+  for (int u = 0; u < kXRows / kXThreads; ++u) {
+    const float mag = isfinite(v[u]) ? fabsf(v[u]) : INFINITY;
+    acc += (double)v[u];
     mx = fmaxf(mx, mag);
     nmn = fmaxf(nmn, mag > 0.f ? -mag : -INFINITY);
   }
@@ -195,9 +198,18 @@ __global__ void dots_scale_kernel(const double* __restrict__ sums, const double*
 {
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (c >= C) return;
-  const double s = warp_sum_partials(sums + (int64_t)c * nblk, nblk);
-  const double a = warp_max_partials(amax + (int64_t)c * nblk, nblk);
-  const double mn = -warp_max_partials(namin + (int64_t)c * nblk, nblk, 1, -INFINITY);
+  double s = 0.0, a = 0.0, mn = -INFINITY;
+  for (int b = threadIdx.x & 31; b < nblk; b += 32) {
+    s += sums[(int64_t)c * nblk + b];
+    a = fmax(a, amax[(int64_t)c * nblk + b]);
+    mn = fmax(mn, namin[(int64_t)c * nblk + b]);
+  }
+  for (int o = 16; o; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    a = fmax(a, __shfl_xor_sync(0xffffffffu, a, o));
+    mn = fmax(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+  }
+  mn = -mn;
   if ((threadIdx.x & 31) == 0) {
     tot[c] = isfinite(a) ? s : NAN;
     exps[c] = digit_exp(a);
@@ -212,12 +224,13 @@ struct DotsPass {
 };
 
 // Their operand.  A non-finite column is stored as zeros (its products come out NaN through its total).
-__global__ void __launch_bounds__(kXThreads)
+constexpr int kOpThreads = 64;   // small blocks: a short column's few threads spread over the SMs
+__global__ void __launch_bounds__(kOpThreads)
 dots_operand_kernel(ExactCols a, int64_t n, int64_t n_pad, const __grid_constant__ DotsPass P, const double* __restrict__ tot,
                     const int* __restrict__ exps, uint8_t* __restrict__ B)
 {
   const int b = blockIdx.y, c = P.c0 + b;
-  const int64_t i = ((int64_t)blockIdx.x * kXThreads + threadIdx.x) * 16;
+  const int64_t i = ((int64_t)blockIdx.x * kOpThreads + threadIdx.x) * 16;
   if (i >= n_pad) return;
   const bool fine = !isnan(tot[c]);
   float v[16];
@@ -266,7 +279,20 @@ void exact_gebv(slemm_geno* g, const double* d_alpha, double amax, double amin, 
   }
 }
 
-void exact_dots(slemm_geno* g, const ExactCols& a, double* dots, double* tot, double* twos)
+int exact_dots_guess(const slemm_geno* g, const ExactCols& a)
+{
+  constexpr int kGuess = 12;
+  return kGuess * a.count() <= 96 && g->n_pad * g->m_pad <= (int64_t)1 << 31 ? kGuess : 0;
+}
+
+bool exact_dots_done(const slemm_geno* g, const ExactCols& a, int guess)
+{
+  for (int c = 0; c < a.count(); ++c)
+    if (guess > 0 && g->scal.h[c] > (double)guess) return false;
+  return true;
+}
+
+void exact_dots(slemm_geno* g, const ExactCols& a, double* dots, double* tot, double* twos, int guess)
 {
   cudaStream_t st = g->stream;
   const int C = a.count();
@@ -276,25 +302,26 @@ void exact_dots(slemm_geno* g, const ExactCols& a, double* dots, double* tot, do
   double* sums = (double*)dst.ensure((size_t)3 * C * nblk * sizeof(double) + C * sizeof(int));
   double *amax = sums + (size_t)C * nblk, *namin = amax + (size_t)C * nblk;
   int* exps = reinterpret_cast<int*>(namin + (size_t)C * nblk);
-  const unsigned rows = (unsigned)ceil_div(g->m, kXThreads), oblk = (unsigned)ceil_div(n_pad, 16 * kXThreads);
+  const unsigned rows = (unsigned)ceil_div(g->m, kXThreads), oblk = (unsigned)ceil_div(n_pad, 16 * kOpThreads);
   dots_stats_kernel<<<dim3(nblk, C), kXThreads, 0, st>>>(a, g->n, sums, amax, namin, nblk);
   LAUNCH_CHECK();
   dots_scale_kernel<<<(unsigned)ceil_div(C * 32, 128), 128, 0, st>>>(sums, amax, namin, nblk, C, tot, exps,
                                                                      g->scal.ensure(C));
   LAUNCH_CHECK();
-  CUDA_TRY(cudaStreamSynchronize(st));   // the columns' numbers of digits
+  if (guess == 0) CUDA_TRY(cudaStreamSynchronize(st));   // the columns' numbers of digits
   auto run = [&](const DotsPass& P, double* out, bool high) {
     const int kp = (int)round_up(P.off[P.count], 8), N = (int)round_up(kp, 16);
     const int splits = exact_splits(m_pad, K_tiles, N);
     uint8_t* B = (uint8_t*)g->ws_B.ensure((size_t)N * n_pad);
     float* D = (float*)g->ws_D.ensure((size_t)splits * kp * m_pad * sizeof(float));
-    dots_operand_kernel<<<dim3(oblk, P.count), kXThreads, 0, st>>>(a, g->n, n_pad, P, tot, exps, B);
+    dots_operand_kernel<<<dim3(oblk, P.count), kOpThreads, 0, st>>>(a, g->n, n_pad, P, tot, exps, B);
     LAUNCH_CHECK();
     gemm_tc({g->G.as<uint8_t>(), m_pad, n_pad, B, N, D, splits, g->err.as<int>(), kp, 1, false, 2, high}, st);
     dots_gather_kernel<<<dim3(rows, P.count), kXThreads, 0, st>>>(D, splits, kp, m_pad, g->m, P, tot, exps, out);
     LAUNCH_CHECK();
   };
-  const std::vector<double> digits(g->scal.h, g->scal.h + C);
+  std::vector<double> digits(C, (double)guess);
+  if (guess == 0) digits.assign(g->scal.h, g->scal.h + C);
   for (int c = 0; c < C;) {   // as many columns per pass as fit
     DotsPass P{c, 0, {0}};
     while (c < C && P.count < kDigitCols && P.off[P.count] + (int)digits[c] <= kDigitRows) {

@@ -129,12 +129,15 @@ int slemm_gpu_score_terms(slemm_geno* g, const float* y, int mac, float* xy, flo
     float* oxx = oxy + m;
     CUDA_TRY(cudaMemcpyAsync(yv, y, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, st));
     row_counts_device(g, pc, n1, n2);
-    exact_dots(g, cols, dots, tot, twos);
-    score_finish_kernel<<<(unsigned)ceil_div(m, 256), 256, 0, st>>>(dots, twos, tot, m, n, n1, n2, c, mac, oxy, oxx);
-    LAUNCH_CHECK();
-    CUDA_TRY(cudaMemcpyAsync(xy, oxy, (size_t)m * sizeof(float), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaMemcpyAsync(xx, oxx, (size_t)m * sizeof(float), cudaMemcpyDeviceToHost, st));
-    check_device_error(g);
+    for (int guess = exact_dots_guess(g, cols);; guess = 0) {
+      exact_dots(g, cols, dots, tot, twos, guess);
+      score_finish_kernel<<<(unsigned)ceil_div(m, 256), 256, 0, st>>>(dots, twos, tot, m, n, n1, n2, c, mac, oxy, oxx);
+      LAUNCH_CHECK();
+      CUDA_TRY(cudaMemcpyAsync(xy, oxy, (size_t)m * sizeof(float), cudaMemcpyDeviceToHost, st));
+      CUDA_TRY(cudaMemcpyAsync(xx, oxx, (size_t)m * sizeof(float), cudaMemcpyDeviceToHost, st));
+      check_device_error(g);
+      if (exact_dots_done(g, cols, guess)) break;
+    }
   });
 }
 

@@ -118,8 +118,14 @@ struct ExactCols {
 };
 // dots[c·m + j] = Σ_i count_ij·column_c(i) for every SNP j, tot[c] = Σ_i column_c(i) (NaN for a column
 // with a non-finite value, and so its dots), and with rr given and twos != nullptr
-// twos[j] = 2·Σ_i rr_i²·[count_ij = 2].  Device pointers; at least one column.
-void exact_dots(slemm_geno* g, const ExactCols& a, double* dots, double* tot, double* twos);
+// twos[j] = 2·Σ_i rr_i²·[count_ij = 2].  Device pointers; at least one column.  The host waits for the columns'
+// numbers of digits, or with a guess > 0 queues passes of that many for each: once the caller has waited for the
+// stream, exact_dots_done says whether they were enough, and if not all of it is to be run again without a guess.
+// The guess of short calls (0: none): score terms at n = 3,000, m = 900 take 112 µs with the wait and 101 without, and 12 digits (36
+// bits between the largest and the smallest value) of all columns cost nothing while the product's N is below 96.
+int exact_dots_guess(const slemm_geno* g, const ExactCols& a);
+bool exact_dots_done(const slemm_geno* g, const ExactCols& a, int guess);
+void exact_dots(slemm_geno* g, const ExactCols& a, double* dots, double* tot, double* twos, int guess = 0);
 
 // MC-REML's criterion terms (ops.cu), device memory: Py = rr∘e and norms[c] = ‖e_c‖², e_0 = P·PV_0 and
 // e_c = P(PV_c + st·PV_{q+c}), c = 1 … q; and X ← √w∘X (m×k), norms[c] = ‖X_c‖².

@@ -136,3 +136,29 @@ def test_score_terms_of_rare_variants_with_small_weights(gpu):
     want = (z * z) @ (rr * rr).astype(np.longdouble)
     # FP64 sums of positive terms, then FP32
     assert np.all(np.abs(xx - want) <= 2.0 ** -23 * want)
+
+
+@pytest.mark.parametrize("bits", [30, 36, 37, 60, 200])
+@pytest.mark.parametrize("unit", [False, True])
+def test_score_terms_of_every_range(gpu, bits, unit):
+    """Short calls guess the columns' digits: phenotypes whose values span up to 2^200, below and above what the guess
+    holds, have the sums of the plain product."""
+    from slemm_gb300 import api
+    n, m = 515, 130
+    rows, _, dec = make_case(n, m, seed=bits)
+    rng = np.random.default_rng(bits)
+    y = np.zeros(n, np.float32)
+    y[:256] = 1.5 * 2.0 ** -(bits - 24)          # a tiny value and its carriers beside one large value
+    y[300] = 2.0 ** 24
+    y[301] = -2.0 ** 24                          # of two individuals with the same genotypes
+    dec = dec.copy()
+    dec[:, 301] = dec[:, 300]
+    rr = np.ones(n, np.float32) if unit else rng.uniform(0.5, 2.0, n).astype(np.float32)
+    with api.Genotypes(synth.encode_bed(dec), n) as g:
+        g.set_weights(dec.mean(1).astype(np.float32), np.ones(m, np.float32), rr)
+        g.set_projection(np.zeros((n, 0), np.float32))
+        xy, _ = g.score_terms(y, 0)
+    z = dec.astype(np.float64) - dec.mean(1, dtype=np.float64)[:, None]
+    want = -(z[:, :256].sum(1) * np.float64(y[0]))
+    # the large pair cancels in the exact sums; the total that centres them is an FP64 sum
+    assert np.all(np.abs(xy - want) <= 2.0 ** -23 * np.abs(want) + 2.0 ** -50 * (np.abs(z) @ np.abs(y).astype(np.float64)))
