@@ -10,17 +10,18 @@
 // re-read from L2, where a column (2 MB at n = 500,000) stays.  So an operator takes three of these
 // kernels and a Lanczos step no more.  Bound by the latency of their four to six cluster-wide reductions
 // for short columns, by L2 and HBM for long ones.  One projected operator at n = 2,000, m = 10,000 with 31
-// columns takes 63 µs (102 with ten kernels), the REML gradient at n = 50,000, m = 25,000 with 30
-// probes 5.6 ms (6.0), an MC-REML fit at n = 50,000, m = 20,000 7.3 ms (7.8); at n = 500,000 with 66 columns,
-// where the products are 95 %, nothing changes.  Clusters of 16 where 8 columns or fewer leave half of the
-// GPU idle with 8: that gradient 5.24 → 5.16 ms, the fit (its samples now drawn on the GPU) 4.58 → 4.52 ms.
+// columns takes 62 µs (102 with ten kernels); the REML gradient at n = 50,000, m = 25,000 with 30
+// probes went from 6.0 to 5.6 ms with them and takes 4.4 now, an MC-REML fit at n = 50,000, m = 20,000 from 7.8 to
+// 7.3 and takes 3.7; at n = 500,000 with 66 columns, where the products are 95 %, nothing changes.  Clusters of 16
+// where 8 columns or fewer leave half of the GPU idle with 8: 1.5 % of that gradient and of the fit.
 //
 // A thread works on half of a packed word, elements 4h … 4h + 3 and 8 + 4h … 11 + 4h: two 4-wide loads,
 // and its digits are 8 contiguous bytes of each operand row (four neighbours' would be single bytes).
 // Whole words (16 rows) took twice the registers, one block per SM, and were slower than the separate
 // kernels from 31 columns on (76 and 98 µs for the operand and the step at n = 50,000).  All sums are
 // double-float per thread and FP64 above, in a fixed order (warps, then blocks by rank), so results are
-// bit-reproducible.
+// bit-reproducible for the same block of columns.  A column's bits depend on how many stand beside it: their number
+// sets the cluster and block sizes here, and up to 32 the products' number format (ops.cu).
 //
 // The operand's padding rows (from k to kp in each piece, and up to N) are left as they are: they only
 // reach product columns that nobody reads (66 columns at n = 100,000, m = 50,000: 1,554 → 1,534 µs).

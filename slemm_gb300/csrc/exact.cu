@@ -2,15 +2,15 @@
 //
 // A dense column v is cut into base-32 digits,
 //   v·2^e = d_0 + 2^−5·d_1 + 2^−10·d_2 + …,   d_p integers, |d_p| ≤ 16,
-// with e such that max|v|·2^e lies in [2^3, 2^4).  An FP64 column takes as many digits as reach the last bit
-// of its smallest nonzero value (11 where all are of one size, 15 for a million between the largest and the
-// smallest; up to 420, in passes of 160), an FP32 one likewise (five to 56; the device finds their number, and the host
-// waits for it to lay out the passes, or guesses it).  Digits are exact in E4M3 and a count is at most 2, so a product row's sum over 2^19 K-elements is an integer of at most 2^24: the
-// tensor cores' FP32 accumulators are exact whatever their order.  K is therefore split every 8,192 K-tiles at
+// with e such that max|v|·2^e lies in [2^3, 2^4), and as many digits as reach the last bit of the smallest nonzero
+// value: for an FP64 column 11 where all values are of one size, 15 for a million between the largest and the smallest,
+// up to 420 (in passes of 160); for an FP32 column five to 56, found on the device.  Digits are exact in E4M3 and a count is at
+// most 2, so a product row's sum over 2^19 K-elements is an integer of at most 2^24: the tensor cores' FP32
+// accumulators are exact whatever their order.  K is therefore split every 8,192 K-tiles at
 // the latest, the partials are added as 64-bit integers, and only the last combination of the digits
 // rounds (in FP64).  Bound by the narrow tensor-core pass.  GB300's FP64 pipe ran the same sums by an
 // FMA per genotype and column: at n = 100,000, m = 50,000 the GEBV took 18,988 µs and takes 415 µs, the
-// score terms with three covariates and residual weights 112,698 µs and 694 µs, with the same or a
+// score terms with three covariates and residual weights 112,698 µs and 691 µs, with the same or a
 // smaller error against 64-bit sums.
 #include "internal.h"
 #include "decode.cuh"

@@ -13,8 +13,8 @@
 // K-elements and row tile: 2.65 ms for the 7.5 GB of n = 500,000, m = 60,000, with 1 column as with 24.
 // E4M3 MMAs take 32 K-elements each, the counts are four masked bytes per LOP instead of two
 // halves, and the dense column is five base-32 digits instead of two halves: half the MMAs and
-// half the decode for the same 24 bits, and sums of integers that FP32 accumulates exactly (2^19 K-elements).  Z_cᵀU of 4
-// columns at n = 200,003, m = 50,021: 990 → 584 µs (error against FP64 2.2e-7 → 1.6e-7).
+// half the decode for the same 24 bits, and sums of integers that FP32 accumulates exactly
+// (2^19 K-elements).  Z_cᵀU of 4 columns at n = 200,003, m = 50,021: 990 → 553 µs (error against FP64 2.2e-7 → 1.6e-7).
 //
 // What limits tcgen05 here is the issuing thread, not the tensor pipe.  Measured on GB300: one
 // thread issuing M=128, N=144, K=16 BF16 MMAs back to back keeps the pipe full (72 cycles per

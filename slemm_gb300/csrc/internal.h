@@ -121,11 +121,12 @@ struct ExactCols {
 // twos[j] = 2·Σ_i rr_i²·[count_ij = 2].  Device pointers; at least one column.  The host waits for the columns'
 // numbers of digits, or with a guess > 0 queues passes of that many for each: once the caller has waited for the
 // stream, exact_dots_done says whether they were enough, and if not all of it is to be run again without a guess.
-// The guess of short calls (0: none): score terms at n = 3,000, m = 900 take 112 µs with the wait and 101 without, and 12 digits (36
-// bits between the largest and the smallest value) of all columns cost nothing while the product's N is below 96.
+void exact_dots(slemm_geno* g, const ExactCols& a, double* dots, double* tot, double* twos, int guess = 0);
+// The guess of short calls (0: none).  Score terms at n = 3,000, m = 900 take 112 µs with the wait and 101 without;
+// 12 digits (36 bits between the largest and the smallest value) of every column cost nothing while the product's N
+// is at most 96, where an MMA takes its least time, and past 2^31 counts (0.12 ms a product) the wait is under 3 %.
 int exact_dots_guess(const slemm_geno* g, const ExactCols& a);
 bool exact_dots_done(const slemm_geno* g, const ExactCols& a, int guess);
-void exact_dots(slemm_geno* g, const ExactCols& a, double* dots, double* tot, double* twos, int guess = 0);
 
 // MC-REML's criterion terms (ops.cu), device memory: Py = rr∘e and norms[c] = ‖e_c‖², e_0 = P·PV_0 and
 // e_c = P(PV_c + st·PV_{q+c}), c = 1 … q; and X ← √w∘X (m×k), norms[c] = ‖X_c‖².

@@ -1201,7 +1201,6 @@ int64_t workspace_bytes(const slemm_geno* g)
                    g->ws_T.bytes + g->ws_in.bytes + g->ws_out.bytes);
 }
 
-// Checks the device error word of the kernels' bounded waits (synchronises the stream).
 void first_order_terms(slemm_geno* g, const float* PV, int q, float st, float* Py, double* norms)
 {
   const int64_t n = g->n, units = round_up(n, 16) / kColRows;
@@ -1217,6 +1216,7 @@ void weighted_norms(slemm_geno* g, float* X, int k, double* norms)
                  g->w.as<float>(), norms);
 }
 
+// Checks the device error word of the kernels' bounded waits (synchronises the stream).
 void check_device_error(slemm_geno* g)
 {
   int h = 0;
