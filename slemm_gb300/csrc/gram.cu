@@ -384,15 +384,15 @@ void gram_rows(const GramSide& R, int64_t s0, int64_t cnt, GramJob& job)
 }
 
 void gram_blocks(slemm_geno* g, const GramSide& R, const GramSide& C, const std::vector<GramJob>& jobs, int cq, const float* rr,
-                 int64_t ldo, GramHalf half)
+                 int64_t ldo, GramHalf half, HostKeep& keep)
 {
   cudaStream_t st = g->stream;
   const int64_t K_pad = g->n_pad, K_tiles = K_pad / kTileK;
   const bool unit = rr == nullptr, sym = half != GramHalf::all;
   // N ≤ 160 keeps two row tiles, each with its own MMA-issuing thread, in one CTA
   const int most = unit ? 160 : 80;
-  std::vector<GramGroup> groups;
-  std::vector<int2> tiles;   // as GemmArgs::table
+  auto& groups = keep.make<std::vector<GramGroup>>();
+  auto& tiles = keep.make<std::vector<int2>>();   // as GemmArgs::table
   int64_t widest = 0, rows = 0;
   for (const GramJob& j : jobs) {
     if (j.ncols <= 0) continue;

@@ -3,6 +3,7 @@
 
 #include "internal.h"
 
+#include <memory>
 #include <vector>
 
 namespace slemm {
@@ -66,10 +67,31 @@ void gram_rows(const GramSide& R, int64_t s0, int64_t cnt, GramJob& job);
 // The blocks of one pair of sides.  g gives the stream, the work buffers and the individuals; rr (n_pad) ==
 // nullptr: all 1.  With R and C the same side and a block's columns among its rows: `lower`
 // wants the rows up to each column's own SNP alone (out's others are left alone), `mirrored` has the columns'
-// SNPs from the other half as well.
+// SNPs from the other half as well.  The host tables of the copies it queues go into `keep`.
 enum class GramHalf { all, lower, mirrored };
+// Host memory that queued copies read: a copy from pageable memory need not be staged on a machine whose GPU reads
+// pageable memory.  Waits for the stream before it lets go, unless the caller has and says so.
+struct HostKeep {
+  cudaStream_t stream;
+  std::vector<std::shared_ptr<void>> held;
+  explicit HostKeep(cudaStream_t st) : stream(st) {}
+  HostKeep(const HostKeep&) = delete;
+  HostKeep& operator=(const HostKeep&) = delete;
+  ~HostKeep()
+  {
+    if (!held.empty()) cudaStreamSynchronize(stream);
+  }
+  template <class T>
+  T& make()
+  {
+    const auto p = std::make_shared<T>();
+    held.push_back(p);
+    return *p;
+  }
+  void waited() { held.clear(); }
+};
 void gram_blocks(slemm_geno* g, const GramSide& R, const GramSide& C, const std::vector<GramJob>& jobs, int cq, const float* rr,
-                 int64_t ldo, GramHalf half);
+                 int64_t ldo, GramHalf half, HostKeep& keep);
 
 // A batch of nb systems of s unknowns (layout in gram.cu); offA, offZ and t are device arrays.
 struct SpdBatch {

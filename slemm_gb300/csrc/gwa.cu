@@ -174,15 +174,22 @@ extern "C" int slemm_gpu_gwa_windows(slemm_geno* g, const float* y, const float*
     double* dq = (double*)d_q.ensure((size_t)ntest * sizeof(double));
     int* status = (int*)d_status.ensure((1 + (size_t)batch) * sizeof(int));
     CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), st));
+    HostKeep keep(st);   // the batches' host tables
     for (int b0 = 0; b0 < nb; b0 += batch) {
       const int bn = std::min(batch, nb - b0);
       const int64_t stride = rows_max * bs;
       float* gram = (float*)d_gram.ensure((size_t)bn * stride * sizeof(float));
       const int64_t tested = hi[b0 + bn - 1] - lo[b0];   // the blocks' tested ranges follow each other
       float* Z = (float*)d_Z.ensure((size_t)std::max<int64_t>(tested, 1) * rows_max * sizeof(float));
-      std::vector<int64_t> off((size_t)2 * bn);   // offA | offZ
-      std::vector<int> tb(bn);
-      std::vector<float> ridge((size_t)bn * bs);
+      struct Tables {
+        std::vector<int64_t> off;   // offA | offZ
+        std::vector<int> tb;
+        std::vector<float> ridge;
+      };
+      auto& [off, tb, ridge] = keep.make<Tables>();
+      off.resize((size_t)2 * bn);
+      tb.resize(bn);
+      ridge.resize((size_t)bn * bs);
       std::vector<GramJob> own, tested_by;   // the blocks' own Gram, and with the variants each serves
       int t_max = 0;
       for (int bi = 0; bi < bn; ++bi) {
@@ -203,8 +210,8 @@ extern "C" int slemm_gpu_gwa_windows(slemm_geno* g, const float* y, const float*
         job.out = Z + off[bn + bi] * rows_max;
         tested_by.push_back(job);
       }
-      gram_blocks(g, model, model, own, c, drr, rows_max, GramHalf::lower);
-      gram_blocks(g, model, all, tested_by, c, drr, rows_max, GramHalf::all);
+      gram_blocks(g, model, model, own, c, drr, rows_max, GramHalf::lower, keep);
+      gram_blocks(g, model, all, tested_by, c, drr, rows_max, GramHalf::all, keep);
       float* dr = (float*)d_ridge.ensure(ridge.size() * sizeof(float));
       int64_t* doff = (int64_t*)d_off.ensure(off.size() * sizeof(int64_t));
       CUDA_TRY(cudaMemcpyAsync(dr, ridge.data(), ridge.size() * sizeof(float), cudaMemcpyHostToDevice, st));
@@ -221,6 +228,7 @@ extern "C" int slemm_gpu_gwa_windows(slemm_geno* g, const float* y, const float*
         snp_var, d_f, d_f + ntest, d_f + 2 * ntest, d_p);
     LAUNCH_CHECK();
     check_device_error(g);
+    keep.waited();
     int hs = 0;
     CUDA_TRY(cudaMemcpy(&hs, status, sizeof(int), cudaMemcpyDeviceToHost));
     if (hs) SLEMM_THROW(SLEMM_ERR_NUMERIC, "a block's BBᵀ + ridge is not positive definite in FP32");

@@ -156,8 +156,10 @@ extern "C" int slemm_gpu_lmm_quadforms(slemm_geno* g, const float* Py, float tau
       idx[k + c] = (int64_t)c * (ws + 1);
       idx[2 * k + c] = j - wds;
     }
-    gram_blocks(g, side, side, jobs, g->c, rr, rows_max, GramHalf::mirrored);
+    HostKeep keep(st);
+    gram_blocks(g, side, side, jobs, g->c, rr, rows_max, GramHalf::mirrored, keep);
     check_device_error(g);
+    keep.waited();
     // batched systems: q_c = zᵀ(ZᵀZ + D)⁻¹z
     float* dvec = (float*)d_d.ensure((size_t)k * ws * sizeof(float));
     const int nq = spd_quadform_blocks(ws);

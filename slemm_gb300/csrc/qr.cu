@@ -241,6 +241,7 @@ void DesignQr::finish()
 {
   CUDA_TRY(cudaMemcpyAsync(head_.data(), Q_ + (size_t)n_ * c_, head_.size() * sizeof(double), cudaMemcpyDeviceToHost, st_));
   CUDA_TRY(cudaStreamSynchronize(st_));
+  waited_ = true;
   work_.release();
   finite = head_[0] == 0.0;
   const double* R = head_.data() + 1;

@@ -7,11 +7,17 @@
 
 namespace slemm {
 
-// QR of rr∘X (host arrays: n×c with leading dimension ldx, rr of n) on a stream; the constructor returns when
-// the inputs are staged, so host work can run until finish().
+// QR of rr∘X (host arrays: n×c with leading dimension ldx, rr of n) on a stream.  The constructor only queues
+// the work, so host work can run until finish(); the arrays have to live until then.
 class DesignQr {
  public:
   DesignQr(const float* X, int64_t ldx, const float* rr, int64_t n, int c, cudaStream_t st);
+  ~DesignQr()   // left early: the copies may still read the inputs
+  {
+    if (!waited_) cudaStreamSynchronize(st_);
+  }
+  DesignQr(const DesignQr&) = delete;
+  DesignQr& operator=(const DesignQr&) = delete;
   // Waits.  rank by Eigen's rule |R_ii| > eps_f32·min(n, c)·|R_00|, R·Pᵀ (rank×c, column-major), and whether
   // every entry of X is finite; Q is that of all c columns if rank == c.
   void finish();
@@ -27,6 +33,7 @@ class DesignQr {
   int64_t n_;
   int c_;
   cudaStream_t st_;
+  bool waited_ = false;
   DevBuf work_, basis_, rr_;
   double *Q_ = nullptr, *v_ = nullptr;
   float* d_rr_ = nullptr;
