@@ -131,13 +131,12 @@ gram_stats_kernel(const double* __restrict__ dots, const double* __restrict__ tw
   s.xx[j] = xx;
 }
 
-void gram_stats(slemm_geno* g, const float* gm, const float* y, const float* rr, const float* Q, int cq,
-                GramStatsBuf& out)
+void gram_stats(slemm_geno* g, const float* gm, const ExactCols& cols, int guess, GramStatsBuf& out)
 {
   cudaStream_t st = g->stream;
   const int64_t m = g->m;
-  const ExactCols cols{y, rr, Q, g->n_pad, cq};
-  const int C = cols.count();
+  const float* rr = cols.rr;
+  const int C = cols.count(), cq = cols.cq;
   DevBuf d(st), dc(st);
   double* dots = (double*)d.ensure(((size_t)(C + 1) * m + C) * sizeof(double));
   double* twos = rr ? dots + (size_t)C * m : nullptr;
@@ -145,9 +144,9 @@ void gram_stats(slemm_geno* g, const float* gm, const float* y, const float* rr,
   int64_t* pc = (int64_t*)dc.ensure((size_t)m * (sizeof(int64_t) + 2 * sizeof(int32_t)));
   int32_t* n1 = reinterpret_cast<int32_t*>(pc + m);
   row_counts_device(g, pc, n1, n1 + m);
-  if (C > 0) exact_dots(g, cols, dots, tot, twos);
+  if (C > 0) exact_dots(g, cols, dots, tot, twos, guess);
   const GramStats s = out.make(m, cq, st);
-  gram_stats_kernel<<<(unsigned)ceil_div(m, 256), 256, 0, st>>>(dots, twos, tot, m, g->n, pc, n1 + m, gm, y ? 1 : 0, cq,
+  gram_stats_kernel<<<(unsigned)ceil_div(m, 256), 256, 0, st>>>(dots, twos, tot, m, g->n, pc, n1 + m, gm, cols.y ? 1 : 0, cq,
                                                                  s);
   LAUNCH_CHECK();
   if (rr == nullptr) return;
@@ -433,7 +432,8 @@ void gram_blocks(slemm_geno* g, const GramSide& R, const GramSide& C, const std:
     float* D = (float*)g->ws_D.ensure((size_t)ng * splits * kp * rows * sizeof(float));
     const uint32_t* Gc = reinterpret_cast<const uint32_t*>(C.G);
     if (unit)
-      gram_counts_kernel<<<dim3((unsigned)ceil_div(K_pad / 16, 256), (unsigned)ceil_div(kp, kCountRows), ng), 256, 0, st>>>(Gc, K_tiles, dg + g0, kp, (uint8_t*)B);
+      gram_counts_kernel<<<dim3((unsigned)ceil_div(K_pad / 16, 256), (unsigned)ceil_div(kp, kCountRows), ng), 256, 0, st>>>(
+          Gc, K_tiles, dg + g0, kp, (uint8_t*)B);
     else
       gram_operand_kernel<<<dim3((unsigned)ceil_div(K_pad / 8, 256), kp, ng), 256, 0, st>>>(
           Gc, K_tiles, dg + g0, kp, C.stats, rr, (__half*)B);

@@ -45,9 +45,8 @@ struct GramStatsBuf {
 };
 
 // Statistics of every SNP of a handle at the centring values gm (m): y (n, may be nullptr), rr (n_pad,
-// nullptr: all 1), Q (n_pad × cq), all on the device.
-void gram_stats(slemm_geno* g, const float* gm, const float* y, const float* rr, const float* Q, int cq,
-                GramStatsBuf& out);
+// nullptr: all 1), Q (n_pad × cq), all on the device; cols = {y, rr, Q, n_pad, cq}, guess as for exact_dots.
+void gram_stats(slemm_geno* g, const float* gm, const ExactCols& cols, int guess, GramStatsBuf& out);
 void gram_stats_gather(const GramStats& src, const int64_t* d_idx, int64_t cnt, int cq, GramStatsBuf& out, cudaStream_t st);
 
 // A packed SNP-major copy of m rows (all with the same individuals) and its rows' statistics.

@@ -162,73 +162,77 @@ extern "C" int slemm_gpu_gwa_windows(slemm_geno* g, const float* y, const float*
     }
     CUDA_TRY(cudaMemcpyAsync(dmean, mean.data(), mean.size() * sizeof(float), cudaMemcpyHostToDevice, st));
     CUDA_TRY(cudaMemcpyAsync(dy, y, n * sizeof(float), cudaMemcpyHostToDevice, st));
-    GramStatsBuf all_stats, model_stats;
-    gram_stats(g, dmean, dy, drr, dQ, c, all_stats);
-    gram_stats_gather(all_stats.s, didx, n_model, c, model_stats, st);
-    const GramSide all{g->G.as<uint8_t>(), m, all_stats.s}, model{Gm, n_model, model_stats.s};
-    const int64_t rows_max = round_up(bs, kPadRows) + kPadRows;
+    const ExactCols cols{dy, drr, dQ, g->n_pad, c};
+    const int batch = 32;   // blocks at a time (bounded memory)
+    DevBuf d_status(st), d_out(st);
     const int64_t ntest = test_end - test_begin + 1;
-    // blocks in batches (bounded memory)
-    const int batch = 32;
-    DevBuf d_gram(st), d_ridge(st), d_off(st), d_status(st), d_Z(st), d_q(st);
-    double* dq = (double*)d_q.ensure((size_t)ntest * sizeof(double));
     int* status = (int*)d_status.ensure((1 + (size_t)batch) * sizeof(int));
-    CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), st));
-    HostKeep keep(st);   // the batches' host tables
-    for (int b0 = 0; b0 < nb; b0 += batch) {
-      const int bn = std::min(batch, nb - b0);
-      const int64_t stride = rows_max * bs;
-      float* gram = (float*)d_gram.ensure((size_t)bn * stride * sizeof(float));
-      const int64_t tested = hi[b0 + bn - 1] - lo[b0];   // the blocks' tested ranges follow each other
-      float* Z = (float*)d_Z.ensure((size_t)std::max<int64_t>(tested, 1) * rows_max * sizeof(float));
-      struct Tables {
-        std::vector<int64_t> off;   // offA | offZ
-        std::vector<int> tb;
-        std::vector<float> ridge;
-      };
-      auto& [off, tb, ridge] = keep.make<Tables>();
-      off.resize((size_t)2 * bn);
-      tb.resize(bn);
-      ridge.resize((size_t)bn * bs);
-      std::vector<GramJob> own, tested_by;   // the blocks' own Gram, and with the variants each serves
-      int t_max = 0;
-      for (int bi = 0; bi < bn; ++bi) {
-        const int64_t s0 = start[b0 + bi];
-        GramJob job{0, 0, s0, bs, gram + (size_t)bi * stride};
-        gram_rows(model, s0, bs, job);
-        own.push_back(job);
-        for (int t = 0; t < bs; ++t) {
-          const float mu = mean[model_idx[s0 + t]];
-          ridge[(size_t)bi * bs + t] = (float)model_snp_ct * tau * ((2.0f - mu) * mu / 2.0f);
-        }
-        off[bi] = s0 - job.r0;
-        off[bn + bi] = lo[b0 + bi] - lo[b0];
-        tb[bi] = (int)(hi[b0 + bi] - lo[b0 + bi]);
-        t_max = std::max(t_max, tb[bi]);
-        job.c0 = lo[b0 + bi];
-        job.ncols = tb[bi];
-        job.out = Z + off[bn + bi] * rows_max;
-        tested_by.push_back(job);
-      }
-      gram_blocks(g, model, model, own, c, drr, rows_max, GramHalf::lower, keep);
-      gram_blocks(g, model, all, tested_by, c, drr, rows_max, GramHalf::all, keep);
-      float* dr = (float*)d_ridge.ensure(ridge.size() * sizeof(float));
-      int64_t* doff = (int64_t*)d_off.ensure(off.size() * sizeof(int64_t));
-      CUDA_TRY(cudaMemcpyAsync(dr, ridge.data(), ridge.size() * sizeof(float), cudaMemcpyHostToDevice, st));
-      CUDA_TRY(cudaMemcpyAsync(doff, off.data(), off.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-      CUDA_TRY(cudaMemcpyAsync(status + 1, tb.data(), (size_t)bn * sizeof(int), cudaMemcpyHostToDevice, st));
-      spd_row_norms({gram, stride, Z, doff, doff + bn, status + 1, rows_max, bs, bn, t_max}, dr,
-                    dq + (lo[b0] - test_begin), status, st);
-    }
-    DevBuf d_out(st);
     double* d_p = (double*)d_out.ensure((size_t)ntest * (sizeof(double) + 3 * sizeof(float)));
     float* d_f = reinterpret_cast<float*>(d_p + ntest);   // beta | se | chisq
-    gwa_final_kernel<<<(unsigned)ceil_div(ntest, 128), 128, 0, st>>>(
-        all_stats.s.xy + test_begin, all_stats.s.xx + test_begin, dq, d_pc + test_begin, n, ntest, mac, tau, cfactor,
-        snp_var, d_f, d_f + ntest, d_f + 2 * ntest, d_p);
-    LAUNCH_CHECK();
-    check_device_error(g);
-    keep.waited();
+    auto attempt = [&](int guess) {   // false: the guess was too small (exact_dots)
+      GramStatsBuf all_stats, model_stats;
+      gram_stats(g, dmean, cols, guess, all_stats);
+      gram_stats_gather(all_stats.s, didx, n_model, c, model_stats, st);
+      const GramSide all{g->G.as<uint8_t>(), m, all_stats.s}, model{Gm, n_model, model_stats.s};
+      const int64_t rows_max = round_up(bs, kPadRows) + kPadRows;
+      DevBuf d_gram(st), d_ridge(st), d_off(st), d_Z(st), d_q(st);
+      double* dq = (double*)d_q.ensure((size_t)ntest * sizeof(double));
+      CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), st));
+      HostKeep keep(st);   // the batches' host tables
+      for (int b0 = 0; b0 < nb; b0 += batch) {
+        const int bn = std::min(batch, nb - b0);
+        const int64_t stride = rows_max * bs;
+        float* gram = (float*)d_gram.ensure((size_t)bn * stride * sizeof(float));
+        const int64_t tested = hi[b0 + bn - 1] - lo[b0];   // the blocks' tested ranges follow each other
+        float* Z = (float*)d_Z.ensure((size_t)std::max<int64_t>(tested, 1) * rows_max * sizeof(float));
+        struct Tables {
+          std::vector<int64_t> off;   // offA | offZ
+          std::vector<int> tb;
+          std::vector<float> ridge;
+        };
+        auto& [off, tb, ridge] = keep.make<Tables>();
+        off.resize((size_t)2 * bn);
+        tb.resize(bn);
+        ridge.resize((size_t)bn * bs);
+        std::vector<GramJob> own, tested_by;   // the blocks' own Gram, and with the variants each serves
+        int t_max = 0;
+        for (int bi = 0; bi < bn; ++bi) {
+          const int64_t s0 = start[b0 + bi];
+          GramJob job{0, 0, s0, bs, gram + (size_t)bi * stride};
+          gram_rows(model, s0, bs, job);
+          own.push_back(job);
+          for (int t = 0; t < bs; ++t) {
+            const float mu = mean[model_idx[s0 + t]];
+            ridge[(size_t)bi * bs + t] = (float)model_snp_ct * tau * ((2.0f - mu) * mu / 2.0f);
+          }
+          off[bi] = s0 - job.r0;
+          off[bn + bi] = lo[b0 + bi] - lo[b0];
+          tb[bi] = (int)(hi[b0 + bi] - lo[b0 + bi]);
+          t_max = std::max(t_max, tb[bi]);
+          job.c0 = lo[b0 + bi];
+          job.ncols = tb[bi];
+          job.out = Z + off[bn + bi] * rows_max;
+          tested_by.push_back(job);
+        }
+        gram_blocks(g, model, model, own, c, drr, rows_max, GramHalf::lower, keep);
+        gram_blocks(g, model, all, tested_by, c, drr, rows_max, GramHalf::all, keep);
+        float* dr = (float*)d_ridge.ensure(ridge.size() * sizeof(float));
+        int64_t* doff = (int64_t*)d_off.ensure(off.size() * sizeof(int64_t));
+        CUDA_TRY(cudaMemcpyAsync(dr, ridge.data(), ridge.size() * sizeof(float), cudaMemcpyHostToDevice, st));
+        CUDA_TRY(cudaMemcpyAsync(doff, off.data(), off.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+        CUDA_TRY(cudaMemcpyAsync(status + 1, tb.data(), (size_t)bn * sizeof(int), cudaMemcpyHostToDevice, st));
+        spd_row_norms({gram, stride, Z, doff, doff + bn, status + 1, rows_max, bs, bn, t_max}, dr,
+                      dq + (lo[b0] - test_begin), status, st);
+      }
+      gwa_final_kernel<<<(unsigned)ceil_div(ntest, 128), 128, 0, st>>>(
+          all_stats.s.xy + test_begin, all_stats.s.xx + test_begin, dq, d_pc + test_begin, n, ntest, mac, tau, cfactor,
+          snp_var, d_f, d_f + ntest, d_f + 2 * ntest, d_p);
+      LAUNCH_CHECK();
+      check_device_error(g);
+      keep.waited();
+      return exact_dots_done(g, cols, guess);
+    };
+    if (!attempt(exact_dots_guess(g, cols))) attempt(0);
     int hs = 0;
     CUDA_TRY(cudaMemcpy(&hs, status, sizeof(int), cudaMemcpyDeviceToHost));
     if (hs) SLEMM_THROW(SLEMM_ERR_NUMERIC, "a block's BBᵀ + ridge is not positive definite in FP32");

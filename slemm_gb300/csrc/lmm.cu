@@ -73,6 +73,13 @@ static std::vector<int64_t> lmm_variants(const std::vector<float>& gm, int64_t n
   return std::vector<int64_t>(v.begin(), v.begin() + k);
 }
 
+// out[c] = xx[rows[c]]
+__global__ void take_xx_kernel(const double* __restrict__ xx, const int64_t* __restrict__ rows, int k, double* __restrict__ out)
+{
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < k) out[c] = xx[rows[c]];
+}
+
 }  // namespace slemm
 
 using namespace slemm;
@@ -135,61 +142,65 @@ extern "C" int slemm_gpu_lmm_quadforms(slemm_geno* g, const float* Py, float tau
     const int64_t stride = rows_max * (ws + 1);   // ws rows and the room for z
     float* gram = (float*)d_gram.ensure((size_t)k * stride * sizeof(float));
     const float* rr = g->rr_one ? nullptr : g->rr.as<float>();
-    GramStatsBuf stats;
-    gram_stats(g, g->gm.as<float>(), nullptr, rr, g->Q.as<float>(), g->c, stats);
-    const GramSide side{g->G.as<uint8_t>(), m, stats.s};
-    std::vector<int64_t> idx((size_t)3 * k);   // offA | offZ | which
-    std::vector<int> one(k, 1);
-    std::vector<GramJob> jobs;
-    std::vector<float> dd((size_t)k * ws);
-    for (int c = 0; c < k; ++c) {
-      const int64_t j = var[c];
-      int64_t wds;
-      if (j < ws / 2) wds = 0;
-      else if (j > m - ws / 2) wds = m - ws;
-      else wds = j - ws / 2;
-      for (int t = 0; t < ws; ++t) dd[(size_t)c * ws + t] = tau1 / gw[wds + t];
-      GramJob job{0, 0, wds, ws, gram + (size_t)c * stride};
-      gram_rows(side, wds, ws, job);
-      jobs.push_back(job);
-      idx[c] = wds - job.r0;   // this window's Gram starts at row wds − r0 of its block
-      idx[k + c] = (int64_t)c * (ws + 1);
-      idx[2 * k + c] = j - wds;
-    }
-    HostKeep keep(st);
-    gram_blocks(g, side, side, jobs, g->c, rr, rows_max, GramHalf::mirrored, keep);
-    check_device_error(g);
-    keep.waited();
-    // batched systems: q_c = zᵀ(ZᵀZ + D)⁻¹z
-    float* dvec = (float*)d_d.ensure((size_t)k * ws * sizeof(float));
-    const int nq = spd_quadform_blocks(ws);
-    double* q = (double*)d_q.ensure((size_t)k * nq * sizeof(double));
-    int* status = (int*)d_status.ensure(((size_t)k + 1) * sizeof(int));
-    int64_t* didx = (int64_t*)d_idx.ensure(idx.size() * sizeof(int64_t));
-    CUDA_TRY(cudaMemcpyAsync(dvec, dd.data(), dd.size() * sizeof(float), cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemcpyAsync(didx, idx.data(), idx.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-    CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), st));
-    CUDA_TRY(cudaMemcpyAsync(status + 1, one.data(), (size_t)k * sizeof(int), cudaMemcpyHostToDevice, st));
-    spd_quadforms({gram, stride, gram + (size_t)ws * rows_max, didx, didx + k, status + 1, rows_max, ws, k, 1}, dvec,
-                  didx + 2 * k, q, status, st);
-    // ‖v‖² as the Gram blocks have it: xBx is its difference from q
-    GramStatsBuf own;
-    gram_stats_gather(stats.s, d_rows.as<int64_t>(), k, g->c, own, st);
-    std::vector<double> h(3 * k), hq((size_t)k * nq), hxx(k);
-    CUDA_TRY(cudaMemcpyAsync(hxx.data(), own.s.xx, k * sizeof(double), cudaMemcpyDeviceToHost, st));
-    int hs = 0;
-    CUDA_TRY(cudaMemcpyAsync(h.data(), sc, 3 * k * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaMemcpyAsync(hq.data(), q, hq.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaMemcpyAsync(&hs, status, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(cudaStreamSynchronize(st));
-    if (hs) SLEMM_THROW(SLEMM_ERR_NUMERIC, "a window's ZᵀZ + τ1·diag(1/gw) is not positive definite in FP32");
-    for (int c = 0; c < k; ++c) {
-      double qc = 0.0;
-      for (int b = 0; b < nq; ++b) qc += hq[(size_t)c * nq + b];
-      xPy[c] = (float)h[c];
-      xPx[c] = (float)h[k + c];
-      xSx[c] = (float)h[2 * k + c];
-      xBx[c] = (float)((hxx[c] - qc) / (double)tau1);
-    }
+    const ExactCols cols{nullptr, rr, g->Q.as<float>(), g->n_pad, g->c};
+    auto attempt = [&](int guess) {   // false: the guess was too small (exact_dots)
+      GramStatsBuf stats;
+      gram_stats(g, g->gm.as<float>(), cols, guess, stats);
+      take_xx_kernel<<<(unsigned)ceil_div(k, 128), 128, 0, st>>>(stats.s.xx, d_rows.as<int64_t>(), k, sc + 3 * k);
+      LAUNCH_CHECK();
+      const GramSide side{g->G.as<uint8_t>(), m, stats.s};
+      std::vector<int64_t> idx((size_t)3 * k);   // offA | offZ | which
+      std::vector<int> one(k, 1);
+      std::vector<GramJob> jobs;
+      std::vector<float> dd((size_t)k * ws);
+      for (int c = 0; c < k; ++c) {
+        const int64_t j = var[c];
+        int64_t wds;
+        if (j < ws / 2) wds = 0;
+        else if (j > m - ws / 2) wds = m - ws;
+        else wds = j - ws / 2;
+        for (int t = 0; t < ws; ++t) dd[(size_t)c * ws + t] = tau1 / gw[wds + t];
+        GramJob job{0, 0, wds, ws, gram + (size_t)c * stride};
+        gram_rows(side, wds, ws, job);
+        jobs.push_back(job);
+        idx[c] = wds - job.r0;   // this window's Gram starts at row wds − r0 of its block
+        idx[k + c] = (int64_t)c * (ws + 1);
+        idx[2 * k + c] = j - wds;
+      }
+      HostKeep keep(st);
+      gram_blocks(g, side, side, jobs, g->c, rr, rows_max, GramHalf::mirrored, keep);
+      check_device_error(g);
+      keep.waited();
+      if (!exact_dots_done(g, cols, guess)) return false;
+      // batched systems: q_c = zᵀ(ZᵀZ + D)⁻¹z
+      float* dvec = (float*)d_d.ensure((size_t)k * ws * sizeof(float));
+      const int nq = spd_quadform_blocks(ws);
+      double* q = (double*)d_q.ensure((size_t)k * nq * sizeof(double));
+      int* status = (int*)d_status.ensure(((size_t)k + 1) * sizeof(int));
+      int64_t* didx = (int64_t*)d_idx.ensure(idx.size() * sizeof(int64_t));
+      CUDA_TRY(cudaMemcpyAsync(dvec, dd.data(), dd.size() * sizeof(float), cudaMemcpyHostToDevice, st));
+      CUDA_TRY(cudaMemcpyAsync(didx, idx.data(), idx.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+      CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), st));
+      CUDA_TRY(cudaMemcpyAsync(status + 1, one.data(), (size_t)k * sizeof(int), cudaMemcpyHostToDevice, st));
+      spd_quadforms({gram, stride, gram + (size_t)ws * rows_max, didx, didx + k, status + 1, rows_max, ws, k, 1}, dvec,
+                    didx + 2 * k, q, status, st);
+      std::vector<double> h(4 * k), hq((size_t)k * nq);
+      int hs = 0;
+      CUDA_TRY(cudaMemcpyAsync(h.data(), sc, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+      CUDA_TRY(cudaMemcpyAsync(hq.data(), q, hq.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+      CUDA_TRY(cudaMemcpyAsync(&hs, status, sizeof(int), cudaMemcpyDeviceToHost, st));
+      CUDA_TRY(cudaStreamSynchronize(st));
+      if (hs) SLEMM_THROW(SLEMM_ERR_NUMERIC, "a window's ZᵀZ + τ1·diag(1/gw) is not positive definite in FP32");
+      for (int c = 0; c < k; ++c) {
+        double qc = 0.0;
+        for (int b = 0; b < nq; ++b) qc += hq[(size_t)c * nq + b];
+        xPy[c] = (float)h[c];
+        xPx[c] = (float)h[k + c];
+        xSx[c] = (float)h[2 * k + c];
+        xBx[c] = (float)((h[3 * k + c] - qc) / (double)tau1);   // ‖v‖² as the Gram blocks have it
+      }
+      return true;
+    };
+    if (!attempt(exact_dots_guess(g, cols))) attempt(0);
   });
 }

@@ -154,3 +154,29 @@ def test_lmm_windows_with_a_zero_weight(gpu):
     assert 0 < holds.sum() < holds.size
     a, b = got[0]["xBx"], got[1]["xBx"]
     assert np.array_equal(np.isnan(b), holds) and np.array_equal(a[~holds], b[~holds])
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+def test_columns_of_wide_range(gpu, weighted):
+    """Phenotypes and covariates over sixteen orders of magnitude: more digits than short calls queue at first."""
+    n, m, n_model, block = 700, 300, 120, 40
+    counts, rows, y, R, X = _data(n, m, 2, weighted, seed=11)
+    rng = np.random.default_rng(2)
+    y = (y * 10.0 ** rng.uniform(-8, 8, n)).astype(np.float32)
+    X[:, 1] *= (10.0 ** rng.uniform(-16, 0, n)).astype(np.float32)   # beside an intercept: of full rank
+    model = np.sort(rng.permutation(m)[:n_model])
+    beta64, xx64 = _gwa_fp64(counts, y, R, X, model, block, 1.5, n_model)
+    gm = orc.genotype_mean(orc.popcounts(counts), n)
+    gw = orc.snp_weights(gm, np.ones(m, np.float32))
+    rr = (1 / np.sqrt(R)).astype(np.float32)
+    Q = np.linalg.qr(rr[:, None] * X.astype(np.float64))[0]
+    ref = orc.LMM_quadforms(counts, y, rr, Q, gm, gw, 1.7, num_qf=9, window_size=130)
+    with api.Genotypes(rows, n) as g:
+        beta, se, _, _ = g.gwa_windows(y, R, X, model, 0, m - 1, block, 1.5, n_model, 1.0, 1.0, -1)
+        g.set_weights(gm, gw, rr)
+        g.set_projection(Q.astype(np.float32))
+        r = g.LMM_quadforms(y, 1.7, num_qf=9, window_size=130)
+    # the bounds of the tests above
+    assert np.allclose(1 / se.astype(np.float64) ** 2, xx64, rtol=1e-5, atol=0)
+    assert np.allclose(beta, beta64, rtol=1e-5, atol=1e-5 * np.abs(beta64).max())
+    assert np.allclose(r["xBx"], ref["xBx"], rtol=2e-5, atol=0)
