@@ -9,7 +9,7 @@
 // accumulators are exact whatever their order.  K is therefore split every 8,192 K-tiles at
 // the latest, the partials are added as 64-bit integers, and only the last combination of the digits
 // rounds (in FP64).  Bound by the narrow tensor-core pass.  GB300's FP64 pipe ran the same sums by an
-// FMA per genotype and column: at n = 100,000, m = 50,000 the GEBV took 18,988 µs and takes 415 µs, the
+// FMA per genotype and column: at n = 100,000, m = 50,000 the GEBV took 18,988 µs and takes 435 µs, the
 // score terms with three covariates and residual weights 112,698 µs and 691 µs, with the same or a
 // smaller error against 64-bit sums.
 #include "internal.h"
